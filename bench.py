@@ -428,10 +428,10 @@ def run_ours(a, rank, world, local_rank):
             tdist.destroy_process_group()
         return
     peak, peak_kind = measured_peak()
-    # A count launches the heavy-pivot kernel when some row is longer than the
-    # light-pivot limit and the light-pivot kernel when some row is not.
-    light_max = (shape or {}).get("light_max", 96)
-    kernels_per_count = 1 + (info["max_row_cardinality"] > light_max)
+    # A count launches the warp kernel, the CTA kernel for rows above light_max,
+    # again for the units of rows above 512, and the giants' kernel above 2,048.
+    limits = [(shape or {}).get("light_max", 96), 512, 2048]
+    kernels_per_count = 1 + sum(info["max_row_cardinality"] > x for x in limits)
     traffic = traffic_per_launch(work)
     fx = fixture_for(a)
     cpu = None

@@ -294,17 +294,18 @@ eh_status eh_bfs_path_length(eh_matrix_t m, uint32_t start, uint64_t max_depth, 
 typedef struct eh_tuning {
   uint32_t light_max;     /* pivots with at most this many entries (2..160) run one
                              per warp                                               */
-  uint32_t unit_span;     /* pivot positions per CTA work unit for larger pivots    */
-  uint32_t ctas_per_sm;   /* resident CTAs per SM of the persistent count kernel     */
+  uint32_t unit_span;     /* pivot positions per CTA work unit for pivots above 512
+                             entries                                                */
+  uint32_t ctas_per_sm;   /* resident CTAs per SM of the persistent count kernels at
+                             most (256 threads each)                                */
   uint32_t core_rows;     /* highest-degree rows kept as a dense bitmap (0 = none)   */
   float ms;               /* median triangle-count time with the chosen shape        */
   uint32_t configs_tried;
-  uint32_t core_hot_words; /* light-pivot probes of the first words of each dense-core
-                              row keep their L2 lines, the rest are evicted first
-                              (0 = no cache hints)                                  */
-  uint32_t core_filter_words; /* words of the per-row hashed filter checked before a
-                              light-pivot probe reads a dense-core word: 0 (none),
-                              16, 32 or 64                                          */
+  uint32_t core_hot_words; /* accepted in a shape and without effect (an L2 hint of
+                              earlier kernels); the tuner reports 0                 */
+  uint32_t core_filter_words; /* 0, 16, 32 or 64: accepted in a shape and without
+                              effect (row filters of earlier kernels); the tuner
+                              reports 0                                             */
 } eh_tuning;
 /* Times the triangle count (EH_SELECT_LOWER) or the lollipop count
  * (EH_SELECT_ALL) on this matrix for a small set of work shapes, coordinate by
@@ -314,8 +315,7 @@ typedef struct eh_tuning {
 eh_status eh_matrix_tune(eh_matrix_t m, void* stream, eh_tuning* result);
 /* As eh_matrix_tune, for matrices that are built, counted counts_per_build
  * times and freed: each shape is ranked by its count time plus the one-shot
- * cost of its own plan parts (heavy work units, dense core, row filters; host
- * time, median of 3 builds) divided by counts_per_build, so a large core that
+ * cost of its own plan parts (work units, dense core; host time, median of 3 builds) divided by counts_per_build, so a large core that
  * saves less per count than it costs to build loses.  0 ranks by count time
  * alone (eh_matrix_tune).  The choice is cached per counts_per_build beside
  * eh_matrix_tune's and is not applied to other matrices by itself: pass it to

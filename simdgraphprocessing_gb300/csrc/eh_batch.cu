@@ -45,7 +45,7 @@ struct Batch {
 namespace {
 
 struct Shape {
-  uint32_t light_max, unit_span, ctas, core, hot, filter;
+  uint32_t light_max, unit_span, ctas, core;
 };
 
 std::mutex g_tune_mutex;
@@ -75,11 +75,10 @@ void load_tune_file() {
   FILE* f = fopen(path, "r");
   if (!f) return;
   char line[1024];
-  while (fgets(line, sizeof(line), f)) {  // key light_max unit_span ctas core [hot [filter]]
+  while (fgets(line, sizeof(line), f)) {  // key light_max unit_span ctas core
     char key[512];
-    unsigned lm, us, ct, co, hot = 0, filt = 0;
-    if (sscanf(line, "%511s %u %u %u %u %u %u", key, &lm, &us, &ct, &co, &hot, &filt) >= 5)
-      g_tune_cache[key] = Shape{lm, us, ct, co, hot, filt};
+    unsigned lm, us, ct, co;
+    if (sscanf(line, "%511s %u %u %u %u", key, &lm, &us, &ct, &co) >= 5) g_tune_cache[key] = Shape{lm, us, ct, co};
   }
   fclose(f);
 }
@@ -90,7 +89,7 @@ void store_tune(const std::string& key, const Shape& s) {
   if (!path) return;
   FILE* f = fopen(path, "a");
   if (!f) return;
-  fprintf(f, "%s %u %u %u %u %u %u\n", key.c_str(), s.light_max, s.unit_span, s.ctas, s.core, s.hot, s.filter);
+  fprintf(f, "%s %u %u %u %u\n", key.c_str(), s.light_max, s.unit_span, s.ctas, s.core);
   fclose(f);
 }
 
@@ -106,15 +105,13 @@ eh_status apply_shape(Matrix* m, const Shape& s, cudaStream_t st) {
   m->light_max = s.light_max;
   m->unit_span = s.unit_span;
   m->core_limit = s.core;
-  m->core_hot_words = s.hot;
-  m->core_filter_words = s.filter;
   m->grid = sms * (int)s.ctas;
   m->shape_set = true;
   return ensure_plan(m, st);
 }
 
 // Host time of building the current shape's own plan parts from nothing (heavy
-// units, dense core, row filters), as a matrix built for a few counts pays
+// units, dense core), as a matrix built for a few counts pays
 // them: median of 3.
 eh_status time_setup(Matrix* m, cudaStream_t st, float* ms) {
   std::vector<float> t;
@@ -182,8 +179,7 @@ eh_status tune(Matrix* m, const uint32_t* graph_rows, uint32_t num_graphs, cudaS
   if (pool_alloc((void**)&out, outn * sizeof(unsigned long long), st) != cudaSuccess)
     return set_error(EH_ERR_OUT_OF_MEMORY, "tuner output allocation failed");
   auto it = g_tune_cache.find(key);
-  Shape best{m->light_max, m->unit_span, (uint32_t)max_ctas_per_sm(m->device), m->core_limit, m->core_hot_words,
-             m->core_filter_words};
+  Shape best{m->light_max, m->unit_span, (uint32_t)max_ctas_per_sm(m->device), m->core_limit};
   float best_ms = 0, best_score = 0;
   uint32_t tried = 0;
   // Count time of the current shape, and its rank (count time plus the
@@ -217,34 +213,19 @@ eh_status tune(Matrix* m, const uint32_t* graph_rows, uint32_t num_graphs, cudaS
       }
     };
     const Shape start = best;
-    // Core size and filters together: a filter makes a larger core pay.
-    for (uint32_t co : {0u, 16384u, 32768u, 65536u, 98304u, 131072u, 196608u, 262144u})
-      for (uint32_t fw : {0u, 32u})
-        if ((co != start.core || fw != start.filter) && co <= kCoreMaxK && (fw == 0 || co > kFilterLo))
-          consider(Shape{start.light_max, start.unit_span, start.ctas, co, start.hot, fw});
-    const Shape after_core0 = best;
-    if (after_core0.core)
-      for (uint32_t hot : {0u, 32u, 64u, 128u})
-        if (hot != after_core0.hot)
-          consider(Shape{after_core0.light_max, after_core0.unit_span, after_core0.ctas, after_core0.core, hot,
-                         after_core0.filter});
-    const Shape after_hot = best;
-    if (after_hot.core > kFilterLo)
-      for (uint32_t fw : {0u, 16u, 32u, 64u})
-        if (fw != after_hot.filter)
-          consider(Shape{after_hot.light_max, after_hot.unit_span, after_hot.ctas, after_hot.core, after_hot.hot, fw});
+    for (uint32_t co : {0u, 8192u, 16384u, 32768u, 65536u, 131072u})
+      if (co != start.core) consider(Shape{start.light_max, start.unit_span, start.ctas, co});
     const Shape after_core = best;
     for (int c = 1; c <= cmax; c++)
       if ((uint32_t)c != after_core.ctas)
-        consider(Shape{after_core.light_max, after_core.unit_span, (uint32_t)c, after_core.core, after_core.hot,
-                         after_core.filter});
+        consider(Shape{after_core.light_max, after_core.unit_span, (uint32_t)c, after_core.core});
     const Shape after_ctas = best;
     for (uint32_t lm : {32u, 64u, 96u, 128u, 160u})
       if (lm != after_ctas.light_max && lm <= kLightMax)
-        consider(Shape{lm, after_ctas.unit_span, after_ctas.ctas, after_ctas.core, after_ctas.hot, after_ctas.filter});
+        consider(Shape{lm, after_ctas.unit_span, after_ctas.ctas, after_ctas.core});
     const Shape after_lm = best;
     for (uint32_t us : {32u, 128u, 256u, 512u, 1024u, 2048u})
-      if (us != after_lm.unit_span) consider(Shape{after_lm.light_max, us, after_lm.ctas, after_lm.core, after_lm.hot, after_lm.filter});
+      if (us != after_lm.unit_span) consider(Shape{after_lm.light_max, us, after_lm.ctas, after_lm.core});
     if (s == EH_OK) {
       s = apply_shape(m, best, st);
       store_tune(key, best);
@@ -259,8 +240,8 @@ eh_status tune(Matrix* m, const uint32_t* graph_rows, uint32_t num_graphs, cudaS
     res->core_rows = best.core;
     res->ms = best_ms;
     res->configs_tried = tried;
-    res->core_hot_words = best.hot;
-    res->core_filter_words = best.filter;
+    res->core_hot_words = 0;
+    res->core_filter_words = 0;
   }
   return EH_OK;
 }
@@ -279,8 +260,6 @@ void apply_cached_shape(Matrix* m) {
   m->light_max = it->second.light_max;
   m->unit_span = it->second.unit_span;
   m->core_limit = it->second.core;
-  m->core_hot_words = it->second.hot;
-  m->core_filter_words = it->second.filter;
   m->grid = sms * (int)it->second.ctas;
 }
 
@@ -324,8 +303,7 @@ eh_status eh_matrix_set_shape(eh_matrix_t mh, const eh_tuning* shape, void* stre
   EH_CHECK_ARG(shape->core_rows <= eh::kCoreMaxK, "core_rows %u above %u", shape->core_rows, eh::kCoreMaxK);
   const uint32_t fw = shape->core_filter_words;
   EH_CHECK_ARG(fw == 0 || fw == 16 || fw == 32 || fw == 64, "core_filter_words %u is not 0, 16, 32 or 64", fw);
-  const eh::Shape s{shape->light_max, shape->unit_span, shape->ctas_per_sm, shape->core_rows, shape->core_hot_words,
-                    fw};
+  const eh::Shape s{shape->light_max, shape->unit_span, shape->ctas_per_sm, shape->core_rows};
   return eh::apply_shape(m, s, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -357,6 +335,7 @@ eh_status eh_batch_build(uint32_t num_graphs, const uint64_t* graph_rows, uint64
   Batch* b = new Batch();
   b->m = reinterpret_cast<eh::Matrix*>(mh);
   b->m->is_batch = true;
+  b->m->core_limit = 0;  // the first rows are one graph's, not the hubs of all
   b->num_graphs = num_graphs;
   std::vector<uint32_t> gr(num_graphs + 1);
   for (uint32_t g = 0; g <= num_graphs; g++) gr[g] = (uint32_t)graph_rows[g];
@@ -396,15 +375,23 @@ eh_status eh_batch_count(eh_batch_t bh, uint32_t k, uint64_t* d_counts, void* st
   return eh::launch_cliques(b->m, k, out, b->d_graph_rows, b->num_graphs, st);
 }
 
+// Triangles and 4-cliques: the triangle kernels take the pivots above
+// kCliqueWarpMax entries, and the clique count's warp kernel adds the others'
+// triangles from the masks it builds anyway.
+static eh_status batch_both(Batch* b, uint64_t* d_triangles, uint64_t* d_cliques4, cudaStream_t st) {
+  unsigned long long* tri = reinterpret_cast<unsigned long long*>(d_triangles);
+  eh_status s = eh::launch_triangle_count(b->m, tri, b->d_graph_rows, b->num_graphs, st, nullptr, true);
+  if (s != EH_OK) return s;
+  return eh::launch_cliques(b->m, 4, reinterpret_cast<unsigned long long*>(d_cliques4), b->d_graph_rows, b->num_graphs,
+                            st, nullptr, false, nullptr, 0, tri);
+}
+
 eh_status eh_batch_run(eh_batch_t bh, uint64_t* d_triangles, uint64_t* d_cliques4, int use_graph, void* stream) {
   EH_CHECK_ARG(bh && d_triangles && d_cliques4, "NULL argument");
   Batch* b = reinterpret_cast<Batch*>(bh);
   cudaSetDevice(b->m->device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (!use_graph) {
-    eh_status s = eh_batch_count(bh, 3, d_triangles, stream);
-    return s != EH_OK ? s : eh_batch_count(bh, 4, d_cliques4, stream);
-  }
+  if (!use_graph) return batch_both(b, d_triangles, d_cliques4, st);
   EH_CHECK_ARG(st != nullptr, "CUDA-graph replay needs a non-default stream");
   if (!b->exec || b->exec_tri != d_triangles || b->exec_clq != d_cliques4) {
     if (b->exec) {
@@ -419,8 +406,7 @@ eh_status eh_batch_run(eh_batch_t bh, uint64_t* d_triangles, uint64_t* d_cliques
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return set_error(EH_ERR_CUDA, "stream capture: %s", cudaGetErrorString(e));
-    eh_status s1 = eh_batch_count(bh, 3, d_triangles, stream);
-    eh_status s2 = s1 == EH_OK ? eh_batch_count(bh, 4, d_cliques4, stream) : s1;
+    eh_status s2 = batch_both(b, d_triangles, d_cliques4, st);
     e = cudaStreamEndCapture(st, &g);
     if (s2 != EH_OK) {
       if (g) cudaGraphDestroy(g);

@@ -563,6 +563,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_encode(uint64_t n, const uint64_t
           const uint32_t x = nbr[k];
           if (is_selected(sel, x, my, mask, k)) *a++ = x;
         }
+        for (uint32_t k = mm.card; k & 3; k++) *a++ = kUintPad;
       } else {
         unsigned long long* words = reinterpret_cast<unsigned long long*>(dst);
         for (uint64_t k = my_b; k < my_e; k++) {
@@ -602,6 +603,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_encode(uint64_t n, const uint64_t
         }
         k_sel += __popc(bal);
       }
+      if (type == TY_UINT && lane < ((0u - k_sel) & 3u)) reinterpret_cast<uint32_t*>(dst)[k_sel + lane] = kUintPad;
     }
   }
 }
@@ -684,6 +686,7 @@ __global__ void __launch_bounds__(kBigBlock) k_encode_big(const uint64_t* __rest
       if (s) reinterpret_cast<uint32_t*>(dst)[k_sel + __popc(bal & ((1u << lane) - 1u))] = x;
       k_sel += __popc(bal);
     }
+    if (threadIdx.x < ((0u - m.card) & 3u)) reinterpret_cast<uint32_t*>(dst)[m.card + threadIdx.x] = kUintPad;
     __syncthreads();  // s_cnt is rewritten for the next row
   }
 }

@@ -230,28 +230,32 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   return EH_OK;
 }
 
-// (Re)builds the heavy-unit list of the plan for (light_max, unit_span).
+// (Re)builds the large pivots' unit list of the plan for (light_max, unit_span).
 eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaStream_t st) {
   Plan& p = m->plan;
-  if (p.units && p.light_max == light_max && p.unit_span == unit_span) return EH_OK;
-  const uint32_t n_heavy = p.above(light_max);
+  if (p.units_ready && p.light_max == light_max && p.unit_span == unit_span) return EH_OK;
+  const uint32_t n_large = p.above(std::max(light_max, kMidMax));
+  p.n_heavy = p.above(light_max);
+  p.n_large = n_large;
+  p.n_units = 0;
+  p.light_max = light_max;
+  p.unit_span = unit_span;
+  p.units_ready = true;
+  if (n_large == 0) return EH_OK;
+  p.units_ready = false;  // until the list below is built
   uint32_t* cnt = nullptr;
   uint32_t* start = nullptr;
   uint32_t* tmp = nullptr;
-  const uint32_t nh = n_heavy ? n_heavy : 1;
-  CU(pool_alloc((void**)&cnt, nh * sizeof(uint32_t), st), "unit scratch");
-  CU(pool_alloc((void**)&start, nh * sizeof(uint32_t), st), "unit scratch");
-  CU(pool_alloc((void**)&tmp, scan_tmp_words(nh) * sizeof(uint32_t), st), "unit scratch");
-  CU(launch_pivot_units(m->desc, p.order, n_heavy, unit_span, cnt, st), "unit count");
-  uint32_t n_units = 0;
-  if (n_heavy) {
-    CU(exclusive_scan_u32(cnt, n_heavy, start, tmp, st), "unit scan");
-    uint32_t last_start = 0, last_cnt = 0;
-    CU(cudaMemcpyAsync(&last_start, start + n_heavy - 1, 4, cudaMemcpyDeviceToHost, st), "unit copy");
-    CU(cudaMemcpyAsync(&last_cnt, cnt + n_heavy - 1, 4, cudaMemcpyDeviceToHost, st), "unit copy");
-    CU(cudaStreamSynchronize(st), "units");
-    n_units = last_start + last_cnt;
-  }
+  CU(pool_alloc((void**)&cnt, n_large * sizeof(uint32_t), st), "unit scratch");
+  CU(pool_alloc((void**)&start, n_large * sizeof(uint32_t), st), "unit scratch");
+  CU(pool_alloc((void**)&tmp, scan_tmp_words(n_large) * sizeof(uint32_t), st), "unit scratch");
+  CU(launch_pivot_units(m->desc, p.order, n_large, unit_span, cnt, st), "unit count");
+  CU(exclusive_scan_u32(cnt, n_large, start, tmp, st), "unit scan");
+  uint32_t last_start = 0, last_cnt = 0;
+  CU(cudaMemcpyAsync(&last_start, start + n_large - 1, 4, cudaMemcpyDeviceToHost, st), "unit copy");
+  CU(cudaMemcpyAsync(&last_cnt, cnt + n_large - 1, 4, cudaMemcpyDeviceToHost, st), "unit copy");
+  CU(cudaStreamSynchronize(st), "units");
+  const uint32_t n_units = last_start + last_cnt;
   if (!p.units || p.units_cap < (uint64_t)n_units) {
     if (p.units) {  // launches on other streams may still read them
       CU(wait_uses(m, st), "units");
@@ -262,57 +266,36 @@ eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaSt
     CU(pool_alloc((void**)&p.units, p.units_cap * sizeof(uint2), st), "unit allocation");
     m->device_bytes += p.units_cap * sizeof(uint2);
   }
-  CU(launch_pivot_unit_fill(cnt, start, n_heavy, p.units, st), "unit fill");
+  CU(launch_pivot_unit_fill(cnt, start, n_large, p.units, st), "unit fill");
   cudaFreeAsync(cnt, st);
   cudaFreeAsync(start, st);
   cudaFreeAsync(tmp, st);
   CU(cudaStreamSynchronize(st), "unit build");
-  p.n_heavy = n_heavy;
   p.n_units = n_units;
-  p.light_max = light_max;
-  p.unit_span = unit_span;
+  p.units_ready = true;
   return EH_OK;
 }
 
 // Dense core of the first min(n, core_limit) rows (rounded down to a multiple of
-// 64); small graphs (under 4,096 rows) go without.
+// 64); graphs under 1,024 rows go without.
 eh_status ensure_core(Matrix* m, cudaStream_t st) {
   Plan& p = m->plan;
   uint32_t want = (uint32_t)std::min<uint64_t>(m->n, m->core_limit) & ~63u;
-  if (m->n < 4096) want = 0;
-  // Row filters cover the core's rows from kFilterLo on.
-  const uint32_t want_fw = (m->core_filter_words && want > kFilterLo) ? m->core_filter_words : 0u;
-  const uint32_t want_fk = want_fw ? want : 0u;
-  if (want == p.core_k && (want == 0 || p.core) && want_fw == p.filter_words && want_fk == p.filter_k)
-    return EH_OK;
-  if (p.core || p.filter) CU(wait_uses(m, st), "core");  // launches on other streams may still read them
-  if (p.filter) {
-    CU(cudaFreeAsync(p.filter, st), "row filters");
-    m->device_bytes -= (uint64_t)(p.filter_k - kFilterLo) * p.filter_words * 8;
-    p.filter = nullptr;
-    p.filter_words = 0;
-    p.filter_k = 0;
-  }
-  if (p.core && want != p.core_k) {
+  if (m->n < 1024) want = 0;
+  if (want == p.core_k && (want == 0 || p.core)) return EH_OK;
+  if (p.core) {
+    CU(wait_uses(m, st), "core");  // launches on other streams may still read it
     CU(cudaFreeAsync(p.core, st), "core");
     m->device_bytes -= core_row_offset(p.core_k) * 8;
     p.core = nullptr;
     p.core_k = 0;
   }
-  if (want && !p.core) {
+  if (want) {
     const uint64_t words = core_row_offset(want);
     CU(pool_alloc((void**)&p.core, words * 8, st, kPoolCore), "core allocation");
     m->device_bytes += words * 8;
     CU(launch_core_build(m->desc, m->arena, want, p.core, st), "core build");
     p.core_k = want;
-  }
-  if (want_fw) {
-    const uint64_t fwords = (uint64_t)(want_fk - kFilterLo) * want_fw;
-    CU(pool_alloc((void**)&p.filter, fwords * 8, st, kPoolCore), "row filter allocation");
-    m->device_bytes += fwords * 8;
-    CU(launch_filter_build(m->desc, m->arena, want_fk, want_fw, p.filter, st), "row filter build");
-    p.filter_words = want_fw;
-    p.filter_k = want_fk;
   }
   CU(cudaStreamSynchronize(st), "core build");
   return EH_OK;
@@ -320,7 +303,8 @@ eh_status ensure_core(Matrix* m, cudaStream_t st) {
 
 eh_status drop_shape_parts(Matrix* m, cudaStream_t st) {
   Plan& p = m->plan;
-  if (!p.units && !p.core && !p.filter) return EH_OK;
+  p.units_ready = false;
+  if (!p.units && !p.core) return EH_OK;
   CU(wait_uses(m, st), "plan parts");  // launches on other streams may still read them
   if (p.units) {
     CU(cudaFreeAsync(p.units, st), "units");
@@ -328,13 +312,6 @@ eh_status drop_shape_parts(Matrix* m, cudaStream_t st) {
     p.units = nullptr;
     p.units_cap = 0;
     p.n_units = 0;
-  }
-  if (p.filter) {
-    CU(cudaFreeAsync(p.filter, st), "row filters");
-    m->device_bytes -= (uint64_t)(p.filter_k - kFilterLo) * p.filter_words * 8;
-    p.filter = nullptr;
-    p.filter_words = 0;
-    p.filter_k = 0;
   }
   if (p.core) {
     CU(cudaFreeAsync(p.core, st), "core");
@@ -441,10 +418,13 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
   a.num_graphs = 0;
   a.core = m->plan.core;
   a.core_k = m->plan.core_k;
-  a.core_hot_words = m->core_hot_words;
-  a.filter = m->plan.filter;
-  a.filter_words = m->plan.filter_words;
-  a.filter_k = m->plan.filter_k;
+  const Plan& p = m->plan;
+  a.n = m->n;
+  a.n_above_tiny = p.above(8);
+  a.n_large = p.n_large;
+  a.max_warp = p.largest_at_most(p.light_max);
+  a.max_mid = p.largest_at_most(kMidMax);
+  a.max_large = p.largest_at_most(kCtaListCap);
   return a;
 }
 
@@ -465,7 +445,7 @@ static eh_status finish_sync(Matrix* m, unsigned long long* d_res, uint64_t* cou
 
 eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const uint32_t* graph_rows,
                          uint32_t num_graphs, cudaStream_t st, Workspace* ws, bool list, uint32_t* tuples,
-                         uint64_t capacity) {
+                         uint64_t capacity, unsigned long long* tri) {
   Workspace own;
   if (!ws) {
     own.counters = m->counters;
@@ -489,9 +469,9 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   const Plan& p = m->plan;
   const uint32_t cap = clique_smem_cap(k, m->device);
   const uint32_t nG = p.above(cap);
-  const uint32_t nB = p.above(32);
-  const uint32_t nL = p.above(k - 2);
-  CliqueArgs a{m->desc, m->arena, p.order, k, out, graph_rows, num_graphs, p.core, p.core_k, tuples, capacity};
+  const uint32_t nB = p.above(kCliqueWarpMax);
+  const uint32_t nL = p.above(tri ? 1 : k - 2);  // triangles need two entries, k-cliques k - 1
+  CliqueArgs a{m->desc, m->arena, p.order, k, out, graph_rows, num_graphs, p.core, p.core_k, tuples, capacity, tri};
   CU(cudaMemsetAsync(w.counters, 0, 16 * sizeof(uint32_t), st), "memset");
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
@@ -523,7 +503,7 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   // occupancy of the largest one.  Band edges where the CTAs per SM change
   // (1 above 1,024 entries, 3 up to 1,024, 5 up to 768, 6 -- the register
   // limit -- up to 512); fewer bands mean fewer drained-GPU tails.
-  const uint32_t bands[] = {cap, 1024, 768, 512, 32};
+  const uint32_t bands[] = {cap, 1024, 768, 512, kCliqueWarpMax};
   for (int b = 0; b + 1 < (int)(sizeof(bands) / sizeof(bands[0])); b++) {
     if (bands[b] <= bands[b + 1]) continue;
     const uint32_t p0 = p.above(bands[b]), p1 = p.above(bands[b + 1]);
@@ -531,10 +511,7 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
     const uint32_t cmax = p.largest_at_most(bands[b]);
     CU(launch_clique_cta(a, p0, p1, w.counters + 3 + b, cmax, nullptr, 0, st, list), "clique kernel (shared)");
   }
-  if (nL > nB) {
-    const int grid = (int)std::min<uint64_t>((nL - nB + 63) / 64, 8ull * sms);
-    CU(launch_clique_light(a, nB, nL, w.counters + 11, grid > 0 ? grid : 1, st, list), "clique kernel (warp)");
-  }
+  if (nL > nB) CU(launch_clique_warp(a, nB, nL, w.counters + 11, sms, st, list), "clique kernel (warp)");
   note_use(m, st);
   return EH_OK;
 }
@@ -549,7 +526,7 @@ eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t
 }
 
 eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32_t* graph_rows, uint32_t num_graphs,
-                                cudaStream_t st, Workspace* ws) {
+                                cudaStream_t st, Workspace* ws, bool large_only) {
   if (m->selection != EH_SELECT_LOWER)
     return set_error(EH_ERR_UNSUPPORTED, "triangle counting needs a matrix built with EH_SELECT_LOWER");
   eh_status s = ensure_plan(m, st);
@@ -558,7 +535,20 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
   if (ws) a.counters = ws->counters;
   a.graph_rows = graph_rows;
   a.num_graphs = num_graphs;
+  if (graph_rows) {
+    // A batch's graphs have no common core and mostly short rows: the clique
+    // count's warp kernel takes the pivots up to kCliqueWarpMax entries.
+    a.n_order = m->plan.above(kCliqueWarpMax);
+    a.n_heavy = std::min(a.n_heavy, a.n_order);
+  }
   CU(launch_triangles(a, m->plan.units, m->plan.n_units, m->grid, st), "triangle kernel");
+  if (graph_rows && !large_only) {
+    CliqueArgs c{m->desc, m->arena, a.order, 3, out, graph_rows, num_graphs, a.core, a.core_k, nullptr, 0, nullptr};
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
+    CU(cudaMemsetAsync(a.counters + 11, 0, sizeof(uint32_t), st), "memset");
+    CU(launch_clique_warp(c, a.n_order, m->plan.above(1), a.counters + 11, sms, st), "triangle kernel (warp)");
+  }
   note_use(m, st);
   return EH_OK;
 }
@@ -803,7 +793,7 @@ void eh_matrix_free(eh_matrix_t mh) {
     st = nullptr;
   }
   void* bufs[] = {m->desc, m->arena, m->counters, m->plan.order, m->plan.units, m->plan.giant_lists,
-                  m->plan.giant_off, m->plan.core, m->plan.filter, m->clique_scratch};
+                  m->plan.giant_off, m->plan.core, m->clique_scratch};
   for (void* b : bufs)
     if (b) cudaFreeAsync(b, st);
   for (auto& u : m->uses) cudaEventDestroy(u.second);

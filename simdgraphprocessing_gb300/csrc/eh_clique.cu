@@ -15,7 +15,7 @@
 //   k = 4: sum_e sum_{t in M[e]} popc(M[e] & M[t])
 //   k > 4: depth-first over the same masks.
 // Tiers by |A_i| (rows sorted by descending size): one warp per pivot with
-// one-word masks (|A_i| <= 32); one CTA per pivot with masks in shared memory
+// two-word masks (|A_i| <= 64); one CTA per pivot with masks in shared memory
 // (up to clique_smem_cap(k), about 1,650-1,850 entries), launched in size bands
 // so that each launch's shared memory (and so its CTAs per SM) fits its own
 // largest pivot; one CTA per pivot with masks in a global scratch slot (larger
@@ -65,95 +65,165 @@ __device__ __forceinline__ void put_tuple(const CliqueArgs& a, unsigned long lon
   if (a.k == 4) o[3] = x3;
 }
 
-// ---- light tier: |A_i| <= 32, one warp per pivot, one-word masks ----
+// ---- warp tier: |A_i| <= kCliqueWarpMax (64), one warp per pivot, two-word masks ----
+// Phase 1 sets bit t of M[e] for every pair with A_i[t] in row(A_i[e]):
+//  * j = A_i[e] < core_k: one lane per pair, two pairs in flight, a word of
+//    core row j each;
+//  * j >= core_k, a uint row: the row is streamed, 8 lanes per row and 16 bytes
+//    per lane, each element tested in a 4,096-bit hash of the pivot; a set bit
+//    is looked up in the list, which gives t;
+//  * other rows, and rows longer than kCliqueProbe e: the e elements below j
+//    are probed, 8 lanes per row.
+// Streaming reads a short row in one step where a probe per pair took a
+// descriptor and a binary search of dependent loads each.  In a batch of 256
+// graphs (37 M entries, rows of 18 on average) the two warp kernels that the
+// triangles and the 4-cliques of the pivots up to 32 entries took were 2.37 +
+// 1.78 ms.
+// Phase 2 counts (or lists) from the masks.  With `tri` set the same masks also
+// give the pivot's triangles (sum of popc M[e]).
+constexpr uint32_t kCliqueHash = 4096;
+constexpr uint32_t kCliqueProbe = 24;
+
 // LIST: write the k = 3 or 4 cliques as tuples instead of counting them.
 template <bool LIST>
-__global__ void __launch_bounds__(kCtaThreads) k_clique_light(CliqueArgs a, uint32_t pos_begin,
-                                                              uint32_t pos_end, uint32_t* counter) {
-  __shared__ uint32_t s_list[NW][32];
-  __shared__ uint32_t s_mask[NW][32];
+__global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, uint32_t pos_begin, uint32_t pos_end,
+                                                                uint32_t grab, uint32_t* counter) {
+  __shared__ unsigned long long s_mask[NW][kCliqueWarpMax];
+  __shared__ uint32_t s_list[NW][kCliqueWarpMax];
+  __shared__ uint32_t s_bm[NW][kCliqueHash / 32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* list = s_list[warp];
-  uint32_t* mask = s_mask[warp];
+  uint32_t* bm = s_bm[warp];
+  unsigned long long* mask = s_mask[warp];
+  uint32_t* mask32 = reinterpret_cast<uint32_t*>(mask);
   const int top = (int)a.k - 3;  // DFS depth at which a popcount finishes the count
-  unsigned long long acc = 0;
+  for (uint32_t k = lane; k < kCliqueHash / 32; k += 32) bm[k] = 0u;
+  unsigned long long acc = 0, tacc = 0;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(counter, 8u);
+    if (lane == 0) base = atomicAdd(counter, grab);
     base = __shfl_sync(FULL, base, 0) + pos_begin;
     if (base >= pos_end) break;
-    const uint32_t end = min(pos_end, base + 8u);
+    const uint32_t end = min(pos_end, base + grab);
     for (uint32_t p = base; p < end; p++) {
       const uint32_t row = a.order[p];
       const RowView A = load_view(a.desc, a.arena, row);
       const uint32_t c = A.card;
-      const unsigned long long acc_before = acc;
       warp_decode(A, list, lane);
-      mask[lane] = 0;
-      __syncwarp();
-      // phase 1: every (e, t < e) pair, one per lane
-      const uint32_t pairs = c * (c - 1) / 2;
-      uint32_t e = 1, t = lane;
-      while (t >= e) { t -= e; e++; }
-      for (uint32_t q = lane; q < pairs; q += 32) {
-        const uint32_t j = list[e], x = list[t];
-        bool hit;
-        if (j < a.core_k) {
-          hit = (__ldg(a.core + core_row_offset(j) + (x >> 6)) >> (x & 63)) & 1ull;
-        } else {
-          const RowView B = load_view(a.desc, a.arena, j);
-          hit = row_contains(B, x);
+      uint32_t ea = 0;  // entries below core_k
+#pragma unroll
+      for (uint32_t h = 0; h < kCliqueWarpMax; h += 32) {
+        const uint32_t e = h + lane, x = e < c ? list[e] : 0xffffffffu;
+        if (e < c) {
+          mask[e] = 0ull;
+          atomicOr(&bm[(x & (kCliqueHash - 1)) >> 5], 1u << (x & 31));
         }
-        if (hit) atomicOr(&mask[e], 1u << t);
-        t += 32;
-        while (t >= e && e < c) { t -= e; e++; }
+        ea += __popc(__ballot_sync(FULL, x < a.core_k));
       }
       __syncwarp();
-      if (LIST) {
-        // Lane e lists the cliques whose two largest members are i and A_i[e]:
-        // (i, A_i[e], A_i[t]) for t in M[e], or (i, A_i[e], A_i[t], A_i[u]) for
-        // u in M[e] & M[t]; one cursor atomic per warp and pivot.
-        const uint32_t m0 = lane < c ? mask[lane] : 0u;
-        uint32_t n = 0;
-        if (top == 0) {
-          n = __popc(m0);
+      // phase 1, j < core_k
+      const uint32_t pairs = ea * (ea - 1) / 2;
+      uint32_t e = 1, t = lane;
+      while (t >= e) { t -= e; e++; }
+      for (uint32_t q = lane; q < pairs; q += 64) {
+        const uint32_t e0 = e, t0 = t, j0 = list[e], x0 = list[t];
+        t += 32;
+        while (t >= e && e < c) { t -= e; e++; }
+        const bool two = q + 32 < pairs;
+        const uint32_t e1 = e, t1 = t, j1 = two ? list[e] : 0u, x1 = two ? list[t] : 0u;
+        t += 32;
+        while (t >= e && e < c) { t -= e; e++; }
+        const unsigned long long v0 = __ldg(a.core + core_row_offset(j0) + (x0 >> 6));
+        const unsigned long long v1 = two ? __ldg(a.core + core_row_offset(j1) + (x1 >> 6)) : 0ull;
+        if ((v0 >> (x0 & 63)) & 1ull) atomicOr(&mask32[2 * e0 + (t0 >> 5)], 1u << (t0 & 31));
+        if ((v1 >> (x1 & 63)) & 1ull) atomicOr(&mask32[2 * e1 + (t1 >> 5)], 1u << (t1 & 31));
+      }
+      // phase 1, j >= core_k
+      const uint32_t sl = lane & 7, first = max(1u, ea) + (lane >> 3);
+      const auto source = [&](uint32_t r) { return __ldg(reinterpret_cast<const uint4*>(a.desc) + list[r]); };
+      uint4 next = make_uint4(0u, 0u, 0u, 0u);
+      if (first < c) next = source(first);
+      for (uint32_t r = first; r < c; r += 4) {
+        const uint4 d = next;
+        if (r + 4 < c) next = source(r + 4);
+        if ((d.w >> 30) == TY_UINT && d.y <= kCliqueProbe * r) {
+          const uint4* p4 = a.arena + d.x;
+          const uint32_t n4 = (d.y + 3) >> 2;  // padded with kUintPad
+          for (uint32_t q0 = sl; q0 < n4; q0 += 16) {
+            const uint4 pad = make_uint4(kUintPad, kUintPad, kUintPad, kUintPad);
+            const uint4 va = __ldg(p4 + q0), vb = q0 + 8 < n4 ? __ldg(p4 + q0 + 8) : pad;
+            const uint32_t y[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+            uint32_t hits = 0;
+#pragma unroll
+            for (int h = 0; h < 8; h++)
+              hits |= ((bm[(y[h] & (kCliqueHash - 1)) >> 5] >> (y[h] & 31)) & 1u) << h;
+            for (; hits; hits &= hits - 1) {
+              const uint32_t h = __ffs(hits) - 1;
+              uint32_t yy = y[0];
+#pragma unroll
+              for (int u = 1; u < 8; u++) yy = h == (uint32_t)u ? y[u] : yy;
+              const uint32_t pos = lower_bound_u32(list, 0, r, yy);
+              if (pos < r && list[pos] == yy) atomicOr(&mask32[2 * r + (pos >> 5)], 1u << (pos & 31));
+            }
+          }
         } else {
-          for (uint32_t m = m0; m; m &= m - 1) n += __popc(m0 & mask[__ffs(m) - 1]);
+          RowView B;
+          B.p = a.arena + d.x;
+          B.card = d.y;
+          B.aux = d.z;
+          B.type = d.w >> 30;
+          B.len = d.w & 0x3fffffffu;
+          for (uint32_t u = sl; u < r; u += 8)
+            if (row_contains(B, list[u])) atomicOr(&mask32[2 * r + (u >> 5)], 1u << (u & 31));
         }
-        const uint32_t ex = warp_exclusive_scan(n, lane);
-        unsigned long long base = 0;
-        if (lane == 31 && ex + n) base = atomicAdd(a.out, (unsigned long long)(ex + n));
-        base = __shfl_sync(FULL, base, 31) + ex;
-        for (uint32_t m = base < a.capacity ? m0 : 0u; m; m &= m - 1) {  // past the capacity: counted only
-          const uint32_t tt = __ffs(m) - 1;
+      }
+      __syncwarp();
+      for (uint32_t u = lane; u < c; u += 32) bm[(list[u] & (kCliqueHash - 1)) >> 5] = 0u;
+      // phase 2: a lane takes the cliques whose two largest members are i and A_i[e]
+      if (LIST) {
+        for (uint32_t h = 0; h < c; h += 32) {
+          // (i, A_i[e], A_i[t]) for t in M[e], or (i, A_i[e], A_i[t], A_i[u]) for
+          // u in M[e] & M[t]; one cursor atomic per warp and 32 entries.
+          const unsigned long long m0 = h + lane < c ? mask[h + lane] : 0ull;
+          uint32_t n = 0;
           if (top == 0) {
-            put_tuple(a, base++, row, list[lane], list[tt], 0u);
+            n = __popcll(m0);
           } else {
-            for (uint32_t r = m0 & mask[tt]; r; r &= r - 1) put_tuple(a, base++, row, list[lane], list[tt], list[__ffs(r) - 1]);
+            for (unsigned long long m = m0; m; m &= m - 1) n += __popcll(m0 & mask[__ffsll((long long)m) - 1]);
+          }
+          const uint32_t ex = warp_exclusive_scan(n, lane);
+          unsigned long long at = 0;
+          if (lane == 31 && ex + n) at = atomicAdd(a.out, (unsigned long long)(ex + n));
+          at = __shfl_sync(FULL, at, 31) + ex;
+          for (unsigned long long m = at < a.capacity ? m0 : 0ull; m; m &= m - 1) {  // past the capacity: counted only
+            const uint32_t tt = __ffsll((long long)m) - 1;
+            if (top == 0) {
+              put_tuple(a, at++, row, list[h + lane], list[tt], 0u);
+            } else {
+              for (unsigned long long r = m0 & mask[tt]; r; r &= r - 1)
+                put_tuple(a, at++, row, list[h + lane], list[tt], list[__ffsll((long long)r) - 1]);
+            }
           }
         }
         __syncwarp();
         continue;
       }
-      // phase 2: lane e counts the cliques whose two largest members are i and A_i[e]
-      if (lane < c) {
-        const uint32_t m0 = mask[lane];
-        if (top == 0) {
-          acc += __popc(m0);
-        } else if (top == 1) {
-          uint32_t m = m0;
-          while (m) {
-            const uint32_t tt = __ffs(m) - 1;
-            m &= m - 1;
-            acc += __popc(m0 & mask[tt]);
-          }
-        } else {
-          uint32_t S[kCliqueMaxK], R[kCliqueMaxK];
+      unsigned long long pc = 0;
+      uint32_t tc = 0;
+      for (uint32_t ee = lane; ee < c; ee += 32) {
+        const unsigned long long m0 = mask[ee];
+        tc += __popcll(m0);
+        if (top == 1) {
+          uint32_t n = 0;
+          for (unsigned long long m = m0; m; m &= m - 1) n += __popcll(m0 & mask[__ffsll((long long)m) - 1]);
+          pc += n;
+        } else if (top > 1) {
+          unsigned long long S[kCliqueMaxK], R[kCliqueMaxK];
           S[0] = R[0] = m0;
           int d = 0;
           while (d >= 0) {
             if (d == top) {
-              acc += __popc(S[d]);
+              pc += __popcll(S[d]);
               d--;
               continue;
             }
@@ -161,26 +231,39 @@ __global__ void __launch_bounds__(kCtaThreads) k_clique_light(CliqueArgs a, uint
               d--;
               continue;
             }
-            const uint32_t tt = __ffs(R[d]) - 1;
+            const uint32_t tt = __ffsll((long long)R[d]) - 1;
             R[d] &= R[d] - 1;
-            const uint32_t nx = S[d] & mask[tt];
-            if ((uint32_t)__popc(nx) >= (uint32_t)(top - d)) {  // enough candidates left
+            const unsigned long long nx = S[d] & mask[tt];
+            if (__popcll(nx) >= top - d) {  // enough candidates left
               S[d + 1] = R[d + 1] = nx;
               d++;
             }
           }
         }
       }
-      if (a.graph_rows) {  // batch: this pivot's cliques go to its graph
-        const unsigned long long pc = warp_sum_u64(acc - acc_before);
-        acc = acc_before;
-        if (lane == 0 && pc) atomicAdd(&a.out[graph_of(a.graph_rows, a.num_graphs, row)], pc);
+      if (top == 0) pc = tc;
+      if (a.graph_rows) {  // batch: this pivot's cliques (and triangles) go to its graph
+        tc = warp_sum_u32(tc);
+        if (tc) {  // no clique without a triangle
+          pc = top <= 1 ? warp_sum_u32((uint32_t)pc) : warp_sum_u64(pc);
+          const uint32_t g = warp_graph_of(a.graph_rows, a.num_graphs, row, lane);
+          if (lane == 0 && pc) atomicAdd(&a.out[g], pc);
+          if (lane == 0 && a.tri) atomicAdd(&a.tri[g], (unsigned long long)tc);
+        }
+      } else {
+        acc += pc;
+        tacc += tc;
       }
       __syncwarp();
     }
   }
+  if (LIST || a.graph_rows) return;
   acc = warp_sum_u64(acc);
-  if (!LIST && lane == 0 && acc) atomicAdd(a.out, acc);
+  if (lane == 0 && acc) atomicAdd(a.out, acc);
+  if (a.tri) {
+    tacc = warp_sum_u64(tacc);
+    if (lane == 0 && tacc) atomicAdd(a.tri, tacc);
+  }
 }
 
 // ---- CTA tiers: one pivot per CTA; masks in shared memory or a global slot ----
@@ -451,11 +534,15 @@ static cudaError_t launch_shared(const CliqueArgs& a, uint32_t pos_begin, uint32
   return cudaGetLastError();
 }
 
-cudaError_t launch_clique_light(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
-                                int grid, cudaStream_t st, bool list) {
+cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
+                               int sms, cudaStream_t st, bool list) {
   if (pos_end <= pos_begin) return cudaSuccess;
-  if (list) k_clique_light<true><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, counter);
-  else k_clique_light<false><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, counter);
+  // Grabs of up to four pivots, small enough that every resident warp gets several.
+  const uint32_t n = pos_end - pos_begin, warps = 5u * NW * (uint32_t)std::max(1, sms);
+  const uint32_t grab = std::max(1u, std::min(4u, n / (16 * warps)));
+  const unsigned grid = std::max(1u, std::min(5u * (uint32_t)std::max(1, sms), (n + NW * grab - 1) / (NW * grab)));
+  if (list) k_clique_warp<true><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, grab, counter);
+  else k_clique_warp<false><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, grab, counter);
   return cudaGetLastError();
 }
 

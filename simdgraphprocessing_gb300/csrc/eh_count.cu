@@ -8,20 +8,16 @@
 // 27-77) run on the full rows and count, for y = A_x[e], the z in A_x ∩ row(y)
 // with z < y -- the same bounded intersection -- each weighted by |A_x|.
 //
-// One persistent kernel does both.  Work comes in two tiers, both handed out
-// dynamically with an atomic counter (the GPU form of par_for_range's block
-// stealing, src/common.hpp:214-276):
-//  * heavy pivots (|A_i| > light_max) are split into units of unit_span values
-//    of e; a CTA stages the pivot's decoded list (and, for bitset rows, its
-//    words) in shared memory and its warps take one j each.  Per pair the warp
-//    picks the cheapest of: AND of overlapping bitset words + popc (bitset ∩
-//    bitset, intersection.hpp:880-955); probing each A_i[t], t < e, into row(j)
-//    (uint ∩ bitset probe, :1023-1058, or the galloping search of :393-584);
-//    streaming row(j) and looking each element up in the staged pivot (merge,
-//    :696-771).
-//  * light pivots run one per warp: the pivot is decoded into the warp's slice
-//    of shared memory and all (e, t) pairs with t < e are probed at once, one
-//    pair per lane, so short rows keep every lane busy.
+// The same kernels do both.  Pivots go by size, largest first, handed out
+// dynamically with atomic counters (the GPU form of par_for_range's block
+// stealing, src/common.hpp:214-276): above 2,048 entries in units of unit_span
+// positions to k_pivots_heavy; above kMidMax in units, and from there down to
+// light_max whole, to a CTA of k_pivots_cta; up to light_max to a warp of
+// k_pivots_warp, which takes the tiniest sixteen at a time.  The per-pair
+// choices stand for the reference's intersection kernels: ANDs of words + popc
+// (bitset ∩ bitset, intersection.hpp:880-955), probes of A_i[t], t < e, into
+// row(j) (uint ∩ bitset, :1023-1058, or the galloping search of :393-584) and
+// streams of row(j) tested against the staged pivot (merge, :696-771).
 // Per-lane counts stay in registers; one u64 atomic per CTA at the end replaces
 // the reference's per-thread padded t_count array.
 #include <algorithm>
@@ -35,15 +31,12 @@ namespace eh {
 namespace {
 
 constexpr int NWARPS = kCtaThreads / 32;
-constexpr uint32_t kLightChunk = 16;  // light pivots per atomic grab
-constexpr uint32_t kTinyPairs = 28;   // chunks of pivots with at most this many pairs (8 entries) share steps
+constexpr int kLargeWarps = 8, kMidWarps = 4;  // warps of a k_pivots_cta CTA for the two tiers
 constexpr uint32_t kStreamMinE = 256;  // core rows: consider streaming row(j) only past this many probes
 
 struct __align__(16) HeavySmem {
   unsigned long long words[kCtaWordCap];
   unsigned long long abits[kCoreAndMax / 64];  // pivot ∩ [0, min(core_k, kCoreAndMax)) as bits
-  uint32_t list[kCtaListCap];
-  uint32_t scan[kCtaThreads];
   uint64_t bar;  // completion of the unit's bulk copy
   uint32_t unit;
 };
@@ -51,15 +44,16 @@ struct __align__(16) HeavySmem {
 constexpr uint32_t kErrWord = 15, kErrBulkWait = 1u;
 
 // Warp, CTA, then one u64 atomic per CTA into the single count.
+template <int NW = NWARPS>
 __device__ __forceinline__ void cta_add(unsigned long long acc, const PivotArgs& a) {
-  __shared__ unsigned long long s_red[NWARPS];
+  __shared__ unsigned long long s_red[NW];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   acc = warp_sum_u64(acc);
   if (lane == 0) s_red[warp] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long tot = 0;
-    for (int w = 0; w < NWARPS; w++) tot += s_red[w];
+    for (int w = 0; w < NW; w++) tot += s_red[w];
     if (tot && !a.graph_rows) atomicAdd(a.out, tot);
   }
 }
@@ -126,8 +120,9 @@ __device__ __forceinline__ uint32_t pair_count_stream(const uint32_t* L, uint32_
   return c;
 }
 
-// Heavy pivots: 6 resident CTAs per SM, 40 registers per thread (the per-pair
-// choice keeps many values live, and at 32 registers it spilled).
+// Pivots above kCtaListCap entries (decoded lists in global memory): 6 resident
+// CTAs per SM, 40 registers per thread (the per-pair choice keeps many values
+// live, and at 32 registers it spilled).
 template <bool LOLLI>
 __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, const uint2* __restrict__ units,
                                                               uint32_t n_units) {
@@ -137,25 +132,20 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
   uint32_t phase = 0;
   if (threadIdx.x == 0) mbar_init(&s.bar);
 
-  // ---- heavy pivots: CTA-wide units ----
   for (;;) {
     if (threadIdx.x == 0) s.unit = atomicAdd(&a.counters[0], 1u);
     __syncthreads();  // also: every thread is done with the previous unit's staging
     const uint32_t unit = s.unit;
     if (unit >= n_units) break;
     const uint2 uu = units[unit];
+    if (uu.x >= a.n_giant) break;  // units come in pivot order, the largest first
     const uint32_t i = a.order[uu.x];
     RowView A = load_view(a.desc, a.arena, i);
-    const uint32_t* L;
-    // uint pivots and bitset words are staged by one bulk (TMA) copy: row
-    // payloads start on 16-byte boundaries and are padded to 16 bytes.
-    const bool bulk_list = uu.x >= a.n_giant && A.type == TY_UINT;
+    // Bitset words are staged by one bulk (TMA) copy: row payloads start on
+    // 16-byte boundaries and are padded to 16 bytes.
     const bool bulk_words = A.type == TY_BITSET && A.len <= kCtaWordCap;
-    if (bulk_list || bulk_words) {
-      if (threadIdx.x == 0) {
-        if (bulk_list) bulk_copy_g2s(s.list, A.p, (4 * A.card + 15) & ~15u, &s.bar);
-        else bulk_copy_g2s(s.words, A.p, (8 * A.len + 15) & ~15u, &s.bar);
-      }
+    if (bulk_words) {
+      if (threadIdx.x == 0) bulk_copy_g2s(s.words, A.p, (8 * A.len + 15) & ~15u, &s.bar);
       if (!mbar_wait(&s.bar, phase)) {
         // Record the failure, then give the copy in flight a second bounded
         // wait before the buffer is used or the CTA exits.
@@ -164,14 +154,8 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
       }
       phase ^= 1u;
     }
-    if (uu.x < a.n_giant) {
-      L = (A.type == TY_UINT) ? static_cast<const uint32_t*>(A.p) : a.giant_lists + a.giant_off[uu.x];
-    } else if (bulk_list) {
-      L = s.list;
-    } else {
-      cta_decode<kCtaThreads>(A, s.list, s.scan);
-      L = s.list;
-    }
+    const uint32_t* L =
+        (A.type == TY_UINT) ? static_cast<const uint32_t*>(A.p) : a.giant_lists + a.giant_off[uu.x];
     if (bulk_words) A.p = s.words;
     // The core path is skipped for pshort pivots of >= 65,536 entries, where the
     // reference's u16 partition count can drop a block (see pshort_pair_drop).
@@ -240,57 +224,374 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
   cta_add(acc, a);
 }
 
-// Word x / 64 of core row j.  With core_hot_words set, words near the start of
-// each core row (the highest-degree columns, where most probes land) keep
-// their L2 lines and the others are evicted first.
-template <bool HOT>
-__device__ __forceinline__ unsigned long long core_word(const PivotArgs& a, uint32_t j, uint32_t x) {
-  const unsigned long long* p = a.core + core_row_offset(j) + (x >> 6);
-  if (!HOT) return __ldg(p);
-  return (x >> 6) < a.core_hot_words ? ld_keep(p) : ld_stream(p);
+// ---- pivots of up to kCtaListCap entries: one warp or one CTA each ----
+// Per pivot, staged in the group's shared-memory slice:
+//  * jc[e] = (word offset of core row j, j) for j = A_i[e];
+//  * word / widx: the non-zero 64-bit words of the pivot's elements below
+//    core_k and their word indices, cfirst[ch] the position of the first
+//    element of word 32 ch;
+//  * bm: the elements of [base, base + win) as bits, base = A_i[0] rounded
+//    down to 64, then kHashBits bits with bit x mod kHashBits set for the
+//    elements x past the window.
+// The pairs (i, j) then take one of two paths, split at the first e with
+// A_i[e] >= core_k (the list is ascending):
+//  * j < core_k: a lane keeps one pivot word of 32 in registers and walks the
+//    e's: core row j's word under it is loaded, ANDed and added to a
+//    carry-save counter.  Nothing is reduced per pair and four pairs' loads are
+//    in flight; only the pivot's non-zero words are touched.  (One warp per
+//    pair, with the whole overlap ANDed or every element probed and a warp sum
+//    per pair, took 6.76 ms for the heavy pivots of an R-MAT scale-22 graph.)
+//  * j >= core_k: row(j) is streamed, 8 lanes per row and 16 bytes per lane,
+//    and each element is tested in bm; a hashed hit past the window is
+//    confirmed by a binary search.  A bitset row of at most 2 e words is ANDed
+//    with the window word by word.  Longer bitset rows, pshort rows and rows of
+//    more than kProbeRatio e entries are probed at the e pivot elements instead.
+// What bounds it: instruction issue (about 11 instructions per 32 words and
+// per 16 streamed entries), and for the core's words the L1: a load in flight
+// holds an L1 line, so shared memory a slice does not need is left to it (at R-MAT
+// scale 22 the warp tier took 4.08 ms with a 32,768-bit window, which leaves
+// L1 28 KB per SM, 2.61 ms with 8,192 + 16,384 hashed bits).
+constexpr uint32_t kProbeRatio = 24;
+constexpr uint32_t kHashBits = 16384;
+
+struct Slice {
+  uint2* jc;
+  unsigned long long* word;
+  uint16_t* widx;
+  uint16_t* cfirst;
+  uint32_t* rcnt;  // CTA groups: per 32 entries, word starts | elements below core_k << 16
+  uint32_t* bm;
+};
+// Bytes of a slice for pivots of up to cap entries (a multiple of 32) and a
+// window of win bits (a multiple of 4,096).
+template <int NW>
+__host__ __device__ constexpr uint32_t slice_bytes(uint32_t cap, uint32_t win) {
+  return (cap * 18 + (cap / 32 + 1) * 2 + (NW > 1 ? cap / 32 * 4 : 0) + (win + kHashBits) / 8 + 31) & ~15u;
+}
+template <int NW>
+__device__ __forceinline__ Slice make_slice(char* p, uint32_t cap, uint32_t win) {
+  Slice s;
+  s.bm = reinterpret_cast<uint32_t*>(p);
+  s.jc = reinterpret_cast<uint2*>(p + (win + kHashBits) / 8);
+  s.word = reinterpret_cast<unsigned long long*>(s.jc + cap);
+  s.rcnt = reinterpret_cast<uint32_t*>(s.word + cap);
+  s.widx = reinterpret_cast<uint16_t*>(s.rcnt + (NW > 1 ? cap / 32 : 0));
+  s.cfirst = s.widx + cap;
+  return s;
+}
+template <int NW>
+__device__ __forceinline__ void group_sync() {
+  if (NW == 1) __syncwarp();
+  else __syncthreads();
 }
 
-// Two light-pivot probes at once, x0 in row(j0) and (if two) x1 in row(j1):
-// the row's filter word first (if the row has a filter; a clear bit means x is
-// not in row(j)), then one word of the core row j when j < core_k, else the
-// row itself.  Both probes' loads are issued before either result is used.
-// Returns the hits as bits 0 and 1.
-template <bool HOT>
-__device__ __forceinline__ uint32_t probe2(const PivotArgs& a, uint32_t j0, uint32_t x0, uint32_t j1, uint32_t x1,
-                                           bool two) {
-  const uint32_t b0 = filter_bit(x0, a.filter_words), b1 = filter_bit(x1, a.filter_words);
-  const unsigned long long f0 = (j0 >= kFilterLo && j0 < a.filter_k)
-                                    ? ld_keep(a.filter + (uint64_t)(j0 - kFilterLo) * a.filter_words + (b0 >> 6))
-                                    : ~0ull;
-  const unsigned long long f1 = (two && j1 >= kFilterLo && j1 < a.filter_k)
-                                    ? ld_keep(a.filter + (uint64_t)(j1 - kFilterLo) * a.filter_words + (b1 >> 6))
-                                    : ~0ull;
-  const bool m0 = (f0 >> (b0 & 63)) & 1ull, m1 = two && ((f1 >> (b1 & 63)) & 1ull);
-  const bool c0 = m0 && j0 < a.core_k, c1 = m1 && j1 < a.core_k;
-  const unsigned long long v0 = c0 ? core_word<HOT>(a, j0, x0) : 0ull;
-  const unsigned long long v1 = c1 ? core_word<HOT>(a, j1, x1) : 0ull;
-  uint32_t h0 = (uint32_t)((v0 >> (x0 & 63)) & 1ull), h1 = (uint32_t)((v1 >> (x1 & 63)) & 1ull);
-  if (m0 && !c0) h0 = row_contains(load_view(a.desc, a.arena, j0), x0);
-  if (m1 && !c1) h1 = row_contains(load_view(a.desc, a.arena, j1), x1);
-  return h0 | (h1 << 1);
+// 32-bit form of core_row_offset (core_k <= kCoreMaxK: below 2^30).
+__device__ __forceinline__ uint32_t core_offset32(uint32_t j) {
+  if (j == 0) return 0;
+  const uint32_t q = (j - 1) >> 6, r = (j - 1) & 63;
+  return (q + 1) * (32 * q + r);
 }
 
-// A chunk of light pivots whose first (largest) pivot has at most kTinyPairs
-// pairs, as one pair space: the pivots' descriptors and rows are loaded by one
-// lane each, and lane q of a step takes pair q of the whole chunk, so a pivot
-// of a few pairs does not hold the warp for a step of its own.  Out of line:
-// its registers do not weigh on the main loop.  Returns the chunk's count
-// (each hit weighted by its pivot's card for lollipops).
-template <bool LOLLI, bool HOT>
-__device__ __noinline__ unsigned long long light_tiny_chunk(const PivotArgs& a, uint32_t base, uint32_t end,
-                                                            uint32_t* list, uint32_t* pstart, uint32_t* poff,
-                                                            uint32_t* pcard, uint32_t lane) {
-  const uint32_t g = end - base;  // <= kLightChunk <= 32
+// Carry-save adder step: (sum, x, y) -> sum, carry out.
+__device__ __forceinline__ uint32_t csa(uint32_t& sum, uint32_t x, uint32_t y) {
+  const uint32_t carry = (sum & x) | (y & (sum ^ x));
+  sum ^= x ^ y;
+  return carry;
+}
+
+// Carry-save counter of 64-bit words, eight at a time: the popcount unit (16
+// lanes per cycle and SM) sees one word in eight.
+struct WordSum {
+  uint32_t one[2], two[2], four[2], eights;
+  __device__ __forceinline__ void clear() { one[0] = one[1] = two[0] = two[1] = four[0] = four[1] = eights = 0; }
+  __device__ __forceinline__ void add8(const unsigned long long (&v)[8], const uint32_t (&w)[2]) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint32_t x[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) x[u] = (uint32_t)(v[u] >> (32 * h)) & w[h];
+      const uint32_t a = csa(one[h], x[0], x[1]), b = csa(one[h], x[2], x[3]), f = csa(two[h], a, b);
+      const uint32_t c = csa(one[h], x[4], x[5]), d = csa(one[h], x[6], x[7]), g = csa(two[h], c, d);
+      eights += __popc(csa(four[h], f, g));
+    }
+  }
+  __device__ __forceinline__ uint32_t total() const {
+    return 8 * eights + 4 * (__popc(four[0]) + __popc(four[1])) + 2 * (__popc(two[0]) + __popc(two[1])) +
+           __popc(one[0]) + __popc(one[1]);
+  }
+};
+
+// This lane's part of the count of pivot i's pairs e in [e0, e1), by a group
+// of NW warps (gw: this warp's index in it): the returned count plus what went
+// into `sum`.  LOLLI: full rows, which hold elements >= j too.  The group's
+// slice is free for the next pivot on return, bm zero.
+template <int NW, bool LOLLI>
+__device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowView& A, uint32_t e0, uint32_t e1,
+                                                const Slice& s, uint32_t win, uint32_t* scan, uint32_t lane,
+                                                uint32_t gw, WordSum& sum) {
+  const uint32_t c = A.card, core_k = a.core_k, lt = (1u << lane) - 1u, tid = gw * 32 + lane;
+  const auto put = [&](uint32_t k, uint32_t x) { s.jc[k] = make_uint2(x < core_k ? core_offset32(x) : 0u, x); };
+  if (NW == 1) warp_decode_to(A, lane, put);
+  else cta_decode_to<NW * 32>(A, scan, put);
+  uint32_t* word32 = reinterpret_cast<uint32_t*>(s.word);
+  if (NW > 1)
+    for (uint32_t k = tid; k < c; k += NW * 32) s.word[k] = 0ull;
+  group_sync<NW>();
+
+  const uint32_t base = s.jc[0].y & ~63u, last = s.jc[c - 1].y;
+  const bool stream_any = last >= core_k, wide = last - base >= win;
+  const uint32_t rounds = (c + 31) >> 5;
+  uint32_t nw = 0, ea = 0, pre0 = 0, pre1 = 0;  // non-zero words; elements below core_k
+  if (NW > 1) {
+    for (uint32_t r = gw; r < rounds; r += NW) {
+      const uint32_t k = 32 * r + lane, x = k < c ? s.jc[k].y : 0xffffffffu;
+      const bool in = x < core_k;  // false past c: core_k <= kCoreMaxK
+      const uint32_t hb = __ballot_sync(FULL, in && (k == 0 || (s.jc[k - 1].y >> 6) != (x >> 6)));
+      const uint32_t ab = __ballot_sync(FULL, in);
+      if (lane == 0) s.rcnt[r] = __popc(hb) | ((uint32_t)__popc(ab) << 16);
+    }
+    group_sync<NW>();
+    const uint32_t v0 = lane < rounds ? s.rcnt[lane] : 0u, v1 = lane + 32 < rounds ? s.rcnt[lane + 32] : 0u;
+    pre0 = warp_exclusive_scan(v0, lane);  // 16-bit halves: sums stay below 2^12
+    const uint32_t t0 = __shfl_sync(FULL, pre0 + v0, 31);
+    pre1 = t0 + warp_exclusive_scan(v1, lane);
+    const uint32_t tot = __shfl_sync(FULL, pre1 + v1, 31);
+    nw = tot & 0xffffu;
+    ea = tot >> 16;
+  }
+  uint32_t run = 0;  // NW == 1: words before this round
+  for (uint32_t r = gw; r < rounds; r += NW) {
+    const uint32_t k = 32 * r + lane, x = k < c ? s.jc[k].y : 0xffffffffu;
+    const bool in = x < core_k;
+    const bool head = in && (k == 0 || (s.jc[k - 1].y >> 6) != (x >> 6));
+    const uint32_t hb = __ballot_sync(FULL, head);
+    if (NW > 1) run = (r < 32 ? __shfl_sync(FULL, pre0, r) : __shfl_sync(FULL, pre1, r - 32)) & 0xffffu;
+    const uint32_t pos = run + __popc(hb & (lt | (1u << lane))) - 1;
+    if (head) {
+      if (NW == 1) s.word[pos] = 0ull;
+      s.widx[pos] = (uint16_t)(x >> 6);
+      if (!(pos & 31)) s.cfirst[pos >> 5] = (uint16_t)k;
+    }
+    if (NW == 1) {
+      ea += __popc(__ballot_sync(FULL, in));
+      run += __popc(hb);
+      __syncwarp();
+    }
+    if (in) atomicOr(&word32[2 * pos + ((x >> 5) & 1)], 1u << (x & 31));
+    if (stream_any && k < c) {
+      const uint32_t d = x - base;
+      atomicOr(&s.bm[(d < win ? d : win + (x & (kHashBits - 1))) >> 5], 1u << (x & 31));
+    }
+  }
+  if (NW == 1) nw = run;
+  group_sync<NW>();
+
+  // ---- j < core_k ----
+  uint32_t cnt = 0;
+  const uint32_t ee = min(e1, ea);
+  for (uint32_t ch = 0; 32 * ch < nw; ch++) {
+    const uint32_t p = 32 * ch + lane;
+    const bool live = p < nw;
+    const unsigned long long word = live ? s.word[p] : 0ull;
+    const uint32_t w[2] = {(uint32_t)word, (uint32_t)(word >> 32)};
+    const uint32_t idx = live ? s.widx[p] : 0u;
+    const uint32_t first = live ? idx << 6 : 0xffffffffu;  // smallest id under this lane's word
+    const unsigned long long* col = a.core + idx;
+    uint32_t e = max(e0, (uint32_t)s.cfirst[ch]) + 8 * gw;
+    unsigned long long v[8];
+    for (; e + 7 < ee; e += 8 * NW) {
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const uint2 q = s.jc[e + u];
+        v[u] = first < q.y ? __ldg(col + q.x) : 0ull;
+      }
+      sum.add8(v, w);
+    }
+    if (e < ee) {  // the last block of fewer than eight belongs to one warp
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const uint2 q = s.jc[e + u];
+        v[u] = (e + u < ee && first < q.y) ? __ldg(col + q.x) : 0ull;
+      }
+      sum.add8(v, w);
+    }
+  }
+
+  // ---- j >= core_k ----
+  if (stream_any && ea < e1) {
+    // Whether L holds y, which lies past the window.
+    const auto search = [&](uint32_t y) -> uint32_t {
+      uint32_t lo = 0, hi = c;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (s.jc[mid].y < y) lo = mid + 1;
+        else hi = mid;
+      }
+      return lo < c && s.jc[lo].y == y;
+    };
+    const uint32_t sl = lane & 7, begin = max(e0, ea) + 4 * gw;
+    const auto source = [&](uint32_t e) { return __ldg(reinterpret_cast<const uint4*>(a.desc) + s.jc[e].y); };
+    uint4 next = make_uint4(0u, 0u, 0u, 0u);
+    if (begin + (lane >> 3) < e1) next = source(begin + (lane >> 3));
+    for (uint32_t eb = begin; eb < e1; eb += 4 * NW) {
+      const uint32_t e = eb + (lane >> 3);
+      const uint4 d = next;
+      if (e + 4 * NW < e1) next = source(e + 4 * NW);
+      uint32_t n = 0, j = 0;
+      const uint32_t* p = nullptr;
+      if (e < e1) {
+        j = s.jc[e].y;
+        const uint32_t type = d.w >> 30;
+        p = reinterpret_cast<const uint32_t*>(a.arena + d.x);
+        n = d.y;
+        if (type == TY_BITSET && (d.w & 0x3fffffffu) <= 2 * e) {
+          // Word pairs of row(j) against the window; words past it element by element.
+          const uint32_t np = ((d.w & 0x3fffffffu) + 1) >> 1, bw = base >> 6, jw = j >> 6, ww = win >> 6;
+          const unsigned long long* bm64 = reinterpret_cast<const unsigned long long*>(s.bm);
+          for (uint32_t q = sl; q < np; q += 8) {
+            const uint32_t w0 = d.z + 2 * q;
+            if (LOLLI && w0 > jw) break;
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + q);
+            const unsigned long long x[2] = {lo64(v), hi64(v)};
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const uint32_t wi = w0 + h;
+              unsigned long long y = x[h];
+              if (LOLLI && wi >= jw) y = wi > jw ? 0ull : y & ((1ull << (j & 63)) - 1ull);
+              if (wi - bw < ww) cnt += __popcll(y & bm64[wi - bw]);
+              else if (wide && wi > bw)
+                for (; y; y &= y - 1ull) cnt += search(64 * wi + (uint32_t)(__ffsll((long long)y) - 1));
+            }
+          }
+          n = 0;
+        } else if (type != TY_UINT || n > kProbeRatio * e) {
+          const RowView B = load_view(a.desc, a.arena, j);
+          for (uint32_t t = sl; t < e; t += 8) cnt += row_contains(B, s.jc[t].y);
+          n = 0;
+        }
+      }
+      // Four 16-byte loads per lane in flight (128 entries of each of the four
+      // rows): the rows come from L2 or DRAM and a lane's chain is one list.
+      const uint32_t most = __reduce_max_sync(FULL, n);
+      for (uint32_t k0 = 0; k0 < most; k0 += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const uint32_t k = k0 + 32 * u + 4 * sl;
+          // uint rows are padded to 16 bytes with an id no row holds (kUintPad).
+          v[u] = k < n ? __ldg(reinterpret_cast<const uint4*>(p + k)) : make_uint4(kUintPad, kUintPad, kUintPad, kUintPad);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          if (k0 + 32 * u >= most) break;
+          const uint32_t y[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+          uint32_t past = 0;  // elements past the window whose hashed bit is set
+#pragma unroll
+          for (int h = 0; h < 4; h++) {
+            const uint32_t dy = y[h] - base;
+            const bool in = dy < win;
+            const uint32_t at = in ? dy : win + (y[h] & (kHashBits - 1));
+            uint32_t bit = (s.bm[at >> 5] >> (y[h] & 31)) & 1u;
+            if (LOLLI) bit = y[h] < j ? bit : 0u;
+            cnt += in ? bit : 0u;
+            past += in ? 0u : bit;
+          }
+          if (past)
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+              if (y[h] - base >= win && (!LOLLI || y[h] < j)) cnt += search(y[h]);
+        }
+      }
+    }
+  }
+  group_sync<NW>();
+  if (stream_any) {
+    for (uint32_t k = tid; k < c; k += NW * 32) {
+      const uint32_t x = s.jc[k].y, d = x - base;
+      s.bm[(d < win ? d : win + (x & (kHashBits - 1))) >> 5] = 0u;
+    }
+    group_sync<NW>();
+  }
+  return cnt;
+}
+
+// A warp's part of a finished pivot (or unit): into its graph's count in a
+// batch (returns 0), weighted by the pivot's card for lollipops, else this
+// lane's part of the one sum, where the carry-save counter may run on.
+template <bool LOLLI>
+__device__ __forceinline__ unsigned long long finish_pivot(const PivotArgs& a, uint32_t i, uint32_t card, uint32_t cnt,
+                                                           WordSum& sum, uint32_t lane) {
+  if (!LOLLI && !a.graph_rows) {
+    const unsigned long long pc = (unsigned long long)cnt + 8ull * sum.eights;
+    sum.eights = 0;
+    return pc;
+  }
+  if (a.core_k) {
+    cnt += sum.total();
+    sum.clear();
+  }
+  if (!a.graph_rows) return (unsigned long long)cnt * card;
+  cnt = warp_sum_u32(cnt);  // below kCtaListCap^2 / 2
+  if (cnt) {
+    const uint32_t g = warp_graph_of(a.graph_rows, a.num_graphs, i, lane);
+    if (lane == 0) atomicAdd(&a.out[g], (unsigned long long)cnt * (LOLLI ? card : 1u));
+  }
+  return 0;
+}
+
+// Pivots above the warp tier and up to kCtaListCap entries, one CTA each, in
+// two launches so that the many mid-sized ones leave their shared memory to
+// L1 and have few warps at a barrier: large pivots as units of unit_span
+// positions (units; the giants' are k_pivots_heavy's), the mid tier
+// order[n_large, n_heavy) whole (units null).
+template <int NW, bool LOLLI>
+__global__ void __launch_bounds__(NW * 32, 32 / NW) k_pivots_cta(PivotArgs a, const uint2* __restrict__ units,
+                                                               uint32_t n_units, uint32_t cap, uint32_t win) {
+  extern __shared__ __align__(16) char dyn[];
+  __shared__ uint32_t s_unit, s_scan[NW];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Slice s = make_slice<NW>(dyn, cap, win);
+  for (uint32_t k = threadIdx.x; k < (win + kHashBits) / 32; k += NW * 32) s.bm[k] = 0u;
+  unsigned long long acc = 0;
+  WordSum sum;
+  sum.clear();
+  for (;;) {
+    if (threadIdx.x == 0) s_unit = atomicAdd(&a.counters[units ? 2 : 4], 1u);
+    __syncthreads();
+    const uint32_t unit = s_unit;
+    __syncthreads();
+    if (unit >= n_units) break;
+    const uint2 uu = units ? units[unit] : make_uint2(a.n_large + unit, 0u);
+    if (units && uu.x < a.n_giant) continue;
+    const uint32_t i = a.order[uu.x];
+    const RowView A = load_view(a.desc, a.arena, i);
+    const uint32_t e0 = 1 + uu.y * a.unit_span, e1 = units ? min(A.card, e0 + a.unit_span) : A.card;
+    const uint32_t cnt = pivot_count<NW, LOLLI>(a, A, e0, e1, s, win, s_scan, lane, warp, sum);
+    acc += finish_pivot<LOLLI>(a, i, A.card, cnt, sum, lane);
+  }
+  cta_add<NW>(acc + sum.total(), a);
+}
+
+// A chunk of pivots of at most kTinyMax entries as one pair space: the pivots'
+// descriptors and rows are loaded by one lane each, and lane q of a step takes
+// pair q of the whole chunk, so a pivot of a few pairs does not hold the warp
+// for a step of its own.  A probe reads one word of core row j when
+// j < core_k, else row(j).  Returns the chunk's count (each hit weighted by its
+// pivot's card for lollipops).
+constexpr uint32_t kTinyMax = 8;
+constexpr uint32_t kTinyChunk = 16;
+template <bool LOLLI>
+__device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32_t base, uint32_t g, uint32_t* mem,
+                                                      uint32_t lane) {
+  uint32_t* list = mem;                               // kTinyChunk * kTinyMax
+  uint32_t* pstart = mem + kTinyChunk * kTinyMax;     // kTinyChunk + 1
+  uint32_t* poff = pstart + kTinyChunk + 1;
+  uint32_t* pcard = poff + kTinyChunk;
   RowView V;
   uint32_t cl = 0;
   if (lane < g) {
-    V = load_view(a.desc, a.arena, a.order[a.n_heavy + base + lane]);
-    cl = V.card;  // <= the first pivot's card: rows in descending card order
+    V = load_view(a.desc, a.arena, a.order[base + lane]);
+    cl = V.card;
   }
   const uint32_t pl = cl * (cl - 1) / 2;
   const uint32_t off = warp_exclusive_scan(cl, lane), pex = warp_exclusive_scan(pl, lane);
@@ -306,95 +607,61 @@ __device__ __noinline__ unsigned long long light_tiny_chunk(const PivotArgs& a, 
   __syncwarp();
   for (uint32_t rest = __ballot_sync(FULL, lane < g && V.type != TY_UINT); rest; rest &= rest - 1) {
     const uint32_t p = __ffs(rest) - 1;
-    warp_decode(load_view(a.desc, a.arena, a.order[a.n_heavy + base + p]), list + poff[p], lane);
+    warp_decode(load_view(a.desc, a.arena, a.order[base + p]), list + poff[p], lane);
   }
   unsigned long long tcnt = 0;
-  for (uint32_t q = lane; q < total; q += 64) {
-    const bool two = q + 32 < total;
-    uint32_t jj[2], xx[2], ww[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const uint32_t qh = (h == 0 || two) ? q + 32u * h : q;
-      uint32_t p = 0;
-      while (pstart[p + 1] <= qh) p++;
-      uint32_t e = 1, t = qh - pstart[p];
-      while (t >= e) { t -= e; e++; }
-      jj[h] = list[poff[p] + e];
-      xx[h] = list[poff[p] + t];
-      ww[h] = LOLLI ? pcard[p] : 1u;
-    }
-    const uint32_t h = probe2<HOT>(a, jj[0], xx[0], jj[1], xx[1], two);
-    tcnt += (unsigned long long)(h & 1u) * ww[0] + (unsigned long long)(h >> 1) * ww[1];
+  for (uint32_t q = lane; q < total; q += 32) {
+    uint32_t p = 0;
+    while (pstart[p + 1] <= q) p++;
+    uint32_t e = 1, t = q - pstart[p];
+    while (t >= e) { t -= e; e++; }
+    const uint32_t j = list[poff[p] + e], x = list[poff[p] + t];
+    bool hit;
+    if (j < a.core_k) hit = (__ldg(a.core + core_offset32(j) + (x >> 6)) >> (x & 63)) & 1ull;
+    else hit = row_contains(load_view(a.desc, a.arena, j), x);
+    if (hit) tcnt += LOLLI ? pcard[p] : 1u;
   }
-  __syncwarp();  // the slice and tables are reused by the next chunk
+  __syncwarp();  // the tables are reused by the next chunk
   return tcnt;
 }
 
-// Light pivots: 8 resident CTAs per SM (64 warps, 32 registers per thread):
-// bound by the latency of scattered probes, so occupancy and two probes in
-// flight per lane pay.
-template <bool LOLLI, bool HOT>  // HOT: core_hot_words != 0
-__global__ void __launch_bounds__(kCtaThreads, 8) k_pivots_light(PivotArgs a) {
-  __shared__ uint32_t wlist[NWARPS][kLightMax];
-  __shared__ uint32_t wtiny[NWARPS][3][kLightChunk + 1];  // tiny chunks: pair starts, list offsets, cards
+// Pivots up to light_max entries, one warp each: order[mid0, mid1) in grabs of
+// mid_chunk, then the tiny ones order[mid1, n_order) in chunks of tiny_chunk.
+template <bool LOLLI>
+__global__ void __launch_bounds__(kCtaThreads, 4) k_pivots_warp(PivotArgs a, uint32_t mid1, uint32_t mid_chunk,
+                                                                uint32_t tiny, uint32_t cap, uint32_t win) {
+  extern __shared__ __align__(16) char dyn[];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  char* mem = dyn + warp * slice_bytes<1>(cap, win);
+  const Slice s = make_slice<1>(mem, cap, win);
+  for (uint32_t k = lane; k < (win + kHashBits) / 32; k += 32) s.bm[k] = 0u;
+  __syncwarp();
   unsigned long long acc = 0;
-
-  // ---- light pivots: one warp each, all (e, t) pairs probed in parallel ----
-  const uint32_t n_light = a.n_order - a.n_heavy;
-  uint32_t* list = wlist[warp];
+  WordSum sum;
+  sum.clear();
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&a.counters[1], kLightChunk);
+    if (lane == 0) base = a.n_heavy + atomicAdd(&a.counters[1], mid_chunk);
     base = __shfl_sync(FULL, base, 0);
-    if (base >= n_light) break;
-    const uint32_t end = min(n_light, base + kLightChunk);
-    // A chunk whose first (largest) pivot has at most kTinyPairs pairs runs as
-    // one pair space: its pivots' descriptors and rows are loaded by one lane
-    // each, and lane q of a step takes pair q of the whole chunk, so a pivot
-    // of a few pairs does not hold the warp for a step of its own.
-    const RowView F = load_view(a.desc, a.arena, a.order[a.n_heavy + base]);
-    if (!a.graph_rows && F.card * (F.card - 1) / 2 <= kTinyPairs) {
-      acc += light_tiny_chunk<LOLLI, HOT>(a, base, end, list, wtiny[warp][0], wtiny[warp][1], wtiny[warp][2], lane);
-      continue;
-    }
+    if (base >= mid1) break;
+    const uint32_t end = min(mid1, base + mid_chunk);
     for (uint32_t k = base; k < end; k++) {
-      const uint32_t i = a.order[a.n_heavy + k];
+      const uint32_t i = a.order[k];
       const RowView A = load_view(a.desc, a.arena, i);
-      const uint32_t c = A.card;
-      warp_decode(A, list, lane);
-      const uint32_t pairs = c * (c - 1) / 2;
-      // Lane q starts at pair q = e(e-1)/2 + t and advances by 32 pairs a step.
-      uint32_t e = 1, t = lane;
-      while (t >= e) { t -= e; e++; }
-      uint32_t cnt = 0;
-      // Two pairs per lane and step (q and q + 32), each probed the same way:
-      // the row's filter word first (if the row has a filter; a clear bit means
-      // x is not in row(j)), then one word of the core row j when j < core_k,
-      // else the row itself.  Both pairs' loads are issued before either
-      // result is used, so two probe chains are in flight per lane.
-      for (uint32_t q = lane; q < pairs; q += 64) {
-        const uint32_t j0 = list[e], x0 = list[t];
-        t += 32;
-        while (t >= e && e < c) { t -= e; e++; }
-        const bool two = q + 32 < pairs;
-        const uint32_t j1 = two ? list[e] : 0u, x1 = two ? list[t] : 0u;
-        t += 32;
-        while (t >= e && e < c) { t -= e; e++; }
-        cnt += __popc(probe2<HOT>(a, j0, x0, j1, x1, two));
-      }
-      unsigned long long pc = LOLLI ? (unsigned long long)cnt * c : (unsigned long long)cnt;
-      if (a.graph_rows) {  // batch: one atomic per pivot into its graph's count
-        pc = warp_sum_u64(pc);
-        if (lane == 0 && pc) atomicAdd(&a.out[graph_of(a.graph_rows, a.num_graphs, i)], pc);
-      } else {
-        acc += pc;
-      }
-      __syncwarp();
+      const uint32_t cnt = pivot_count<1, LOLLI>(a, A, 1, A.card, s, win, nullptr, lane, 0, sum);
+      acc += finish_pivot<LOLLI>(a, i, A.card, cnt, sum, lane);
     }
   }
-
-  cta_add(acc, a);
+  __syncwarp();
+  const uint32_t tiny0 = max(mid1, a.n_heavy);
+  for (;;) {
+    uint32_t base = 0;
+    if (lane == 0) base = tiny0 + atomicAdd(&a.counters[3], tiny);
+    base = __shfl_sync(FULL, base, 0);
+    if (base >= a.n_order) break;
+    acc += tiny_chunk<LOLLI>(a, base, min(tiny, a.n_order - base), reinterpret_cast<uint32_t*>(mem), lane);
+  }
+  cta_add(acc + sum.total(), a);
 }
 
 // Dense core build: one warp per row j < core_k writes row(j) ∩ [0, j) as bits.
@@ -420,26 +687,6 @@ __global__ void __launch_bounds__(256) k_core_build(const RowDesc* __restrict__ 
     } else {
       warp_for_each(B, j, lane, [&](uint32_t x) { atomicOr(&row[x >> 6], 1ull << (x & 63)); });
     }
-    __syncwarp();
-  }
-}
-
-// Row filters: one warp per row j in [kFilterLo, filter_k) sets
-// filter_bit(x) for each x in row(j) ∩ [0, j).
-__global__ void __launch_bounds__(256) k_filter_build(const RowDesc* __restrict__ desc,
-                                                      const uint4* __restrict__ arena, uint32_t filter_k,
-                                                      uint32_t filter_words, unsigned long long* __restrict__ filter) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t nw = gridDim.x * (blockDim.x / 32);
-  for (uint32_t j = kFilterLo + blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); j < filter_k; j += nw) {
-    unsigned long long* row = filter + (uint64_t)(j - kFilterLo) * filter_words;
-    for (uint32_t w = lane; w < filter_words; w += 32) row[w] = 0ull;
-    __syncwarp();
-    const RowView B = load_view(desc, arena, j);
-    warp_for_each(B, j, lane, [&](uint32_t x) {
-      const uint32_t b = filter_bit(x, filter_words);
-      atomicOr(&row[b >> 6], 1ull << (b & 63));
-    });
     __syncwarp();
   }
 }
@@ -500,40 +747,89 @@ __global__ void __launch_bounds__(256) k_intersect_rows(uint64_t n, const RowDes
 
 }  // namespace
 
-// Persistent grid sizes per device: SMs x resident CTAs of the light kernel
-// (the tunable grid) and of the heavy kernel (its cap), looked up once.
-static int grid_of(int device, bool heavy) {
-  static std::atomic<int> cache[64][2];
+// Resident CTAs per SM that a shape may ask for (eh_matrix_set_shape).
+constexpr int kMaxCtasPerSm = 8;
+
+static int sm_count(int device) {
+  static std::atomic<int> cache[64];
   if (device < 0 || device >= 64) return 152;
-  int g = cache[device][heavy].load();
+  int g = cache[device].load();
   if (g > 0) return g;
-  int sms = 0, per = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (heavy) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pivots_heavy<false>, kCtaThreads, 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pivots_light<false, false>, kCtaThreads, 0);
-  g = std::max(1, sms) * std::max(1, per);
-  cache[device][heavy].store(g);
+  cudaDeviceGetAttribute(&g, cudaDevAttrMultiProcessorCount, device);
+  g = std::max(1, g);
+  cache[device].store(g);
   return g;
 }
 
-int pivot_grid(int device) { return grid_of(device, false); }
+int pivot_grid(int device) { return sm_count(device) * kMaxCtasPerSm; }
+
+// Resident CTAs of a kernel with `bytes` of dynamic shared memory and at most
+// `regs` CTAs per SM by registers (a larger grid would only queue).
+static int resident_grid(int device, uint32_t bytes, int regs) {
+  constexpr uint32_t kSmemPerSm = 228u << 10;
+  return sm_count(device) * std::max(1, std::min<int>(regs, (int)(kSmemPerSm / (bytes + 2048))));
+}
+
+// Window bits of the tiers' membership bitmaps: the id range up to the tier's most.
+static uint32_t window_bits(uint64_t n, uint32_t most) {
+  uint32_t w = 4096;
+  while (w < most && w < n) w *= 2;
+  return w;
+}
+
+// Dynamic shared memory above 48 KB has to be allowed once per kernel and device.
+template <bool LOLLI>
+static cudaError_t allow_warp_smem(int device) {
+  static std::atomic<bool> done[64];
+  if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+  if (done[device].load()) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(k_pivots_warp<LOLLI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(NWARPS * slice_bytes<1>(kLightMax, kWarpWindow)));
+  if (e == cudaSuccess) done[device].store(true);
+  return e;
+}
 
 template <bool LOLLI>
 static cudaError_t launch_pivots(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
                                  cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(a.counters, 0, 2 * sizeof(uint32_t), st);
+  cudaError_t e = cudaMemsetAsync(a.counters, 0, 5 * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(a.out, 0, sizeof(unsigned long long) * (a.graph_rows ? a.num_graphs : 1), st);
   if (e != cudaSuccess) return e;
   int device = 0;
   if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
-  if (n_units) {
-    const int gh = std::min(grid, grid_of(device, true));
+  const auto cap_of = [](uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); };
+  if (n_units && a.n_giant) {
+    const int gh = std::min(grid, resident_grid(device, (uint32_t)sizeof(HeavySmem), 6));
     k_pivots_heavy<LOLLI><<<std::max(gh, 1), kCtaThreads, 0, st>>>(a, units, n_units);
   }
+  if (n_units && a.n_large > a.n_giant) {
+    const uint32_t cap = cap_of(a.max_large), win = window_bits(a.n, kCtaWindow);
+    const uint32_t bytes = slice_bytes<kLargeWarps>(cap, win);
+    const int g = std::min<int64_t>(n_units, std::min(grid, resident_grid(device, bytes, 32 / kLargeWarps)));
+    k_pivots_cta<kLargeWarps, LOLLI><<<std::max(g, 1), kLargeWarps * 32, bytes, st>>>(a, units, n_units, cap, win);
+  }
+  if (a.n_heavy > a.n_large) {
+    const uint32_t cap = cap_of(a.max_mid), win = window_bits(a.n, kWarpWindow);
+    const uint32_t bytes = slice_bytes<kMidWarps>(cap, win);
+    const int per = std::max(1, std::min(32 / kMidWarps, grid / sm_count(device) * (NWARPS / kMidWarps)));
+    const int g = std::min<int64_t>(a.n_heavy - a.n_large, resident_grid(device, bytes, per));
+    k_pivots_cta<kMidWarps, LOLLI><<<std::max(g, 1), kMidWarps * 32, bytes, st>>>(a, nullptr, a.n_heavy - a.n_large, cap,
+                                                                                 win);
+  }
   if (a.n_order > a.n_heavy) {
-    if (a.core_hot_words) k_pivots_light<LOLLI, true><<<std::max(grid, 1), kCtaThreads, 0, st>>>(a);
-    else k_pivots_light<LOLLI, false><<<std::max(grid, 1), kCtaThreads, 0, st>>>(a);
+    if ((e = allow_warp_smem<LOLLI>(device)) != cudaSuccess) return e;
+    const uint32_t cap = cap_of(a.max_warp), win = window_bits(a.n, kWarpWindow);
+    const uint32_t bytes = NWARPS * slice_bytes<1>(cap, win);
+    const uint32_t mid1 = std::min(a.n_order, std::max(a.n_heavy, a.n_above_tiny)), mid = mid1 - a.n_heavy, tiny = a.n_order - mid1;
+    int gw = std::min(grid, resident_grid(device, bytes, 4));
+    // Grabs small enough that every warp gets several; one pivot at least.
+    const uint32_t warps = (uint32_t)std::max(gw, 1) * NWARPS;
+    const uint32_t mid_chunk = std::max(1u, std::min(4u, mid / (16 * warps)));
+    const uint32_t tiny_grab = std::max(1u, std::min(kTinyChunk, tiny / (4 * warps)));
+    const uint64_t grabs = (uint64_t)mid / mid_chunk + tiny / tiny_grab + 1;
+    gw = (int)std::min<uint64_t>(std::max(gw, 1), (grabs + NWARPS - 1) / NWARPS);
+    k_pivots_warp<LOLLI><<<gw, kCtaThreads, bytes, st>>>(a, mid1, mid_chunk, tiny_grab, cap, win);
   }
   return cudaGetLastError();
 }
@@ -565,14 +861,6 @@ cudaError_t launch_core_build(const RowDesc* desc, const uint4* arena, uint32_t 
   if (core_k == 0) return cudaSuccess;
   const uint32_t blocks = std::min<uint32_t>((core_k + 7) / 8, 152u * 16u);
   k_core_build<<<blocks, 256, 0, st>>>(desc, arena, core_k, core);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_filter_build(const RowDesc* desc, const uint4* arena, uint32_t filter_k, uint32_t filter_words,
-                                unsigned long long* filter, cudaStream_t st) {
-  if (filter_k <= kFilterLo || filter_words == 0) return cudaSuccess;
-  const uint32_t blocks = std::min<uint32_t>((filter_k - kFilterLo + 7) / 8, 152u * 16u);
-  k_filter_build<<<blocks, 256, 0, st>>>(desc, arena, filter_k, filter_words, filter);
   return cudaGetLastError();
 }
 

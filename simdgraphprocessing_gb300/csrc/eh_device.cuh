@@ -50,6 +50,10 @@ __device__ __forceinline__ RowView load_view(const RowDesc* __restrict__ desc,
 }
 
 constexpr uint32_t FULL = 0xffffffffu;
+// uint payloads are padded to 16 bytes with this id, which no row holds (ids
+// are below n < 2^32), so that 128-bit loads need no tail test; the other
+// layouts' padding is zero.
+constexpr uint32_t kUintPad = 0xffffffffu;
 
 // ---- Bulk (TMA) copies from global to shared memory, completing on an mbarrier ----
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -86,27 +90,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     if (done) return true;
   }
   return false;
-}
-
-// ---- L2 eviction priority of single loads (createpolicy + L2::cache_hint) ----
-// ld_keep marks the line to be evicted last, ld_stream to be evicted first:
-// probes into a small, hot region keep it in L2 while scattered one-off probes
-// do not displace it.  Read-only data (the non-coherent path).
-__device__ __forceinline__ unsigned long long ld_keep(const unsigned long long* p) {
-  unsigned long long v;
-  asm("{\n .reg .b64 pol;\n createpolicy.fractional.L2::evict_last.b64 pol, 1.0;\n"
-      " ld.global.nc.L2::cache_hint.u64 %0, [%1], pol;\n}"
-      : "=l"(v)
-      : "l"(p));
-  return v;
-}
-__device__ __forceinline__ unsigned long long ld_stream(const unsigned long long* p) {
-  unsigned long long v;
-  asm("{\n .reg .b64 pol;\n createpolicy.fractional.L2::evict_first.b64 pol, 1.0;\n"
-      " ld.global.nc.L2::cache_hint.u64 %0, [%1], pol;\n}"
-      : "=l"(v)
-      : "l"(p));
-  return v;
 }
 
 __device__ __forceinline__ uint32_t warp_sum_u32(uint32_t x) { return __reduce_add_sync(FULL, x); }
@@ -181,16 +164,17 @@ __device__ __forceinline__ uint32_t warp_exclusive_scan(uint32_t x, uint32_t lan
   return inc - x;
 }
 
-// Writes the elements of word pair (lo, hi) -- absolute word index w0 for lo --
-// to list[pos...] in ascending order.
+// Calls put(pos, x) for the elements of word pair (lo, hi) -- absolute word
+// index w0 for lo -- in ascending order, pos counting up.
+template <class Put>
 __device__ __forceinline__ void emit_pair_bits(unsigned long long lo, unsigned long long hi, uint32_t w0,
-                                               uint32_t* list, uint32_t pos) {
+                                               uint32_t pos, Put&& put) {
   while (lo) {
-    list[pos++] = 64u * w0 + (uint32_t)(__ffsll((long long)lo) - 1);
+    put(pos++, 64u * w0 + (uint32_t)(__ffsll((long long)lo) - 1));
     lo &= lo - 1ull;
   }
   while (hi) {
-    list[pos++] = 64u * (w0 + 1) + (uint32_t)(__ffsll((long long)hi) - 1);
+    put(pos++, 64u * (w0 + 1) + (uint32_t)(__ffsll((long long)hi) - 1));
     hi &= hi - 1ull;
   }
 }
@@ -472,6 +456,19 @@ __device__ __forceinline__ uint32_t graph_of(const uint32_t* graph_rows, uint32_
   return lo;
 }
 
+// The same by a whole warp: 32 boundaries are compared per step.
+__device__ __forceinline__ uint32_t warp_graph_of(const uint32_t* graph_rows, uint32_t num_graphs, uint32_t row,
+                                                  uint32_t lane) {
+  uint32_t lo = 0, hi = num_graphs;
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 31) >> 5;
+    const uint32_t at = lo + (lane + 1) * step;
+    lo += step * __popc(__ballot_sync(FULL, at < hi && graph_rows[at] <= row));
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
 // Layout payload bytes of a row as the algorithmic-bytes formula counts them:
 // uint 4|S|, bitset 8 (words + 1), pshort 2 (|S| + 2 partitions).
 __device__ __forceinline__ uint64_t payload_bytes(const RowView& V) {
@@ -480,13 +477,15 @@ __device__ __forceinline__ uint64_t payload_bytes(const RowView& V) {
   return 2ull * V.len;
 }
 
-// CTA-cooperative decode of a row into a sorted u32 list in shared memory.
-template <uint32_t kThreads>
-__device__ inline void cta_decode(const RowView& A, uint32_t* list, uint32_t* scan) {
+// CTA-cooperative decode of a row: put(k, x) for the k-th smallest element x of
+// every k < card, each from one thread (put uses no collectives).  The caller
+// synchronizes.  scan: kThreads / 32 words of shared memory.
+template <uint32_t kThreads, class Put>
+__device__ __forceinline__ void cta_decode_to(const RowView& A, uint32_t* scan, Put&& put) {
   const uint32_t tid = threadIdx.x;
   if (A.type == TY_UINT) {
     const uint32_t* a = static_cast<const uint32_t*>(A.p);
-    for (uint32_t k = tid; k < A.card; k += kThreads) list[k] = a[k];
+    for (uint32_t k = tid; k < A.card; k += kThreads) put(k, a[k]);
     return;
   }
   if (A.type == TY_BITSET) {
@@ -511,7 +510,7 @@ __device__ inline void cta_decode(const RowView& A, uint32_t* list, uint32_t* sc
         woff += w < warp ? t : 0u;
         total += t;
       }
-      if (c) emit_pair_bits(x0, x1, A.aux + 2u * (uint32_t)q, list, base_pos + woff + ex);
+      if (c) emit_pair_bits(x0, x1, A.aux + 2u * (uint32_t)q, base_pos + woff + ex, put);
       base_pos += total;
     }
     return;
@@ -521,18 +520,26 @@ __device__ inline void cta_decode(const RowView& A, uint32_t* list, uint32_t* sc
     uint32_t i = 0, pos = 0;
     while (i < A.len) {
       const uint32_t hb = (uint32_t)s[i] << 16, cnt = (uint32_t)s[i + 1] + 1;
-      for (uint32_t k = tid; k < cnt; k += 32) list[pos + k] = hb | s[i + 2 + k];
+      for (uint32_t k = tid; k < cnt; k += 32) put(pos + k, hb | s[i + 2 + k]);
       pos += cnt;
       i += cnt + 2;
     }
   }
 }
 
-// Warp-cooperative decode into the warp's slice (card <= kLightMax).
-__device__ __forceinline__ void warp_decode(const RowView& A, uint32_t* list, uint32_t lane) {
+// As cta_decode_to into a sorted u32 list in shared memory.
+template <uint32_t kThreads>
+__device__ inline void cta_decode(const RowView& A, uint32_t* list, uint32_t* scan) {
+  cta_decode_to<kThreads>(A, scan, [&](uint32_t k, uint32_t x) { list[k] = x; });
+}
+
+// Warp-cooperative decode: put(k, x) for the k-th smallest element x, each from
+// one lane.  The caller synchronizes.
+template <class Put>
+__device__ __forceinline__ void warp_decode_to(const RowView& A, uint32_t lane, Put&& put) {
   if (A.type == TY_UINT) {
     const uint32_t* a = static_cast<const uint32_t*>(A.p);
-    for (uint32_t k = lane; k < A.card; k += 32) list[k] = a[k];
+    for (uint32_t k = lane; k < A.card; k += 32) put(k, a[k]);
   } else if (A.type == TY_BITSET) {
     // 16-byte loads (32 word pairs = 512 bytes per warp round); rounds whose
     // words are all zero cost one vote.
@@ -544,7 +551,7 @@ __device__ __forceinline__ void warp_decode(const RowView& A, uint32_t* list, ui
       const uint32_t c = __popcll(lo64(v)) + __popcll(hi64(v));
       if (!__any_sync(FULL, c != 0)) continue;
       const uint32_t ex = warp_exclusive_scan(c, lane);
-      if (c) emit_pair_bits(lo64(v), hi64(v), A.aux + 2u * (uint32_t)q, list, pos + ex);
+      if (c) emit_pair_bits(lo64(v), hi64(v), A.aux + 2u * (uint32_t)q, pos + ex, put);
       pos += __shfl_sync(FULL, ex + c, 31);
     }
   } else {
@@ -552,11 +559,14 @@ __device__ __forceinline__ void warp_decode(const RowView& A, uint32_t* list, ui
     uint32_t i = 0, pos = 0;
     while (i < A.len) {
       const uint32_t hb = (uint32_t)s[i] << 16, cnt = (uint32_t)s[i + 1] + 1;
-      for (uint32_t k = lane; k < cnt; k += 32) list[pos + k] = hb | s[i + 2 + k];
+      for (uint32_t k = lane; k < cnt; k += 32) put(pos + k, hb | s[i + 2 + k]);
       pos += cnt;
       i += cnt + 2;
     }
   }
+}
+__device__ __forceinline__ void warp_decode(const RowView& A, uint32_t* list, uint32_t lane) {
+  warp_decode_to(A, lane, [&](uint32_t k, uint32_t x) { list[k] = x; });
   __syncwarp();
 }
 

@@ -76,26 +76,31 @@ struct PivotArgs {
   const uint4* arena;
   const uint32_t* order;   // rows sorted by descending card
   uint32_t n_order;        // rows in the plan
-  uint32_t n_heavy;        // order[0, n_heavy) are processed CTA-wide
+  uint32_t n_heavy;        // order[0, n_heavy) are processed CTA-wide, the rest by a warp each
   uint32_t n_giant;        // order[0, n_giant) have decoded lists in giant_lists
   const uint32_t* giant_lists;
   const unsigned long long* giant_off;
-  uint32_t* counters;      // [0] next heavy unit, [1] next light chunk, [15] device error flags
+  // [0] next unit (pivots above kCtaListCap), [1] next warp pivot, [2] next
+  // unit (the other large pivots), [3] next tiny pivot, [4] next mid pivot,
+  // [15] device error flags
+  uint32_t* counters;
   unsigned long long* out; // result; in batch mode out[num_graphs]
-  uint32_t unit_span;      // pivot positions e per heavy unit
+  uint32_t unit_span;      // pivot positions e per unit of a large pivot
   const uint32_t* graph_rows;  // batch mode: graph g owns rows [graph_rows[g], graph_rows[g+1]); else null
   uint32_t num_graphs;
   const unsigned long long* core;  // dense core bitmap of rows j < core_k (see core_row_offset), or null
   uint32_t core_k;
-  uint32_t core_hot_words;  // light-pivot core probes of words below this keep their L2 lines (0: no hints)
-  const unsigned long long* filter;  // row filters of rows [kFilterLo, filter_k), or null (see filter_bit)
-  uint32_t filter_words;             // words per row filter (16, 32 or 64)
-  uint32_t filter_k;
+  uint64_t n;              // rows of the matrix
+  uint32_t n_above_tiny;   // rows in the plan with more than 8 entries
+  uint32_t n_large;        // order[0, n_large) have units (the rest up to n_heavy run whole)
+  uint32_t max_warp, max_mid, max_large;  // largest pivot of each tier
 };
 constexpr uint32_t kCtaThreads = 256;
 constexpr uint32_t kLightMax = 160;    // largest light_max: warp-wide pivots fit a slice of this size
+constexpr uint32_t kMidMax = 512;      // heavy pivots up to this size run whole, larger ones in units
+constexpr uint32_t kWarpWindow = 8192, kCtaWindow = 65536;  // bits of the pivots' membership windows
 constexpr uint32_t kDefaultLightMax = 96;
-constexpr uint32_t kDefaultUnitSpan = 128;
+constexpr uint32_t kDefaultUnitSpan = 1024;
 constexpr uint32_t kCtaListCap = 2048; // CTA-staged list capacity (elements)
 constexpr uint32_t kCtaWordCap = 1024; // CTA-staged bitset words capacity
 cudaError_t launch_pivot_units(const RowDesc* desc, const uint32_t* order, uint32_t n_heavy,
@@ -124,25 +129,6 @@ __host__ __device__ inline uint64_t core_row_offset(uint32_t j) {
 cudaError_t launch_core_build(const RowDesc* desc, const uint4* arena, uint32_t core_k, unsigned long long* core,
                               cudaStream_t st);
 
-// Core row filters: for every core row j in [kFilterLo, filter_k = core_k), a
-// bitmap of filter_words * 64 bits with bit filter_bit(x) set for each x in
-// row(j) ∩ [0, j) (Fibonacci hashing: the top bits of x * 2^32 / phi).  A light
-// pivot's probe (j, x) reads the filter word first and the core word only when
-// the bit is set, so a probe that misses (about 91% of them at R-MAT scale 22)
-// costs one word of the small filter, loaded with the L2 keep hint, instead of
-// a DRAM sector of the core; that makes a larger core pay (at scale 22 the
-// tuner picks 262,144 rows with filters, 8.35 ms per count, against 98,304
-// rows without, 8.86 ms).  A set bit is only a hint: the core word decides, so
-// counts are exact.  Rows below kFilterLo form a core block small enough to
-// stay in L2 and have no filter.  (Filters on rows past the core, falling back
-// to the row's binary search, measured no faster.)
-constexpr uint32_t kFilterLo = 4096;
-__host__ __device__ inline uint32_t filter_bit(uint32_t x, uint32_t filter_words) {
-  const uint32_t log2_bits = filter_words == 16 ? 10u : filter_words == 32 ? 11u : 12u;
-  return (x * 2654435769u) >> (32 - log2_bits);
-}
-cudaError_t launch_filter_build(const RowDesc* desc, const uint4* arena, uint32_t filter_k, uint32_t filter_words,
-                                unsigned long long* filter, cudaStream_t st);
 cudaError_t launch_similar(uint64_t n, const RowDesc* desc, const uint4* arena, uint32_t vstar,
                            uint32_t threshold, unsigned long long* out, cudaStream_t st);
 cudaError_t launch_intersect_rows(uint64_t n, const RowDesc* desc, const uint4* arena, const uint32_t* a,
@@ -165,17 +151,19 @@ struct CliqueArgs {
   // cursor that hands out j.
   uint32_t* tuples;
   uint64_t capacity;
+  unsigned long long* tri;  // also the triangles of the pivots the warp kernel takes (laid out as out), or null
 };
 constexpr uint32_t kCliqueMaxK = 16;
 // Largest pivot row a clique count accepts: a pivot's packed masks are indexed
 // with 32-bit word offsets, which stay exact below 2^18 entries (a degree-
 // ordered graph reaches that only past 2^35 edges).
 constexpr uint32_t kCliqueMaxPivot = 1u << 18;
+constexpr uint32_t kCliqueWarpMax = 64;    // pivots up to this size are a warp's
 constexpr uint32_t kCliqueSmemMax = 2048;  // no pivot above this size keeps its masks in shared memory
 // Words of one pivot's working set (list, masks, per-warp DFS stacks).
 uint64_t clique_slot_words(uint32_t cmax, uint32_t k);
-cudaError_t launch_clique_light(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
-                                int grid, cudaStream_t st, bool list = false);
+cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
+                               int sms, cudaStream_t st, bool list = false);
 // Largest pivot (<= kCliqueSmemMax) whose k-clique working set fits one CTA's
 // opt-in shared memory on `device`; larger pivots use global scratch slots.
 uint32_t clique_smem_cap(uint32_t k, int device);

@@ -20,16 +20,15 @@ struct Plan {
   uint32_t* giant_lists = nullptr;
   unsigned long long* giant_off = nullptr;
   std::vector<uint32_t> starts;  // bin starts: rows with card > x are order[0, starts[65535 - x])
-  // Heavy units for the current (light_max, unit_span).
+  // Units of the large pivots (above light_max and kMidMax) for the current (light_max, unit_span).
   uint32_t light_max = 0, unit_span = 0;
-  uint32_t n_heavy = 0;           // order[0, n_heavy) have card > light_max
+  uint32_t n_heavy = 0, n_large = 0;  // order[0, n_heavy) have card > light_max, [0, n_large) units
+  bool units_ready = false;
   uint2* units = nullptr;         // (order position, part)
   uint32_t n_units = 0;
   uint64_t units_cap = 0;
   unsigned long long* core = nullptr;  // dense core bitmap (rows j < core_k)
   uint32_t core_k = 0;
-  unsigned long long* filter = nullptr;  // row filters (rows [kFilterLo, filter_k))
-  uint32_t filter_words = 0, filter_k = 0;
   // rows in the plan with card > x (x < 65535)
   uint32_t above(uint32_t x) const { return starts.empty() ? 0 : starts[65535 - x]; }
   // largest card <= x present in the plan (0 if none)
@@ -70,8 +69,6 @@ struct Matrix {
   uint32_t light_max = kDefaultLightMax;
   uint32_t unit_span = kDefaultUnitSpan;
   uint32_t core_limit = kCoreDefaultK;  // rows in the dense core at most (0 = no core)
-  uint32_t core_hot_words = 0;          // see PivotArgs::core_hot_words
-  uint32_t core_filter_words = 0;       // words per core row filter (0: no filters)
   bool is_batch = false;            // the union matrix of an eh_batch_t
   bool shape_set = false;           // a shape was given (eh_matrix_set_shape, the tuner): no cached shape
   // Where the matrix's buffers are read: one event per stream, recorded after
@@ -92,7 +89,7 @@ struct Matrix {
 // 400 MB again costs about 1 ms on GB300.  16 GiB holds a rebuilt scale-22
 // matrix with its largest tuned core (4.3 GB) and its build scratch.
 constexpr uint64_t kPoolKeep = 16ull << 30;
-// Which pool: the dense cores and row filters of work plans (large, and kept
+// Which pool: the dense cores of work plans (large, and kept
 // for the matrix's life) come from a pool of their own.  In the same pool as
 // the other buffers, a resident 4.3 GB core made every later build and plan
 // of another matrix 0.6 + 0.6 ms slower at scale 22; in their own pool (or
@@ -120,8 +117,7 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
 eh_status ensure_plan(Matrix* m, cudaStream_t st);
 eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaStream_t st);
 eh_status ensure_core(Matrix* m, cudaStream_t st);
-// Frees the parts of the plan that depend on the work shape (heavy units, dense
-// core, row filters), so that the next ensure_plan builds them from nothing.
+// Frees the parts of the plan that depend on the work shape (units, dense core), so that the next ensure_plan builds them from nothing.
 eh_status drop_shape_parts(Matrix* m, cudaStream_t st);
 // Records that launches reading m's buffers were just queued on st.
 void note_use(Matrix* m, cudaStream_t st);
@@ -133,12 +129,14 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out);
 // Count launches; graph_rows / num_graphs != null selects per-graph outputs
 // out[num_graphs].  ws == null uses the matrix's own workspace.  The plan must
 // already exist when ws != null (launches with a workspace never allocate it).
+// large_only (batches): only the pivots above kCliqueWarpMax entries.
 eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32_t* graph_rows, uint32_t num_graphs,
-                                cudaStream_t st, Workspace* ws = nullptr);
+                                cudaStream_t st, Workspace* ws = nullptr, bool large_only = false);
 eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st);
 // tuples != null or list: write the k = 3 or 4 cliques as tuples (CliqueArgs::tuples).
+// tri: the triangles of the pivots of up to kCliqueWarpMax entries are added there.
 eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const uint32_t* graph_rows,
                          uint32_t num_graphs, cudaStream_t st, Workspace* ws = nullptr, bool list = false,
-                         uint32_t* tuples = nullptr, uint64_t capacity = 0);
+                         uint32_t* tuples = nullptr, uint64_t capacity = 0, unsigned long long* tri = nullptr);
 
 }  // namespace eh

@@ -100,14 +100,14 @@ extern "C" eh_status eh_count_cliques_noalloc(eh_matrix_t mh, uint32_t k, uint64
   const Plan& p = m->plan;
   const uint32_t cap = clique_smem_cap(k, m->device);
   const uint32_t nG = p.above(cap);
-  const uint32_t nB = p.above(32);
+  const uint32_t nB = p.above(kCliqueWarpMax);
   const uint32_t nL = p.above(k - 2);
   uint32_t* counters = scratch;
   uint32_t* slots = scratch + kCounterWords;
   const uint64_t slot_capacity = kNoAllocScratchWords - kCounterWords;
   // No dense core here: the counts probe the rows themselves.
   CliqueArgs a{m->desc, m->arena, p.order, k, reinterpret_cast<unsigned long long*>(d_count), nullptr, 0,
-               nullptr, 0};
+               nullptr, 0, nullptr, 0, nullptr};
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
   uint64_t grid_g = 0;
@@ -134,8 +134,7 @@ extern "C" eh_status eh_count_cliques_noalloc(eh_matrix_t mh, uint32_t k, uint64
     if (e != cudaSuccess) return set_error(EH_ERR_CUDA, "clique kernel (shared): %s", cudaGetErrorString(e));
   }
   if (nL > nB) {
-    const int grid = (int)std::min<uint64_t>((nL - nB + 63) / 64, 8ull * sms);
-    e = launch_clique_light(a, nB, nL, counters + 4, grid > 0 ? grid : 1, st);
+    e = launch_clique_warp(a, nB, nL, counters + 4, sms, st);
     if (e != cudaSuccess) return set_error(EH_ERR_CUDA, "clique kernel (warp): %s", cudaGetErrorString(e));
   }
   return EH_OK;
