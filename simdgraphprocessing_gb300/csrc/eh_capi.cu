@@ -555,6 +555,27 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
 
 }  // namespace eh
 
+namespace eh {
+eh_status ensure_vbits(Matrix* m) {
+  if (m->vbits) return EH_OK;
+  uint32_t v = 0;
+  eh_status s = eh_matrix_get_max_row_id(reinterpret_cast<eh_matrix_t>(m), &v);
+  if (s != EH_OK) return s;
+  unsigned long long* bits = nullptr;
+  const uint64_t bytes = row_bits_words(m->n) * sizeof(unsigned long long);
+  CU(pool_alloc((void**)&bits, bytes, nullptr), "similar_nodes bitmap");
+  cudaError_t e = launch_row_bits(m->n, m->desc, m->arena, v, bits, nullptr);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // queries may run on any stream
+  if (e != cudaSuccess) {
+    cudaFreeAsync(bits, nullptr);
+    return cuda_fail(e, "similar_nodes bitmap");
+  }
+  m->vbits = bits;
+  m->device_bytes += bytes;
+  return EH_OK;
+}
+}  // namespace eh
+
 using eh::Matrix;
 using eh::set_error;
 
@@ -793,7 +814,7 @@ void eh_matrix_free(eh_matrix_t mh) {
     st = nullptr;
   }
   void* bufs[] = {m->desc, m->arena, m->counters, m->plan.order, m->plan.units, m->plan.giant_lists,
-                  m->plan.giant_off, m->plan.core, m->clique_scratch};
+                  m->plan.giant_off, m->plan.core, m->clique_scratch, m->vbits};
   for (void* b : bufs)
     if (b) cudaFreeAsync(b, st);
   for (auto& u : m->uses) cudaEventDestroy(u.second);
@@ -832,11 +853,10 @@ eh_status eh_similar_nodes_async(eh_matrix_t mh, uint32_t threshold, uint64_t* d
   CHECK_MATRIX(mh);
   EH_CHECK_ARG(d_count, "d_count is NULL");
   Matrix* m = MX(mh);
-  uint32_t vstar = 0;
-  eh_status s = eh_matrix_get_max_row_id(mh, &vstar);
+  eh_status s = eh::ensure_vbits(m);
   if (s != EH_OK) return s;
-  CU(eh::launch_similar(m->n, m->desc, m->arena, vstar, threshold, reinterpret_cast<unsigned long long*>(d_count),
-                        ST(stream)),
+  CU(eh::launch_similar(m->n, m->desc, m->arena, (uint32_t)m->vstar, m->vbits, threshold,
+                        reinterpret_cast<unsigned long long*>(d_count), ST(stream)),
      "similar_nodes kernel");
   eh::note_use(m, ST(stream));
   return EH_OK;

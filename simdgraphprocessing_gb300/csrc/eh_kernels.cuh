@@ -129,8 +129,14 @@ __host__ __device__ inline uint64_t core_row_offset(uint32_t j) {
 cudaError_t launch_core_build(const RowDesc* desc, const uint4* arena, uint32_t core_k, unsigned long long* core,
                               cudaStream_t st);
 
+// A row as a bitmap over all n ids, for similar_nodes (one spare word: bitset
+// payloads are read in word pairs).
+__host__ __device__ inline uint64_t row_bits_words(uint64_t n) { return (n + 63) / 64 + 1; }
+cudaError_t launch_row_bits(uint64_t n, const RowDesc* desc, const uint4* arena, uint32_t v, unsigned long long* bits,
+                            cudaStream_t st);
 cudaError_t launch_similar(uint64_t n, const RowDesc* desc, const uint4* arena, uint32_t vstar,
-                           uint32_t threshold, unsigned long long* out, cudaStream_t st);
+                           const unsigned long long* bits, uint32_t threshold, unsigned long long* out,
+                           cudaStream_t st);
 cudaError_t launch_intersect_rows(uint64_t n, const RowDesc* desc, const uint4* arena, const uint32_t* a,
                                   const uint32_t* b, uint64_t np, uint32_t* counts, cudaStream_t st);
 cudaError_t launch_max_row(uint64_t n, const RowDesc* desc, unsigned long long* out, cudaStream_t st);

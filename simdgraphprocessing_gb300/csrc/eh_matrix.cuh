@@ -62,6 +62,7 @@ struct Matrix {
   unsigned long long* result = nullptr;
   int grid = 0;
   int64_t vstar = -1;
+  unsigned long long* vbits = nullptr;  // row vstar as a bitmap (similar_nodes), built with its first query
   uint64_t device_bytes = 0;
   uint32_t* clique_scratch = nullptr;  // global slots for the largest clique pivots
   uint64_t clique_scratch_words = 0;
@@ -119,6 +120,8 @@ eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaSt
 eh_status ensure_core(Matrix* m, cudaStream_t st);
 // Frees the parts of the plan that depend on the work shape (units, dense core), so that the next ensure_plan builds them from nothing.
 eh_status drop_shape_parts(Matrix* m, cudaStream_t st);
+// The largest row's id and its bitmap (Matrix::vstar, vbits).
+eh_status ensure_vbits(Matrix* m);
 // Records that launches reading m's buffers were just queued on st.
 void note_use(Matrix* m, cudaStream_t st);
 // Makes st wait for every launch note_use has recorded on m, on any stream.

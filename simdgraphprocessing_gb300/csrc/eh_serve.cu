@@ -69,7 +69,6 @@ struct Slot {
 struct GraphEntry {
   Matrix* low = nullptr;  // nbr < node rows: triangles, cliques
   Matrix* all = nullptr;  // full rows: similar_nodes
-  uint32_t vstar = 0;
   uint64_t bytes = 0;
 };
 
@@ -124,7 +123,8 @@ eh_status launch_query(Server* s, Slot& sl, const Query& q) {
   } else if (q.kind == EH_QUERY_CLIQUES) {
     st = launch_cliques(ge.low, q.param, sl.d_out, nullptr, 0, sl.st, &sl.ws);
   } else {
-    cudaError_t e = launch_similar(ge.all->n, ge.all->desc, ge.all->arena, ge.vstar, q.param, sl.d_out, sl.st);
+    cudaError_t e = launch_similar(ge.all->n, ge.all->desc, ge.all->arena, (uint32_t)ge.all->vstar, ge.all->vbits, q.param,
+                                   sl.d_out, sl.st);
     if (e != cudaSuccess) st = set_error(EH_ERR_CUDA, "similar_nodes kernel: %s", cudaGetErrorString(e));
   }
   if (st != EH_OK) return st;
@@ -314,7 +314,7 @@ eh_status eh_server_add_graph(eh_server_t sh, uint64_t n, const uint64_t* offset
   eh::GraphEntry ge;
   ge.low = reinterpret_cast<eh::Matrix*>(low);
   ge.all = reinterpret_cast<eh::Matrix*>(all);
-  if ((st = eh::ensure_plan(ge.low, nullptr)) == EH_OK) st = eh_matrix_get_max_row_id(all, &ge.vstar);
+  if ((st = eh::ensure_plan(ge.low, nullptr)) == EH_OK) st = eh::ensure_vbits(ge.all);
   if (st != EH_OK) {
     eh_matrix_free(low);
     eh_matrix_free(all);
