@@ -464,6 +464,10 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   if (m->tot.max_card >= kCliqueMaxPivot)
     return set_error(EH_ERR_UNSUPPORTED, "a row of %llu selected entries is above the clique kernels' limit of %u",
                      (unsigned long long)m->tot.max_card, kCliqueMaxPivot - 1);
+  // 3-cliques are triangles.  (Rows of 2^16 entries stay here: a pshort row that
+  // long is where the triangle count follows the reference's u16 counts.)
+  if (k == 3 && !list && !graph_rows && m->tot.max_card < 65536u)
+    return launch_triangle_count(m, out, nullptr, 0, st, ws);
   eh_status s = ensure_plan(m, st);
   if (s != EH_OK) return s;
   const Plan& p = m->plan;
@@ -500,16 +504,23 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   }
   // The shared-memory tier runs in size bands, each launch sized for its own
   // largest pivot, so that the many small pivots are not held to the
-  // occupancy of the largest one.  Band edges where the CTAs per SM change
-  // (1 above 1,024 entries, 3 up to 1,024, 5 up to 768, 6 -- the register
-  // limit -- up to 512); fewer bands mean fewer drained-GPU tails.
-  const uint32_t bands[] = {cap, 1024, 768, 512, kCliqueWarpMax};
-  for (int b = 0; b + 1 < (int)(sizeof(bands) / sizeof(bands[0])); b++) {
+  // occupancy of the largest one; fewer bands mean fewer drained-GPU tails.
+  // k = 4 has its own kernel up to kCliqueMidMax entries; otherwise the edges
+  // are where the CTAs per SM change (1 above 1,024 entries, 3 up to 1,024, 5 up
+  // to 768, 6 -- the register limit -- up to 512).
+  const bool mid = k == 4 && !list;
+  const uint32_t bands_mid[] = {cap, kCliqueMidMax, 512, 256, kCliqueWarpMax};
+  const uint32_t bands_dfs[] = {cap, 1024, 768, 512, kCliqueWarpMax};
+  const uint32_t* bands = mid ? bands_mid : bands_dfs;
+  for (int b = 0; b + 1 < 5; b++) {
     if (bands[b] <= bands[b + 1]) continue;
     const uint32_t p0 = p.above(bands[b]), p1 = p.above(bands[b + 1]);
     if (p1 <= p0) continue;
     const uint32_t cmax = p.largest_at_most(bands[b]);
-    CU(launch_clique_cta(a, p0, p1, w.counters + 3 + b, cmax, nullptr, 0, st, list), "clique kernel (shared)");
+    if (mid && bands[b] <= kCliqueMidMax)
+      CU(launch_clique_mid(a, p0, p1, w.counters + 3 + b, cmax, sms, st), "clique kernel (mid)");
+    else
+      CU(launch_clique_cta(a, p0, p1, w.counters + 3 + b, cmax, nullptr, 0, st, list), "clique kernel (shared)");
   }
   if (nL > nB) CU(launch_clique_warp(a, nB, nL, w.counters + 11, sms, st, list), "clique kernel (warp)");
   note_use(m, st);

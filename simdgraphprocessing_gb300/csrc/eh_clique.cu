@@ -266,6 +266,189 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, ui
   }
 }
 
+// ---- mid tier, k = 4: kCliqueWarpMax < |A_i| <= kCliqueMidMax, one CTA per pivot ----
+// The masks in shared memory as rows of 16-byte quads: row e holds bits < e in
+// ceil(e / 128) quads, from quad quad_off(e) on.
+//  Phase 1, j = A_i[e] < core_k: a lane keeps one t of 32 (its element's word and
+//    bit in a core row) and walks the e's, eight words in flight; a ballot per e
+//    gives a mask word, which lane e - e0 keeps and stores once per 16 e's.  That
+//    is about half the instructions of a warp per e, which recomputed every
+//    element's address for every e.  j >= core_k: a warp per e probes or streams
+//    row(j).
+//  Phase 2: the sum over e and t in M[e] of popc(M[e] & M[t]).  A lane keeps the
+//    quad of M[t] for one t of 32, and the e's quads are broadcast: three LDS and
+//    a masked AND per word into a carry-save counter, whatever the density, no
+//    bank conflicts, and the popcount unit (16 lanes per cycle and SM) sees one
+//    word in eight.
+// Bound by instruction issue.  Tensor cores do not help: the one-bit mma.sync
+// (m16n8k256, and.popc) takes 545 cycles a warp on this chip, fewer bits per cycle
+// than the AND loop.  R-MAT, 1 M vertices, 4-cliques: phase 1 / phase 2 took 1.49 /
+// 2.73 ms with a warp per e in both.
+__host__ __device__ __forceinline__ uint32_t quad_off(uint32_t e) {
+  if (e == 0) return 0;
+  const uint32_t m = (e - 1) >> 7, r = (e - 1) & 127;
+  return (64 * m + r) * (m + 1);
+}
+
+__host__ __device__ constexpr uint32_t mid_slots(uint32_t c) { return (c + 31) & ~31u; }
+static uint32_t mid_bytes(uint32_t cmax) { return quad_off(cmax) * 16 + mid_slots(cmax) * (4 + 4 + 2); }
+
+struct MaskSum {  // carry-save counter of 32-bit words
+  uint32_t one, two, four, eights;
+  __device__ __forceinline__ void clear() { one = two = four = eights = 0; }
+  __device__ __forceinline__ void add8(const uint32_t (&x)[8]) {
+    const uint32_t a = csa(one, x[0], x[1]), b = csa(one, x[2], x[3]), f = csa(two, a, b);
+    const uint32_t c = csa(one, x[4], x[5]), d = csa(one, x[6], x[7]), g = csa(two, c, d);
+    eights += __popc(csa(four, f, g));
+  }
+  __device__ __forceinline__ uint32_t total() const {
+    return 8 * eights + 4 * __popc(four) + 2 * __popc(two) + __popc(one);
+  }
+};
+
+// Phase 2 for one quad of 32 t's (mt: this lane's, W words of it in use), e = e0,
+// e0 + NW, ... < c: quad q of M[e] against mt where bit `lane` of M[e]'s word r is set.
+template <int W>
+__device__ __forceinline__ void and_quads(const uint4* m4, const uint16_t* ro, uint4 mt, uint32_t q, uint32_t r,
+                                          uint32_t e0, uint32_t c, uint32_t lane, MaskSum& sum) {
+  constexpr int E = W == 1 ? 8 : W == 2 ? 4 : 2;  // e's per step: eight words or six
+  const uint32_t m[4] = {mt.x, mt.y, mt.z, mt.w};
+  for (uint32_t e = e0; e < c; e += E * NW) {
+    uint32_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < E; u++) {
+      const uint32_t eu = e + u * NW;
+      const bool in = eu < c;
+      const uint4* row = m4 + ro[in ? eu : e];
+      const uint32_t bits = in ? reinterpret_cast<const uint32_t*>(row)[r] : 0u;
+      const uint32_t sel = (uint32_t)((int32_t)(bits << (31 - lane)) >> 31);
+      const uint4 v = row[q];
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < W; k++) x[u * W + k] = w[k] & m[k] & sel;
+    }
+    sum.add8(x);
+  }
+}
+
+__global__ void __launch_bounds__(kCtaThreads, 5) k_clique_mid(CliqueArgs a, uint32_t pos_begin, uint32_t pos_end,
+                                                               uint32_t* counter, uint32_t cmax) {
+  extern __shared__ __align__(16) uint4 m4[];
+  __shared__ uint32_t s_unit, s_scan[NW];
+  uint32_t* m32 = reinterpret_cast<uint32_t*>(m4);
+  uint32_t* list = reinterpret_cast<uint32_t*>(m4 + quad_off(cmax));
+  uint32_t* off = list + mid_slots(cmax);  // word (32-bit) offset of core row A_i[e]
+  uint16_t* ro = reinterpret_cast<uint16_t*>(off + mid_slots(cmax));
+  const uint32_t* core32 = reinterpret_cast<const uint32_t*>(a.core);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long acc = 0;
+  MaskSum sum;
+  sum.clear();
+  for (;;) {
+    if (threadIdx.x == 0) s_unit = atomicAdd(counter, 1u) + pos_begin;
+    __syncthreads();  // also: every thread is done with the previous pivot's masks
+    const uint32_t unit = s_unit;
+    if (unit >= pos_end) break;
+    const uint32_t row = a.order[unit];
+    const RowView A = load_view(a.desc, a.arena, row);
+    const uint32_t c = A.card;
+    cta_decode_to<kCtaThreads>(A, s_scan, [&](uint32_t k, uint32_t x) {
+      list[k] = x;
+      off[k] = x < a.core_k ? 2 * core_offset32(x) : 0u;
+    });
+    const uint32_t quads = quad_off(c);
+    for (uint32_t k = threadIdx.x; k < quads; k += kCtaThreads) m4[k] = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t k = threadIdx.x; k < c; k += kCtaThreads) ro[k] = (uint16_t)quad_off(k);
+    __syncthreads();
+    const uint32_t ea = lower_bound_u32(list, 0, c, a.core_k);
+    // phase 1, j < core_k: tasks (32 t's from 32 r, 16 e's from 16 b), b >= 2 r
+    const uint32_t nb = (ea + 15) >> 4;
+    for (uint32_t r = 0, id = warp;;) {
+      while (2 * r < nb && id >= nb - 2 * r) {
+        id -= nb - 2 * r;
+        r++;
+      }
+      if (2 * r >= nb) break;
+      const uint32_t e0 = 16 * (2 * r + id), t = 32 * r + lane;
+      const uint32_t x = t < ea ? list[t] : 0u;
+      const uint32_t* col = core32 + (x >> 5);
+      const uint32_t bit = 1u << (x & 31);
+      uint32_t word = 0;
+      const bool whole = e0 >= 32 * (r + 1) && e0 + 16 <= ea;  // every t < e
+#pragma unroll
+      for (int h = 0; h < 16; h += 8) {
+        uint32_t v[8];
+        if (whole) {
+#pragma unroll
+          for (int u = 0; u < 8; u++) v[u] = __ldg(col + off[e0 + h + u]);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            const uint32_t e = e0 + h + u;
+            v[u] = (t < e && e < ea) ? __ldg(col + off[e]) : 0u;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const uint32_t bal = __ballot_sync(FULL, v[u] & bit);
+          if (lane == (uint32_t)(h + u)) word = bal;
+        }
+      }
+      const uint32_t e = e0 + lane;
+      if (lane < 16 && e < ea && e > 32 * r) m32[4 * (uint32_t)ro[e] + r] = word;
+      id += NW;
+    }
+    // phase 1, j >= core_k: a warp per e
+    for (uint32_t e = max(1u, ea) + warp; e < c; e += NW) {
+      const uint32_t j = list[e];
+      uint32_t* Me = m32 + 4 * (uint32_t)ro[e];
+      const RowView B = load_view(a.desc, a.arena, j);
+      if (B.card == 0) continue;
+      bool stream = false;
+      if (B.type == TY_UINT) stream = (uint64_t)B.card * ilog2p1_c(e) < (uint64_t)e * ilog2p1_c(B.card) * 4u;
+      else if (B.type == TY_PSHORT) stream = (uint64_t)B.card * ilog2p1_c(e) < (uint64_t)e * (B.aux + ilog2p1_c(B.card)) * 4u;
+      if (!stream) {
+        for (uint32_t b = 0; b < e; b += 32) {
+          const uint32_t t = b + lane;
+          const uint32_t word = __ballot_sync(FULL, t < e && row_contains(B, list[t]));
+          if (lane == 0) Me[b >> 5] = word;
+        }
+      } else {
+        warp_for_each(B, j, lane, [&](uint32_t y) {
+          const uint32_t t = lower_bound_u32(list, 0, e, y);
+          if (t < e && list[t] == y) atomicOr(&Me[t >> 5], 1u << (t & 31));
+        });
+      }
+    }
+    __syncthreads();
+    // phase 2
+    for (uint32_t r = 0; 32 * r < c; r++) {
+      const uint32_t t = 32 * r + lane, e0 = 32 * r + 1 + warp, last = r >> 2;
+      for (uint32_t q = 0; q <= last; q++) {
+        const uint4 mt = (t < c && 128 * q < t) ? m4[ro[t] + q] : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t words = q < last ? 4u : (r & 3) + 1;
+        if (words == 1) and_quads<1>(m4, ro, mt, q, r, e0, c, lane, sum);
+        else if (words == 2) and_quads<2>(m4, ro, mt, q, r, e0, c, lane, sum);
+        else if (words == 3) and_quads<3>(m4, ro, mt, q, r, e0, c, lane, sum);
+        else and_quads<4>(m4, ro, mt, q, r, e0, c, lane, sum);
+      }
+    }
+    if (a.graph_rows) {  // batch: each warp's share of this pivot goes to its graph
+      const uint32_t pc = warp_sum_u32(sum.total());  // below 2^28
+      sum.clear();
+      if (pc) {
+        const uint32_t g = warp_graph_of(a.graph_rows, a.num_graphs, row, lane);
+        if (lane == 0) atomicAdd(&a.out[g], (unsigned long long)pc);
+      }
+    } else {
+      acc += 8ull * sum.eights;
+      sum.eights = 0;
+    }
+  }
+  acc = warp_sum_u64(acc + sum.total());
+  if (lane == 0 && acc) atomicAdd(a.out, acc);
+}
+
 // ---- CTA tiers: one pivot per CTA; masks in shared memory or a global slot ----
 // Per CTA working set (words): list[cmax] | masks[mask_off(cmax)] | stacks[NW][2 * (k-2) * W]
 // (stacks only for k >= 5); W = mask_len(cmax) is the DFS stack row length.
@@ -543,6 +726,25 @@ cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t
   const unsigned grid = std::max(1u, std::min(5u * (uint32_t)std::max(1, sms), (n + NW * grab - 1) / (NW * grab)));
   if (list) k_clique_warp<true><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, grab, counter);
   else k_clique_warp<false><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, grab, counter);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_clique_mid(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
+                              uint32_t cmax, int sms, cudaStream_t st) {
+  if (pos_end <= pos_begin) return cudaSuccess;
+  static std::atomic<bool> allowed[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!allowed[dev].load()) {
+    const cudaError_t e = cudaFuncSetAttribute(k_clique_mid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)mid_bytes(kCliqueMidMax));
+    if (e != cudaSuccess) return e;
+    allowed[dev].store(true);
+  }
+  const uint32_t bytes = mid_bytes(cmax), per = std::max(1u, std::min(5u, (228u << 10) / (bytes + 2048)));
+  const unsigned grid = std::min<unsigned>(pos_end - pos_begin, per * (unsigned)std::max(1, sms));
+  k_clique_mid<<<grid, kCtaThreads, bytes, st>>>(a, pos_begin, pos_end, counter, cmax);
   return cudaGetLastError();
 }
 

@@ -285,20 +285,6 @@ __device__ __forceinline__ void group_sync() {
   else __syncthreads();
 }
 
-// 32-bit form of core_row_offset (core_k <= kCoreMaxK: below 2^30).
-__device__ __forceinline__ uint32_t core_offset32(uint32_t j) {
-  if (j == 0) return 0;
-  const uint32_t q = (j - 1) >> 6, r = (j - 1) & 63;
-  return (q + 1) * (32 * q + r);
-}
-
-// Carry-save adder step: (sum, x, y) -> sum, carry out.
-__device__ __forceinline__ uint32_t csa(uint32_t& sum, uint32_t x, uint32_t y) {
-  const uint32_t carry = (sum & x) | (y & (sum ^ x));
-  sum ^= x ^ y;
-  return carry;
-}
-
 // Carry-save counter of 64-bit words, eight at a time: the popcount unit (16
 // lanes per cycle and SM) sees one word in eight.
 struct WordSum {

@@ -98,6 +98,13 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long x)
   return x;
 }
 
+// Carry-save adder step: (sum, x, y) -> sum, carry out.
+__device__ __forceinline__ uint32_t csa(uint32_t& sum, uint32_t x, uint32_t y) {
+  const uint32_t carry = (sum & x) | (y & (sum ^ x));
+  sum ^= x ^ y;
+  return carry;
+}
+
 // ---- Bitset words as 16-byte pairs ----
 // Every payload starts on a 16-byte boundary and is zero-padded to a multiple
 // of 16 bytes (in the arena and in shared-memory copies of it), so words

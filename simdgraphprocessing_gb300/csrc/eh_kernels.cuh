@@ -126,6 +126,13 @@ __host__ __device__ inline uint64_t core_row_offset(uint32_t j) {
   const uint64_t a = (uint64_t)(j - 1) >> 6, b = (uint64_t)(j - 1) & 63;
   return 32 * a * (a + 1) + b * (a + 1);  // sum over x < j of ceil(x / 64)
 }
+// 32-bit form of core_row_offset (core_k <= kCoreMaxK: below 2^30).
+__device__ __forceinline__ uint32_t core_offset32(uint32_t j) {
+  if (j == 0) return 0;
+  const uint32_t q = (j - 1) >> 6, r = (j - 1) & 63;
+  return (q + 1) * (32 * q + r);
+}
+
 cudaError_t launch_core_build(const RowDesc* desc, const uint4* arena, uint32_t core_k, unsigned long long* core,
                               cudaStream_t st);
 
@@ -173,6 +180,11 @@ cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t
 // Largest pivot (<= kCliqueSmemMax) whose k-clique working set fits one CTA's
 // opt-in shared memory on `device`; larger pivots use global scratch slots.
 uint32_t clique_smem_cap(uint32_t k, int device);
+// 4-cliques of pivots of kCliqueWarpMax < entries <= kCliqueMidMax (cmax the
+// largest of them), one CTA each, masks in shared memory.
+constexpr uint32_t kCliqueMidMax = 1024;
+cudaError_t launch_clique_mid(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
+                              uint32_t cmax, int sms, cudaStream_t st);
 // gscratch == nullptr: masks in dynamic shared memory (grid <= 0: as many CTAs
 // as fit on the GPU, at most one per pivot); else grid slots of
 // clique_slot_words(cmax, k) words each in global memory.
