@@ -3,24 +3,22 @@
 //
 // symbiosity: one warp per row i intersects out(i) (the row matrix) with in(i)
 // (the column matrix) and tests the Jaccard ratio in double precision, as
-// symbiosity.cpp:46-58 does.  Rows too long for a warp (hubs) are listed and
-// taken one per CTA, with the probed row staged in shared memory when it is a
-// uint row that fits.
+// symbiosity.cpp:46-58 does.  Short rows take a lane each, longer ones a warp; rows too
+// long for a warp (hubs) are listed and taken one per CTA, a slice per warp.
 //
 // n_path: level-synchronous BFS on a visited bitset of (n + 64) / 64 words,
 // the reference's bs_size (n_path.cpp:45-53).  A level is two launches:
-//   expand  ORs into `next` every element of the frontier's rows whose visited
-//           bit is clear (set_union of the rows into the visited set,
-//           union.hpp:6-127, minus what was already visited); a bitset row is
-//           ORed word by word;
-//   collect takes next AND NOT visited as the new frontier (set_difference,
-//           difference.hpp:5-84), merges it into visited and clears next.
+//   expand  ORs the frontier's rows into `seen`, which starts as the visited set
+//           (set_union, union.hpp:6-127); a bitset row is ORed word by word;
+//   collect takes seen AND NOT visited as the new frontier (set_difference,
+//           difference.hpp:5-84) and merges it into visited.
 // Frontier rows longer than kBfsHeavy entries are split over every warp of
 // the grid; shorter ones are taken one per warp.  Levels are launched
 // kBfsChunk at a time: each kernel reads its frontier size from device memory
 // and does nothing once a frontier is empty, so the host checks the sizes
 // once per chunk instead of once per level.
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <vector>
 
@@ -32,15 +30,17 @@ namespace eh {
 namespace {
 
 constexpr uint32_t kBfsHeavy = 4096;
+constexpr uint32_t kBfsGroup = 256;
+constexpr uint32_t kBfsListed = 1024;
 constexpr uint32_t kBfsChunk = 8;
 constexpr int kBfsThreads = 256;
 
 // A row pair whose intersection is too long for one warp: streamed side (the
-// smaller row) above kSymLight entries, or two bitsets sharing more than
-// 8 * kSymLight words.  Such rows go to a list that whole CTAs work through.
+// smaller row) above kSymLight entries (two uint rows of sizes within 32x: the
+// larger above kSymMerge), or two bitsets sharing more than 8 * kSymLight words.  Such rows go
+// to a list that whole CTAs work through.
 constexpr uint32_t kSymLight = 256;
-// Probed uint rows of up to kSymStage entries are staged in shared memory.
-constexpr uint32_t kSymStage = 12288;
+constexpr uint32_t kSymMerge = 2048;
 
 __device__ __forceinline__ bool sym_heavy(const RowView& A, const RowView& B) {
   if (!A.card || !B.card) return false;
@@ -48,15 +48,48 @@ __device__ __forceinline__ bool sym_heavy(const RowView& A, const RowView& B) {
     const int64_t lo = max(A.aux, B.aux), hi = min((int64_t)A.aux + A.len, (int64_t)B.aux + B.len);
     return hi - lo > 8 * (int64_t)kSymLight;
   }
-  return min(A.card, B.card) > kSymLight;
+  const uint32_t lo = min(A.card, B.card), hi = max(A.card, B.card);
+  if (A.type == TY_UINT && B.type == TY_UINT && hi <= 32u * lo) return hi > kSymMerge;
+  return lo > kSymLight;
 }
 
 constexpr uint32_t kSymChunk = 32;  // rows a warp takes per grab (one per lane)
-constexpr uint32_t kSymTiny = 64;   // uint rows a single lane intersects by merging
+constexpr uint32_t kSymTiny = 32;   // uint rows a single lane intersects by merging
 
-__device__ __forceinline__ bool sym_above(uint32_t both, const RowView& A, const RowView& B, double threshold) {
-  // 0 / 0 is NaN, which is not above any threshold (as in the reference).
-  return (double)both / (double)((uint64_t)A.card + B.card - both) > threshold;
+// The test both / (|A| + |B| - both) > threshold, the quotient rounded to double
+// as the reference rounds it, without FP64 (a division took 30-odd instructions of
+// a pipe with two lanes per SM: two divisions a row were 170 us for 2^21 rows).  For
+// 2^-30 <= threshold < 1, threshold = m 2^-s' with 2^52 <= m < 2^53, the rounded
+// quotient is above it when the quotient is above the middle (2m + 1) 2^-(s' + 1) to
+// the next double, or on it when that rounds up (m odd, ties to even): an exact
+// 128-bit comparison of both 2^shift with m2 (|A| + |B| - both).
+struct SymTest {
+  double threshold;
+  unsigned long long m2;  // 2m + 1, 0: outside the range above
+  int shift;              // s' + 1: 54 .. 84
+  bool tie;               // m odd
+};
+SymTest sym_test(double threshold) {
+  SymTest t{threshold, 0, 0, false};
+  if (threshold >= 0x1p-30 && threshold < 1.0) {
+    int e = 0;
+    const unsigned long long m = (unsigned long long)std::ldexp(std::frexp(threshold, &e), 53);
+    t.m2 = 2 * m + 1;
+    t.shift = 53 - e + 1;
+    t.tie = m & 1;
+  }
+  return t;
+}
+__device__ __forceinline__ bool sym_above(uint32_t both, const RowView& A, const RowView& B, const SymTest& t) {
+  const unsigned long long all = (unsigned long long)A.card + B.card - both;
+  if (!t.m2) return (double)both / (double)all > t.threshold;  // 0 / 0 is NaN, above nothing (as in the reference)
+  if (!both) return false;
+  const unsigned long long rl = t.m2 * all, rh = __umul64hi(t.m2, all);
+  // shift is 54 .. 84: both << shift as two words.
+  const unsigned long long ll = t.shift < 64 ? (unsigned long long)both << t.shift : 0ull;
+  const unsigned long long lh = t.shift < 64 ? (unsigned long long)both >> (64 - t.shift)
+                                             : (unsigned long long)both << (t.shift - 64);
+  return lh != rh ? lh > rh : ll != rl ? ll > rl : t.tie;
 }
 
 // |A ∩ B| of two sorted uint rows by one thread (a merge).
@@ -71,47 +104,112 @@ __device__ __forceinline__ uint32_t merge_count(const uint32_t* a, uint32_t na, 
   return c;
 }
 
-// Rows are taken kSymChunk at a time from a shared cursor, one row per lane.
-// A lane finishes its row alone when both sides are uint rows of at most
-// kSymTiny entries (most rows of a sparse graph) or one side is empty; rows
-// above that go to the whole warp, and rows too long for a warp to the list
-// of k_symbiosity_heavy.
+// Per-lane part of |A ∩ B| of two ascending uint lists, by a warp.  A block of 32
+// entries of each list is held one per lane; each a is looked up in the b block
+// by a binary search over the lanes (shuffles), then the block with the smaller
+// last entry is replaced (both when equal), so that overlapping blocks meet
+// exactly once.  Loads are coalesced and
+// the next three blocks of each list are in flight; a merge path per lane read
+// one entry at a time.
+__device__ __forceinline__ uint32_t block_merge(const uint32_t* A, uint32_t na, const uint32_t* B, uint32_t nb,
+                                                uint32_t lane) {
+  uint32_t ia = 0, ib = 0, c = 0;
+  const auto at = [&](const uint32_t* p, uint32_t n, uint32_t k) { return k < n ? __ldg(p + k) : kUintPad; };
+  uint32_t x = at(A, na, lane), x1 = at(A, na, 32 + lane), x2 = at(A, na, 64 + lane), x3 = at(A, na, 96 + lane);
+  uint32_t y = at(B, nb, lane), y1 = at(B, nb, 32 + lane), y2 = at(B, nb, 64 + lane), y3 = at(B, nb, 96 + lane);
+  while (ia < na && ib < nb) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (int h = 16; h; h >>= 1) pos += __shfl_sync(FULL, y, pos + h - 1) < x ? h : 0;
+    c += __shfl_sync(FULL, y, pos) == x && x != kUintPad;
+    const uint32_t xm = __shfl_sync(FULL, x, 31), ym = __shfl_sync(FULL, y, 31);
+    if (xm <= ym) {
+      ia += 32;
+      x = x1;
+      x1 = x2;
+      x2 = x3;
+      x3 = at(A, na, ia + 96 + lane);
+    }
+    if (ym <= xm) {
+      ib += 32;
+      y = y1;
+      y1 = y2;
+      y2 = y3;
+      y3 = at(B, nb, ib + 96 + lane);
+    }
+  }
+  return c;
+}
+
+// Rows are taken kSymChunk at a time from a shared cursor, one row per lane.  A
+// row that could not pass with min(|out|, |in|) common entries is not read (the
+// ratio grows with their number).  Two uint rows of at most kSymTiny entries are
+// merged by the lane alone, longer ones and the other layouts go to the warp,
+// rows too long for a warp to the list of k_symbiosity_heavy.  Half-reciprocal
+// R-MAT scale 21, hybrid: 223 us here (latency of the lane merges and of the
+// warp rows' first blocks, about equal) and 74 us for the listed rows, where
+// binary searches in a staged row took 335 us; both together 538 -> 305 us a call.
 __global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc* __restrict__ dr,
                                                     const uint4* __restrict__ ar, const RowDesc* __restrict__ dc,
-                                                    const uint4* __restrict__ ac, double threshold,
+                                                    const uint4* __restrict__ ac, SymTest test,
                                                     unsigned long long* out, uint32_t* heavy, uint32_t* n_heavy,
                                                     uint32_t* cursor) {
   __shared__ PshortHdr s_hdr[8];
   const uint32_t lane = threadIdx.x & 31;
   unsigned long long acc = 0;
+  const uint32_t chunks = (n + kSymChunk - 1) / kSymChunk;
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(cursor, kSymChunk);
-    base = __shfl_sync(FULL, base, 0);
-    if (base >= n) break;
-    const uint32_t r = base + lane;
+    uint32_t q = 0;
+    if (lane == 0) q = atomicAdd(cursor, 1u);
+    q = __shfl_sync(FULL, q, 0);
+    if (q >= chunks) break;
+    // Pairs of rows, 2 * chunks apart: the long rows at the front of a degree-ordered graph spread over the chunks.
+    const auto row_of = [&](uint32_t l) { return 2 * q + (l & 1) + (uint64_t)(l >> 1) * 2 * chunks; };
+    const uint64_t r = row_of(lane);
     bool warp_row = false;
+    RowView A, B;
+    A.p = B.p = nullptr;
+    A.card = B.card = 0;
+    A.type = B.type = TY_UINT;
     if (r < n) {
-      const RowView A = load_view(dr, ar, r);
-      const RowView B = load_view(dc, ac, r);
+      A = load_view(dr, ar, (uint32_t)r);
+      B = load_view(dc, ac, (uint32_t)r);
+      const uint32_t most = max(A.card, B.card);
+      const bool both_uint = A.type == TY_UINT && B.type == TY_UINT;
       if (!A.card || !B.card) {  // ratio 0, or 0/0 (NaN, never above)
-        acc += sym_above(0, A, B, threshold);
-      } else if (A.type == TY_UINT && B.type == TY_UINT && max(A.card, B.card) <= kSymTiny) {
+        acc += sym_above(0, A, B, test);
+      } else if (!sym_above(min(A.card, B.card), A, B, test)) {
+        // not even with every entry of the shorter row
+      } else if (both_uint && most <= kSymTiny) {
         const uint32_t both = merge_count(static_cast<const uint32_t*>(A.p), A.card,
                                           static_cast<const uint32_t*>(B.p), B.card);
-        acc += sym_above(both, A, B, threshold);
+        acc += sym_above(both, A, B, test);
       } else if (sym_heavy(A, B)) {
-        heavy[atomicAdd(n_heavy, 1u)] = r;
+        heavy[atomicAdd(n_heavy, 1u)] = (uint32_t)r;
       } else {
         warp_row = true;
       }
     }
-    for (uint32_t wm = __ballot_sync(FULL, warp_row); wm; wm &= wm - 1) {
-      const uint32_t r2 = base + (__ffs(wm) - 1);
-      const RowView A = load_view(dr, ar, r2);
-      const RowView B = load_view(dc, ac, r2);
-      const uint32_t both = warp_intersect_size(A, B, lane, &s_hdr[threadIdx.x >> 5]);  // header table: pshort rows
-      if (lane == 0) acc += sym_above(both, A, B, threshold);
+    const bool mergeable =
+        A.type == TY_UINT && B.type == TY_UINT && max(A.card, B.card) <= 32u * min(A.card, B.card);
+    for (uint32_t m = __ballot_sync(FULL, warp_row && mergeable); m; m &= m - 1) {
+      const uint32_t src = __ffs(m) - 1;
+      RowView A2, B2;
+      A2.card = __shfl_sync(FULL, A.card, src);
+      B2.card = __shfl_sync(FULL, B.card, src);
+      const uint32_t* a = reinterpret_cast<const uint32_t*>(
+          __shfl_sync(FULL, reinterpret_cast<unsigned long long>(A.p), src));
+      const uint32_t* b = reinterpret_cast<const uint32_t*>(
+          __shfl_sync(FULL, reinterpret_cast<unsigned long long>(B.p), src));
+      const uint32_t both = warp_sum_u32(block_merge(a, A2.card, b, B2.card, lane));
+      if (lane == 0) acc += sym_above(both, A2, B2, test);
+    }
+    for (uint32_t wm = __ballot_sync(FULL, warp_row && !mergeable); wm; wm &= wm - 1) {
+      const uint32_t r2 = (uint32_t)row_of(__ffs(wm) - 1);
+      const RowView A2 = load_view(dr, ar, r2);
+      const RowView B2 = load_view(dc, ac, r2);
+      const uint32_t both = warp_intersect_size(A2, B2, lane, &s_hdr[threadIdx.x >> 5]);  // header table: pshort rows
+      if (lane == 0) acc += sym_above(both, A2, B2, test);
     }
   }
   acc = warp_sum_u64(acc);
@@ -148,17 +246,16 @@ __device__ __forceinline__ void cta_for_each(const RowView& V, F&& f) {
 // The heavy rows of k_symbiosity, one CTA per row taken from a shared cursor.
 __global__ void __launch_bounds__(256) k_symbiosity_heavy(const RowDesc* __restrict__ dr, const uint4* __restrict__ ar,
                                                           const RowDesc* __restrict__ dc, const uint4* __restrict__ ac,
-                                                          double threshold, unsigned long long* out,
+                                                          SymTest test, unsigned long long* out,
                                                           const uint32_t* __restrict__ heavy,
                                                           const uint32_t* n_heavy, uint32_t* cursor) {
-  __shared__ uint32_t stage[kSymStage];
   __shared__ uint32_t s_sum[8];
   __shared__ uint32_t s_idx;
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const uint32_t nh = *n_heavy;
   unsigned long long acc = 0;
   for (;;) {
-    __syncthreads();  // the previous row is finished with stage / s_sum / s_idx
+    __syncthreads();  // the previous row is finished with s_sum / s_idx
     if (tid == 0) s_idx = atomicAdd(cursor, 1u);
     __syncthreads();
     const uint32_t idx = s_idx;
@@ -179,14 +276,15 @@ __global__ void __launch_bounds__(256) k_symbiosity_heavy(const RowDesc* __restr
         A = B;
         B = T;
       }
-      if (B.type == TY_UINT && B.card <= kSymStage) {
-        const uint32_t* b = static_cast<const uint32_t*>(B.p);
-        for (uint32_t k = tid; k < B.card; k += blockDim.x) stage[k] = b[k];
-        __syncthreads();
-        cta_for_each(A, [&](uint32_t y) {
-          const uint32_t pos = lower_bound_u32(stage, 0, B.card, y);
-          c += pos < B.card && stage[pos] == y;
-        });
+      if (A.type == TY_UINT && B.type == TY_UINT && B.card <= 32u * A.card) {
+        // Each warp merges a slice of the larger row with the part of the other in its range.
+        const uint32_t* p = static_cast<const uint32_t*>(A.p);
+        const uint32_t* q = static_cast<const uint32_t*>(B.p);
+        const uint32_t nwarp = blockDim.x >> 5, per = (B.card + nwarp - 1) / nwarp;
+        const uint32_t b0 = min(B.card, (tid >> 5) * per), b1 = min(B.card, b0 + per);
+        const uint32_t a0 = b0 < b1 ? lower_bound_u32(p, 0, A.card, q[b0]) : 0u;
+        const uint32_t a1 = b0 < b1 ? (b1 < B.card ? lower_bound_u32(p, a0, A.card, q[b1]) : A.card) : 0u;
+        c = block_merge(p + a0, a1 - a0, q + b0, b1 - b0, lane);
       } else {
         cta_for_each(A, [&](uint32_t y) { c += row_contains(B, y); });
       }
@@ -198,7 +296,7 @@ __global__ void __launch_bounds__(256) k_symbiosity_heavy(const RowDesc* __restr
       uint32_t both = 0;
       for (uint32_t w = 0; w < (blockDim.x >> 5); w++) both += s_sum[w];
       both -= (uint32_t)pshort_pair_drop(A0, B0, ~0ull);
-      if (sym_above(both, A0, B0, threshold)) acc++;
+      if (sym_above(both, A0, B0, test)) acc++;
     }
   }
   if (tid == 0 && acc) atomicAdd(out, acc);
@@ -213,32 +311,54 @@ struct BfsArgs {
   const uint4* arena;
   uint32_t n;
   uint64_t words;
-  unsigned long long* vis;
-  unsigned long long* next;
+  unsigned long long* vis;   // visited up to the current frontier
+  unsigned long long* seen;  // and what the current expansion has reached
   uint32_t* lists;     // two frontier lists of n entries: light rows from the front, heavy from the back
   LevelCount* counts;  // counts[j]: frontier sizes of the j-th level of the current chunk
   unsigned long long* reached;
 };
 
-__device__ __forceinline__ void visit(const unsigned long long* vis, unsigned long long* next, uint32_t x) {
-  const uint32_t wi = x >> 6;
+// A word of `seen` through L1, possibly an older value of it: bits are only ever
+// set, so a set bit is never wrong and a clear one is looked up again in L2.
+__device__ __forceinline__ unsigned long long ld_seen(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
+}
+// Sets x's bit in `seen` unless it is set.
+__device__ __forceinline__ void visit(unsigned long long* seen, uint32_t x) {
+  unsigned long long* at = seen + (x >> 6);
   const unsigned long long bit = 1ull << (x & 63);
-  if (!((vis[wi] | __ldcg(next + wi)) & bit)) atomicOr(next + wi, bit);
+  if (!(ld_seen(at) & bit) && !(__ldcg(at) & bit)) atomicOr(at, bit);
 }
 
-// Marks in `next` the unvisited elements of slice `part` (of `nparts`) of row V;
-// the warp's lanes share the slice.
-__device__ __forceinline__ void expand_slice(const unsigned long long* vis, unsigned long long* next,
-                                             const RowView& V, uint32_t part, uint32_t nparts, uint32_t lane) {
+// Sets the bits of slice `part` (of `nparts`) of row V in `seen`; a group of W
+// lanes (lane: the index in the group) shares the slice.
+template <uint32_t W>
+__device__ __forceinline__ void expand_slice(unsigned long long* seen, uint32_t n, const RowView& V, uint32_t part,
+                                             uint32_t nparts, uint32_t lane) {
   if (V.type == TY_UINT) {
-    const uint32_t* e = static_cast<const uint32_t*>(V.p);
-    for (uint32_t k = part * 32 + lane; k < V.card; k += nparts * 32) visit(vis, next, e[k]);
+    const uint4* e4 = static_cast<const uint4*>(V.p);
+    const uint32_t n4 = (V.card + 3) >> 2;
+    for (uint32_t k = part * W + lane; k < n4; k += nparts * W) {
+      const uint4 v = __ldg(e4 + k);
+      const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+      unsigned long long w[4];
+#pragma unroll
+      for (int h = 0; h < 4; h++) w[h] = x[h] < n ? ld_seen(seen + (x[h] >> 6)) : ~0ull;  // padding: kUintPad
+#pragma unroll
+      for (int h = 0; h < 4; h++) {
+        const unsigned long long bit = 1ull << (x[h] & 63);
+        unsigned long long* at = seen + (x[h] >> 6);
+        if (!(w[h] & bit) && !(__ldcg(at) & bit)) atomicOr(at, bit);
+      }
+    }
   } else if (V.type == TY_BITSET) {
     const unsigned long long* w = static_cast<const unsigned long long*>(V.p);
-    for (uint32_t k = part * 32 + lane; k < V.len; k += nparts * 32) {
-      const uint32_t wi = V.aux + k;
-      const unsigned long long x = w[k] & ~vis[wi];
-      if (x & ~__ldcg(next + wi)) atomicOr(next + wi, x);
+    for (uint32_t k = part * W + lane; k < V.len; k += nparts * W) {
+      unsigned long long* at = seen + V.aux + k;
+      const unsigned long long x = w[k];
+      if ((x & ~ld_seen(at)) && (x & ~__ldcg(at))) atomicOr(at, x);
     }
   } else {
     const uint16_t* s = static_cast<const uint16_t*>(V.p);
@@ -246,7 +366,7 @@ __device__ __forceinline__ void expand_slice(const unsigned long long* vis, unsi
     while (i < V.len) {
       const uint32_t hb = (uint32_t)s[i] << 16, cnt = (uint32_t)s[i + 1] + 1;
       if (p % nparts == part)
-        for (uint32_t k = lane; k < cnt; k += 32) visit(vis, next, hb | s[i + 2 + k]);
+        for (uint32_t k = lane; k < cnt; k += W) visit(seen, hb | s[i + 2 + k]);
       i += cnt + 2;
       p++;
     }
@@ -254,7 +374,7 @@ __device__ __forceinline__ void expand_slice(const unsigned long long* vis, unsi
 }
 
 __global__ void k_bfs_init(BfsArgs a, uint32_t start) {
-  a.vis[start >> 6] = 1ull << (start & 63);
+  a.vis[start >> 6] = a.seen[start >> 6] = 1ull << (start & 63);
   if (a.desc[start].card > kBfsHeavy) {
     a.lists[a.n - 1] = start;
     a.counts[0] = LevelCount{0, 1};
@@ -265,7 +385,11 @@ __global__ void k_bfs_init(BfsArgs a, uint32_t start) {
   *a.reached = 1;
 }
 
-// Level j of the chunk: frontier F (sizes counts[j]) -> next.
+// Level j of the chunk: frontier F (sizes counts[j]) -> seen.  Most entries lead to
+// the same few hubs, whose words every SM asked the same L2 slice for (423 of
+// 520 us at R-MAT scale 21 were one level's): the words now come through L1
+// first, and no row is longer than its group of lanes, CTA or grid can share:
+// 520 -> 260 us for all levels.
 __global__ void __launch_bounds__(kBfsThreads) k_bfs_expand(BfsArgs a, uint32_t j, const uint32_t* __restrict__ F) {
   const LevelCount c = a.counts[j];
   if (c.light + c.heavy == 0) return;
@@ -278,12 +402,40 @@ __global__ void __launch_bounds__(kBfsThreads) k_bfs_expand(BfsArgs a, uint32_t 
     const uint32_t groups = min(c.heavy, nw), gsz = nw / groups, g = gw / gsz;
     if (g < groups)
       for (uint32_t h = g; h < c.heavy; h += groups)
-        expand_slice(a.vis, a.next, load_view(a.desc, a.arena, F[a.n - 1 - h]), gw % gsz, gsz, lane);
+        expand_slice<32>(a.seen, a.n, load_view(a.desc, a.arena, F[a.n - 1 - h]), gw % gsz, gsz, lane);
   }
-  for (uint32_t f = gw; f < c.light; f += nw) expand_slice(a.vis, a.next, load_view(a.desc, a.arena, F[f]), 0, 1, lane);
+  // Light rows: 8 lanes each up to kBfsGroup entries; longer ones wait in a list
+  // that the whole CTA shares at the end.  The ids and descriptors of a group's
+  // next rows are fetched ahead.
+  __shared__ uint32_t s_row[kBfsListed], s_n;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  const uint32_t step = 4 * nw;
+  const auto id = [&](uint32_t f) { return f < c.light ? F[f] : 0u; };
+  const uint32_t f0 = 4 * gw + (lane >> 3);
+  uint32_t r1 = id(f0), r2 = id(f0 + step);
+  RowView next = load_view(a.desc, a.arena, r1);
+  for (uint32_t f = f0; f < c.light; f += step) {
+    const RowView V = next;
+    const uint32_t row = r1;
+    r1 = r2;
+    next = load_view(a.desc, a.arena, r1);
+    r2 = id(f + 2 * step);
+    uint32_t at = kBfsListed;
+    if (V.card > kBfsGroup) {
+      if ((lane & 7) == 0) at = atomicAdd(&s_n, 1u);
+      at = __shfl_sync(0xffu << (lane & 24), at, 0, 8);
+      if (at < kBfsListed && (lane & 7) == 0) s_row[at] = row;
+    }
+    if (at >= kBfsListed) expand_slice<8>(a.seen, a.n, V, 0, 1, lane & 7);
+  }
+  __syncthreads();
+  const uint32_t listed = min(s_n, kBfsListed);
+  for (uint32_t k = 0; k < listed; k++)
+    expand_slice<32>(a.seen, a.n, load_view(a.desc, a.arena, s_row[k]), threadIdx.x >> 5, kBfsThreads / 32, lane);
 }
 
-// Level j of the chunk: next AND NOT visited -> frontier F (sizes counts[j + 1]).
+// Level j of the chunk: seen AND NOT visited -> frontier F (sizes counts[j + 1]).
 __global__ void __launch_bounds__(kBfsThreads) k_bfs_collect(BfsArgs a, uint32_t j, uint32_t* __restrict__ F) {
   const LevelCount c = a.counts[j];
   if (c.light + c.heavy == 0) return;
@@ -291,45 +443,37 @@ __global__ void __launch_bounds__(kBfsThreads) k_bfs_collect(BfsArgs a, uint32_t
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x / 32);
   unsigned long long found = 0;
-  // Whole warps step together (the appends below use warp collectives).
-  for (uint64_t w0 = ((uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * 32; w0 < a.words;
-       w0 += nw * 32) {
+  // One byte of the bitsets per lane, so that a lane has at most 8 vertices to
+  // look up; whole warps step together (the appends below use warp collectives).
+  const unsigned char* seen8 = reinterpret_cast<const unsigned char*>(a.seen);
+  unsigned char* vis8 = reinterpret_cast<unsigned char*>(a.vis);
+  const uint64_t bytes = a.words * 8;
+  for (uint64_t w0 = ((uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * 32; w0 < bytes; w0 += nw * 32) {
     const uint64_t w = w0 + lane;
-    unsigned long long x = 0, heavy = 0;
-    if (w < a.words) {
-      const unsigned long long nx = a.next[w];
-      if (nx) {
-        x = nx & ~a.vis[w];
-        a.next[w] = 0;
-        a.vis[w] |= x;
-      }
+    uint32_t x = 0, heavy = 0;
+    if (w < bytes) {
+      const uint32_t now = seen8[w];
+      x = now & ~(uint32_t)vis8[w];
+      if (x) vis8[w] = (unsigned char)now;
     }
-    for (unsigned long long y = x; y; y &= y - 1) {
-      const uint32_t v = (uint32_t)(64 * w) + (uint32_t)(__ffsll((long long)y) - 1);
-      if (a.desc[v].card > kBfsHeavy) heavy |= y & (~y + 1);
-    }
-    found += __popcll(x);
-    const uint32_t nh = __popcll(heavy), nl = __popcll(x) - nh;
-    // Warp-exclusive prefix of nl and nh, one atomic per list and warp.
-    uint32_t il = nl, ih = nh;
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t tl = __shfl_up_sync(FULL, il, d), th = __shfl_up_sync(FULL, ih, d);
-      if (lane >= (uint32_t)d) {
-        il += tl;
-        ih += th;
-      }
-    }
-    const uint32_t tot_l = __shfl_sync(FULL, il, 31), tot_h = __shfl_sync(FULL, ih, 31);
+    if (!__any_sync(FULL, x)) continue;
+    uint32_t card[8];
+#pragma unroll
+    for (int h = 0; h < 8; h++) card[h] = (x >> h) & 1u ? a.desc[8 * w + h].card : 0u;
+#pragma unroll
+    for (int h = 0; h < 8; h++) heavy |= (card[h] > kBfsHeavy ? 1u : 0u) << h;
+    found += __popc(x);
+    const uint32_t nh = __popc(heavy), nl = __popc(x) - nh;
+    const uint32_t il = warp_exclusive_scan(nl, lane), ih = warp_exclusive_scan(nh, lane);
     uint32_t base_l = 0, base_h = 0;
-    if (lane == 0) {
-      if (tot_l) base_l = atomicAdd(&out->light, tot_l);
-      if (tot_h) base_h = atomicAdd(&out->heavy, tot_h);
+    if (lane == 31) {
+      if (il + nl) base_l = atomicAdd(&out->light, il + nl);
+      if (ih + nh) base_h = atomicAdd(&out->heavy, ih + nh);
     }
-    uint32_t pl = __shfl_sync(FULL, base_l, 0) + il - nl, ph = __shfl_sync(FULL, base_h, 0) + ih - nh;
-    for (unsigned long long y = x; y; y &= y - 1) {
-      const unsigned long long b = y & (~y + 1);
-      const uint32_t v = (uint32_t)(64 * w) + (uint32_t)(__ffsll((long long)y) - 1);
-      if (heavy & b) F[a.n - 1 - ph++] = v;
+    uint32_t pl = __shfl_sync(FULL, base_l, 31) + il, ph = __shfl_sync(FULL, base_h, 31) + ih;
+    for (uint32_t y = x; y; y &= y - 1) {
+      const uint32_t v = (uint32_t)(8 * w) + (__ffs(y) - 1);
+      if (heavy & y & (0u - y)) F[a.n - 1 - ph++] = v;
       else F[pl++] = v;
     }
   }
@@ -374,11 +518,12 @@ extern "C" eh_status eh_symbiosity_async(eh_matrix_t rh, eh_matrix_t ch, double 
   if (e == cudaSuccess) {
     const uint64_t g = std::min<uint64_t>((r->n + 8 * kSymChunk - 1) / (8 * kSymChunk), (uint64_t)sms * 8);
     unsigned long long* out = reinterpret_cast<unsigned long long*>(d_count);
+    const SymTest test = sym_test(threshold);
     k_symbiosity<<<(unsigned)std::max<uint64_t>(g, 1), 256, 0, st>>>((uint32_t)r->n, r->desc, r->arena, c->desc,
-                                                                     c->arena, threshold, out, scratch, counts,
+                                                                     c->arena, test, out, scratch, counts,
                                                                      counts + 2);
     k_symbiosity_heavy<<<(unsigned)(sms * std::max(per, 1)), 256, 0, st>>>(r->desc, r->arena, c->desc, c->arena,
-                                                                           threshold, out, scratch, counts,
+                                                                           test, out, scratch, counts,
                                                                            counts + 1);
     e = cudaGetLastError();
   }
@@ -426,24 +571,28 @@ extern "C" eh_status eh_bfs_path_length(eh_matrix_t mh, uint32_t start, uint64_t
   a.n = (uint32_t)n;
   a.words = words;
   a.vis = reinterpret_cast<unsigned long long*>(base);
-  a.next = a.vis + words;
-  a.lists = reinterpret_cast<uint32_t*>(a.next + words);
-  a.reached = reinterpret_cast<unsigned long long*>(a.lists + 2 * n);
+  a.seen = a.vis + words;
+  a.reached = a.seen + words;
   a.counts = reinterpret_cast<LevelCount*>(a.reached + 1);
+  a.lists = reinterpret_cast<uint32_t*>(a.counts + kBfsChunk + 1);
   auto done = [&](eh_status s) {
     cudaFreeAsync(base, st);
     return s;
   };
-  if ((e = cudaMemsetAsync(a.vis, 0, 2 * words * 8, st)) != cudaSuccess ||
-      (e = cudaMemsetAsync(a.counts, 0, (kBfsChunk + 1) * sizeof(LevelCount), st)) != cudaSuccess)
+  // vis, seen, reached, counts: everything before the lists starts at zero.
+  if ((e = cudaMemsetAsync(base, 0, reinterpret_cast<char*>(a.lists) - base, st)) != cudaSuccess)
     return done(cuda_err(e, "memset"));
   k_bfs_init<<<1, 1, 0, st>>>(a, start);
   int sms = 0, per = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bfs_expand, kBfsThreads, 0);
   const unsigned grid = (unsigned)std::max(1, sms * std::max(per, 1));
-  const unsigned cgrid = (unsigned)std::min<uint64_t>((words + kBfsThreads - 1) / kBfsThreads, grid);
-  LevelCount hc[kBfsChunk + 1];
+  const unsigned cgrid = (unsigned)std::min<uint64_t>((words * 8 + kBfsThreads - 1) / kBfsThreads, grid);
+  struct {  // as on the device
+    unsigned long long reached;
+    LevelCount counts[kBfsChunk + 1];
+  } h;
+  const LevelCount* hc = h.counts;
   uint64_t level = 0, path = 0;
   for (;;) {
     // Expansions level .. level + k - 1; expansion L produces the frontier of level L + 1.
@@ -455,7 +604,7 @@ extern "C" eh_status eh_bfs_path_length(eh_matrix_t mh, uint32_t start, uint64_t
       k_bfs_collect<<<cgrid, kBfsThreads, 0, st>>>(a, j, nxt);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return done(cuda_err(e, "BFS kernels"));
-    if ((e = cudaMemcpyAsync(hc, a.counts, (k + 1) * sizeof(LevelCount), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+    if ((e = cudaMemcpyAsync(&h, a.reached, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
       return done(cuda_err(e, "BFS level sizes"));
     bool stop = false;
@@ -475,12 +624,8 @@ extern "C" eh_status eh_bfs_path_length(eh_matrix_t mh, uint32_t start, uint64_t
         (e = cudaMemsetAsync(a.counts + 1, 0, kBfsChunk * sizeof(LevelCount), st)) != cudaSuccess)
       return done(cuda_err(e, "BFS level sizes"));
   }
-  uint64_t r = 0;
-  if ((e = cudaMemcpyAsync(&r, a.reached, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(st)) != cudaSuccess)
-    return done(cuda_err(e, "BFS result"));
   *path_length = path;
-  if (reached) *reached = r;
+  if (reached) *reached = h.reached;
   return done(EH_OK);
 }
 
