@@ -691,29 +691,29 @@ __global__ void __launch_bounds__(kBigBlock) k_encode_big(const uint64_t* __rest
   }
 }
 
-// Row order by descending card: a histogram over 65,536 card buckets, a scan,
+// Row order by descending card (cards[r * stride]): a histogram over 65,536 card buckets, a scan,
 // then a scatter.  Most rows share a few small cards, so lanes of a warp with
 // the same bucket combine their atomics (one per bucket and warp).
-__global__ void k_plan_hist(uint64_t n, const RowDesc* __restrict__ desc, uint32_t min_card,
+__global__ void k_plan_hist(uint64_t n, const uint32_t* __restrict__ cards, uint32_t stride, uint32_t min_card,
                             uint32_t* __restrict__ hist) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t r0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); r0 < n; r0 += step) {
     const uint64_t r = r0 + lane;
-    const uint32_t c = r < n ? desc[r].card : 0u;
+    const uint32_t c = r < n ? cards[r * stride] : 0u;
     const bool take = r < n && c >= min_card;
     const uint32_t bucket = take ? 65535u - min(c, 65535u) : 0xffffffffu;
     const uint32_t peers = __match_any_sync(FULL, bucket);
     if (take && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&hist[bucket], (uint32_t)__popc(peers));
   }
 }
-__global__ void k_plan_scatter(uint64_t n, const RowDesc* __restrict__ desc, uint32_t min_card,
+__global__ void k_plan_scatter(uint64_t n, const uint32_t* __restrict__ cards, uint32_t stride, uint32_t min_card,
                                uint32_t* __restrict__ cursor, uint32_t* __restrict__ order) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t r0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); r0 < n; r0 += step) {
     const uint64_t r = r0 + lane;
-    const uint32_t c = r < n ? desc[r].card : 0u;
+    const uint32_t c = r < n ? cards[r * stride] : 0u;
     const bool take = r < n && c >= min_card;
     const uint32_t bucket = take ? 65535u - min(c, 65535u) : 0xffffffffu;
     const uint32_t peers = __match_any_sync(FULL, bucket);
@@ -723,6 +723,99 @@ __global__ void k_plan_scatter(uint64_t n, const RowDesc* __restrict__ desc, uin
     base = __shfl_sync(FULL, base, leader);
     if (take) order[base + __popc(peers & ((1u << lane) - 1u))] = (uint32_t)r;
   }
+}
+
+// Rows as pivots of the symmetric lollipop count: lcard[r] = |row(r) ∩ [0, r)|, and
+// whether the matrix is symmetric without self-loops: check[0] sums a keyed hash
+// of the pair (larger id, smaller id) over the entries below the diagonal minus
+// the same over those above it (0 for a symmetric matrix; for any other, 0 with
+// probability 2^-64 over the key), check[1] counts self-loops.  Pairs of rows are
+// dealt to warps round-robin; a lane takes its row of up to kLaneRow entries, the
+// warp longer ones, and a CTA of k_orient_big those over kBigRow entries, so that
+// no hub is one warp's (one row a warp, 8 rows a CTA: 614 us at R-MAT scale 20).
+__device__ __forceinline__ unsigned long long pair_hash(unsigned long long key, uint32_t hi, uint32_t lo) {
+  unsigned long long z = (((unsigned long long)hi << 32) | lo) ^ key;  // SplitMix64's finalizer (Steele, Lea, Flood 2014)
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  return (z ^ (z >> 31)) * (key | 1ull);
+}
+struct OrientSum {
+  unsigned long long sum = 0, self = 0;
+  uint32_t low = 0;
+  __device__ __forceinline__ void visit(unsigned long long key, uint32_t r, uint32_t x) {
+    if (x < r) {
+      low++;
+      sum += pair_hash(key, r, x);
+    } else if (x > r) {
+      sum -= pair_hash(key, x, r);
+    } else {
+      self++;
+    }
+  }
+  __device__ __forceinline__ void flush(unsigned long long* check, uint32_t lane) {
+    sum = warp_sum_u64(sum);
+    self = warp_sum_u64(self);
+    if (lane == 0 && sum) atomicAdd(check, sum);
+    if (lane == 0 && self) atomicAdd(check + 1, self);
+  }
+};
+__global__ void __launch_bounds__(kBlock) k_orient(uint64_t n, const RowDesc* __restrict__ desc,
+                                                   const uint4* __restrict__ arena, unsigned long long key,
+                                                   uint32_t* __restrict__ lcard, unsigned long long* check,
+                                                   uint32_t* __restrict__ big, uint32_t* __restrict__ n_big) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t nw = (uint64_t)gridDim.x * (kBlock / 32);
+  const uint64_t w = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+  OrientSum t;
+  for (uint64_t base = 2 * w; base < n; base += nw * 32) {
+    const uint64_t r = base + (lane & 1) + (lane >> 1) * 2 * nw;
+    RowView V;
+    V.card = 0;
+    if (r < n) V = load_view(desc, arena, (uint32_t)r);
+    const bool lane_row = r < n && (V.card == 0 || (V.type == TY_UINT && V.card <= kLaneRow));
+    if (lane_row) {
+      const uint32_t* e = static_cast<const uint32_t*>(V.p);
+      t.low = 0;
+      for (uint32_t k = 0; k < V.card; k++) t.visit(key, (uint32_t)r, __ldg(e + k));
+      lcard[r] = t.low;
+    }
+    for (uint32_t m = __ballot_sync(FULL, r < n && !lane_row); m; m &= m - 1) {
+      const uint32_t q = __ffs(m) - 1;
+      const uint32_t rq = (uint32_t)(base + (q & 1) + (uint64_t)(q >> 1) * 2 * nw);
+      const RowView B = load_view(desc, arena, rq);
+      if (B.card > kBigRow) {
+        if (lane == 0) big[atomicAdd(n_big, 1u)] = rq;
+        continue;
+      }
+      t.low = 0;
+      warp_for_each(B, 0xffffffffu, lane, [&](uint32_t x) { t.visit(key, rq, x); });
+      const uint32_t low = warp_sum_u32(t.low);
+      if (lane == 0) lcard[rq] = low;
+    }
+  }
+  t.flush(check, lane);
+}
+__global__ void __launch_bounds__(kBigBlock) k_orient_big(const RowDesc* __restrict__ desc,
+                                                          const uint4* __restrict__ arena, unsigned long long key,
+                                                          uint32_t* __restrict__ lcard, unsigned long long* check,
+                                                          const uint32_t* __restrict__ big,
+                                                          const uint32_t* __restrict__ n_big) {
+  __shared__ uint32_t s_low;
+  const uint32_t lane = threadIdx.x & 31, nb = *n_big;
+  OrientSum t;
+  for (uint32_t i = blockIdx.x; i < nb; i += gridDim.x) {
+    const uint32_t r = big[i];
+    if (threadIdx.x == 0) s_low = 0;
+    __syncthreads();
+    t.low = 0;
+    cta_for_each(load_view(desc, arena, r), [&](uint32_t x) { t.visit(key, r, x); });
+    const uint32_t low = warp_sum_u32(t.low);
+    if (lane == 0 && low) atomicAdd(&s_low, low);
+    __syncthreads();
+    if (threadIdx.x == 0) lcard[r] = s_low;
+    __syncthreads();
+  }
+  t.flush(check, lane);
 }
 
 // Decodes whole rows into plain sorted u32 lists (one block per row).
@@ -855,19 +948,30 @@ cudaError_t launch_encode(uint64_t n, const uint64_t* off, const uint32_t* nbr, 
 
 // hist: 65536 + scan tmp words; counts[0] = rows in plan (host reads order count
 // from the scanned histogram).
-cudaError_t launch_plan(uint64_t n, const RowDesc* desc, uint32_t min_card, uint32_t* hist,
+cudaError_t launch_plan(uint64_t n, const uint32_t* cards, uint32_t stride, uint32_t min_card, uint32_t* hist,
                         uint32_t* order, uint32_t* cursor, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(hist, 0, 65536 * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   if (n == 0) return cudaSuccess;
-  k_plan_hist<<<grid_for(n, 256), 256, 0, st>>>(n, desc, min_card, hist);
+  k_plan_hist<<<grid_for(n, 256), 256, 0, st>>>(n, cards, stride, min_card, hist);
   e = exclusive_scan(Plain{hist}, 65536, cursor, hist + 65536, st);
   if (e != cudaSuccess) return e;
   // Keep the scanned starts (cursor is advanced by the scatter): copy them after the
   // histogram so that the host can read bin starts.
   e = cudaMemcpyAsync(hist, cursor, 65536 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) return e;
-  k_plan_scatter<<<grid_for(n, 256), 256, 0, st>>>(n, desc, min_card, cursor, order);
+  k_plan_scatter<<<grid_for(n, 256), 256, 0, st>>>(n, cards, stride, min_card, cursor, order);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_orient(uint64_t n, const RowDesc* desc, const uint4* arena, unsigned long long key, uint32_t* lcard,
+                          unsigned long long* check, uint32_t* big, uint32_t* n_big, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(check, 0, 2 * sizeof(unsigned long long), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(n_big, 0, sizeof(uint32_t), st);
+  if (e != cudaSuccess || n == 0) return e;
+  const uint64_t g = std::min<uint64_t>((n + kBlock - 1) / kBlock, 152 * 8);
+  k_orient<<<(unsigned)g, kBlock, 0, st>>>(n, desc, arena, key, lcard, check, big, n_big);
+  k_orient_big<<<2 * 152, kBigBlock, 0, st>>>(desc, arena, key, lcard, check, big, n_big);
   return cudaGetLastError();
 }
 

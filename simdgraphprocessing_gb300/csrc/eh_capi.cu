@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <random>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -335,7 +336,7 @@ eh_status ensure_plan(Matrix* m, cudaStream_t st) {
     m->device_bytes += nn * sizeof(uint32_t);
     CU(pool_alloc((void**)&hist, (65536 + scan_tmp_words(65536)) * sizeof(uint32_t), st), "plan scratch");
     CU(pool_alloc((void**)&cursor, 65536 * sizeof(uint32_t), st), "plan scratch");
-    CU(launch_plan(m->n, m->desc, 2, hist, p.order, cursor, st), "plan kernels");
+    CU(launch_plan(m->n, &m->desc->card, sizeof(RowDesc) / 4, 2, hist, p.order, cursor, st), "plan kernels");
     std::vector<uint32_t> starts(65536);
     uint32_t total = 0;
     CU(cudaMemcpyAsync(starts.data(), hist, 65536 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "plan copy");
@@ -425,6 +426,7 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
   a.max_warp = p.largest_at_most(p.light_max);
   a.max_mid = p.largest_at_most(kMidMax);
   a.max_large = p.largest_at_most(kCtaListCap);
+  a.lcard = nullptr;
   return a;
 }
 
@@ -527,9 +529,90 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   return EH_OK;
 }
 
+// Looks at the matrix once: symmetric without self-loops and with at most
+// kCtaListCap entries below the diagonal in any row, it gets the pivots of the
+// symmetric lollipop count (Oriented); any other keeps the count by definition.
+static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
+  Oriented& o = m->oriented;
+  if (o.state) return EH_OK;
+  if (!m->shape_set && !m->plan.ready) apply_cached_shape(m);
+  if (m->n == 0) {
+    o.state = 2;
+    return EH_OK;
+  }
+  static const unsigned long long key = [] {
+    std::random_device r;
+    return ((unsigned long long)r() << 32) ^ r();
+  }();
+  uint32_t *hist = nullptr, *cursor = nullptr;
+  unsigned long long* check = nullptr;
+  auto drop = [&]() {
+    cudaFreeAsync(hist, st);
+    cudaFreeAsync(cursor, st);
+    cudaFreeAsync(check, st);
+  };
+  auto fail = [&](cudaError_t e) {
+    drop();
+    cudaFreeAsync(o.lcard, st);
+    cudaFreeAsync(o.order, st);
+    o.lcard = o.order = nullptr;
+    return cuda_fail(e, "lollipop plan");
+  };
+  cudaError_t e;
+  unsigned long long sums[2] = {0, 0};
+  uint32_t total = 0;
+  std::vector<uint32_t> starts(65536);
+  if ((e = pool_alloc((void**)&o.lcard, m->n * sizeof(uint32_t), st)) != cudaSuccess ||
+      (e = pool_alloc((void**)&o.order, m->n * sizeof(uint32_t), st)) != cudaSuccess ||
+      (e = pool_alloc((void**)&hist, (65536 + scan_tmp_words(65536)) * sizeof(uint32_t), st)) != cudaSuccess ||
+      (e = pool_alloc((void**)&cursor, 65536 * sizeof(uint32_t), st)) != cudaSuccess ||
+      (e = pool_alloc((void**)&check, sizeof(sums), st)) != cudaSuccess ||
+      // (the order's buffer lists the long rows until the order is made)
+      (e = launch_orient(m->n, m->desc, m->arena, key, o.lcard, check, o.order, cursor, st)) != cudaSuccess ||
+      (e = launch_plan(m->n, o.lcard, 1, 2, hist, o.order, cursor, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(starts.data(), hist, 65536 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(&total, cursor + 65535, sizeof(uint32_t), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(sums, check, sizeof(sums), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(st)) != cudaSuccess)
+    return fail(e);
+  drop();
+  o.starts = std::move(starts);
+  o.n_order = total;
+  if (sums[0] || sums[1] || o.above(kCtaListCap)) {
+    cudaFreeAsync(o.lcard, st);
+    cudaFreeAsync(o.order, st);
+    o.lcard = o.order = nullptr;
+    o.starts.clear();
+    o.state = 2;
+    return EH_OK;
+  }
+  m->device_bytes += 2 * m->n * sizeof(uint32_t);
+  o.state = 1;
+  return EH_OK;
+}
+
 eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st) {
-  eh_status s = ensure_plan(m, st);
+  eh_status s = ensure_oriented(m, st);
   if (s != EH_OK) return s;
+  if (m->oriented.state == 1) {
+    if ((s = ensure_core(m, st)) != EH_OK) return s;
+    const Oriented& o = m->oriented;
+    PivotArgs a = pivot_args(m, out);
+    a.lcard = o.lcard;
+    a.order = o.order;
+    a.n_order = o.n_order;
+    a.n_giant = 0;
+    a.n_heavy = o.above(m->light_max);
+    a.n_large = o.above(std::max(m->light_max, kMidMax));
+    a.n_above_tiny = o.above(8);
+    a.max_warp = o.largest_at_most(m->light_max);
+    a.max_mid = o.largest_at_most(kMidMax);
+    a.max_large = o.largest_at_most(kCtaListCap);
+    CU(launch_lollipops(a, nullptr, 0, m->grid, st), "lollipop kernel");
+    note_use(m, st);
+    return EH_OK;
+  }
+  if ((s = ensure_plan(m, st)) != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
   CU(launch_lollipops(a, m->plan.units, m->plan.n_units, m->grid, st), "lollipop kernel");
   note_use(m, st);
@@ -825,7 +908,8 @@ void eh_matrix_free(eh_matrix_t mh) {
     st = nullptr;
   }
   void* bufs[] = {m->desc, m->arena, m->counters, m->plan.order, m->plan.units, m->plan.giant_lists,
-                  m->plan.giant_off, m->plan.core, m->clique_scratch, m->vbits};
+                  m->plan.giant_off, m->plan.core, m->clique_scratch, m->vbits,
+                  m->oriented.lcard, m->oriented.order};
   for (void* b : bufs)
     if (b) cudaFreeAsync(b, st);
   for (auto& u : m->uses) cudaEventDestroy(u.second);

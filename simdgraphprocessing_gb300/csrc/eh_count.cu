@@ -224,6 +224,13 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
   cta_add(acc, a);
 }
 
+// What the kernels below count: triangles; lollipops by the definition (full
+// rows, each hit weighted by its pivot's card); or lollipops of a symmetric
+// matrix without self-loops, where every triangle {i > j > k} counts |A_i| +
+// |A_j| + |A_k|: pivots then hold only their entries below i (PivotArgs::lcard),
+// so hubs are no pivots of 10^5 entries (R-MAT scale 20: 4.8 ms by definition).
+enum Mode { kTri = 0, kFull = 1, kSym = 2 };
+
 // ---- pivots of up to kCtaListCap entries: one warp or one CTA each ----
 // Per pivot, staged in the group's shared-memory slice:
 //  * jc[e] = (word offset of core row j, j) for j = A_i[e];
@@ -261,22 +268,27 @@ struct Slice {
   uint16_t* cfirst;
   uint32_t* rcnt;  // CTA groups: per 32 entries, word starts | elements below core_k << 16
   uint32_t* bm;
+  // kSym: |A_i| + |A_j| of entry e, and its word's position mod 32.
+  uint32_t* wt;
+  uint8_t* wp;
 };
 // Bytes of a slice for pivots of up to cap entries (a multiple of 32) and a
 // window of win bits (a multiple of 4,096).
-template <int NW>
+template <int NW, int MODE>
 __host__ __device__ constexpr uint32_t slice_bytes(uint32_t cap, uint32_t win) {
-  return (cap * 18 + (cap / 32 + 1) * 2 + (NW > 1 ? cap / 32 * 4 : 0) + (win + kHashBits) / 8 + 31) & ~15u;
+  return (cap * (MODE == kSym ? 23 : 18) + (cap / 32 + 1) * 2 + (NW > 1 ? cap / 32 * 4 : 0) + (win + kHashBits) / 8 + 31) & ~15u;
 }
-template <int NW>
+template <int NW, int MODE>
 __device__ __forceinline__ Slice make_slice(char* p, uint32_t cap, uint32_t win) {
   Slice s;
   s.bm = reinterpret_cast<uint32_t*>(p);
   s.jc = reinterpret_cast<uint2*>(p + (win + kHashBits) / 8);
   s.word = reinterpret_cast<unsigned long long*>(s.jc + cap);
   s.rcnt = reinterpret_cast<uint32_t*>(s.word + cap);
-  s.widx = reinterpret_cast<uint16_t*>(s.rcnt + (NW > 1 ? cap / 32 : 0));
+  s.wt = s.rcnt + (NW > 1 ? cap / 32 : 0);
+  s.widx = reinterpret_cast<uint16_t*>(s.wt + (MODE == kSym ? cap : 0));
   s.cfirst = s.widx + cap;
+  s.wp = reinterpret_cast<uint8_t*>(s.cfirst + cap / 32 + 1);
   return s;
 }
 template <int NW>
@@ -307,16 +319,46 @@ struct WordSum {
   }
 };
 
+// Bit-sliced counters of hits per bit of a lane's word over a chunk's e's: at most
+// 256 per warp (a CTA tier's e's are shared by its warps, a warp's pivot has 160).
+constexpr int kPlanes = 9;
+__device__ __forceinline__ void add_planes(uint32_t (&plane)[2][kPlanes], const unsigned long long (&v)[8],
+                                           const uint32_t (&w)[2]) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    uint32_t x[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) x[u] = (uint32_t)(v[u] >> (32 * h)) & w[h];
+    uint32_t* p = plane[h];
+    const uint32_t a = csa(p[0], x[0], x[1]), b = csa(p[0], x[2], x[3]), f = csa(p[1], a, b);
+    const uint32_t c = csa(p[0], x[4], x[5]), d = csa(p[0], x[6], x[7]), g = csa(p[1], c, d);
+    uint32_t carry = csa(p[2], f, g);
+#pragma unroll
+    for (int q = 3; q < kPlanes; q++) {
+      const uint32_t t = p[q] & carry;
+      p[q] ^= carry;
+      carry = t;
+    }
+  }
+}
+
 // This lane's part of the count of pivot i's pairs e in [e0, e1), by a group
 // of NW warps (gw: this warp's index in it): the returned count plus what went
-// into `sum`.  LOLLI: full rows, which hold elements >= j too.  The group's
-// slice is free for the next pivot on return, bm zero.
-template <int NW, bool LOLLI>
+// into `sum`; kSym: everything goes into `wsum`, weighted.  But for kTri the rows
+// are full ones, which hold elements >= j too.  The group's slice is free for the
+// next pivot on return, bm zero.
+template <int NW, int MODE>
 __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowView& A, uint32_t e0, uint32_t e1,
                                                 const Slice& s, uint32_t win, uint32_t* scan, uint32_t lane,
-                                                uint32_t gw, WordSum& sum) {
+                                                uint32_t gw, WordSum& sum, uint32_t card_i,
+                                                unsigned long long& wsum) {
+  constexpr bool LOLLI = MODE != kTri, SYM = MODE == kSym;
   const uint32_t c = A.card, core_k = a.core_k, lt = (1u << lane) - 1u, tid = gw * 32 + lane;
-  const auto put = [&](uint32_t k, uint32_t x) { s.jc[k] = make_uint2(x < core_k ? core_offset32(x) : 0u, x); };
+  const auto put = [&](uint32_t k, uint32_t x) {
+    if (SYM && k >= c) return;  // entries past the pivot itself
+    s.jc[k] = make_uint2(x < core_k ? core_offset32(x) : 0u, x);
+    if (SYM) s.wt[k] = card_i + a.desc[x].card;
+  };
   if (NW == 1) warp_decode_to(A, lane, put);
   else cta_decode_to<NW * 32>(A, scan, put);
   uint32_t* word32 = reinterpret_cast<uint32_t*>(s.word);
@@ -364,6 +406,7 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
       __syncwarp();
     }
     if (in) atomicOr(&word32[2 * pos + ((x >> 5) & 1)], 1u << (x & 31));
+    if (SYM && in) s.wp[k] = (uint8_t)(pos & 31);
     if (stream_any && k < c) {
       const uint32_t d = x - base;
       atomicOr(&s.bm[(d < win ? d : win + (x & (kHashBits - 1))) >> 5], 1u << (x & 31));
@@ -385,13 +428,28 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
     const unsigned long long* col = a.core + idx;
     uint32_t e = max(e0, (uint32_t)s.cfirst[ch]) + 8 * gw;
     unsigned long long v[8];
+    uint32_t plane[2][kPlanes];  // kSym: hits per bit of this lane's word, bit-sliced
+    if (SYM) {
+#pragma unroll
+      for (int q = 0; q < kPlanes; q++) plane[0][q] = plane[1][q] = 0;
+    }
+    const auto add = [&](uint32_t eb) {
+      if (!SYM) {
+        sum.add8(v, w);
+        return;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        wsum += (unsigned long long)(__popc((uint32_t)v[u] & w[0]) + __popc((uint32_t)(v[u] >> 32) & w[1])) * s.wt[eb + u];
+      add_planes(plane, v, w);
+    };
     for (; e + 7 < ee; e += 8 * NW) {
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         const uint2 q = s.jc[e + u];
         v[u] = first < q.y ? __ldg(col + q.x) : 0ull;
       }
-      sum.add8(v, w);
+      add(e);
     }
     if (e < ee) {  // the last block of fewer than eight belongs to one warp
 #pragma unroll
@@ -399,13 +457,31 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
         const uint2 q = s.jc[e + u];
         v[u] = (e + u < ee && first < q.y) ? __ldg(col + q.x) : 0ull;
       }
-      sum.add8(v, w);
+      add(e);
+    }
+    if (SYM) {
+      // Each element under the chunk's words takes its hits from the lane that holds its word.
+      const uint32_t k1 = 32 * (ch + 1) < nw ? s.cfirst[ch + 1] : ea;
+      for (uint32_t k0 = s.cfirst[ch]; k0 < k1; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        const bool has = k < k1;
+        const uint32_t owner = has ? s.wp[k] : 0u, x = has ? s.jc[k].y : 0u;
+        uint32_t hits = 0;
+#pragma unroll
+        for (int q = 0; q < kPlanes; q++) {
+          const uint32_t p0 = __shfl_sync(FULL, plane[0][q], owner), p1 = __shfl_sync(FULL, plane[1][q], owner);
+          hits |= (((x & 32 ? p1 : p0) >> (x & 31)) & 1u) << q;
+        }
+        if (has) wsum += (unsigned long long)hits * (s.wt[k] - card_i);
+      }
     }
   }
 
   // ---- j >= core_k ----
   if (stream_any && ea < e1) {
     // Whether L holds y, which lies past the window.
+    // (Hits of kSym are weighed as they are found: wt of the row's entry plus |A_y|.)
+    const auto weigh = [&](uint32_t e, uint32_t y) { wsum += (unsigned long long)s.wt[e] + a.desc[y].card; };
     const auto search = [&](uint32_t y) -> uint32_t {
       uint32_t lo = 0, hi = c;
       while (lo < hi) {
@@ -444,15 +520,28 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
               const uint32_t wi = w0 + h;
               unsigned long long y = x[h];
               if (LOLLI && wi >= jw) y = wi > jw ? 0ull : y & ((1ull << (j & 63)) - 1ull);
-              if (wi - bw < ww) cnt += __popcll(y & bm64[wi - bw]);
-              else if (wide && wi > bw)
-                for (; y; y &= y - 1ull) cnt += search(64 * wi + (uint32_t)(__ffsll((long long)y) - 1));
+              if (wi - bw < ww) {
+                y &= bm64[wi - bw];
+                if (!SYM) cnt += __popcll(y);
+                else
+                  for (; y; y &= y - 1ull) weigh(e, 64 * wi + (uint32_t)(__ffsll((long long)y) - 1));
+              } else if (wide && wi > bw) {
+                for (; y; y &= y - 1ull) {
+                  const uint32_t id = 64 * wi + (uint32_t)(__ffsll((long long)y) - 1), hit = search(id);
+                  if (!SYM) cnt += hit;
+                  else if (hit) weigh(e, id);
+                }
+              }
             }
           }
           n = 0;
         } else if (type != TY_UINT || n > kProbeRatio * e) {
           const RowView B = load_view(a.desc, a.arena, j);
-          for (uint32_t t = sl; t < e; t += 8) cnt += row_contains(B, s.jc[t].y);
+          for (uint32_t t = sl; t < e; t += 8) {
+            const bool hit = row_contains(B, s.jc[t].y);
+            if (!SYM) cnt += hit;
+            else if (hit) wsum += s.wt[e] + (unsigned long long)(s.wt[t] - card_i);
+          }
           n = 0;
         }
       }
@@ -471,6 +560,7 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
         for (int u = 0; u < 4; u++) {
           if (k0 + 32 * u >= most) break;
           const uint32_t y[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+          uint32_t near = 0;  // kSym: hits in the window
           uint32_t past = 0;  // elements past the window whose hashed bit is set
 #pragma unroll
           for (int h = 0; h < 4; h++) {
@@ -479,13 +569,23 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
             const uint32_t at = in ? dy : win + (y[h] & (kHashBits - 1));
             uint32_t bit = (s.bm[at >> 5] >> (y[h] & 31)) & 1u;
             if (LOLLI) bit = y[h] < j ? bit : 0u;
-            cnt += in ? bit : 0u;
+            if (!SYM) cnt += in ? bit : 0u;
+            else near |= (in ? bit : 0u) << h;
             past += in ? 0u : bit;
           }
+          if (SYM)
+            for (; near; near &= near - 1) {
+              const uint32_t h = __ffs(near) - 1;
+              weigh(e, h == 0 ? y[0] : h == 1 ? y[1] : h == 2 ? y[2] : y[3]);
+            }
           if (past)
 #pragma unroll
             for (int h = 0; h < 4; h++)
-              if (y[h] - base >= win && (!LOLLI || y[h] < j)) cnt += search(y[h]);
+              if (y[h] - base >= win && (!LOLLI || y[h] < j)) {
+                const uint32_t hit = search(y[h]);
+                if (!SYM) cnt += hit;
+                else if (hit) weigh(e, y[h]);
+              }
         }
       }
     }
@@ -504,9 +604,11 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
 // A warp's part of a finished pivot (or unit): into its graph's count in a
 // batch (returns 0), weighted by the pivot's card for lollipops, else this
 // lane's part of the one sum, where the carry-save counter may run on.
-template <bool LOLLI>
+template <int MODE>
 __device__ __forceinline__ unsigned long long finish_pivot(const PivotArgs& a, uint32_t i, uint32_t card, uint32_t cnt,
                                                            WordSum& sum, uint32_t lane) {
+  constexpr bool LOLLI = MODE != kTri;
+  if (MODE == kSym) return 0;
   if (!LOLLI && !a.graph_rows) {
     const unsigned long long pc = (unsigned long long)cnt + 8ull * sum.eights;
     sum.eights = 0;
@@ -525,35 +627,45 @@ __device__ __forceinline__ unsigned long long finish_pivot(const PivotArgs& a, u
   return 0;
 }
 
+// kSym: cuts a pivot's view to its entries below i (bitset rows: the words that
+// hold some; what a word or a pshort row holds past them is dropped as it is decoded).
+__device__ __forceinline__ void keep_below(const PivotArgs& a, RowView& A, uint32_t i) {
+  A.card = a.lcard[i];
+  if (A.type == TY_BITSET) A.len = min(A.len, (i >> 6) + 1 - A.aux);
+}
+
 // Pivots above the warp tier and up to kCtaListCap entries, one CTA each, in
 // two launches so that the many mid-sized ones leave their shared memory to
 // L1 and have few warps at a barrier: large pivots as units of unit_span
-// positions (units; the giants' are k_pivots_heavy's), the mid tier
-// order[n_large, n_heavy) whole (units null).
-template <int NW, bool LOLLI>
-__global__ void __launch_bounds__(NW * 32, 32 / NW) k_pivots_cta(PivotArgs a, const uint2* __restrict__ units,
-                                                               uint32_t n_units, uint32_t cap, uint32_t win) {
+// positions (units; the giants' are k_pivots_heavy's), or a range of the order
+// from pos0 on whole (units null).
+template <int NW, int MODE>
+__global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivots_cta(PivotArgs a, const uint2* __restrict__ units,
+                                                               uint32_t n_units, uint32_t pos0, uint32_t* counter,
+                                                               uint32_t cap, uint32_t win) {
   extern __shared__ __align__(16) char dyn[];
   __shared__ uint32_t s_unit, s_scan[NW];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const Slice s = make_slice<NW>(dyn, cap, win);
+  const Slice s = make_slice<NW, MODE>(dyn, cap, win);
   for (uint32_t k = threadIdx.x; k < (win + kHashBits) / 32; k += NW * 32) s.bm[k] = 0u;
   unsigned long long acc = 0;
   WordSum sum;
   sum.clear();
   for (;;) {
-    if (threadIdx.x == 0) s_unit = atomicAdd(&a.counters[units ? 2 : 4], 1u);
+    if (threadIdx.x == 0) s_unit = atomicAdd(counter, 1u);
     __syncthreads();
     const uint32_t unit = s_unit;
     __syncthreads();
     if (unit >= n_units) break;
-    const uint2 uu = units ? units[unit] : make_uint2(a.n_large + unit, 0u);
+    const uint2 uu = units ? units[unit] : make_uint2(pos0 + unit, 0u);
     if (units && uu.x < a.n_giant) continue;
     const uint32_t i = a.order[uu.x];
-    const RowView A = load_view(a.desc, a.arena, i);
+    RowView A = load_view(a.desc, a.arena, i);
+    const uint32_t card = A.card;
+    if (MODE == kSym) keep_below(a, A, i);
     const uint32_t e0 = 1 + uu.y * a.unit_span, e1 = units ? min(A.card, e0 + a.unit_span) : A.card;
-    const uint32_t cnt = pivot_count<NW, LOLLI>(a, A, e0, e1, s, win, s_scan, lane, warp, sum);
-    acc += finish_pivot<LOLLI>(a, i, A.card, cnt, sum, lane);
+    const uint32_t cnt = pivot_count<NW, MODE>(a, A, e0, e1, s, win, s_scan, lane, warp, sum, card, acc);
+    acc += finish_pivot<MODE>(a, i, card, cnt, sum, lane);
   }
   cta_add<NW>(acc + sum.total(), a);
 }
@@ -566,7 +678,7 @@ __global__ void __launch_bounds__(NW * 32, 32 / NW) k_pivots_cta(PivotArgs a, co
 // pivot's card for lollipops).
 constexpr uint32_t kTinyMax = 8;
 constexpr uint32_t kTinyChunk = 16;
-template <bool LOLLI>
+template <int MODE>
 __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32_t base, uint32_t g, uint32_t* mem,
                                                       uint32_t lane) {
   uint32_t* list = mem;                               // kTinyChunk * kTinyMax
@@ -574,9 +686,12 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
   uint32_t* poff = pstart + kTinyChunk + 1;
   uint32_t* pcard = poff + kTinyChunk;
   RowView V;
-  uint32_t cl = 0;
+  uint32_t cl = 0, card = 0;
   if (lane < g) {
-    V = load_view(a.desc, a.arena, a.order[base + lane]);
+    const uint32_t i = a.order[base + lane];
+    V = load_view(a.desc, a.arena, i);
+    card = V.card;
+    if (MODE == kSym) keep_below(a, V, i);
     cl = V.card;
   }
   const uint32_t pl = cl * (cl - 1) / 2;
@@ -585,7 +700,7 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
   if (lane < g) {
     pstart[lane] = pex;
     poff[lane] = off;
-    pcard[lane] = cl;
+    pcard[lane] = card;
   }
   if (lane == 0) pstart[g] = total;
   if (lane < g && V.type == TY_UINT)
@@ -593,7 +708,14 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
   __syncwarp();
   for (uint32_t rest = __ballot_sync(FULL, lane < g && V.type != TY_UINT); rest; rest &= rest - 1) {
     const uint32_t p = __ffs(rest) - 1;
-    warp_decode(load_view(a.desc, a.arena, a.order[base + p]), list + poff[p], lane);
+    const uint32_t i = a.order[base + p];
+    RowView W = load_view(a.desc, a.arena, i);
+    if (MODE == kSym) keep_below(a, W, i);
+    uint32_t* to = list + poff[p];
+    warp_decode_to(W, lane, [&](uint32_t k, uint32_t x) {
+      if (k < W.card) to[k] = x;
+    });
+    __syncwarp();
   }
   unsigned long long tcnt = 0;
   for (uint32_t q = lane; q < total; q += 32) {
@@ -605,7 +727,8 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
     bool hit;
     if (j < a.core_k) hit = (__ldg(a.core + core_offset32(j) + (x >> 6)) >> (x & 63)) & 1ull;
     else hit = row_contains(load_view(a.desc, a.arena, j), x);
-    if (hit) tcnt += LOLLI ? pcard[p] : 1u;
+    if (hit && MODE == kSym) tcnt += (unsigned long long)pcard[p] + a.desc[j].card + a.desc[x].card;
+    else if (hit) tcnt += MODE == kFull ? pcard[p] : 1u;
   }
   __syncwarp();  // the tables are reused by the next chunk
   return tcnt;
@@ -613,13 +736,13 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
 
 // Pivots up to light_max entries, one warp each: order[mid0, mid1) in grabs of
 // mid_chunk, then the tiny ones order[mid1, n_order) in chunks of tiny_chunk.
-template <bool LOLLI>
-__global__ void __launch_bounds__(kCtaThreads, 4) k_pivots_warp(PivotArgs a, uint32_t mid1, uint32_t mid_chunk,
+template <int MODE>
+__global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_warp(PivotArgs a, uint32_t mid1, uint32_t mid_chunk,
                                                                 uint32_t tiny, uint32_t cap, uint32_t win) {
   extern __shared__ __align__(16) char dyn[];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  char* mem = dyn + warp * slice_bytes<1>(cap, win);
-  const Slice s = make_slice<1>(mem, cap, win);
+  char* mem = dyn + warp * slice_bytes<1, MODE>(cap, win);
+  const Slice s = make_slice<1, MODE>(mem, cap, win);
   for (uint32_t k = lane; k < (win + kHashBits) / 32; k += 32) s.bm[k] = 0u;
   __syncwarp();
   unsigned long long acc = 0;
@@ -633,9 +756,11 @@ __global__ void __launch_bounds__(kCtaThreads, 4) k_pivots_warp(PivotArgs a, uin
     const uint32_t end = min(mid1, base + mid_chunk);
     for (uint32_t k = base; k < end; k++) {
       const uint32_t i = a.order[k];
-      const RowView A = load_view(a.desc, a.arena, i);
-      const uint32_t cnt = pivot_count<1, LOLLI>(a, A, 1, A.card, s, win, nullptr, lane, 0, sum);
-      acc += finish_pivot<LOLLI>(a, i, A.card, cnt, sum, lane);
+      RowView A = load_view(a.desc, a.arena, i);
+      const uint32_t card = A.card;
+      if (MODE == kSym) keep_below(a, A, i);
+      const uint32_t cnt = pivot_count<1, MODE>(a, A, 1, A.card, s, win, nullptr, lane, 0, sum, card, acc);
+      acc += finish_pivot<MODE>(a, i, card, cnt, sum, lane);
     }
   }
   __syncwarp();
@@ -645,7 +770,7 @@ __global__ void __launch_bounds__(kCtaThreads, 4) k_pivots_warp(PivotArgs a, uin
     if (lane == 0) base = tiny0 + atomicAdd(&a.counters[3], tiny);
     base = __shfl_sync(FULL, base, 0);
     if (base >= a.n_order) break;
-    acc += tiny_chunk<LOLLI>(a, base, min(tiny, a.n_order - base), reinterpret_cast<uint32_t*>(mem), lane);
+    acc += tiny_chunk<MODE>(a, base, min(tiny, a.n_order - base), reinterpret_cast<uint32_t*>(mem), lane);
   }
   cta_add(acc + sum.total(), a);
 }
@@ -888,18 +1013,34 @@ static uint32_t window_bits(uint64_t n, uint32_t most) {
 }
 
 // Dynamic shared memory above 48 KB has to be allowed once per kernel and device.
-template <bool LOLLI>
-static cudaError_t allow_warp_smem(int device) {
-  static std::atomic<bool> done[64];
+static cudaError_t allow_smem(const void* kernel, uint32_t bytes, std::atomic<bool>* done, int device) {
   if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
   if (done[device].load()) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(k_pivots_warp<LOLLI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(NWARPS * slice_bytes<1>(kLightMax, kWarpWindow)));
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) done[device].store(true);
   return e;
 }
 
-template <bool LOLLI>
+static uint32_t cap_of(uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); }
+
+// n pivots of k_pivots_cta: units, or order[pos0, pos0 + n) whole.
+template <int NW, int MODE>
+static cudaError_t launch_cta_pivots(const PivotArgs& a, const uint2* units, uint32_t n, uint32_t pos0,
+                                     uint32_t* counter, uint32_t largest, uint32_t window, int grid, int device,
+                                     cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  cudaError_t e = allow_smem((const void*)k_pivots_cta<NW, MODE>, slice_bytes<NW, MODE>(kCtaListCap, kCtaWindow), done,
+                             device);
+  if (e != cudaSuccess) return e;
+  const uint32_t cap = cap_of(largest), win = window_bits(a.n, window), bytes = slice_bytes<NW, MODE>(cap, win);
+  const int regs = (MODE == kSym ? 24 : 32) / NW;
+  const int per = std::max(1, std::min(regs, grid / sm_count(device) * (NWARPS / NW)));
+  const int g = (int)std::min<int64_t>(n, resident_grid(device, bytes, per));
+  k_pivots_cta<NW, MODE><<<std::max(g, 1), NW * 32, bytes, st>>>(a, units, n, pos0, counter, cap, win);
+  return cudaGetLastError();
+}
+
+template <int MODE>
 static cudaError_t launch_pivots(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
                                  cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(a.counters, 0, 5 * sizeof(uint32_t), st);
@@ -908,38 +1049,40 @@ static cudaError_t launch_pivots(const PivotArgs& a, const uint2* units, uint32_
   if (e != cudaSuccess) return e;
   int device = 0;
   if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
-  const auto cap_of = [](uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); };
-  if (n_units && a.n_giant) {
+  if (MODE != kSym && n_units && a.n_giant) {
     const int gh = std::min(grid, resident_grid(device, (uint32_t)sizeof(HeavySmem), 6));
-    k_pivots_heavy<LOLLI><<<std::max(gh, 1), kCtaThreads, 0, st>>>(a, units, n_units);
+    k_pivots_heavy<MODE == kFull><<<std::max(gh, 1), kCtaThreads, 0, st>>>(a, units, n_units);
   }
-  if (n_units && a.n_large > a.n_giant) {
-    const uint32_t cap = cap_of(a.max_large), win = window_bits(a.n, kCtaWindow);
-    const uint32_t bytes = slice_bytes<kLargeWarps>(cap, win);
-    const int g = std::min<int64_t>(n_units, std::min(grid, resident_grid(device, bytes, 32 / kLargeWarps)));
-    k_pivots_cta<kLargeWarps, LOLLI><<<std::max(g, 1), kLargeWarps * 32, bytes, st>>>(a, units, n_units, cap, win);
+  if (MODE == kSym) {
+    if (a.n_large && (e = launch_cta_pivots<kLargeWarps, MODE>(a, nullptr, a.n_large, 0, a.counters + 2, a.max_large,
+                                                               kCtaWindow, grid, device, st)) != cudaSuccess)
+      return e;
+  } else if (n_units && a.n_large > a.n_giant) {
+    if ((e = launch_cta_pivots<kLargeWarps, MODE>(a, units, n_units, 0, a.counters + 2, a.max_large, kCtaWindow, grid,
+                                                  device, st)) != cudaSuccess)
+      return e;
   }
-  if (a.n_heavy > a.n_large) {
-    const uint32_t cap = cap_of(a.max_mid), win = window_bits(a.n, kWarpWindow);
-    const uint32_t bytes = slice_bytes<kMidWarps>(cap, win);
-    const int per = std::max(1, std::min(32 / kMidWarps, grid / sm_count(device) * (NWARPS / kMidWarps)));
-    const int g = std::min<int64_t>(a.n_heavy - a.n_large, resident_grid(device, bytes, per));
-    k_pivots_cta<kMidWarps, LOLLI><<<std::max(g, 1), kMidWarps * 32, bytes, st>>>(a, nullptr, a.n_heavy - a.n_large, cap,
-                                                                                 win);
-  }
+  if (a.n_heavy > a.n_large &&
+      (e = launch_cta_pivots<kMidWarps, MODE>(a, nullptr, a.n_heavy - a.n_large, a.n_large, a.counters + 4, a.max_mid,
+                                              kWarpWindow, grid, device, st)) != cudaSuccess)
+    return e;
   if (a.n_order > a.n_heavy) {
-    if ((e = allow_warp_smem<LOLLI>(device)) != cudaSuccess) return e;
+    static std::atomic<bool> done[64];
+    if ((e = allow_smem((const void*)k_pivots_warp<MODE>, NWARPS * slice_bytes<1, MODE>(kLightMax, kWarpWindow), done,
+                        device)) != cudaSuccess)
+      return e;
     const uint32_t cap = cap_of(a.max_warp), win = window_bits(a.n, kWarpWindow);
-    const uint32_t bytes = NWARPS * slice_bytes<1>(cap, win);
-    const uint32_t mid1 = std::min(a.n_order, std::max(a.n_heavy, a.n_above_tiny)), mid = mid1 - a.n_heavy, tiny = a.n_order - mid1;
-    int gw = std::min(grid, resident_grid(device, bytes, 4));
+    const uint32_t bytes = NWARPS * slice_bytes<1, MODE>(cap, win);
+    const uint32_t mid1 = std::min(a.n_order, std::max(a.n_heavy, a.n_above_tiny)), mid = mid1 - a.n_heavy,
+                   tiny = a.n_order - mid1;
+    int gw = std::min(grid, resident_grid(device, bytes, MODE == kSym ? 3 : 4));
     // Grabs small enough that every warp gets several; one pivot at least.
     const uint32_t warps = (uint32_t)std::max(gw, 1) * NWARPS;
     const uint32_t mid_chunk = std::max(1u, std::min(4u, mid / (16 * warps)));
     const uint32_t tiny_grab = std::max(1u, std::min(kTinyChunk, tiny / (4 * warps)));
     const uint64_t grabs = (uint64_t)mid / mid_chunk + tiny / tiny_grab + 1;
     gw = (int)std::min<uint64_t>(std::max(gw, 1), (grabs + NWARPS - 1) / NWARPS);
-    k_pivots_warp<LOLLI><<<gw, kCtaThreads, bytes, st>>>(a, mid1, mid_chunk, tiny_grab, cap, win);
+    k_pivots_warp<MODE><<<gw, kCtaThreads, bytes, st>>>(a, mid1, mid_chunk, tiny_grab, cap, win);
   }
   return cudaGetLastError();
 }
@@ -959,11 +1102,11 @@ cudaError_t launch_pivot_unit_fill(const uint32_t* cnt, const uint32_t* start, u
 
 cudaError_t launch_triangles(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
                              cudaStream_t st) {
-  return launch_pivots<false>(a, units, n_units, grid, st);
+  return launch_pivots<kTri>(a, units, n_units, grid, st);
 }
 cudaError_t launch_lollipops(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
                              cudaStream_t st) {
-  return launch_pivots<true>(a, units, n_units, grid, st);
+  return a.lcard ? launch_pivots<kSym>(a, units, n_units, grid, st) : launch_pivots<kFull>(a, units, n_units, grid, st);
 }
 
 cudaError_t launch_core_build(const RowDesc* desc, const uint4* arena, uint32_t core_k, unsigned long long* core,

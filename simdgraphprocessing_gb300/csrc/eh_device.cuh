@@ -361,6 +361,33 @@ __device__ __forceinline__ void warp_for_each(const RowView& V, uint32_t lim, ui
   }
 }
 
+// f(x) for every element of V, spread over the CTA (pshort: warps take
+// partitions round-robin, lanes the entries of a partition).
+template <class F>
+__device__ __forceinline__ void cta_for_each(const RowView& V, F&& f) {
+  const uint32_t tid = threadIdx.x, nt = blockDim.x;
+  if (V.type == TY_UINT) {
+    const uint32_t* a = static_cast<const uint32_t*>(V.p);
+    for (uint32_t k = tid; k < V.card; k += nt) f(a[k]);
+  } else if (V.type == TY_BITSET) {
+    const unsigned long long* w = static_cast<const unsigned long long*>(V.p);
+    for (uint32_t k = tid; k < V.len; k += nt)
+      for (unsigned long long x = w[k]; x; x &= x - 1ull)
+        f(64u * (V.aux + k) + (uint32_t)(__ffsll((long long)x) - 1));
+  } else {
+    const uint16_t* s = static_cast<const uint16_t*>(V.p);
+    const uint32_t lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
+    uint32_t i = 0, p = 0;
+    while (i < V.len) {
+      const uint32_t hb = (uint32_t)s[i] << 16, cnt = (uint32_t)s[i + 1] + 1;
+      if (p % nwarps == warp)
+        for (uint32_t k = lane; k < cnt; k += 32) f(hb | s[i + 2 + k]);
+      i += cnt + 2;
+      p++;
+    }
+  }
+}
+
 // The reference's pshort ∩ pshort kernel keeps each partition's intersection
 // size in a uint16_t (intersection.hpp:857-865), so a partition pair whose
 // 65,536 values are all common adds 0 and none of those values reach its

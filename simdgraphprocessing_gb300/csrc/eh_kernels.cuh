@@ -55,10 +55,15 @@ uint64_t scan_tmp_words(uint64_t n);
 cudaError_t launch_encode(uint64_t n, const uint64_t* off, const uint32_t* nbr, const uint8_t* mask,
                           int sel, const RowMeasure* meas, const uint32_t* off16, RowDesc* desc,
                           uint4* arena, const uint32_t* big, const uint32_t* n_big, cudaStream_t st);
-// Work plan: rows with card >= min_card sorted by descending card.
+// Entries below the diagonal per row, and check[0] == check[1] == 0 for a symmetric
+// matrix without self-loops (key: random; see k_orient).  big / n_big: a list of
+// up to n row ids, scratch.
+cudaError_t launch_orient(uint64_t n, const RowDesc* desc, const uint4* arena, unsigned long long key, uint32_t* lcard,
+                          unsigned long long* check, uint32_t* big, uint32_t* n_big, cudaStream_t st);
+// Work plan: rows with cards[r * stride] >= min_card sorted by descending card.
 // hist: 65536 + scan_tmp_words(65536) words; after the call hist[0..65536) holds
 // the bin starts and cursor[0..65536) the bin ends (bin b = card 65535 - b).
-cudaError_t launch_plan(uint64_t n, const RowDesc* desc, uint32_t min_card, uint32_t* hist,
+cudaError_t launch_plan(uint64_t n, const uint32_t* cards, uint32_t stride, uint32_t min_card, uint32_t* hist,
                         uint32_t* order, uint32_t* cursor, cudaStream_t st);
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint64_t n, uint32_t* out, uint32_t* tmp,
                                cudaStream_t st);
@@ -94,6 +99,7 @@ struct PivotArgs {
   uint32_t n_above_tiny;   // rows in the plan with more than 8 entries
   uint32_t n_large;        // order[0, n_large) have units (the rest up to n_heavy run whole)
   uint32_t max_warp, max_mid, max_large;  // largest pivot of each tier
+  const uint32_t* lcard;   // lollipops of a symmetric matrix: entries of each row below it; else null
 };
 constexpr uint32_t kCtaThreads = 256;
 constexpr uint32_t kLightMax = 160;    // largest light_max: warp-wide pivots fit a slice of this size

@@ -13,13 +13,34 @@
 
 namespace eh {
 
-struct Plan {
+// Positions of an order of rows by descending size, from the bin starts of launch_plan.
+struct SizeOrder {
+  std::vector<uint32_t> starts;  // rows of size > x are order[0, starts[65535 - x])
+  // rows in the order of size > x (x < 65535)
+  uint32_t above(uint32_t x) const { return starts.empty() ? 0 : starts[65535 - x]; }
+  // largest size <= x present (0 if none)
+  uint32_t largest_at_most(uint32_t x) const {
+    if (starts.empty()) return 0;
+    for (uint32_t b = 65535 - x; b < 65535; b++)
+      if (starts[b + 1] > starts[b]) return 65535 - b;
+    return 0;
+  }
+};
+
+// Pivots of the symmetric lollipop count: rows by their entries below the diagonal.
+struct Oriented : SizeOrder {
+  int state = 0;              // 0: not looked at; 1: in use; 2: not symmetric, self-loops or a row too long
+  uint32_t* lcard = nullptr;  // entries of each row below it
+  uint32_t* order = nullptr;
+  uint32_t n_order = 0;
+};
+
+struct Plan : SizeOrder {
   bool ready = false;
   uint32_t* order = nullptr;  // rows with card >= 2, descending card
   uint32_t n_order = 0, n_giant = 0;
   uint32_t* giant_lists = nullptr;
   unsigned long long* giant_off = nullptr;
-  std::vector<uint32_t> starts;  // bin starts: rows with card > x are order[0, starts[65535 - x])
   // Units of the large pivots (above light_max and kMidMax) for the current (light_max, unit_span).
   uint32_t light_max = 0, unit_span = 0;
   uint32_t n_heavy = 0, n_large = 0;  // order[0, n_heavy) have card > light_max, [0, n_large) units
@@ -29,15 +50,6 @@ struct Plan {
   uint64_t units_cap = 0;
   unsigned long long* core = nullptr;  // dense core bitmap (rows j < core_k)
   uint32_t core_k = 0;
-  // rows in the plan with card > x (x < 65535)
-  uint32_t above(uint32_t x) const { return starts.empty() ? 0 : starts[65535 - x]; }
-  // largest card <= x present in the plan (0 if none)
-  uint32_t largest_at_most(uint32_t x) const {
-    if (starts.empty()) return 0;
-    for (uint32_t b = 65535 - x; b < 65535; b++)
-      if (starts[b + 1] > starts[b]) return 65535 - b;
-    return 0;
-  }
 };
 
 // Per-launch scratch: work-queue counters and the clique kernel's global slots.
@@ -58,6 +70,7 @@ struct Matrix {
   uint64_t arena_units = 0;
   BuildTotals tot{};
   Plan plan;
+  Oriented oriented;
   uint32_t* counters = nullptr;  // 16 work-queue counters, then `result`
   unsigned long long* result = nullptr;
   int grid = 0;

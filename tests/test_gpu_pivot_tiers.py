@@ -84,3 +84,35 @@ def test_batch_triangles_from_the_clique_masks(eh, oracle, layout):
     tri = [m.triangles() for m in lows]
     assert out[0].tolist() == tri and out[2].tolist() == tri
     assert out[1].tolist() == [m.cliques(4) for m in lows]
+
+
+@pytest.mark.parametrize("layout", ["hybrid", "uint", "pshort"])
+@pytest.mark.parametrize("kind", ["symmetric", "one entry missing", "one moved", "self-loop", "long rows below"])
+def test_lollipops_by_triangles_only_where_symmetric(eh, oracle, graph, layout, kind):
+    """Lollipops of a symmetric matrix without self-loops come from its
+    triangles, weighted; anything else keeps the definition.  Both equal the
+    oracle, twice in a row and at other shapes."""
+    off, nbr = graph
+    row = np.repeat(np.arange(N, dtype=np.int64), np.diff(off).astype(np.int64))
+    key = row * N + nbr
+    if kind == "one entry missing":
+        key = np.delete(key, len(key) // 2)
+    elif kind == "one moved":                            # as many entries below the diagonal as above
+        free = np.setdiff1d(np.arange(1, 400) * N, key)
+        key = np.append(np.delete(key, np.flatnonzero(nbr < row)[1234]), free[0])
+    elif kind == "self-loop":
+        key = np.append(key, 40 * N + 40)
+    elif kind == "long rows below":                      # symmetric, but no pivot may hold 2,600 smaller neighbours
+        far, some = np.int64(N - 200), np.arange(2600)
+        key = np.concatenate([key, far * N + some, some * N + far])
+    key = np.unique(key)
+    off = np.zeros(N + 1, np.uint64)
+    off[1:] = np.cumsum(np.bincount(key // N, minlength=N))
+    nbr = (key % N).astype(np.uint32)
+    m = eh.Matrix.build(off, nbr, "all", layout)
+    want = oracle.Matrix(off, nbr, oracle.SELECT_ALL, oracle.UINTEGER).lollipops()
+    assert m.count_lollipops() == want and m.count_lollipops() == want
+    m.set_shape(8, 64, 8, 0)
+    assert m.count_lollipops() == want
+    m.set_shape(160, 64, 2, 4096)
+    assert m.count_lollipops() == want
