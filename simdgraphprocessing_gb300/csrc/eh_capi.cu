@@ -207,13 +207,12 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   m->arena_units = m->tot.payload_units;
   if ((e = pool_alloc((void**)&m->desc, nn * sizeof(RowDesc), st)) != cudaSuccess ||
       (e = pool_alloc((void**)&m->arena, (m->arena_units + 1) * 16, st)) != cudaSuccess ||
-      (e = pool_alloc((void**)&m->counters, 128, st)) != cudaSuccess)
+      (e = pool_alloc((void**)&m->counters, kMatrixCounters * sizeof(uint32_t), st)) != cudaSuccess)
     return fail(set_error(EH_ERR_OUT_OF_MEMORY, "matrix allocation (%llu bytes) failed: %s",
                           (unsigned long long)((m->arena_units + 1) * 16 + nn * 16), cudaGetErrorString(e)));
-  // Words 0..15: work-queue counters; 16..17: the u64 result of the synchronous calls.
   m->result = reinterpret_cast<unsigned long long*>(m->counters + 16);
   m->device_bytes = nn * sizeof(RowDesc) + (m->arena_units + 1) * 16 + 128;
-  cudaMemsetAsync(m->counters, 0, 128, st);
+  cudaMemsetAsync(m->counters, 0, kMatrixCounters * sizeof(uint32_t), st);
   cudaMemsetAsync(m->arena, 0, (m->arena_units + 1) * 16, st);
   if ((e = launch_encode(n, d_off, d_nbr, d_mask, sel, meas, off16, m->desc, m->arena, big, big + big_cap, st)) !=
       cudaSuccess)
@@ -345,7 +344,7 @@ eh_status ensure_plan(Matrix* m, cudaStream_t st) {
     cudaFreeAsync(hist, st);
     cudaFreeAsync(cursor, st);
     p.n_order = m->n ? total : 0;
-    if (m->n) p.starts = starts;
+    if (m->n) p.set(std::move(starts));
     p.n_giant = p.above(kCtaListCap);
     // Giant pivots that are not uint rows get a decoded list.
     std::vector<uint32_t> grows(p.n_giant);
@@ -412,7 +411,10 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
   a.n_giant = m->plan.n_giant;
   a.giant_lists = m->plan.giant_lists;
   a.giant_off = m->plan.giant_off;
-  a.counters = m->counters;
+  a.queue = m->counters + kQueueWord;
+  a.flags = m->counters + kFlagWord;
+  a.ctas = 0;
+  a.report = false;
   a.out = out;
   a.unit_span = m->plan.unit_span;
   a.graph_rows = nullptr;
@@ -430,19 +432,78 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
   return a;
 }
 
-// Copies the result back and checks the kernels' device error flags
-// (counters[15]; e.g. a bulk copy whose bounded wait ran out), which are
-// cleared when reported.
-static eh_status finish_sync(Matrix* m, unsigned long long* d_res, uint64_t* count, cudaStream_t st) {
-  uint32_t flags = 0;
-  CU(cudaMemcpyAsync(count, d_res, sizeof(uint64_t), cudaMemcpyDeviceToHost, st), "result copy");
-  CU(cudaMemcpyAsync(&flags, m->counters + 15, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "flag copy");
-  CU(cudaStreamSynchronize(st), "count");
-  if (flags) {
-    CU(cudaMemsetAsync(m->counters + 15, 0, sizeof(uint32_t), st), "flag reset");
-    return set_error(EH_ERR_DEVICE_CHECK, "a device-side wait ran out (flags 0x%x); the count is not valid", flags);
+namespace {
+// Pinned words that blocking calls get their result and flags in: [0] the count,
+// [1] device error flags.  One block per process, handed out a slot at a time.
+struct HostSlots {
+  static constexpr int kSlots = 64;
+  std::mutex mu;
+  uint64_t* block = nullptr;
+  bool tried = false;
+  std::vector<uint64_t*> free;
+  uint64_t* take() {
+    std::lock_guard<std::mutex> g(mu);
+    if (!tried) {
+      tried = true;
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, kSlots * 64, cudaHostAllocPortable) == cudaSuccess) {
+        block = static_cast<uint64_t*>(p);
+        for (int k = 0; k < kSlots; k++) free.push_back(block + 8 * k);
+      } else {
+        cudaGetLastError();
+      }
+    }
+    if (free.empty()) return nullptr;
+    uint64_t* s = free.back();
+    free.pop_back();
+    return s;
   }
-  return EH_OK;
+  void give(uint64_t* s) {
+    std::lock_guard<std::mutex> g(mu);
+    free.push_back(s);
+  }
+};
+HostSlots g_slots;
+}  // namespace
+
+static eh_status check_flags(uint32_t flags) {
+  if (!flags) return EH_OK;
+  return set_error(EH_ERR_DEVICE_CHECK, "a device-side wait ran out (flags 0x%x); the count is not valid", flags);
+}
+
+// Copies m->result and the device error flags back (one copy: words 15 to 17);
+// the flags are cleared when reported.
+static eh_status finish_sync(Matrix* m, uint64_t* count, cudaStream_t st) {
+  uint32_t words[3] = {0, 0, 0};
+  CU(cudaMemcpyAsync(words, m->counters + kFlagWord, sizeof(words), cudaMemcpyDeviceToHost, st), "result copy");
+  CU(cudaStreamSynchronize(st), "count");
+  memcpy(count, words + 1, sizeof(uint64_t));
+  if (words[0]) CU(cudaMemsetAsync(m->counters + kFlagWord, 0, sizeof(uint32_t), st), "flag reset");
+  return check_flags(words[0]);
+}
+
+// Runs a count into `out` (launch(out, report)), waits and returns it: the
+// kernels write the count and their error flags (e.g. a bulk copy whose bounded
+// wait ran out) to a pinned slot.  Without a free slot they go through m->result.
+template <class Launch>
+static eh_status count_sync(Matrix* m, uint64_t* count, cudaStream_t st, Launch&& launch) {
+  uint64_t* slot = g_slots.take();
+  if (!slot) {
+    eh_status s = launch(m->result, false);
+    return s != EH_OK ? s : finish_sync(m, count, st);
+  }
+  eh_status s = launch(reinterpret_cast<unsigned long long*>(slot), true);
+  if (s != EH_OK && s != EH_ERR_CUDA) {  // refused: nothing was launched
+    g_slots.give(slot);
+    return s;
+  }
+  const cudaError_t e = cudaStreamSynchronize(st);  // the slot is the kernels' until then
+  const uint64_t got = slot[0], flags = slot[1];
+  g_slots.give(slot);
+  if (s != EH_OK) return s;
+  if (e != cudaSuccess) return cuda_fail(e, "count");
+  *count = got;
+  return check_flags((uint32_t)flags);
 }
 
 eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const uint32_t* graph_rows,
@@ -514,17 +575,19 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   const uint32_t bands_mid[] = {cap, kCliqueMidMax, 512, 256, kCliqueWarpMax};
   const uint32_t bands_dfs[] = {cap, 1024, 768, 512, kCliqueWarpMax};
   const uint32_t* bands = mid ? bands_mid : bands_dfs;
+  bool overlap = nG > 0;  // a kernel of this call came before
   for (int b = 0; b + 1 < 5; b++) {
     if (bands[b] <= bands[b + 1]) continue;
     const uint32_t p0 = p.above(bands[b]), p1 = p.above(bands[b + 1]);
     if (p1 <= p0) continue;
     const uint32_t cmax = p.largest_at_most(bands[b]);
     if (mid && bands[b] <= kCliqueMidMax)
-      CU(launch_clique_mid(a, p0, p1, w.counters + 3 + b, cmax, sms, st), "clique kernel (mid)");
+      CU(launch_clique_mid(a, p0, p1, w.counters + 3 + b, cmax, sms, st, overlap), "clique kernel (mid)");
     else
       CU(launch_clique_cta(a, p0, p1, w.counters + 3 + b, cmax, nullptr, 0, st, list), "clique kernel (shared)");
+    overlap = true;
   }
-  if (nL > nB) CU(launch_clique_warp(a, nB, nL, w.counters + 11, sms, st, list), "clique kernel (warp)");
+  if (nL > nB) CU(launch_clique_warp(a, nB, nL, w.counters + 11, sms, st, list, overlap), "clique kernel (warp)");
   note_use(m, st);
   return EH_OK;
 }
@@ -576,7 +639,7 @@ static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
       (e = cudaStreamSynchronize(st)) != cudaSuccess)
     return fail(e);
   drop();
-  o.starts = std::move(starts);
+  o.set(std::move(starts));
   o.n_order = total;
   if (sums[0] || sums[1] || o.above(kCtaListCap)) {
     cudaFreeAsync(o.lcard, st);
@@ -591,13 +654,14 @@ static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
   return EH_OK;
 }
 
-eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st) {
+eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st, bool report) {
   eh_status s = ensure_oriented(m, st);
   if (s != EH_OK) return s;
   if (m->oriented.state == 1) {
     if ((s = ensure_core(m, st)) != EH_OK) return s;
     const Oriented& o = m->oriented;
     PivotArgs a = pivot_args(m, out);
+    a.report = report;
     a.lcard = o.lcard;
     a.order = o.order;
     a.n_order = o.n_order;
@@ -614,19 +678,23 @@ eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t
   }
   if ((s = ensure_plan(m, st)) != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
+  a.report = report;
   CU(launch_lollipops(a, m->plan.units, m->plan.n_units, m->grid, st), "lollipop kernel");
   note_use(m, st);
   return EH_OK;
 }
 
 eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32_t* graph_rows, uint32_t num_graphs,
-                                cudaStream_t st, Workspace* ws, bool large_only) {
+                                cudaStream_t st, Workspace* ws, bool large_only, bool report) {
   if (m->selection != EH_SELECT_LOWER)
     return set_error(EH_ERR_UNSUPPORTED, "triangle counting needs a matrix built with EH_SELECT_LOWER");
   eh_status s = ensure_plan(m, st);
   if (s != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
-  if (ws) a.counters = ws->counters;
+  a.report = report;
+  uint32_t* counters = ws ? ws->counters : m->counters;
+  a.queue = counters + kQueueWord;
+  a.flags = counters + kFlagWord;
   a.graph_rows = graph_rows;
   a.num_graphs = num_graphs;
   if (graph_rows) {
@@ -640,8 +708,8 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
     CliqueArgs c{m->desc, m->arena, a.order, 3, out, graph_rows, num_graphs, a.core, a.core_k, nullptr, 0, nullptr};
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    CU(cudaMemsetAsync(a.counters + 11, 0, sizeof(uint32_t), st), "memset");
-    CU(launch_clique_warp(c, a.n_order, m->plan.above(1), a.counters + 11, sms, st), "triangle kernel (warp)");
+    CU(cudaMemsetAsync(counters + 11, 0, sizeof(uint32_t), st), "memset");
+    CU(launch_clique_warp(c, a.n_order, m->plan.above(1), counters + 11, sms, st), "triangle kernel (warp)");
   }
   note_use(m, st);
   return EH_OK;
@@ -925,9 +993,9 @@ eh_status eh_count_triangles_async(eh_matrix_t mh, uint64_t* d_count, void* stre
 eh_status eh_count_triangles(eh_matrix_t mh, uint64_t* count, void* stream) {
   CHECK_MATRIX(mh);
   EH_CHECK_ARG(count, "count is NULL");
-  eh_status s = eh_count_triangles_async(mh, reinterpret_cast<uint64_t*>(MX(mh)->result), stream);
-  if (s != EH_OK) return s;
-  return eh::finish_sync(MX(mh), MX(mh)->result, count, ST(stream));
+  return eh::count_sync(MX(mh), count, ST(stream), [&](unsigned long long* out, bool report) {
+    return eh::launch_triangle_count(MX(mh), out, nullptr, 0, ST(stream), nullptr, false, report);
+  });
 }
 
 eh_status eh_count_lollipops_async(eh_matrix_t mh, uint64_t* d_count, void* stream) {
@@ -939,9 +1007,9 @@ eh_status eh_count_lollipops_async(eh_matrix_t mh, uint64_t* d_count, void* stre
 eh_status eh_count_lollipops(eh_matrix_t mh, uint64_t* count, void* stream) {
   CHECK_MATRIX(mh);
   EH_CHECK_ARG(count, "count is NULL");
-  eh_status s = eh_count_lollipops_async(mh, reinterpret_cast<uint64_t*>(MX(mh)->result), stream);
-  if (s != EH_OK) return s;
-  return eh::finish_sync(MX(mh), MX(mh)->result, count, ST(stream));
+  return eh::count_sync(MX(mh), count, ST(stream), [&](unsigned long long* out, bool report) {
+    return eh::launch_lollipop_count(MX(mh), out, ST(stream), report);
+  });
 }
 
 eh_status eh_similar_nodes_async(eh_matrix_t mh, uint32_t threshold, uint64_t* d_count, void* stream) {
@@ -962,7 +1030,7 @@ eh_status eh_similar_nodes(eh_matrix_t mh, uint32_t threshold, uint64_t* count, 
   EH_CHECK_ARG(count, "count is NULL");
   eh_status s = eh_similar_nodes_async(mh, threshold, reinterpret_cast<uint64_t*>(MX(mh)->result), stream);
   if (s != EH_OK) return s;
-  return eh::finish_sync(MX(mh), MX(mh)->result, count, ST(stream));
+  return eh::finish_sync(MX(mh), count, ST(stream));
 }
 
 eh_status eh_intersect_rows(eh_matrix_t mh, const uint32_t* d_a, const uint32_t* d_b, uint64_t npairs,
@@ -996,7 +1064,7 @@ eh_status eh_count_cliques(eh_matrix_t mh, uint32_t k, uint64_t* count, void* st
   EH_CHECK_ARG(count, "count is NULL");
   eh_status s = eh_count_cliques_async(mh, k, reinterpret_cast<uint64_t*>(MX(mh)->result), stream);
   if (s != EH_OK) return s;
-  return eh::finish_sync(MX(mh), MX(mh)->result, count, ST(stream));
+  return eh::finish_sync(MX(mh), count, ST(stream));
 }
 
 }  // extern "C"

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, ui
   __shared__ unsigned long long s_mask[NW][kCliqueWarpMax];
   __shared__ uint32_t s_list[NW][kCliqueWarpMax];
   __shared__ uint32_t s_bm[NW][kCliqueHash / 32];
+  overlap_begin();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* list = s_list[warp];
   uint32_t* bm = s_bm[warp];
@@ -257,13 +258,13 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, ui
       __syncwarp();
     }
   }
-  if (LIST || a.graph_rows) return;
-  acc = warp_sum_u64(acc);
-  if (lane == 0 && acc) atomicAdd(a.out, acc);
-  if (a.tri) {
-    tacc = warp_sum_u64(tacc);
+  if (!LIST && !a.graph_rows) {
+    acc = warp_sum_u64(acc);
+    if (lane == 0 && acc) atomicAdd(a.out, acc);
+    tacc = a.tri ? warp_sum_u64(tacc) : 0ull;
     if (lane == 0 && tacc) atomicAdd(a.tri, tacc);
   }
+  overlap_end();
 }
 
 // ---- mid tier, k = 4: kCliqueWarpMax < |A_i| <= kCliqueMidMax, one CTA per pivot ----
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_mid(CliqueArgs a, uin
                                                                uint32_t* counter, uint32_t cmax) {
   extern __shared__ __align__(16) uint4 m4[];
   __shared__ uint32_t s_unit, s_scan[NW];
+  overlap_begin();
   uint32_t* m32 = reinterpret_cast<uint32_t*>(m4);
   uint32_t* list = reinterpret_cast<uint32_t*>(m4 + quad_off(cmax));
   uint32_t* off = list + mid_slots(cmax);  // word (32-bit) offset of core row A_i[e]
@@ -447,6 +449,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_mid(CliqueArgs a, uin
   }
   acc = warp_sum_u64(acc + sum.total());
   if (lane == 0 && acc) atomicAdd(a.out, acc);
+  overlap_end();
 }
 
 // ---- CTA tiers: one pivot per CTA; masks in shared memory or a global slot ----
@@ -718,19 +721,18 @@ static cudaError_t launch_shared(const CliqueArgs& a, uint32_t pos_begin, uint32
 }
 
 cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
-                               int sms, cudaStream_t st, bool list) {
+                               int sms, cudaStream_t st, bool list, bool overlap) {
   if (pos_end <= pos_begin) return cudaSuccess;
   // Grabs of up to four pivots, small enough that every resident warp gets several.
   const uint32_t n = pos_end - pos_begin, warps = 5u * NW * (uint32_t)std::max(1, sms);
   const uint32_t grab = std::max(1u, std::min(4u, n / (16 * warps)));
   const unsigned grid = std::max(1u, std::min(5u * (uint32_t)std::max(1, sms), (n + NW * grab - 1) / (NW * grab)));
-  if (list) k_clique_warp<true><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, grab, counter);
-  else k_clique_warp<false><<<grid, kCtaThreads, 0, st>>>(a, pos_begin, pos_end, grab, counter);
-  return cudaGetLastError();
+  return launch_overlapped(list ? k_clique_warp<true> : k_clique_warp<false>, grid, kCtaThreads, 0, st, overlap, a,
+                           pos_begin, pos_end, grab, counter);
 }
 
 cudaError_t launch_clique_mid(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
-                              uint32_t cmax, int sms, cudaStream_t st) {
+                              uint32_t cmax, int sms, cudaStream_t st, bool overlap) {
   if (pos_end <= pos_begin) return cudaSuccess;
   static std::atomic<bool> allowed[64];
   int dev = 0;
@@ -744,8 +746,7 @@ cudaError_t launch_clique_mid(const CliqueArgs& a, uint32_t pos_begin, uint32_t 
   }
   const uint32_t bytes = mid_bytes(cmax), per = std::max(1u, std::min(5u, (228u << 10) / (bytes + 2048)));
   const unsigned grid = std::min<unsigned>(pos_end - pos_begin, per * (unsigned)std::max(1, sms));
-  k_clique_mid<<<grid, kCtaThreads, bytes, st>>>(a, pos_begin, pos_end, counter, cmax);
-  return cudaGetLastError();
+  return launch_overlapped(k_clique_mid, grid, kCtaThreads, bytes, st, overlap, a, pos_begin, pos_end, counter, cmax);
 }
 
 template <bool LIST>

@@ -40,10 +40,12 @@ struct __align__(16) HeavySmem {
   uint64_t bar;  // completion of the unit's bulk copy
   uint32_t unit;
 };
-// Device error flag (PivotArgs::counters[kErrWord]): a bulk copy's wait ran out.
-constexpr uint32_t kErrWord = 15, kErrBulkWait = 1u;
+// Device error flag (PivotArgs::flags): a bulk copy's wait ran out.
+constexpr uint32_t kErrBulkWait = 1u;
 
-// Warp, CTA, then one u64 atomic per CTA into the single count.
+// Warp, CTA, then one u64 atomic per CTA into the single count; the last CTA of
+// the call's kernels writes the result and resets the queue, so that a call needs
+// no memset before it and a blocking call no copy after it (out is then host memory).
 template <int NW = NWARPS>
 __device__ __forceinline__ void cta_add(unsigned long long acc, const PivotArgs& a) {
   __shared__ unsigned long long s_red[NW];
@@ -54,7 +56,15 @@ __device__ __forceinline__ void cta_add(unsigned long long acc, const PivotArgs&
   if (threadIdx.x == 0) {
     unsigned long long tot = 0;
     for (int w = 0; w < NW; w++) tot += s_red[w];
-    if (tot && !a.graph_rows) atomicAdd(a.out, tot);
+    unsigned long long* sum = reinterpret_cast<unsigned long long*>(a.queue + 6);
+    if (tot && !a.graph_rows) atomicAdd(sum, tot);
+    __threadfence();
+    if (atomicAdd(&a.queue[5], 1u) == a.ctas - 1) {
+      __threadfence();
+      if (!a.graph_rows) a.out[0] = atomicExch(sum, 0ull);
+      if (a.report) a.out[1] = atomicExch(a.flags, 0u);
+      for (int k = 0; k < 6; k++) a.queue[k] = 0u;
+    }
   }
 }
 
@@ -127,13 +137,14 @@ template <bool LOLLI>
 __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, const uint2* __restrict__ units,
                                                               uint32_t n_units) {
   __shared__ HeavySmem s;
+  overlap_begin();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long acc = 0;
   uint32_t phase = 0;
   if (threadIdx.x == 0) mbar_init(&s.bar);
 
   for (;;) {
-    if (threadIdx.x == 0) s.unit = atomicAdd(&a.counters[0], 1u);
+    if (threadIdx.x == 0) s.unit = atomicAdd(&a.queue[0], 1u);
     __syncthreads();  // also: every thread is done with the previous unit's staging
     const uint32_t unit = s.unit;
     if (unit >= n_units) break;
@@ -149,7 +160,7 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
       if (!mbar_wait(&s.bar, phase)) {
         // Record the failure, then give the copy in flight a second bounded
         // wait before the buffer is used or the CTA exits.
-        if (threadIdx.x == 0) atomicOr(&a.counters[kErrWord], kErrBulkWait);
+        if (threadIdx.x == 0) atomicOr(a.flags, kErrBulkWait);
         mbar_wait(&s.bar, phase);
       }
       phase ^= 1u;
@@ -222,6 +233,7 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
   }
 
   cta_add(acc, a);
+  overlap_end();
 }
 
 // What the kernels below count: triangles; lollipops by the definition (full
@@ -645,6 +657,7 @@ __global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivo
                                                                uint32_t cap, uint32_t win) {
   extern __shared__ __align__(16) char dyn[];
   __shared__ uint32_t s_unit, s_scan[NW];
+  overlap_begin();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Slice s = make_slice<NW, MODE>(dyn, cap, win);
   for (uint32_t k = threadIdx.x; k < (win + kHashBits) / 32; k += NW * 32) s.bm[k] = 0u;
@@ -668,6 +681,7 @@ __global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivo
     acc += finish_pivot<MODE>(a, i, card, cnt, sum, lane);
   }
   cta_add<NW>(acc + sum.total(), a);
+  overlap_end();
 }
 
 // A chunk of pivots of at most kTinyMax entries as one pair space: the pivots'
@@ -740,6 +754,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_warp(PivotArgs a, uint32_t mid1, uint32_t mid_chunk,
                                                                 uint32_t tiny, uint32_t cap, uint32_t win) {
   extern __shared__ __align__(16) char dyn[];
+  overlap_begin();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   char* mem = dyn + warp * slice_bytes<1, MODE>(cap, win);
   const Slice s = make_slice<1, MODE>(mem, cap, win);
@@ -750,7 +765,7 @@ __global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_wa
   sum.clear();
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = a.n_heavy + atomicAdd(&a.counters[1], mid_chunk);
+    if (lane == 0) base = a.n_heavy + atomicAdd(&a.queue[1], mid_chunk);
     base = __shfl_sync(FULL, base, 0);
     if (base >= mid1) break;
     const uint32_t end = min(mid1, base + mid_chunk);
@@ -767,12 +782,13 @@ __global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_wa
   const uint32_t tiny0 = max(mid1, a.n_heavy);
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = tiny0 + atomicAdd(&a.counters[3], tiny);
+    if (lane == 0) base = tiny0 + atomicAdd(&a.queue[3], tiny);
     base = __shfl_sync(FULL, base, 0);
     if (base >= a.n_order) break;
     acc += tiny_chunk<MODE>(a, base, min(tiny, a.n_order - base), reinterpret_cast<uint32_t*>(mem), lane);
   }
   cta_add(acc + sum.total(), a);
+  overlap_end();
 }
 
 // Dense core build: one warp per row j < core_k writes row(j) ∩ [0, j) as bits.
@@ -1023,68 +1039,85 @@ static cudaError_t allow_smem(const void* kernel, uint32_t bytes, std::atomic<bo
 
 static uint32_t cap_of(uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); }
 
-// n pivots of k_pivots_cta: units, or order[pos0, pos0 + n) whole.
+// One launch of k_pivots_cta: n units, or order[pos0, pos0 + n) whole.
 template <int NW, int MODE>
-static cudaError_t launch_cta_pivots(const PivotArgs& a, const uint2* units, uint32_t n, uint32_t pos0,
-                                     uint32_t* counter, uint32_t largest, uint32_t window, int grid, int device,
-                                     cudaStream_t st) {
-  static std::atomic<bool> done[64];
-  cudaError_t e = allow_smem((const void*)k_pivots_cta<NW, MODE>, slice_bytes<NW, MODE>(kCtaListCap, kCtaWindow), done,
-                             device);
-  if (e != cudaSuccess) return e;
-  const uint32_t cap = cap_of(largest), win = window_bits(a.n, window), bytes = slice_bytes<NW, MODE>(cap, win);
-  const int regs = (MODE == kSym ? 24 : 32) / NW;
-  const int per = std::max(1, std::min(regs, grid / sm_count(device) * (NWARPS / NW)));
-  const int g = (int)std::min<int64_t>(n, resident_grid(device, bytes, per));
-  k_pivots_cta<NW, MODE><<<std::max(g, 1), NW * 32, bytes, st>>>(a, units, n, pos0, counter, cap, win);
-  return cudaGetLastError();
-}
+struct CtaLaunch {
+  uint32_t n = 0, pos0 = 0, cap = 0, win = 0, bytes = 0;
+  unsigned grid = 0;
+  CtaLaunch(const PivotArgs& a, uint32_t n_, uint32_t pos0_, uint32_t largest, uint32_t window, int most, int device)
+      : n(n_), pos0(pos0_) {
+    if (!n) return;
+    cap = cap_of(largest);
+    win = window_bits(a.n, window);
+    bytes = slice_bytes<NW, MODE>(cap, win);
+    const int regs = (MODE == kSym ? 24 : 32) / NW;
+    const int per = std::max(1, std::min(regs, most / sm_count(device) * (NWARPS / NW)));
+    grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n, resident_grid(device, bytes, per)));
+  }
+  cudaError_t run(const PivotArgs& a, const uint2* units, uint32_t* next, int device, cudaStream_t st,
+                  bool& overlap) const {
+    if (!n) return cudaSuccess;
+    static std::atomic<bool> done[64];
+    cudaError_t e = allow_smem((const void*)k_pivots_cta<NW, MODE>, slice_bytes<NW, MODE>(kCtaListCap, kCtaWindow),
+                               done, device);
+    if (e != cudaSuccess) return e;
+    e = launch_overlapped(k_pivots_cta<NW, MODE>, grid, NW * 32, bytes, st, overlap, a, units, n, pos0, next, cap, win);
+    overlap = true;
+    return e;
+  }
+};
 
 template <int MODE>
-static cudaError_t launch_pivots(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
-                                 cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(a.counters, 0, 5 * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(a.out, 0, sizeof(unsigned long long) * (a.graph_rows ? a.num_graphs : 1), st);
-  if (e != cudaSuccess) return e;
+static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_units, int most, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
   int device = 0;
   if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
-  if (MODE != kSym && n_units && a.n_giant) {
-    const int gh = std::min(grid, resident_grid(device, (uint32_t)sizeof(HeavySmem), 6));
-    k_pivots_heavy<MODE == kFull><<<std::max(gh, 1), kCtaThreads, 0, st>>>(a, units, n_units);
-  }
-  if (MODE == kSym) {
-    if (a.n_large && (e = launch_cta_pivots<kLargeWarps, MODE>(a, nullptr, a.n_large, 0, a.counters + 2, a.max_large,
-                                                               kCtaWindow, grid, device, st)) != cudaSuccess)
-      return e;
-  } else if (n_units && a.n_large > a.n_giant) {
-    if ((e = launch_cta_pivots<kLargeWarps, MODE>(a, units, n_units, 0, a.counters + 2, a.max_large, kCtaWindow, grid,
-                                                  device, st)) != cudaSuccess)
-      return e;
-  }
-  if (a.n_heavy > a.n_large &&
-      (e = launch_cta_pivots<kMidWarps, MODE>(a, nullptr, a.n_heavy - a.n_large, a.n_large, a.counters + 4, a.max_mid,
-                                              kWarpWindow, grid, device, st)) != cudaSuccess)
+  if (a.graph_rows && (e = cudaMemsetAsync(a.out, 0, sizeof(unsigned long long) * a.num_graphs, st)) != cudaSuccess)
     return e;
+  // Largest pivots first; the kernels overlap, their CTAs counted for the last one to finish.
+  const bool giants = MODE != kSym && n_units && a.n_giant;
+  const unsigned g_heavy =
+      giants ? (unsigned)std::max(1, std::min(most, resident_grid(device, (uint32_t)sizeof(HeavySmem), 6))) : 0u;
+  const uint32_t n_large = MODE == kSym ? a.n_large : a.n_large > a.n_giant ? n_units : 0u;
+  const CtaLaunch<kLargeWarps, MODE> large(a, n_large, 0, a.max_large, kCtaWindow, most, device);
+  const CtaLaunch<kMidWarps, MODE> mid(a, a.n_heavy > a.n_large ? a.n_heavy - a.n_large : 0u, a.n_large, a.max_mid,
+                                       kWarpWindow, most, device);
+  const uint32_t cap = cap_of(a.max_warp), win = window_bits(a.n, kWarpWindow);
+  const uint32_t bytes = NWARPS * slice_bytes<1, MODE>(cap, win);
+  uint32_t mid1 = 0, mid_chunk = 1, tiny_grab = 1;
+  int gw = 0;
   if (a.n_order > a.n_heavy) {
-    static std::atomic<bool> done[64];
-    if ((e = allow_smem((const void*)k_pivots_warp<MODE>, NWARPS * slice_bytes<1, MODE>(kLightMax, kWarpWindow), done,
-                        device)) != cudaSuccess)
-      return e;
-    const uint32_t cap = cap_of(a.max_warp), win = window_bits(a.n, kWarpWindow);
-    const uint32_t bytes = NWARPS * slice_bytes<1, MODE>(cap, win);
-    const uint32_t mid1 = std::min(a.n_order, std::max(a.n_heavy, a.n_above_tiny)), mid = mid1 - a.n_heavy,
-                   tiny = a.n_order - mid1;
-    int gw = std::min(grid, resident_grid(device, bytes, MODE == kSym ? 3 : 4));
+    mid1 = std::min(a.n_order, std::max(a.n_heavy, a.n_above_tiny));
+    const uint32_t warp_pivots = mid1 - a.n_heavy, tiny = a.n_order - mid1;
+    gw = std::max(1, std::min(most, resident_grid(device, bytes, MODE == kSym ? 3 : 4)));
     // Grabs small enough that every warp gets several; one pivot at least.
-    const uint32_t warps = (uint32_t)std::max(gw, 1) * NWARPS;
-    const uint32_t mid_chunk = std::max(1u, std::min(4u, mid / (16 * warps)));
-    const uint32_t tiny_grab = std::max(1u, std::min(kTinyChunk, tiny / (4 * warps)));
-    const uint64_t grabs = (uint64_t)mid / mid_chunk + tiny / tiny_grab + 1;
-    gw = (int)std::min<uint64_t>(std::max(gw, 1), (grabs + NWARPS - 1) / NWARPS);
-    k_pivots_warp<MODE><<<gw, kCtaThreads, bytes, st>>>(a, mid1, mid_chunk, tiny_grab, cap, win);
+    const uint32_t warps = (uint32_t)gw * NWARPS;
+    mid_chunk = std::max(1u, std::min(4u, warp_pivots / (16 * warps)));
+    tiny_grab = std::max(1u, std::min(kTinyChunk, tiny / (4 * warps)));
+    const uint64_t grabs = (uint64_t)warp_pivots / mid_chunk + tiny / tiny_grab + 1;
+    gw = (int)std::min<uint64_t>(gw, (grabs + NWARPS - 1) / NWARPS);
   }
-  return cudaGetLastError();
+  a.ctas = g_heavy + large.grid + mid.grid + (unsigned)gw;
+  if (a.ctas == 0)  // no row with a pair
+    return a.graph_rows ? cudaSuccess : cudaMemsetAsync(a.out, 0, (a.report ? 2 : 1) * sizeof(unsigned long long), st);
+  bool overlap = false;
+  if (g_heavy) {
+    e = launch_overlapped(k_pivots_heavy<MODE == kFull>, g_heavy, kCtaThreads, 0, st, false, a, units, n_units);
+    overlap = true;
+  }
+  if (e == cudaSuccess) e = large.run(a, MODE == kSym ? nullptr : units, a.queue + 2, device, st, overlap);
+  if (e == cudaSuccess) e = mid.run(a, nullptr, a.queue + 4, device, st, overlap);
+  if (e == cudaSuccess && gw) {
+    static std::atomic<bool> done[64];
+    e = allow_smem((const void*)k_pivots_warp<MODE>, NWARPS * slice_bytes<1, MODE>(kLightMax, kWarpWindow), done,
+                   device);
+    if (e == cudaSuccess)
+      e = launch_overlapped(k_pivots_warp<MODE>, (unsigned)gw, kCtaThreads, bytes, st, overlap, a, mid1, mid_chunk,
+                            tiny_grab, cap, win);
+  }
+  // A launch that failed leaves the others short of the last CTA: clear the queue for the next call.
+  if (e != cudaSuccess) cudaMemsetAsync(a.queue, 0, kPivotQueueWords * sizeof(uint32_t), st);
+  return e;
 }
 
 cudaError_t launch_pivot_units(const RowDesc* desc, const uint32_t* order, uint32_t n_heavy,
@@ -1100,11 +1133,11 @@ cudaError_t launch_pivot_unit_fill(const uint32_t* cnt, const uint32_t* start, u
   return cudaGetLastError();
 }
 
-cudaError_t launch_triangles(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
+cudaError_t launch_triangles(PivotArgs a, const uint2* units, uint32_t n_units, int grid,
                              cudaStream_t st) {
   return launch_pivots<kTri>(a, units, n_units, grid, st);
 }
-cudaError_t launch_lollipops(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
+cudaError_t launch_lollipops(PivotArgs a, const uint2* units, uint32_t n_units, int grid,
                              cudaStream_t st) {
   return a.lcard ? launch_pivots<kSym>(a, units, n_units, grid, st) : launch_pivots<kFull>(a, units, n_units, grid, st);
 }

@@ -55,6 +55,29 @@ constexpr uint32_t FULL = 0xffffffffu;
 // layouts' padding is zero.
 constexpr uint32_t kUintPad = 0xffffffffu;
 
+// ---- Kernels of one call that do not depend on each other ----
+// A call's later kernels are launched with programmatic stream serialization
+// (launch_overlapped): every CTA lets the next kernel's CTAs start as room frees
+// up (overlap_begin) and a kernel's CTAs leave only after the kernel before has
+// finished (overlap_end), so that whatever follows in the stream waits for all.
+__device__ __forceinline__ void overlap_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void overlap_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... Params, class... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem,
+                                     cudaStream_t st, bool overlap, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // ---- Bulk (TMA) copies from global to shared memory, completing on an mbarrier ----
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

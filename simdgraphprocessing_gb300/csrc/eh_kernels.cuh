@@ -85,10 +85,14 @@ struct PivotArgs {
   uint32_t n_giant;        // order[0, n_giant) have decoded lists in giant_lists
   const uint32_t* giant_lists;
   const unsigned long long* giant_off;
-  // [0] next unit (pivots above kCtaListCap), [1] next warp pivot, [2] next
-  // unit (the other large pivots), [3] next tiny pivot, [4] next mid pivot,
-  // [15] device error flags
-  uint32_t* counters;
+  // kPivotQueueWords, all zero between launches: [0] next unit (pivots above
+  // kCtaListCap), [1] next warp pivot, [2] next unit (the other large pivots),
+  // [3] next tiny pivot, [4] next mid pivot, [5] CTAs done, [6..7] the sum so far.
+  // The last CTA writes the result and leaves the words zero again.
+  uint32_t* queue;
+  uint32_t* flags;         // device error flags
+  uint32_t ctas;           // CTAs of all the call's kernels
+  bool report;             // also move the flags to out[1] (and clear them)
   unsigned long long* out; // result; in batch mode out[num_graphs]
   uint32_t unit_span;      // pivot positions e per unit of a large pivot
   const uint32_t* graph_rows;  // batch mode: graph g owns rows [graph_rows[g], graph_rows[g+1]); else null
@@ -101,6 +105,7 @@ struct PivotArgs {
   uint32_t max_warp, max_mid, max_large;  // largest pivot of each tier
   const uint32_t* lcard;   // lollipops of a symmetric matrix: entries of each row below it; else null
 };
+constexpr uint32_t kPivotQueueWords = 8;
 constexpr uint32_t kCtaThreads = 256;
 constexpr uint32_t kLightMax = 160;    // largest light_max: warp-wide pivots fit a slice of this size
 constexpr uint32_t kMidMax = 512;      // heavy pivots up to this size run whole, larger ones in units
@@ -113,9 +118,9 @@ cudaError_t launch_pivot_units(const RowDesc* desc, const uint32_t* order, uint3
                                uint32_t unit_span, uint32_t* cnt, cudaStream_t st);
 cudaError_t launch_pivot_unit_fill(const uint32_t* cnt, const uint32_t* start, uint32_t n_heavy,
                                    uint2* units, cudaStream_t st);
-cudaError_t launch_triangles(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
+cudaError_t launch_triangles(PivotArgs a, const uint2* units, uint32_t n_units, int grid,
                              cudaStream_t st);
-cudaError_t launch_lollipops(const PivotArgs& a, const uint2* units, uint32_t n_units, int grid,
+cudaError_t launch_lollipops(PivotArgs a, const uint2* units, uint32_t n_units, int grid,
                              cudaStream_t st);
 int pivot_grid(int device);  // persistent grid: SMs x resident CTAs of the pivot kernel
 
@@ -181,8 +186,9 @@ constexpr uint32_t kCliqueWarpMax = 64;    // pivots up to this size are a warp'
 constexpr uint32_t kCliqueSmemMax = 2048;  // no pivot above this size keeps its masks in shared memory
 // Words of one pivot's working set (list, masks, per-warp DFS stacks).
 uint64_t clique_slot_words(uint32_t cmax, uint32_t k);
+// overlap: a kernel of the same call came before (see launch_overlapped).
 cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
-                               int sms, cudaStream_t st, bool list = false);
+                               int sms, cudaStream_t st, bool list = false, bool overlap = false);
 // Largest pivot (<= kCliqueSmemMax) whose k-clique working set fits one CTA's
 // opt-in shared memory on `device`; larger pivots use global scratch slots.
 uint32_t clique_smem_cap(uint32_t k, int device);
@@ -190,7 +196,7 @@ uint32_t clique_smem_cap(uint32_t k, int device);
 // largest of them), one CTA each, masks in shared memory.
 constexpr uint32_t kCliqueMidMax = 1024;
 cudaError_t launch_clique_mid(const CliqueArgs& a, uint32_t pos_begin, uint32_t pos_end, uint32_t* counter,
-                              uint32_t cmax, int sms, cudaStream_t st);
+                              uint32_t cmax, int sms, cudaStream_t st, bool overlap = false);
 // gscratch == nullptr: masks in dynamic shared memory (grid <= 0: as many CTAs
 // as fit on the GPU, at most one per pivot); else grid slots of
 // clique_slot_words(cmax, k) words each in global memory.

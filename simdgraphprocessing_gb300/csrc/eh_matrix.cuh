@@ -18,13 +18,17 @@ struct SizeOrder {
   std::vector<uint32_t> starts;  // rows of size > x are order[0, starts[65535 - x])
   // rows in the order of size > x (x < 65535)
   uint32_t above(uint32_t x) const { return starts.empty() ? 0 : starts[65535 - x]; }
-  // largest size <= x present (0 if none)
-  uint32_t largest_at_most(uint32_t x) const {
-    if (starts.empty()) return 0;
-    for (uint32_t b = 65535 - x; b < 65535; b++)
-      if (starts[b + 1] > starts[b]) return 65535 - b;
-    return 0;
+  // largest size <= x present (0 if none), x <= kCtaListCap
+  uint32_t largest_at_most(uint32_t x) const { return starts.empty() ? 0 : largest[x]; }
+  void set(std::vector<uint32_t> s) {
+    starts = std::move(s);
+    largest.assign(kCtaListCap + 1, 0);
+    for (uint32_t x = 1; x <= kCtaListCap; x++)
+      largest[x] = starts[65536 - x] > starts[65535 - x] ? x : largest[x - 1];
   }
+
+ private:
+  std::vector<uint32_t> largest;
 };
 
 // Pivots of the symmetric lollipop count: rows by their entries below the diagonal.
@@ -52,11 +56,13 @@ struct Plan : SizeOrder {
   uint32_t core_k = 0;
 };
 
+constexpr uint32_t kMatrixCounters = 32, kFlagWord = 15, kQueueWord = 18;
+
 // Per-launch scratch: work-queue counters and the clique kernel's global slots.
 // A matrix has its own; concurrent launches on one matrix (the serving loop)
 // each bring theirs.
 struct Workspace {
-  uint32_t* counters = nullptr;        // >= 16 words
+  uint32_t* counters = nullptr;        // kMatrixCounters: as Matrix::counters
   uint32_t* clique_scratch = nullptr;
   uint64_t clique_scratch_words = 0;
 };
@@ -71,7 +77,9 @@ struct Matrix {
   BuildTotals tot{};
   Plan plan;
   Oriented oriented;
-  uint32_t* counters = nullptr;  // 16 work-queue counters, then `result`
+  // kMatrixCounters words: 0..14 the clique and list kernels' work queues, 15 device
+  // error flags, 16..17 `result`, 18..25 the pivot kernels' queue (PivotArgs::queue).
+  uint32_t* counters = nullptr;
   unsigned long long* result = nullptr;
   int grid = 0;
   int64_t vstar = -1;
@@ -145,10 +153,12 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out);
 // Count launches; graph_rows / num_graphs != null selects per-graph outputs
 // out[num_graphs].  ws == null uses the matrix's own workspace.  The plan must
 // already exist when ws != null (launches with a workspace never allocate it).
-// large_only (batches): only the pivots above kCliqueWarpMax entries.
+// large_only (batches): only the pivots above kCliqueWarpMax entries.  report: the
+// device error flags go to out[1].
 eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32_t* graph_rows, uint32_t num_graphs,
-                                cudaStream_t st, Workspace* ws = nullptr, bool large_only = false);
-eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st);
+                                cudaStream_t st, Workspace* ws = nullptr, bool large_only = false,
+                                bool report = false);
+eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st, bool report = false);
 // tuples != null or list: write the k = 3 or 4 cliques as tuples (CliqueArgs::tuples).
 // tri: the triangles of the pivots of up to kCliqueWarpMax entries are added there.
 eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const uint32_t* graph_rows,

@@ -131,8 +131,8 @@ eh_status launch_query(Server* s, Slot& sl, const Query& q) {
   cudaMemcpyAsync(sl.h_out, sl.d_out, sizeof(uint64_t), cudaMemcpyDeviceToHost, sl.st);
   // The pivot kernels' flags word (a bounded wait that ran out), cleared for the slot's next query.
   sl.h_out[1] = 0;
-  cudaMemcpyAsync(sl.h_out + 1, sl.ws.counters + 15, sizeof(uint32_t), cudaMemcpyDeviceToHost, sl.st);
-  cudaMemsetAsync(sl.ws.counters + 15, 0, sizeof(uint32_t), sl.st);
+  cudaMemcpyAsync(sl.h_out + 1, sl.ws.counters + kFlagWord, sizeof(uint32_t), cudaMemcpyDeviceToHost, sl.st);
+  cudaMemsetAsync(sl.ws.counters + kFlagWord, 0, sizeof(uint32_t), sl.st);
   cudaEventRecord(sl.ev, sl.st);
   return EH_OK;
 }
@@ -285,8 +285,8 @@ eh_status eh_server_create(const eh_server_config* cfg, eh_server_t* out) {
   for (auto& sl : s->slots) {
     if (cudaStreamCreateWithFlags(&sl.st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMalloc((void**)&sl.ws.counters, 64) != cudaSuccess ||
-        cudaMemset(sl.ws.counters, 0, 64) != cudaSuccess ||
+        cudaMalloc((void**)&sl.ws.counters, eh::kMatrixCounters * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemset(sl.ws.counters, 0, eh::kMatrixCounters * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc((void**)&sl.d_out, sizeof(unsigned long long)) != cudaSuccess ||
         cudaMallocHost((void**)&sl.h_out, 2 * sizeof(uint64_t)) != cudaSuccess) {
       eh_server_free(reinterpret_cast<eh_server_t>(s));

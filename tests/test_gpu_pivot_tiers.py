@@ -77,7 +77,12 @@ def test_batch_triangles_from_the_clique_masks(eh, oracle, layout):
     b = eh.Batch(gr, off, nbr, layout=layout)
     out = torch.full((3, len(csrs)), -1, dtype=torch.int64, device="cuda")
     st = torch.cuda.Stream()
-    b.run(out[0].data_ptr(), out[1].data_ptr(), use_graph=False, stream=st)
+    for use_graph in (True, True, False, True):          # captured, replayed, direct
+        out.fill_(-1)
+        torch.cuda.synchronize()
+        b.run(out[0].data_ptr(), out[1].data_ptr(), use_graph=use_graph, stream=st)
+        st.synchronize()
+        assert [int(x) for x in out[0][:4]] == [0, 1, 4, 10] and (out[1] >= 0).all()
     b.count(3, out[2].data_ptr(), stream=st)
     st.synchronize()
     lows = [oracle.Matrix(o, x, oracle.SELECT_LOWER, oracle.UINTEGER) for o, x in csrs]
