@@ -179,6 +179,27 @@ struct Totals {
     n_pshort = __reduce_add_sync(FULL, n_pshort);
     n_bitset = __reduce_add_sync(FULL, n_bitset);
   }
+  // One flush per CTA of kBlock threads (all of them call it): the warps' atomics on
+  // the same few words were most of the measure pass (312 of 340 us for 1.2 M rows).
+  __device__ __forceinline__ void cta_flush(BuildTotals* tot) {
+    __shared__ Totals s_tot[kBlock / 32];
+    warp_reduce();
+    if ((threadIdx.x & 31) == 0) s_tot[threadIdx.x >> 5] = *this;
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int w = 1; w < kBlock / 32; w++) {
+      const Totals& o = s_tot[w];
+      card += o.card;
+      ref += o.ref;
+      units += o.units;
+      n_uint += o.n_uint;
+      n_pshort += o.n_pshort;
+      n_bitset += o.n_bitset;
+      max_full = max(max_full, o.max_full);
+      max_card = max(max_card, o.max_card);
+    }
+    flush(tot);
+  }
   __device__ __forceinline__ void flush(BuildTotals* tot) const {
     if (card) atomicAdd(&tot->cardinality, card);
     if (ref) atomicAdd(&tot->ref_bytes, ref);
@@ -254,12 +275,9 @@ __global__ void __launch_bounds__(kBlock) k_measure(uint64_t n, uint64_t total, 
       }
     }
   }
-  t.warp_reduce();
+  t.cta_flush(tot);
   flags = __reduce_or_sync(FULL, flags);
-  if (lane == 0) {
-    t.flush(tot);
-    if (flags) atomicOr(err, flags);
-  }
+  if (lane == 0 && flags) atomicOr(err, flags);
 }
 
 // Rows longer than kBigRow, one CTA of kBigBlock threads each: warp w measures
@@ -313,6 +331,250 @@ __global__ void __launch_bounds__(kBigBlock) k_measure_big(uint64_t n, const uin
   if (threadIdx.x == 0) {
     t.flush(tot);
     if (flags) atomicOr(err, flags);
+  }
+}
+
+// ---- the common case: all entries, or those below the row, and no pshort row ----
+// Row q (of 32) of a warp whose first is base: runs of 8 consecutive rows (whose
+// offsets, entries and payloads share sectors), dealt round-robin so that the hubs
+// at the front of a degree-ordered graph spread over the grid of nw warps.
+__device__ __forceinline__ uint64_t dealt_row(uint64_t base, uint32_t q, uint64_t nw) {
+  return base + (q & 7) + (uint64_t)(q >> 3) * 8 * nw;
+}
+
+// Rows are ascending (checked as they are measured), so the selected entries are a
+// prefix: its length, first and last entry are all that the other layouts need,
+// and encoding is a copy of the prefix (or one bit per entry of it).  A lane takes
+// its row of up to kLaneRow entries, 8 lanes one of up to kGroupRow, the warp
+// longer ones; every load of a step is in flight before the first is used.  (A
+// warp per row over 8 entries, with ballots for selections and 16-bit partitions,
+// took 545 us to measure 46 M entries, 316 us of it after the last chunk's upload.)
+constexpr uint32_t kGroupRow = 256;
+__host__ __device__ inline bool prefix_build(int sel, int layout) {
+  return (sel == 0 || sel == 1) && (layout == TY_UINT || layout == TY_BITSET || layout == 5);
+}
+
+// Selected entries of r[0, len) (row id `row`) seen by one of W lanes, and flags.
+template <uint32_t W, class Index>
+__device__ __forceinline__ uint32_t measure_prefix(const uint32_t* __restrict__ r, Index len, uint64_t n,
+                                                   uint64_t row, int sel, uint32_t sl, uint32_t& flags) {
+  uint32_t cnt = 0;
+  for (Index k0 = sl; k0 < len; k0 += 4 * W) {
+    uint32_t x[4], p[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      const Index k = k0 + u * W;
+      x[u] = k < len ? __ldg(r + k) : 0u;
+      p[u] = k < len && k > 0 ? __ldg(r + k - 1) : 0u;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      const Index k = k0 + u * W;
+      if (k >= len) break;
+      if (x[u] >= n) flags |= ERRF_RANGE;
+      if (k > 0 && p[u] >= x[u]) flags |= ERRF_UNSORTED;
+      cnt += sel == 0 || x[u] < row;
+    }
+  }
+  return cnt;
+}
+__device__ __forceinline__ RowResult finish_prefix(const uint32_t* __restrict__ r, uint32_t cnt, int layout) {
+  return finish_row(cnt, 0, cnt ? __ldg(r) : 0xffffffffu, cnt ? __ldg(r + cnt - 1) : 0u, layout);
+}
+
+__global__ void __launch_bounds__(kBlock) k_measure_prefix(uint64_t n, uint64_t total, uint64_t r_begin,
+                                                           uint64_t r_end, const uint64_t* __restrict__ off,
+                                                           const uint32_t* __restrict__ nbr, int sel, int layout,
+                                                           RowMeasure* __restrict__ meas,
+                                                           BuildTotals* __restrict__ tot, uint32_t* __restrict__ err,
+                                                           uint32_t* __restrict__ big, uint32_t* __restrict__ n_big) {
+  const uint32_t lane = threadIdx.x & 31, sl = lane & 7, grp = lane >> 3;
+  const uint64_t nw = (uint64_t)gridDim.x * (kBlock / 32);
+  uint32_t flags = 0;
+  Totals t;
+  for (uint64_t row0 = r_begin + 8 * ((uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)); row0 < r_end;
+       row0 += nw * 32) {
+    const uint64_t my = dealt_row(row0, lane, nw);
+    uint64_t my_b = my < r_end ? off[my] : 0, my_e = my < r_end ? off[my + 1] : 0;
+    if (my_e < my_b || my_e > total) {  // offsets must rise monotonically within the nbr array
+      flags |= ERRF_OFFSETS;
+      my_b = my_e = 0;
+    }
+    const uint64_t len = my_e - my_b;
+    const uint32_t* r = nbr + my_b;
+    if (my < r_end && len <= kLaneRow) {
+      uint32_t x[kLaneRow];
+#pragma unroll
+      for (uint32_t u = 0; u < kLaneRow; u++) x[u] = u < len ? __ldg(r + u) : 0u;
+      uint32_t cnt = 0, last = 0;
+#pragma unroll
+      for (uint32_t u = 0; u < kLaneRow; u++)
+        if (u < len) {
+          if (x[u] >= n) flags |= ERRF_RANGE;
+          if (u && x[u - 1] >= x[u]) flags |= ERRF_UNSORTED;
+          if (sel == 0 || x[u] < my) {
+            cnt++;
+            last = x[u];
+          }
+        }
+      const RowResult res = finish_row(cnt, 0, cnt ? x[0] : 0xffffffffu, last, layout);
+      meas[my] = res.m;
+      t.add(res, len);
+    }
+    for (uint32_t m = __ballot_sync(FULL, my < r_end && len > kLaneRow && len <= kGroupRow); m;) {
+      uint32_t own = m;  // group g takes the g-th row left
+      for (uint32_t u = 0; u < 4; u++) {
+        if (u < grp) own &= own - 1;
+        m &= m - 1;
+      }
+      const uint32_t q = own ? __ffs(own) - 1 : 0u;
+      const uint64_t b = __shfl_sync(FULL, my_b, q);
+      const uint32_t lq = (uint32_t)__shfl_sync(FULL, len, q), l = own ? lq : 0u;
+      const uint64_t row = dealt_row(row0, q, nw);
+      uint32_t cnt = measure_prefix<8, uint32_t>(nbr + b, l, n, row, sel, sl, flags);
+      cnt += __shfl_xor_sync(FULL, cnt, 1);
+      cnt += __shfl_xor_sync(FULL, cnt, 2);
+      cnt += __shfl_xor_sync(FULL, cnt, 4);
+      if (sl == 0 && own) {
+        const RowResult res = finish_prefix(nbr + b, cnt, layout);
+        meas[row] = res.m;
+        t.add(res, l);
+      }
+    }
+    for (uint32_t m = __ballot_sync(FULL, my < r_end && len > kGroupRow); m; m &= m - 1) {
+      const uint32_t q = __ffs(m) - 1;
+      const uint64_t row = dealt_row(row0, q, nw), b = __shfl_sync(FULL, my_b, q), l = __shfl_sync(FULL, len, q);
+      if (l > kBigRow) {
+        if (lane == 0) big[atomicAdd(n_big, 1u)] = (uint32_t)row;
+        continue;
+      }
+      const uint32_t cnt = warp_sum_u32(measure_prefix<32, uint32_t>(nbr + b, (uint32_t)l, n, row, sel, lane, flags));
+      if (lane == 0) {
+        const RowResult res = finish_prefix(nbr + b, cnt, layout);
+        meas[row] = res.m;
+        t.add(res, l);
+      }
+    }
+  }
+  t.cta_flush(tot);
+  flags = __reduce_or_sync(FULL, flags);
+  if (lane == 0 && flags) atomicOr(err, flags);
+}
+
+__global__ void __launch_bounds__(kBigBlock) k_measure_prefix_big(uint64_t n, const uint64_t* __restrict__ off,
+                                                                  const uint32_t* __restrict__ nbr, int sel,
+                                                                  int layout, RowMeasure* __restrict__ meas,
+                                                                  BuildTotals* __restrict__ tot,
+                                                                  uint32_t* __restrict__ err,
+                                                                  const uint32_t* __restrict__ big,
+                                                                  const uint32_t* __restrict__ big_begin,
+                                                                  const uint32_t* __restrict__ big_end) {
+  __shared__ uint32_t s_cnt;
+  const uint32_t lane = threadIdx.x & 31, nb = *big_end;
+  Totals t;
+  uint32_t flags = 0;
+  for (uint32_t i = *big_begin + blockIdx.x; i < nb; i += gridDim.x) {
+    const uint64_t row = big[i], b = off[row], len = off[row + 1] - b;
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    const uint32_t c = warp_sum_u32(measure_prefix<kBigBlock, uint64_t>(nbr + b, len, n, row, sel, threadIdx.x, flags));
+    if (lane == 0 && c) atomicAdd(&s_cnt, c);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const uint32_t cnt = s_cnt;
+      if (cnt >= (1u << 28)) flags |= ERRF_ROW_TOO_LONG;
+      const RowResult res = finish_prefix(nbr + b, cnt, layout);
+      meas[row] = res.m;
+      t.add(res, len);
+    }
+    __syncthreads();
+  }
+  flags = __reduce_or_sync(FULL, flags);
+  if (threadIdx.x == 0) t.flush(tot);
+  if (lane == 0 && flags) atomicOr(err, flags);
+}
+
+// The prefix r[0, card) of a row into its payload, by W lanes.
+template <uint32_t W>
+__device__ __forceinline__ void encode_prefix(const uint32_t* __restrict__ r, uint32_t card, uint32_t type,
+                                              uint32_t aux, uint4* dst, uint32_t sl) {
+  if (type == TY_UINT) {
+    uint32_t* a = reinterpret_cast<uint32_t*>(dst);
+    const uint32_t padded = (card + 3) & ~3u;
+    for (uint32_t k0 = sl; k0 < padded; k0 += 4 * W) {
+      uint32_t x[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++) x[u] = k0 + u * W < card ? __ldg(r + k0 + u * W) : kUintPad;
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++)
+        if (k0 + u * W < padded) a[k0 + u * W] = x[u];
+    }
+  } else {
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(dst);
+    for (uint32_t k = sl; k < card; k += W) {
+      const uint32_t x = __ldg(r + k);
+      atomicOr(&words[(x >> 6) - aux], 1ull << (x & 63));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) k_encode_prefix(uint64_t n, const uint64_t* __restrict__ off,
+                                                          const uint32_t* __restrict__ nbr,
+                                                          const RowMeasure* __restrict__ meas,
+                                                          const uint32_t* __restrict__ off16,
+                                                          RowDesc* __restrict__ desc, uint4* __restrict__ arena) {
+  const uint32_t lane = threadIdx.x & 31, sl = lane & 7, grp = lane >> 3;
+  const uint64_t nw = (uint64_t)gridDim.x * (kBlock / 32);
+  for (uint64_t row0 = 8 * ((uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)); row0 < n; row0 += nw * 32) {
+    const uint64_t my = dealt_row(row0, lane, nw);
+    RowMeasure mm{0, 0, 0, 0};
+    uint64_t my_b = 0;
+    uint32_t my_o = 0;
+    if (my < n) {
+      mm = meas[my];
+      my_o = off16[my];
+      my_b = off[my];
+      desc[my] = RowDesc{my_o, mm.card, mm.aux, mm.lt};
+    }
+    const uint32_t type = mm.lt >> 30;
+    if (mm.card && mm.card <= kLaneRow) encode_prefix<1>(nbr + my_b, mm.card, type, mm.aux, arena + my_o, 0);
+    __syncwarp();
+    for (uint32_t m = __ballot_sync(FULL, mm.card > kLaneRow && mm.card <= kGroupRow); m;) {
+      uint32_t own = m;
+      for (uint32_t u = 0; u < 4; u++) {
+        if (u < grp) own &= own - 1;
+        m &= m - 1;
+      }
+      const uint32_t q = own ? __ffs(own) - 1 : 0u;
+      const uint64_t b = __shfl_sync(FULL, my_b, q);
+      const uint32_t card = __shfl_sync(FULL, mm.card, q), ty = __shfl_sync(FULL, type, q);
+      const uint32_t aux = __shfl_sync(FULL, mm.aux, q), o = __shfl_sync(FULL, my_o, q);
+      if (own) encode_prefix<8>(nbr + b, card, ty, aux, arena + o, sl);
+      __syncwarp();
+    }
+    for (uint32_t m = __ballot_sync(FULL, mm.card > kGroupRow); m; m &= m - 1) {
+      const uint32_t q = __ffs(m) - 1;
+      const uint64_t b = __shfl_sync(FULL, my_b, q);
+      const uint32_t card = __shfl_sync(FULL, mm.card, q), ty = __shfl_sync(FULL, type, q);
+      const uint32_t aux = __shfl_sync(FULL, mm.aux, q), o = __shfl_sync(FULL, my_o, q);
+      if (card <= kBigRow) encode_prefix<32>(nbr + b, card, ty, aux, arena + o, lane);
+    }
+  }
+}
+// Rows listed by the measure pass whose prefix is longer than kBigRow, a CTA each.
+__global__ void __launch_bounds__(kBigBlock) k_encode_prefix_big(const uint64_t* __restrict__ off,
+                                                                 const uint32_t* __restrict__ nbr,
+                                                                 const RowMeasure* __restrict__ meas,
+                                                                 const uint32_t* __restrict__ off16,
+                                                                 uint4* __restrict__ arena,
+                                                                 const uint32_t* __restrict__ big,
+                                                                 const uint32_t* __restrict__ n_big) {
+  const uint32_t nb = *n_big;
+  for (uint32_t i = blockIdx.x; i < nb; i += gridDim.x) {
+    const uint64_t row = big[i];
+    const RowMeasure m = meas[row];
+    if (m.card > kBigRow)
+      encode_prefix<kBigBlock>(nbr + off[row], m.card, m.lt >> 30, m.aux, arena + off16[row], threadIdx.x);
   }
 }
 
@@ -913,7 +1175,14 @@ cudaError_t launch_measure_rows(uint64_t n, uint64_t total, uint64_t r_begin, ui
                                 const uint32_t* nbr, const uint8_t* mask, int sel, int layout, RowMeasure* meas,
                                 BuildTotals* totals, uint32_t* err, uint32_t* big, uint32_t* n_big, cudaStream_t st) {
   if (r_end <= r_begin) return cudaSuccess;
-  k_measure<<<grid_for(r_end - r_begin, kBlock / 32), kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, mask, sel,
+  if (prefix_build(sel, layout)) {
+    const unsigned grid = (unsigned)std::min<uint64_t>((r_end - r_begin + kBlock - 1) / kBlock, 152 * 8);
+    k_measure_prefix<<<grid, kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, sel,
+                                                                                layout, meas, totals, err, big, n_big);
+    return cudaGetLastError();
+  }
+  const unsigned grid = (unsigned)std::min<uint64_t>((r_end - r_begin + kBlock / 32 - 1) / (kBlock / 32), 152 * 8);
+  k_measure<<<grid, kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, mask, sel,
                                                                         layout, meas, totals, err, big, n_big);
   return cudaGetLastError();
 }
@@ -922,6 +1191,11 @@ cudaError_t launch_measure_big(uint64_t n, const uint64_t* off, const uint32_t* 
                                int layout, RowMeasure* meas, BuildTotals* totals, uint32_t* err, const uint32_t* big,
                                const uint32_t* big_begin, const uint32_t* big_end, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
+  if (prefix_build(sel, layout)) {
+    k_measure_prefix_big<<<2 * 152, kBigBlock, 0, st>>>(n, off, nbr, sel, layout, meas, totals, err, big, big_begin,
+                                                        big_end);
+    return cudaGetLastError();
+  }
   k_measure_big<<<2 * 152, kBigBlock, 0, st>>>(n, off, nbr, mask, sel, layout, meas, totals, err, big, big_begin,
                                                big_end);
   return cudaGetLastError();
@@ -938,9 +1212,14 @@ cudaError_t launch_scan_units(uint64_t n, const RowMeasure* meas, uint32_t* off1
 }
 
 cudaError_t launch_encode(uint64_t n, const uint64_t* off, const uint32_t* nbr, const uint8_t* mask,
-                          int sel, const RowMeasure* meas, const uint32_t* off16, RowDesc* desc,
+                          int sel, int layout, const RowMeasure* meas, const uint32_t* off16, RowDesc* desc,
                           uint4* arena, const uint32_t* big, const uint32_t* n_big, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
+  if (prefix_build(sel, layout)) {
+    k_encode_prefix<<<(unsigned)std::min<uint64_t>((n + kBlock - 1) / kBlock, 152 * 16), kBlock, 0, st>>>(n, off, nbr, meas, off16, desc, arena);
+    k_encode_prefix_big<<<2 * 152, kBigBlock, 0, st>>>(off, nbr, meas, off16, arena, big, n_big);
+    return cudaGetLastError();
+  }
   k_encode<<<grid_for(n, kBlock / 32), kBlock, 0, st>>>(n, off, nbr, mask, sel, meas, off16, desc, arena);
   k_encode_big<<<2 * 152, kBigBlock, 0, st>>>(off, nbr, mask, sel, meas, off16, arena, big, n_big);
   return cudaGetLastError();

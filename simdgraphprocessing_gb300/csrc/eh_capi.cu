@@ -129,10 +129,11 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   m->n = n;
   m->layout = layout;
   m->selection = sel;
+  m->light_max = default_light_max(n);
+  m->core_limit = default_core_rows(n);
   cudaGetDevice(&m->device);
   RowMeasure* meas = nullptr;
   BuildTotals* tot = nullptr;
-  uint32_t* err = nullptr;
   uint32_t* off16 = nullptr;
   uint32_t* tmp = nullptr;
   // big: rows over 4,096 entries (big_cap slots), their count n_big, then
@@ -144,7 +145,6 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   auto cleanup = [&]() {
     cudaFreeAsync(meas, st);
     cudaFreeAsync(tot, st);
-    cudaFreeAsync(err, st);
     cudaFreeAsync(off16, st);
     cudaFreeAsync(tmp, st);
     cudaFreeAsync(big, st);
@@ -161,15 +161,14 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   cudaError_t e;
   const uint64_t nn = n ? n : 1;
   if ((e = pool_alloc((void**)&meas, nn * sizeof(RowMeasure), st)) != cudaSuccess ||
-      (e = pool_alloc((void**)&tot, sizeof(BuildTotals), st)) != cudaSuccess ||
-      (e = pool_alloc((void**)&err, sizeof(uint32_t), st)) != cudaSuccess ||
+      (e = pool_alloc((void**)&tot, sizeof(BuildTotals) + 8, st)) != cudaSuccess ||  // then the error word
       (e = pool_alloc((void**)&off16, nn * sizeof(uint32_t), st)) != cudaSuccess ||
       (e = pool_alloc((void**)&tmp, scan_tmp_words(nn) * sizeof(uint32_t), st)) != cudaSuccess ||
       (e = pool_alloc((void**)&big, (big_cap + 1 + n_marks) * sizeof(uint32_t), st)) != cudaSuccess)
     return fail(e == cudaErrorMemoryAllocation ? set_error(EH_ERR_OUT_OF_MEMORY, "build scratch allocation failed")
                                                : cuda_fail(e, "cudaMallocAsync"));
-  cudaMemsetAsync(tot, 0, sizeof(BuildTotals), st);
-  cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
+  uint32_t* err = reinterpret_cast<uint32_t*>(tot + 1);
+  cudaMemsetAsync(tot, 0, sizeof(BuildTotals) + 8, st);
   uint32_t* n_big = big + big_cap;
   uint32_t* mark = n_big + 1;
   cudaMemsetAsync(n_big, 0, 2 * sizeof(uint32_t), st);  // n_big, mark[0]
@@ -189,10 +188,14 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
                  cudaSuccess) {
     return fail(cuda_fail(e, "measure kernel"));
   }
-  uint32_t herr = 0;
-  cudaMemcpyAsync(&m->tot, tot, sizeof(BuildTotals), cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(&herr, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+  struct {
+    BuildTotals tot;
+    uint32_t err, pad;
+  } h{};
+  cudaMemcpyAsync(&h, tot, sizeof(h), cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(cuda_fail(e, "measure"));
+  m->tot = h.tot;
+  const uint32_t herr = h.err;
   if (herr) {
     return fail(set_error(EH_ERR_INVALID_ARGUMENT, "adjacency rejected:%s%s%s%s",
                           (herr & ERRF_OFFSETS) ? " offsets fall or run past offsets[n];" : "",
@@ -214,7 +217,7 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   m->device_bytes = nn * sizeof(RowDesc) + (m->arena_units + 1) * 16 + 128;
   cudaMemsetAsync(m->counters, 0, kMatrixCounters * sizeof(uint32_t), st);
   cudaMemsetAsync(m->arena, 0, (m->arena_units + 1) * 16, st);
-  if ((e = launch_encode(n, d_off, d_nbr, d_mask, sel, meas, off16, m->desc, m->arena, big, big + big_cap, st)) !=
+  if ((e = launch_encode(n, d_off, d_nbr, d_mask, sel, layout, meas, off16, m->desc, m->arena, big, big + big_cap, st)) !=
       cudaSuccess)
     return fail(cuda_fail(e, "encode kernel"));
   cleanup();
@@ -241,7 +244,9 @@ eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaSt
   p.light_max = light_max;
   p.unit_span = unit_span;
   p.units_ready = true;
-  if (n_large == 0) return EH_OK;
+  // Without giants, and with a span that no large pivot exceeds, a pivot is a unit.
+  p.whole_large = p.n_giant == 0 && p.largest_at_most(kCtaListCap) <= unit_span + 1;
+  if (n_large == 0 || p.whole_large) return EH_OK;
   p.units_ready = false;  // until the list below is built
   uint32_t* cnt = nullptr;
   uint32_t* start = nullptr;
@@ -278,11 +283,12 @@ eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaSt
 
 // Dense core of the first min(n, core_limit) rows (rounded down to a multiple of
 // 64); graphs under 1,024 rows go without.
-eh_status ensure_core(Matrix* m, cudaStream_t st) {
+static eh_status start_core(Matrix* m, cudaStream_t st) {
   Plan& p = m->plan;
   uint32_t want = (uint32_t)std::min<uint64_t>(m->n, m->core_limit) & ~63u;
   if (m->n < 1024) want = 0;
   if (want == p.core_k && (want == 0 || p.core)) return EH_OK;
+  p.core_ready = false;
   if (p.core) {
     CU(wait_uses(m, st), "core");  // launches on other streams may still read it
     CU(cudaFreeAsync(p.core, st), "core");
@@ -294,10 +300,17 @@ eh_status ensure_core(Matrix* m, cudaStream_t st) {
     const uint64_t words = core_row_offset(want);
     CU(pool_alloc((void**)&p.core, words * 8, st, kPoolCore), "core allocation");
     m->device_bytes += words * 8;
-    CU(launch_core_build(m->desc, m->arena, want, p.core, st), "core build");
     p.core_k = want;
+    CU(launch_core_build(m->desc, m->arena, want, p.core, st), "core build");
   }
-  CU(cudaStreamSynchronize(st), "core build");
+  return EH_OK;
+}
+
+eh_status ensure_core(Matrix* m, cudaStream_t st) {
+  eh_status s = start_core(m, st);
+  if (s != EH_OK || m->plan.core_ready) return s;
+  CU(cudaStreamSynchronize(st), "core build");  // counts may run on any stream
+  m->plan.core_ready = true;
   return EH_OK;
 }
 
@@ -336,16 +349,20 @@ eh_status ensure_plan(Matrix* m, cudaStream_t st) {
     CU(pool_alloc((void**)&hist, (65536 + scan_tmp_words(65536)) * sizeof(uint32_t), st), "plan scratch");
     CU(pool_alloc((void**)&cursor, 65536 * sizeof(uint32_t), st), "plan scratch");
     CU(launch_plan(m->n, &m->desc->card, sizeof(RowDesc) / 4, 2, hist, p.order, cursor, st), "plan kernels");
-    std::vector<uint32_t> starts(65536);
-    uint32_t total = 0;
-    CU(cudaMemcpyAsync(starts.data(), hist, 65536 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "plan copy");
-    CU(cudaMemcpyAsync(&total, cursor + 65535, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "plan copy");
+    // The core does not depend on the order: it is built behind it, before the host waits.
+    eh_status s = start_core(m, st);
+    if (s != EH_OK) return s;
+    std::vector<uint32_t> starts(65537);  // bin starts, then the end of the last bin
+    CU(cudaMemcpyAsync(hist + 65536, cursor + 65535, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st), "plan copy");
+    CU(cudaMemcpyAsync(starts.data(), hist, 65537 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "plan copy");
     CU(cudaStreamSynchronize(st), "plan");
     cudaFreeAsync(hist, st);
     cudaFreeAsync(cursor, st);
-    p.n_order = m->n ? total : 0;
+    p.n_order = m->n ? starts[65536] : 0;
+    starts.resize(65536);
     if (m->n) p.set(std::move(starts));
     p.n_giant = p.above(kCtaListCap);
+    p.core_ready = true;
     // Giant pivots that are not uint rows get a decoded list.
     std::vector<uint32_t> grows(p.n_giant);
     std::vector<unsigned long long> goff(p.n_giant ? p.n_giant : 1, 0);
@@ -375,6 +392,10 @@ eh_status ensure_plan(Matrix* m, cudaStream_t st) {
         }
       }
     }
+    if (p.n_giant == 0) {
+      p.ready = true;
+      return ensure_units(m, m->light_max, m->unit_span, st);
+    }
     CU(pool_alloc((void**)&p.giant_off, goff.size() * sizeof(unsigned long long), st), "giant allocation");
     CU(pool_alloc((void**)&p.giant_lists, (gtotal ? gtotal : 1) * sizeof(uint32_t), st), "giant allocation");
     m->device_bytes += goff.size() * 8 + (gtotal ? gtotal : 1) * 4;
@@ -397,8 +418,7 @@ eh_status ensure_plan(Matrix* m, cudaStream_t st) {
     p.ready = true;
   }
   eh_status s = ensure_core(m, st);
-  if (s != EH_OK) return s;
-  return ensure_units(m, m->light_max, m->unit_span, st);
+  return s != EH_OK ? s : ensure_units(m, m->light_max, m->unit_span, st);
 }
 
 PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
@@ -679,7 +699,7 @@ eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t
   if ((s = ensure_plan(m, st)) != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
   a.report = report;
-  CU(launch_lollipops(a, m->plan.units, m->plan.n_units, m->grid, st), "lollipop kernel");
+  CU(launch_lollipops(a, m->plan.unit_list(), m->plan.n_units, m->grid, st), "lollipop kernel");
   note_use(m, st);
   return EH_OK;
 }
@@ -703,7 +723,7 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
     a.n_order = m->plan.above(kCliqueWarpMax);
     a.n_heavy = std::min(a.n_heavy, a.n_order);
   }
-  CU(launch_triangles(a, m->plan.units, m->plan.n_units, m->grid, st), "triangle kernel");
+  CU(launch_triangles(a, m->plan.unit_list(), m->plan.n_units, m->grid, st), "triangle kernel");
   if (graph_rows && !large_only) {
     CliqueArgs c{m->desc, m->arena, a.order, 3, out, graph_rows, num_graphs, a.core, a.core_k, nullptr, 0, nullptr};
     int sms = 0;

@@ -649,8 +649,8 @@ __device__ __forceinline__ void keep_below(const PivotArgs& a, RowView& A, uint3
 // Pivots above the warp tier and up to kCtaListCap entries, one CTA each, in
 // two launches so that the many mid-sized ones leave their shared memory to
 // L1 and have few warps at a barrier: large pivots as units of unit_span
-// positions (units; the giants' are k_pivots_heavy's), or a range of the order
-// from pos0 on whole (units null).
+// positions (units; the giants' are k_pivots_heavy's) where some have more, or
+// a range of the order from pos0 on whole (units null).
 template <int NW, int MODE>
 __global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivots_cta(PivotArgs a, const uint2* __restrict__ units,
                                                                uint32_t n_units, uint32_t pos0, uint32_t* counter,
@@ -1078,7 +1078,7 @@ static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_uni
   const bool giants = MODE != kSym && n_units && a.n_giant;
   const unsigned g_heavy =
       giants ? (unsigned)std::max(1, std::min(most, resident_grid(device, (uint32_t)sizeof(HeavySmem), 6))) : 0u;
-  const uint32_t n_large = MODE == kSym ? a.n_large : a.n_large > a.n_giant ? n_units : 0u;
+  const uint32_t n_large = !units ? a.n_large : a.n_large > a.n_giant ? n_units : 0u;  // no list: whole pivots
   const CtaLaunch<kLargeWarps, MODE> large(a, n_large, 0, a.max_large, kCtaWindow, most, device);
   const CtaLaunch<kMidWarps, MODE> mid(a, a.n_heavy > a.n_large ? a.n_heavy - a.n_large : 0u, a.n_large, a.max_mid,
                                        kWarpWindow, most, device);
@@ -1105,7 +1105,7 @@ static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_uni
     e = launch_overlapped(k_pivots_heavy<MODE == kFull>, g_heavy, kCtaThreads, 0, st, false, a, units, n_units);
     overlap = true;
   }
-  if (e == cudaSuccess) e = large.run(a, MODE == kSym ? nullptr : units, a.queue + 2, device, st, overlap);
+  if (e == cudaSuccess) e = large.run(a, units, a.queue + 2, device, st, overlap);
   if (e == cudaSuccess) e = mid.run(a, nullptr, a.queue + 4, device, st, overlap);
   if (e == cudaSuccess && gw) {
     static std::atomic<bool> done[64];

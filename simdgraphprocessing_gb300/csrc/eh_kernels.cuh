@@ -53,7 +53,7 @@ cudaError_t launch_scan_units(uint64_t n, const RowMeasure* meas, uint32_t* off1
                               uint64_t n_block_tmp, cudaStream_t st);
 uint64_t scan_tmp_words(uint64_t n);
 cudaError_t launch_encode(uint64_t n, const uint64_t* off, const uint32_t* nbr, const uint8_t* mask,
-                          int sel, const RowMeasure* meas, const uint32_t* off16, RowDesc* desc,
+                          int sel, int layout, const RowMeasure* meas, const uint32_t* off16, RowDesc* desc,
                           uint4* arena, const uint32_t* big, const uint32_t* n_big, cudaStream_t st);
 // Entries below the diagonal per row, and check[0] == check[1] == 0 for a symmetric
 // matrix without self-loops (key: random; see k_orient).  big / n_big: a list of
@@ -110,8 +110,17 @@ constexpr uint32_t kCtaThreads = 256;
 constexpr uint32_t kLightMax = 160;    // largest light_max: warp-wide pivots fit a slice of this size
 constexpr uint32_t kMidMax = 512;      // heavy pivots up to this size run whole, larger ones in units
 constexpr uint32_t kWarpWindow = 8192, kCtaWindow = 65536;  // bits of the pivots' membership windows
-constexpr uint32_t kDefaultLightMax = 96;
-constexpr uint32_t kDefaultUnitSpan = 1024;
+// Work shape of a matrix the tuner has not seen.  R-MAT, edge factor 16, us per
+// count: 32,768 / 40,960 / 65,536 core rows take 704 / 721 / 780 at 1 M rows, 1,193 /
+// 1,239 / 1,453 at 1.5 M (67 MB of core words stay in L2), 3,625 / 3,257 / 3,738 at
+// 3 M and 6,487 / 5,927 / 5,557 at 2^22, where streaming the bitset rows behind a
+// smaller core costs more.  A warp per pivot as far as its slice goes (light_max
+// 160; one launch for most small graphs: 2^14 rows 37 -> 21 us, 2^18 185 -> 164)
+// except at the largest sizes, where smaller slices leave more L1 for loads in flight
+// (2^22: 5,557 at 160, 5,410 at 96).
+inline uint32_t default_light_max(uint64_t n) { return n < 3500000 ? 160 : 96; }
+inline uint32_t default_core_rows(uint64_t n) { return n < 1750000 ? 32768 : n < 3500000 ? 40960 : 65536; }
+constexpr uint32_t kDefaultUnitSpan = 2048;
 constexpr uint32_t kCtaListCap = 2048; // CTA-staged list capacity (elements)
 constexpr uint32_t kCtaWordCap = 1024; // CTA-staged bitset words capacity
 cudaError_t launch_pivot_units(const RowDesc* desc, const uint32_t* order, uint32_t n_heavy,
@@ -128,7 +137,6 @@ int pivot_grid(int device);  // persistent grid: SMs x resident CTAs of the pivo
 // ceil(j/64) words starting at word core_row_offset(j) (a lower-triangular
 // bitmap of the highest-degree rows, which degree ordering puts first).
 constexpr uint32_t kCoreMaxK = 262144;     // 4.3 GB of bits, the largest core a shape may ask for
-constexpr uint32_t kCoreDefaultK = 65536;  // 268 MB: the core of a matrix the tuner has not seen
 // Heavy pivots keep their elements below min(core_k, kCoreAndMax) as bits in
 // shared memory, to AND with core rows in that range.
 constexpr uint32_t kCoreAndMax = 65536;

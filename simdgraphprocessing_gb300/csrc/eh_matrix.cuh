@@ -51,9 +51,12 @@ struct Plan : SizeOrder {
   bool units_ready = false;
   uint2* units = nullptr;         // (order position, part)
   uint32_t n_units = 0;
+  const uint2* unit_list() const { return whole_large ? nullptr : units; }
   uint64_t units_cap = 0;
+  bool whole_large = false;       // no large pivot has two units: no list
   unsigned long long* core = nullptr;  // dense core bitmap (rows j < core_k)
   uint32_t core_k = 0;
+  bool core_ready = false;  // built, and waited for
 };
 
 constexpr uint32_t kMatrixCounters = 32, kFlagWord = 15, kQueueWord = 18;
@@ -88,9 +91,9 @@ struct Matrix {
   uint32_t* clique_scratch = nullptr;  // global slots for the largest clique pivots
   uint64_t clique_scratch_words = 0;
   // Work-shape parameters of the pivot kernel (set by the autotuner).
-  uint32_t light_max = kDefaultLightMax;
+  uint32_t light_max = 96;  // default_light_max(n) once built
   uint32_t unit_span = kDefaultUnitSpan;
-  uint32_t core_limit = kCoreDefaultK;  // rows in the dense core at most (0 = no core)
+  uint32_t core_limit = 0;              // rows in the dense core at most (default_core_rows(n) once built)
   bool is_batch = false;            // the union matrix of an eh_batch_t
   bool shape_set = false;           // a shape was given (eh_matrix_set_shape, the tuner): no cached shape
   // Where the matrix's buffers are read: one event per stream, recorded after
