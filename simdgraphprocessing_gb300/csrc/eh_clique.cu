@@ -274,8 +274,10 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, ui
 //    bit in a core row) and walks the e's, eight words in flight; a ballot per e
 //    gives a mask word, which lane e - e0 keeps and stores once per 16 e's.  That
 //    is about half the instructions of a warp per e, which recomputed every
-//    element's address for every e.  j >= core_k: a warp per e probes or streams
-//    row(j).
+//    element's address for every e.  j >= core_k: 8 lanes stream row(j) and find
+//    each element's position in a chained hash of the list (two or three words of
+//    shared memory, where a binary search took eight), or probe a longer row or
+//    another layout at the e elements.
 //  Phase 2: the sum over e and t in M[e] of popc(M[e] & M[t]).  A lane keeps the
 //    quad of M[t] for one t of 32, and the e's quads are broadcast: three LDS and
 //    a masked AND per word into a carry-save counter, whatever the density, no
@@ -292,7 +294,15 @@ __host__ __device__ __forceinline__ uint32_t quad_off(uint32_t e) {
 }
 
 __host__ __device__ constexpr uint32_t mid_slots(uint32_t c) { return (c + 31) & ~31u; }
-static uint32_t mid_bytes(uint32_t cmax) { return quad_off(cmax) * 16 + mid_slots(cmax) * (4 + 4 + 2); }
+// Heads of the list's hash chains: two per entry at least.
+__host__ __device__ inline uint32_t mid_heads(uint32_t cmax) {
+  uint32_t h = 128;
+  while (h < 2 * cmax) h *= 2;
+  return h;
+}
+static uint32_t mid_bytes(uint32_t cmax) {
+  return quad_off(cmax) * 16 + mid_slots(cmax) * (4 + 4 + 2 + 2) + mid_heads(cmax) * 4;
+}
 
 struct MaskSum {  // carry-save counter of 32-bit words
   uint32_t one, two, four, eights;
@@ -340,7 +350,11 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_mid(CliqueArgs a, uin
   uint32_t* m32 = reinterpret_cast<uint32_t*>(m4);
   uint32_t* list = reinterpret_cast<uint32_t*>(m4 + quad_off(cmax));
   uint32_t* off = list + mid_slots(cmax);  // word (32-bit) offset of core row A_i[e]
-  uint16_t* ro = reinterpret_cast<uint16_t*>(off + mid_slots(cmax));
+  constexpr uint32_t kNone = 0xffffu;
+  const uint32_t hmask = mid_heads(cmax) - 1;
+  uint32_t* head = off + mid_slots(cmax);  // first position of each chain (positions are below 2^16), or kNone
+  uint16_t* ro = reinterpret_cast<uint16_t*>(head + hmask + 1);
+  uint16_t* next = ro + mid_slots(cmax);
   const uint32_t* core32 = reinterpret_cast<const uint32_t*>(a.core);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long acc = 0;
@@ -363,6 +377,13 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_mid(CliqueArgs a, uin
     for (uint32_t k = threadIdx.x; k < c; k += kCtaThreads) ro[k] = (uint16_t)quad_off(k);
     __syncthreads();
     const uint32_t ea = lower_bound_u32(list, 0, c, a.core_k);
+    if (ea < c) {  // rows to stream: hash the list
+      for (uint32_t k = threadIdx.x; k <= hmask; k += kCtaThreads) head[k] = kNone;
+      __syncthreads();
+      for (uint32_t k = threadIdx.x; k < c; k += kCtaThreads)
+        next[k] = (uint16_t)atomicExch(&head[list[k] & hmask], k);
+      __syncthreads();
+    }
     // phase 1, j < core_k: tasks (32 t's from 32 r, 16 e's from 16 b), b >= 2 r
     const uint32_t nb = (ea + 15) >> 4;
     for (uint32_t r = 0, id = warp;;) {
@@ -400,26 +421,31 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_mid(CliqueArgs a, uin
       if (lane < 16 && e < ea && e > 32 * r) m32[4 * (uint32_t)ro[e] + r] = word;
       id += NW;
     }
-    // phase 1, j >= core_k: a warp per e
-    for (uint32_t e = max(1u, ea) + warp; e < c; e += NW) {
-      const uint32_t j = list[e];
+    // phase 1, j >= core_k: 8 lanes per e
+    const uint32_t sl = lane & 7;
+    for (uint32_t e = max(1u, ea) + 4 * warp + (lane >> 3); e < c; e += 4 * NW) {
       uint32_t* Me = m32 + 4 * (uint32_t)ro[e];
-      const RowView B = load_view(a.desc, a.arena, j);
-      if (B.card == 0) continue;
-      bool stream = false;
-      if (B.type == TY_UINT) stream = (uint64_t)B.card * ilog2p1_c(e) < (uint64_t)e * ilog2p1_c(B.card) * 4u;
-      else if (B.type == TY_PSHORT) stream = (uint64_t)B.card * ilog2p1_c(e) < (uint64_t)e * (B.aux + ilog2p1_c(B.card)) * 4u;
-      if (!stream) {
-        for (uint32_t b = 0; b < e; b += 32) {
-          const uint32_t t = b + lane;
-          const uint32_t word = __ballot_sync(FULL, t < e && row_contains(B, list[t]));
-          if (lane == 0) Me[b >> 5] = word;
+      const RowView B = load_view(a.desc, a.arena, list[e]);
+      if (B.type == TY_UINT && B.card <= kCliqueProbe * e) {
+        const uint4* p4 = static_cast<const uint4*>(B.p);
+        const uint32_t n4 = (B.card + 3) >> 2;  // padded with kUintPad
+        for (uint32_t q0 = sl; q0 < n4; q0 += 16) {
+          const uint4 pad = make_uint4(kUintPad, kUintPad, kUintPad, kUintPad);
+          const uint4 va = __ldg(p4 + q0), vb = q0 + 8 < n4 ? __ldg(p4 + q0 + 8) : pad;
+          const uint32_t y[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+          uint32_t at[8];
+#pragma unroll
+          for (int h = 0; h < 8; h++) at[h] = head[y[h] & hmask];
+#pragma unroll
+          for (int h = 0; h < 8; h++) {
+            uint32_t k = at[h];
+            while (k != kNone && list[k] != y[h]) k = next[k];
+            if (k < e) atomicOr(&Me[k >> 5], 1u << (k & 31));
+          }
         }
       } else {
-        warp_for_each(B, j, lane, [&](uint32_t y) {
-          const uint32_t t = lower_bound_u32(list, 0, e, y);
-          if (t < e && list[t] == y) atomicOr(&Me[t >> 5], 1u << (t & 31));
-        });
+        for (uint32_t t = sl; t < e; t += 8)
+          if (row_contains(B, list[t])) atomicOr(&Me[t >> 5], 1u << (t & 31));
       }
     }
     __syncthreads();
