@@ -66,7 +66,8 @@ __device__ __forceinline__ void put_tuple(const CliqueArgs& a, unsigned long lon
 }
 
 // ---- warp tier: |A_i| <= kCliqueWarpMax (64), one warp per pivot, two-word masks ----
-// Phase 1 sets bit t of M[e] for every pair with A_i[t] in row(A_i[e]):
+// Phase 1 sets bit t of M[e] for every pair with A_i[t] in row(A_i[e]); it has two forms,
+// find_masks by work area.  HashArea, for a matrix with a core:
 //  * j = A_i[e] < core_k: one lane per pair, two pairs in flight, a word of
 //    core row j each;
 //  * j >= core_k, a uint row: the row is streamed, 8 lanes per row and 16 bytes
@@ -74,112 +75,340 @@ __device__ __forceinline__ void put_tuple(const CliqueArgs& a, unsigned long lon
 //    is looked up in the list, which gives t;
 //  * other rows, and rows longer than kCliqueProbe e: the e elements below j
 //    are probed, 8 lanes per row.
-// Streaming reads a short row in one step where a probe per pair took a
-// descriptor and a binary search of dependent loads each.  In a batch of 256
-// graphs (37 M entries, rows of 18 on average) the two warp kernels that the
-// triangles and the 4-cliques of the pivots up to 32 entries took were 2.37 +
-// 1.78 ms.
+// RowsArea, for a batch of graphs, which has no core and all its pivots here.  The
+// rows are gathered by kind first, so that a warp's lanes stay together:
+//  * bitset rows: a lane per t, a row per step, four in flight: the row's word under
+//    x_t, a ballot, and a lane in 32 keeps it;
+//  * uint rows are streamed as one sequence of 16-byte quads, two per lane and step
+//    (rows of 17 entries on average, but of any length side by side), and each element
+//    x looked up in a hash table of the pivot: kSlots 16-bit entries, ten bits of the
+//    element stored there over its position, so that one shared-memory word answers
+//    nearly every miss and gives t for a hit (the list confirms it).  Entries whose
+//    slot another one took (18 entries: 0.15 of them) are compared with every x;
+//  * other rows, and uint rows longer than kCliqueProbe e: the e elements below j
+//    are probed, 4 lanes per row.
+// Both are bound by instruction issue (80% of the slots with RowsArea).  A batch of
+// 256 graphs (37 M entries, rows of 18 on average): 2.24 ms with HashArea, 15.7 of 32
+// lanes active, as nearly every step met a bitset row beside a uint one and a hit to
+// look up; 1.70 ms with RowsArea, 26.7 lanes.  Where a core answers most pairs HashArea
+// is the better one: 4-cliques of an R-MAT graph of 1 M vertices 0.340 against 0.347 ms
+// in this kernel, of 21,288 vertices 34 against 51 us in all, as the table's shared
+// memory (158 KB per SM against 51) keeps it from starting beside the larger pivots'
+// kernel.
 // Phase 2 counts (or lists) from the masks.  With `tri` set the same masks also
 // give the pivot's triangles (sum of popc M[e]).
 constexpr uint32_t kCliqueHash = 4096;
 constexpr uint32_t kCliqueProbe = 24;
+constexpr uint32_t kSlots = 1024;
+constexpr uint32_t kFreeSlot = 0x803fu;  // no t: bit 63 is past every row's masks
+__device__ __forceinline__ uint32_t slot_of(uint32_t x) { return (x * 0x9e3779b1u) >> 22; }
+__device__ __forceinline__ uint32_t slot_tag(uint32_t x) { return (x >> 4) & 0xffc0u; }
+
+// A warp's work area.
+struct HashArea {
+  // Draws from the queue a chunk ahead?  Not where that would set large pivots aside:
+  // planted cliques 2.33 against 2.25 ms, 4-cliques of 21,288 vertices 37 against 34 us.
+  static constexpr bool kAhead = false;
+  uint32_t bm[kCliqueHash / 32];
+  __device__ __forceinline__ void clear(uint32_t lane) {
+    for (uint32_t k = lane; k < kCliqueHash / 32; k += 32) bm[k] = 0u;
+  }
+};
+struct RowsArea {
+  static constexpr bool kAhead = true;
+  uint4 src[kCliqueWarpMax + 3];
+  uint16_t tab[kSlots];
+  uint8_t bit_e[kCliqueWarpMax];
+  __device__ __forceinline__ void clear(uint32_t lane) {
+    for (uint32_t k = lane; k < kSlots; k += 32) tab[k] = kFreeSlot;
+  }
+};
+
+// The masks of the pivot whose c entries are in list; the work area is clear again on return.
+__device__ __forceinline__ void find_masks(const CliqueArgs& a, HashArea& w, const uint32_t* list,
+                                           unsigned long long* mask, uint32_t c, uint32_t lane) {
+  uint32_t* bm = w.bm;
+  uint32_t* mask32 = reinterpret_cast<uint32_t*>(mask);
+  uint32_t ea = 0;  // entries below core_k
+#pragma unroll
+  for (uint32_t h = 0; h < kCliqueWarpMax; h += 32) {
+    const uint32_t e = h + lane, x = e < c ? list[e] : 0xffffffffu;
+    if (e < c) {
+      mask[e] = 0ull;
+      atomicOr(&bm[(x & (kCliqueHash - 1)) >> 5], 1u << (x & 31));
+    }
+    ea += __popc(__ballot_sync(FULL, x < a.core_k));
+  }
+  __syncwarp();
+  // j < core_k
+  const uint32_t pairs = ea * (ea - 1) / 2;
+  uint32_t e = 1, t = lane;
+  while (t >= e) { t -= e; e++; }
+  for (uint32_t q = lane; q < pairs; q += 64) {
+    const uint32_t e0 = e, t0 = t, j0 = list[e], x0 = list[t];
+    t += 32;
+    while (t >= e && e < c) { t -= e; e++; }
+    const bool two = q + 32 < pairs;
+    const uint32_t e1 = e, t1 = t, j1 = two ? list[e] : 0u, x1 = two ? list[t] : 0u;
+    t += 32;
+    while (t >= e && e < c) { t -= e; e++; }
+    const unsigned long long v0 = __ldg(a.core + core_row_offset(j0) + (x0 >> 6));
+    const unsigned long long v1 = two ? __ldg(a.core + core_row_offset(j1) + (x1 >> 6)) : 0ull;
+    if ((v0 >> (x0 & 63)) & 1ull) atomicOr(&mask32[2 * e0 + (t0 >> 5)], 1u << (t0 & 31));
+    if ((v1 >> (x1 & 63)) & 1ull) atomicOr(&mask32[2 * e1 + (t1 >> 5)], 1u << (t1 & 31));
+  }
+  // j >= core_k
+  const uint32_t sl = lane & 7, first = max(1u, ea) + (lane >> 3);
+  const auto source = [&](uint32_t r) { return __ldg(reinterpret_cast<const uint4*>(a.desc) + list[r]); };
+  uint4 next = make_uint4(0u, 0u, 0u, 0u);
+  if (first < c) next = source(first);
+  for (uint32_t r = first; r < c; r += 4) {
+    const uint4 d = next;
+    if (r + 4 < c) next = source(r + 4);
+    if ((d.w >> 30) == TY_UINT && d.y <= kCliqueProbe * r) {
+      const uint4* p4 = a.arena + d.x;
+      const uint32_t n4 = (d.y + 3) >> 2;  // padded with kUintPad
+      for (uint32_t q0 = sl; q0 < n4; q0 += 16) {
+        const uint4 pad = make_uint4(kUintPad, kUintPad, kUintPad, kUintPad);
+        const uint4 va = __ldg(p4 + q0), vb = q0 + 8 < n4 ? __ldg(p4 + q0 + 8) : pad;
+        const uint32_t y[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+        uint32_t hits = 0;
+#pragma unroll
+        for (int h = 0; h < 8; h++)
+          hits |= ((bm[(y[h] & (kCliqueHash - 1)) >> 5] >> (y[h] & 31)) & 1u) << h;
+        for (; hits; hits &= hits - 1) {
+          const uint32_t h = __ffs(hits) - 1;
+          uint32_t yy = y[0];
+#pragma unroll
+          for (int u = 1; u < 8; u++) yy = h == (uint32_t)u ? y[u] : yy;
+          const uint32_t pos = lower_bound_u32(list, 0, r, yy);
+          if (pos < r && list[pos] == yy) atomicOr(&mask32[2 * r + (pos >> 5)], 1u << (pos & 31));
+        }
+      }
+    } else {
+      RowView B;
+      B.p = a.arena + d.x;
+      B.card = d.y;
+      B.aux = d.z;
+      B.type = d.w >> 30;
+      B.len = d.w & 0x3fffffffu;
+      for (uint32_t u = sl; u < r; u += 8)
+        if (row_contains(B, list[u])) atomicOr(&mask32[2 * r + (u >> 5)], 1u << (u & 31));
+    }
+  }
+  __syncwarp();
+  for (uint32_t u = lane; u < c; u += 32) bm[(list[u] & (kCliqueHash - 1)) >> 5] = 0u;
+}
+
+__device__ __forceinline__ void find_masks(const CliqueArgs& a, RowsArea& w, const uint32_t* list,
+                                           unsigned long long* mask, uint32_t c, uint32_t lane) {
+  uint4* src = w.src;
+  uint16_t* tab = w.tab;
+  uint8_t* bit_e = w.bit_e;
+  uint32_t* mask32 = reinterpret_cast<uint32_t*>(mask);
+  // The entries by kind: uint rows in src[0, ns) (payload, first quad in the sequence, e),
+  // bitset rows in src[np, nr) (payload, first 32-bit word, words) and three empty ones, the others between (e).
+  uint4 d[2];
+  uint32_t kind[2] = {0u, 0u}, quads[2] = {0u, 0u}, lost[2] = {0u, 0u};  // entries whose slot another one took
+#pragma unroll
+  for (uint32_t h = 0; h < 2; h++) {
+    const uint32_t e = 32 * h + lane;
+    if (e < c) {
+      const uint32_t x = list[e];
+      mask[e] = 0ull;
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.desc) + x);
+      const uint32_t type = v.w >> 30;
+      if (type == TY_BITSET) {
+        d[h] = make_uint4(v.x, 0u, 2 * v.z, 2 * (v.w & 0x3fffffffu));
+        kind[h] = 3;
+      } else {
+        d[h] = make_uint4(v.x, v.y, e, 0u);
+        kind[h] = type == TY_UINT && v.y <= kCliqueProbe * e ? 1 : 2;
+        if (kind[h] == 1) quads[h] = (v.y + 3) >> 2;  // padded with kUintPad
+      }
+      if (e == 0 || (kind[h] == 1 && quads[h] == 0)) kind[h] = quads[h] = 0;
+    }
+    if (c <= 32) break;
+  }
+  // The hash table and the sequence of quads, if there are uint rows.
+  uint32_t start[2] = {0xffffffffu, 0xffffffffu}, total = 0;
+  if (__any_sync(FULL, quads[0] + quads[1])) {
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+      const uint32_t e = 32 * h + lane;
+      if (e < c) {
+        const uint32_t x = list[e];
+        tab[slot_of(x)] = (uint16_t)(slot_tag(x) | e);
+      }
+      const uint32_t s = total + warp_exclusive_scan(quads[h], lane);
+      total = __shfl_sync(FULL, s + quads[h], 31);
+      if (quads[h]) start[h] = d[h].y = s;
+      if (c <= 32) break;
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+      const uint32_t e = 32 * h + lane;
+      lost[h] = __ballot_sync(FULL, e < c && (tab[slot_of(list[e])] & 63u) != e);
+      if (c <= 32) break;
+    }
+  }
+  uint32_t ns = 0, np = 0, np1 = 0, nr = 0;  // np1: the first bit row of an entry past 31
+#pragma unroll
+  for (uint32_t k = 1; k <= 3; k++) {
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+      const uint32_t bits = __ballot_sync(FULL, kind[h] == k), at = nr + __popc(bits & ((1u << lane) - 1u));
+      if (kind[h] == k) {
+        src[at] = d[h];
+        if (k == 3) bit_e[at] = (uint8_t)(32 * h + lane);
+      }
+      nr += __popc(bits);
+      if (k == 3 && h == 0) np1 = nr;
+      if (c <= 32) break;
+    }
+    if (k == 1) ns = nr;
+    if (k == 2) np = nr;
+  }
+  if (lane < 3) src[nr + lane] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  // bitset rows
+#pragma unroll 1
+  for (uint32_t h = 0; h < 2 && 32 * h < c; h++) {
+    const uint32_t t = 32 * h + lane, x = t < c ? list[t] : 0u, xw = x >> 5, sh = x & 31;
+#pragma unroll 1
+    for (uint32_t i0 = h ? np1 : np; i0 < nr; i0 += 32) {
+      uint32_t keep = 0;
+      const uint32_t iend = min(nr - i0, 32u);
+      for (uint32_t i = 0; i < iend; i += 4) {
+        uint32_t v[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+          const uint4 b = src[i0 + i + u];
+          const uint32_t* words = reinterpret_cast<const uint32_t*>(a.arena + b.x);
+          v[u] = xw - b.z < b.w ? __ldg(words + (xw - b.z)) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+          const uint32_t m = __ballot_sync(FULL, (v[u] >> sh) & 1u);
+          if (lane == i + u) keep = m;
+        }
+      }
+      if (lane < iend) {
+        const uint32_t e = bit_e[i0 + lane];  // bits t < e
+        if (h) mask32[2 * e + 1] = keep & ((1u << (e - 32)) - 1u);
+        else mask32[2 * e] = e < 32 ? keep & ((1u << e) - 1u) : keep;
+      }
+    }
+  }
+  // uint rows
+  const uint32_t upto = (2u << lane) - 1u;
+  uint32_t rows = 0xffffffffu;  // the last row that starts before the step
+  for (uint32_t q0 = 0; q0 < total; q0 += 64) {
+    uint32_t e[2], y[8], at[8], least = 64;
+#pragma unroll
+    for (int v = 0; v < 2; v++) {
+      const uint32_t first = q0 + 32 * v, q = first + lane;
+      const uint32_t begins = __reduce_or_sync(FULL, __funnelshift_lc(0u, 1u, start[0] - first) |
+                                                         __funnelshift_lc(0u, 1u, start[1] - first));
+      const uint4 b = src[rows + __popc(begins & upto)];
+      rows += __popc(begins);
+      uint4 w = make_uint4(kUintPad, kUintPad, kUintPad, kUintPad);
+      if (q < total) w = __ldg(a.arena + b.x + (q - b.y));
+      e[v] = b.z;
+      y[4 * v] = w.x;
+      y[4 * v + 1] = w.y;
+      y[4 * v + 2] = w.z;
+      y[4 * v + 3] = w.w;
+    }
+#pragma unroll
+    for (int h = 0; h < 8; h++) {
+      at[h] = tab[slot_of(y[h])] ^ slot_tag(y[h]);
+      least = min(least, at[h]);
+    }
+    uint32_t m[4] = {0u, 0u, 0u, 0u};  // the quads' masks, low and high words
+    if (least < 64) {
+#pragma unroll
+      for (int h = 0; h < 8; h++)
+        if (at[h] < 64 && list[at[h]] == y[h]) {
+          m[h >> 2] |= __funnelshift_lc(0u, 1u, at[h]);  // 0 from 32 on
+          m[2 + (h >> 2)] |= __funnelshift_lc(0u, 1u, at[h] - 32u);
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+      for (uint32_t o = lost[g]; o; o &= o - 1) {
+        const uint32_t pos = __ffs((int)o) - 1, x = list[32 * g + pos];
+#pragma unroll
+        for (int h = 0; h < 8; h++) m[2 * g + (h >> 2)] |= y[h] == x ? 1u << pos : 0u;
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 2; v++) {  // bits t < e
+      if (m[v]) atomicOr(&mask32[2 * e[v]], m[v] & (__funnelshift_lc(0u, 1u, e[v]) - 1u));
+      if (m[2 + v] && e[v] > 32) atomicOr(&mask32[2 * e[v] + 1], m[2 + v] & ((1u << (e[v] - 32)) - 1u));
+    }
+  }
+  // the other rows, eight at a time
+  const uint32_t sl = lane & 3;
+  for (uint32_t i0 = ns; i0 < np; i0 += 8) {
+    const uint32_t i = i0 + (lane >> 2);
+    unsigned long long m = 0;
+    uint32_t r = 0;
+    if (i < np) {
+      r = src[i].z;
+      const RowView B = load_view(a.desc, a.arena, list[r]);
+      for (uint32_t u = sl; u < r; u += 4)
+        if (row_contains(B, list[u])) m |= 1ull << u;
+    }
+    m |= __shfl_xor_sync(FULL, m, 1);
+    m |= __shfl_xor_sync(FULL, m, 2);
+    if (sl == 0 && r) mask[r] = m;
+  }
+  __syncwarp();
+  if (total)
+    for (uint32_t u = lane; u < c; u += 32) tab[slot_of(list[u])] = kFreeSlot;
+}
 
 // LIST: write the k = 3 or 4 cliques as tuples instead of counting them.
-template <bool LIST>
+template <bool LIST, class Area>
 __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, uint32_t pos_begin, uint32_t pos_end,
                                                                 uint32_t grab, uint32_t* counter) {
   __shared__ unsigned long long s_mask[NW][kCliqueWarpMax];
   __shared__ uint32_t s_list[NW][kCliqueWarpMax];
-  __shared__ uint32_t s_bm[NW][kCliqueHash / 32];
+  __shared__ Area s_work[NW];
   overlap_begin();
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* list = s_list[warp];
-  uint32_t* bm = s_bm[warp];
+  Area& work = s_work[warp];
   unsigned long long* mask = s_mask[warp];
   uint32_t* mask32 = reinterpret_cast<uint32_t*>(mask);
   const int top = (int)a.k - 3;  // DFS depth at which a popcount finishes the count
-  for (uint32_t k = lane; k < kCliqueHash / 32; k += 32) bm[k] = 0u;
+  work.clear(lane);
   unsigned long long acc = 0, tacc = 0;
+  const bool ahead = Area::kAhead && grab > 1;
+  uint32_t drawn = 0;
+  if (lane == 0 && ahead) drawn = atomicAdd(counter, grab);
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(counter, grab);
-    base = __shfl_sync(FULL, base, 0) + pos_begin;
+    if (lane == 0 && !ahead) drawn = atomicAdd(counter, grab);
+    const uint32_t base = __shfl_sync(FULL, drawn, 0) + pos_begin;
     if (base >= pos_end) break;
+    if (lane == 0 && ahead) drawn = atomicAdd(counter, grab);
     const uint32_t end = min(pos_end, base + grab);
+    const uint32_t my_row = base + lane < end ? a.order[base + lane] : a.order[base];
+    const uint4 my_desc = __ldg(reinterpret_cast<const uint4*>(a.desc) + my_row);
     for (uint32_t p = base; p < end; p++) {
-      const uint32_t row = a.order[p];
-      const RowView A = load_view(a.desc, a.arena, row);
+      const uint32_t row = __shfl_sync(FULL, my_row, p - base);
+      RowView A;
+      A.p = a.arena + __shfl_sync(FULL, my_desc.x, p - base);
+      A.card = __shfl_sync(FULL, my_desc.y, p - base);
+      A.aux = __shfl_sync(FULL, my_desc.z, p - base);
+      A.len = __shfl_sync(FULL, my_desc.w, p - base);
+      A.type = A.len >> 30;
+      A.len &= 0x3fffffffu;
       const uint32_t c = A.card;
       warp_decode(A, list, lane);
-      uint32_t ea = 0;  // entries below core_k
-#pragma unroll
-      for (uint32_t h = 0; h < kCliqueWarpMax; h += 32) {
-        const uint32_t e = h + lane, x = e < c ? list[e] : 0xffffffffu;
-        if (e < c) {
-          mask[e] = 0ull;
-          atomicOr(&bm[(x & (kCliqueHash - 1)) >> 5], 1u << (x & 31));
-        }
-        ea += __popc(__ballot_sync(FULL, x < a.core_k));
-      }
-      __syncwarp();
-      // phase 1, j < core_k
-      const uint32_t pairs = ea * (ea - 1) / 2;
-      uint32_t e = 1, t = lane;
-      while (t >= e) { t -= e; e++; }
-      for (uint32_t q = lane; q < pairs; q += 64) {
-        const uint32_t e0 = e, t0 = t, j0 = list[e], x0 = list[t];
-        t += 32;
-        while (t >= e && e < c) { t -= e; e++; }
-        const bool two = q + 32 < pairs;
-        const uint32_t e1 = e, t1 = t, j1 = two ? list[e] : 0u, x1 = two ? list[t] : 0u;
-        t += 32;
-        while (t >= e && e < c) { t -= e; e++; }
-        const unsigned long long v0 = __ldg(a.core + core_row_offset(j0) + (x0 >> 6));
-        const unsigned long long v1 = two ? __ldg(a.core + core_row_offset(j1) + (x1 >> 6)) : 0ull;
-        if ((v0 >> (x0 & 63)) & 1ull) atomicOr(&mask32[2 * e0 + (t0 >> 5)], 1u << (t0 & 31));
-        if ((v1 >> (x1 & 63)) & 1ull) atomicOr(&mask32[2 * e1 + (t1 >> 5)], 1u << (t1 & 31));
-      }
-      // phase 1, j >= core_k
-      const uint32_t sl = lane & 7, first = max(1u, ea) + (lane >> 3);
-      const auto source = [&](uint32_t r) { return __ldg(reinterpret_cast<const uint4*>(a.desc) + list[r]); };
-      uint4 next = make_uint4(0u, 0u, 0u, 0u);
-      if (first < c) next = source(first);
-      for (uint32_t r = first; r < c; r += 4) {
-        const uint4 d = next;
-        if (r + 4 < c) next = source(r + 4);
-        if ((d.w >> 30) == TY_UINT && d.y <= kCliqueProbe * r) {
-          const uint4* p4 = a.arena + d.x;
-          const uint32_t n4 = (d.y + 3) >> 2;  // padded with kUintPad
-          for (uint32_t q0 = sl; q0 < n4; q0 += 16) {
-            const uint4 pad = make_uint4(kUintPad, kUintPad, kUintPad, kUintPad);
-            const uint4 va = __ldg(p4 + q0), vb = q0 + 8 < n4 ? __ldg(p4 + q0 + 8) : pad;
-            const uint32_t y[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-            uint32_t hits = 0;
-#pragma unroll
-            for (int h = 0; h < 8; h++)
-              hits |= ((bm[(y[h] & (kCliqueHash - 1)) >> 5] >> (y[h] & 31)) & 1u) << h;
-            for (; hits; hits &= hits - 1) {
-              const uint32_t h = __ffs(hits) - 1;
-              uint32_t yy = y[0];
-#pragma unroll
-              for (int u = 1; u < 8; u++) yy = h == (uint32_t)u ? y[u] : yy;
-              const uint32_t pos = lower_bound_u32(list, 0, r, yy);
-              if (pos < r && list[pos] == yy) atomicOr(&mask32[2 * r + (pos >> 5)], 1u << (pos & 31));
-            }
-          }
-        } else {
-          RowView B;
-          B.p = a.arena + d.x;
-          B.card = d.y;
-          B.aux = d.z;
-          B.type = d.w >> 30;
-          B.len = d.w & 0x3fffffffu;
-          for (uint32_t u = sl; u < r; u += 8)
-            if (row_contains(B, list[u])) atomicOr(&mask32[2 * r + (u >> 5)], 1u << (u & 31));
-        }
-      }
-      __syncwarp();
-      for (uint32_t u = lane; u < c; u += 32) bm[(list[u] & (kCliqueHash - 1)) >> 5] = 0u;
+      find_masks(a, work, list, mask, c, lane);
       // phase 2: a lane takes the cliques whose two largest members are i and A_i[e]
       if (LIST) {
         for (uint32_t h = 0; h < c; h += 32) {
@@ -211,7 +440,14 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, ui
       }
       unsigned long long pc = 0;
       uint32_t tc = 0;
-      for (uint32_t ee = lane; ee < c; ee += 32) {
+      if (c <= 32 && top <= 1) {
+        const uint32_t m0 = lane < c ? mask32[2 * lane] : 0u;
+        tc = __popc(m0);
+        uint32_t n = 0;
+        for (uint32_t m = top == 1 ? m0 : 0u; m; m &= m - 1) n += __popc(m0 & mask32[2 * (__ffs(m) - 1)]);
+        pc = n;
+      }
+      for (uint32_t ee = c <= 32 && top <= 1 ? c : lane; ee < c; ee += 32) {
         const unsigned long long m0 = mask[ee];
         tc += __popcll(m0);
         if (top == 1) {
@@ -753,7 +989,10 @@ cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t
   const uint32_t n = pos_end - pos_begin, warps = 5u * NW * (uint32_t)std::max(1, sms);
   const uint32_t grab = std::max(1u, std::min(4u, n / (16 * warps)));
   const unsigned grid = std::max(1u, std::min(5u * (uint32_t)std::max(1, sms), (n + NW * grab - 1) / (NW * grab)));
-  return launch_overlapped(list ? k_clique_warp<true> : k_clique_warp<false>, grid, kCtaThreads, 0, st, overlap, a,
+  // The batch's form where there is no core (see above).
+  const auto kernel = list ? k_clique_warp<true, HashArea>
+                           : a.core ? k_clique_warp<false, HashArea> : k_clique_warp<false, RowsArea>;
+  return launch_overlapped(kernel, grid, kCtaThreads, 0, st, overlap, a,
                            pos_begin, pos_end, grab, counter);
 }
 
