@@ -992,7 +992,7 @@ cudaError_t launch_clique_warp(const CliqueArgs& a, uint32_t pos_begin, uint32_t
   // The batch's form where there is no core (see above).
   const auto kernel = list ? k_clique_warp<true, HashArea>
                            : a.core ? k_clique_warp<false, HashArea> : k_clique_warp<false, RowsArea>;
-  return launch_overlapped(kernel, grid, kCtaThreads, 0, st, overlap, a,
+  return launch_overlapped(kernel, grid, kCtaThreads, 0, st, overlap, 0, a,
                            pos_begin, pos_end, grab, counter);
 }
 
@@ -1011,7 +1011,7 @@ cudaError_t launch_clique_mid(const CliqueArgs& a, uint32_t pos_begin, uint32_t 
   }
   const uint32_t bytes = mid_bytes(cmax), per = std::max(1u, std::min(5u, (228u << 10) / (bytes + 2048)));
   const unsigned grid = std::min<unsigned>(pos_end - pos_begin, per * (unsigned)std::max(1, sms));
-  return launch_overlapped(k_clique_mid, grid, kCtaThreads, bytes, st, overlap, a, pos_begin, pos_end, counter, cmax);
+  return launch_overlapped(k_clique_mid, grid, kCtaThreads, bytes, st, overlap, 0, a, pos_begin, pos_end, counter, cmax);
 }
 
 template <bool LIST>

@@ -1037,6 +1037,13 @@ static cudaError_t allow_smem(const void* kernel, uint32_t bytes, std::atomic<bo
   return e;
 }
 
+// Kernels that ask for different splits of L1 and shared memory do not run on an SM
+// at the same time, and a short call is mostly the tails of its tiers: below
+// kSplitRows rows, if there are several, all ask for the whole of it.  R-MAT, 14 edges a vertex, uint: 60 K
+// vertices 46.9 -> 43.4 us, 130 K 80.5 -> 79.3 (hybrid 90.3 -> 86.7), 260 K even; above
+// that L1 counts for more (520 K 247 -> 270, 1 M 544 -> 623).
+constexpr uint64_t kSplitRows = 196608;
+
 static uint32_t cap_of(uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); }
 
 // One launch of k_pivots_cta: n units, or order[pos0, pos0 + n) whole.
@@ -1055,13 +1062,14 @@ struct CtaLaunch {
     grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(n, resident_grid(device, bytes, per)));
   }
   cudaError_t run(const PivotArgs& a, const uint2* units, uint32_t* next, int device, cudaStream_t st,
-                  bool& overlap) const {
+                  unsigned split, bool& overlap) const {
     if (!n) return cudaSuccess;
     static std::atomic<bool> done[64];
     cudaError_t e = allow_smem((const void*)k_pivots_cta<NW, MODE>, slice_bytes<NW, MODE>(kCtaListCap, kCtaWindow),
                                done, device);
     if (e != cudaSuccess) return e;
-    e = launch_overlapped(k_pivots_cta<NW, MODE>, grid, NW * 32, bytes, st, overlap, a, units, n, pos0, next, cap, win);
+    e = launch_overlapped(k_pivots_cta<NW, MODE>, grid, NW * 32, bytes, st, overlap, split, a, units, n, pos0, next,
+                          cap, win);
     overlap = true;
     return e;
   }
@@ -1100,20 +1108,21 @@ static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_uni
   a.ctas = g_heavy + large.grid + mid.grid + (unsigned)gw;
   if (a.ctas == 0)  // no row with a pair
     return a.graph_rows ? cudaSuccess : cudaMemsetAsync(a.out, 0, (a.report ? 2 : 1) * sizeof(unsigned long long), st);
+  const unsigned split = a.n < kSplitRows && g_heavy + large.grid + mid.grid ? 100u : 0u;
   bool overlap = false;
   if (g_heavy) {
-    e = launch_overlapped(k_pivots_heavy<MODE == kFull>, g_heavy, kCtaThreads, 0, st, false, a, units, n_units);
+    e = launch_overlapped(k_pivots_heavy<MODE == kFull>, g_heavy, kCtaThreads, 0, st, false, split, a, units, n_units);
     overlap = true;
   }
-  if (e == cudaSuccess) e = large.run(a, units, a.queue + 2, device, st, overlap);
-  if (e == cudaSuccess) e = mid.run(a, nullptr, a.queue + 4, device, st, overlap);
+  if (e == cudaSuccess) e = large.run(a, units, a.queue + 2, device, st, split, overlap);
+  if (e == cudaSuccess) e = mid.run(a, nullptr, a.queue + 4, device, st, split, overlap);
   if (e == cudaSuccess && gw) {
     static std::atomic<bool> done[64];
     e = allow_smem((const void*)k_pivots_warp<MODE>, NWARPS * slice_bytes<1, MODE>(kLightMax, kWarpWindow), done,
                    device);
     if (e == cudaSuccess)
-      e = launch_overlapped(k_pivots_warp<MODE>, (unsigned)gw, kCtaThreads, bytes, st, overlap, a, mid1, mid_chunk,
-                            tiny_grab, cap, win);
+      e = launch_overlapped(k_pivots_warp<MODE>, (unsigned)gw, kCtaThreads, bytes, st, overlap, split, a, mid1,
+                            mid_chunk, tiny_grab, cap, win);
   }
   // A launch that failed leaves the others short of the last CTA: clear the queue for the next call.
   if (e != cudaSuccess) cudaMemsetAsync(a.queue, 0, kPivotQueueWords * sizeof(uint32_t), st);

@@ -60,21 +60,30 @@ constexpr uint32_t kUintPad = 0xffffffffu;
 // (launch_overlapped): every CTA lets the next kernel's CTAs start as room frees
 // up (overlap_begin) and a kernel's CTAs leave only after the kernel before has
 // finished (overlap_end), so that whatever follows in the stream waits for all.
+// carveout: percent of an SM's L1 that the launch prefers as shared memory, 0 for
+// the runtime's choice by the launch's own need.
 __device__ __forceinline__ void overlap_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void overlap_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... Params, class... Args>
 inline cudaError_t launch_overlapped(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem,
-                                     cudaStream_t st, bool overlap, Args... args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+                                     cudaStream_t st, bool overlap, unsigned carveout, Args... args) {
+  cudaLaunchAttribute attr[2];
+  unsigned attrs = 0;
+  if (overlap) {
+    attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (carveout) {
+    attr[attrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[attrs++].val.sharedMemCarveout = carveout;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
+  cfg.numAttrs = attrs;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
