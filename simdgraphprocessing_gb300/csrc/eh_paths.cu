@@ -1,10 +1,11 @@
 // Apps over directed graphs: symbiosity (apps/symbiosity.cpp) and the n_path
 // breadth-first search (apps/n_path.cpp).
 //
-// symbiosity: one warp per row i intersects out(i) (the row matrix) with in(i)
-// (the column matrix) and tests the Jaccard ratio in double precision, as
-// symbiosity.cpp:46-58 does.  Short rows take a lane each, longer ones a warp; rows too
-// long for a warp (hubs) are listed and taken one per CTA, a slice per warp.
+// symbiosity: for each row i, out(i) (the row matrix) is intersected with in(i)
+// (the column matrix) and the Jaccard ratio tested as symbiosity.cpp:46-58 does in
+// double precision (here exactly, in integers).  Short rows take a lane each, longer
+// ones a warp; rows too long for a warp (hubs) are listed first and taken one per CTA, a
+// slice per warp.
 //
 // n_path: level-synchronous BFS on a visited bitset of (n + 64) / 64 words,
 // the reference's bs_size (n_path.cpp:45-53).  A level is two launches:
@@ -141,20 +142,37 @@ __device__ __forceinline__ uint32_t block_merge(const uint32_t* A, uint32_t na, 
   return c;
 }
 
+// Lists the rows whose intersection CTAs take (sym_heavy).  A kernel of its own, so that
+// those rows come first and k_symbiosity fills the GPU as they run out: with the list made
+// by k_symbiosity the two ran one after the other (half-reciprocal R-MAT scale 21, hybrid:
+// 328 against 299 us a call, 50,000 vertices 65 against 56).  Bound by reading the row
+// descriptors; the column matrix is only looked at where the row's own size allows a heavy pair.
+__global__ void k_symbiosity_find(uint32_t n, const RowDesc* __restrict__ dr, const uint4* __restrict__ ar,
+                                  const RowDesc* __restrict__ dc, const uint4* __restrict__ ac, SymTest test,
+                                  uint32_t* heavy, uint32_t* n_heavy) {
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
+    const RowView A = load_view(dr, ar, (uint32_t)r);
+    // Uint rows: the larger above kSymMerge and within 32 x of the smaller, or the smaller above kSymLight.
+    if (A.type != TY_BITSET && A.card <= kSymMerge / 32) continue;
+    const RowView B = load_view(dc, ac, (uint32_t)r);
+    if (sym_heavy(A, B) && sym_above(min(A.card, B.card), A, B, test)) heavy[atomicAdd(n_heavy, 1u)] = (uint32_t)r;
+  }
+}
+
 // Rows are taken kSymChunk at a time from a shared cursor, one row per lane.  A
 // row that could not pass with min(|out|, |in|) common entries is not read (the
 // ratio grows with their number).  Two uint rows of at most kSymTiny entries are
 // merged by the lane alone, longer ones and the other layouts go to the warp,
-// rows too long for a warp to the list of k_symbiosity_heavy.  Half-reciprocal
-// R-MAT scale 21, hybrid: 223 us here (latency of the lane merges and of the
-// warp rows' first blocks, about equal) and 74 us for the listed rows, where
-// binary searches in a staged row took 335 us; both together 538 -> 305 us a call.
+// rows too long for a warp are k_symbiosity_heavy's.  Half-reciprocal R-MAT scale 21,
+// hybrid: 223 us here (latency of the lane merges and of the warp rows' first
+// blocks, about equal) and 74 us for the listed rows, where binary searches in a
+// staged row took 335 us; 541 -> 299 us a call with the two overlapped.
 __global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc* __restrict__ dr,
                                                     const uint4* __restrict__ ar, const RowDesc* __restrict__ dc,
                                                     const uint4* __restrict__ ac, SymTest test,
-                                                    unsigned long long* out, uint32_t* heavy, uint32_t* n_heavy,
-                                                    uint32_t* cursor) {
+                                                    unsigned long long* out, uint32_t* cursor) {
   __shared__ PshortHdr s_hdr[8];
+  overlap_begin();
   const uint32_t lane = threadIdx.x & 31;
   unsigned long long acc = 0;
   const uint32_t chunks = (n + kSymChunk - 1) / kSymChunk;
@@ -185,7 +203,7 @@ __global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc
                                           static_cast<const uint32_t*>(B.p), B.card);
         acc += sym_above(both, A, B, test);
       } else if (sym_heavy(A, B)) {
-        heavy[atomicAdd(n_heavy, 1u)] = (uint32_t)r;
+        // in the list
       } else {
         warp_row = true;
       }
@@ -214,9 +232,10 @@ __global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc
   }
   acc = warp_sum_u64(acc);
   if (lane == 0 && acc) atomicAdd(out, acc);
+  overlap_end();
 }
 
-// The heavy rows of k_symbiosity, one CTA per row taken from a shared cursor.
+// The listed rows, one CTA per row taken from a shared cursor.
 __global__ void __launch_bounds__(256) k_symbiosity_heavy(const RowDesc* __restrict__ dr, const uint4* __restrict__ ar,
                                                           const RowDesc* __restrict__ dc, const uint4* __restrict__ ac,
                                                           SymTest test, unsigned long long* out,
@@ -224,6 +243,7 @@ __global__ void __launch_bounds__(256) k_symbiosity_heavy(const RowDesc* __restr
                                                           const uint32_t* n_heavy, uint32_t* cursor) {
   __shared__ uint32_t s_sum[8];
   __shared__ uint32_t s_idx;
+  overlap_begin();
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const uint32_t nh = *n_heavy;
   unsigned long long acc = 0;
@@ -492,13 +512,16 @@ extern "C" eh_status eh_symbiosity_async(eh_matrix_t rh, eh_matrix_t ch, double 
     const uint64_t g = std::min<uint64_t>((r->n + 8 * kSymChunk - 1) / (8 * kSymChunk), (uint64_t)sms * 8);
     unsigned long long* out = reinterpret_cast<unsigned long long*>(d_count);
     const SymTest test = sym_test(threshold);
-    k_symbiosity<<<(unsigned)std::max<uint64_t>(g, 1), 256, 0, st>>>((uint32_t)r->n, r->desc, r->arena, c->desc,
-                                                                     c->arena, test, out, scratch, counts,
-                                                                     counts + 2);
+    const unsigned blocks = (unsigned)std::min<uint64_t>((r->n + 255) / 256, (uint64_t)sms * 8);
+    k_symbiosity_find<<<blocks, 256, 0, st>>>((uint32_t)r->n, r->desc, r->arena, c->desc, c->arena, test, scratch,
+                                              counts);
     k_symbiosity_heavy<<<(unsigned)(sms * std::max(per, 1)), 256, 0, st>>>(r->desc, r->arena, c->desc, c->arena,
                                                                            test, out, scratch, counts,
                                                                            counts + 1);
-    e = cudaGetLastError();
+    e = launch_overlapped(k_symbiosity, (unsigned)std::max<uint64_t>(g, 1), 256, 0, st, true, 0, (uint32_t)r->n,
+                          r->desc, r->arena, c->desc, c->arena, test, out, counts + 2);
+    const cudaError_t el = cudaGetLastError();
+    if (e == cudaSuccess) e = el;
   }
   const cudaError_t ef = cudaFreeAsync(scratch, st);
   if (e == cudaSuccess) e = ef;
