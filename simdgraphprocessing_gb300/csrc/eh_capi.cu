@@ -437,6 +437,7 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
   a.report = false;
   a.out = out;
   a.unit_span = m->plan.unit_span;
+  a.long_rows = m->layout != EH_LAYOUT_HYBRID && m->layout != EH_LAYOUT_UINTEGER;
   a.graph_rows = nullptr;
   a.num_graphs = 0;
   a.core = m->plan.core;

@@ -354,12 +354,44 @@ __device__ __forceinline__ void add_planes(uint32_t (&plane)[2][kPlanes], const 
   }
 }
 
+// This lane's part (of 8: sl) of the members of a pivot, as bm and jc hold them, in a
+// pshort row of u16 stream h, below j unless kTri; kSym: the sum of we + |A_y| over
+// them.  Partition by partition, where a probe walks the headers for each of the
+// pivot's elements (R-MAT scale 22, pshort: 8.06 -> 7.05 ms a count).  Out of line: in
+// it, the uint rows' loop loses 2%.
+template <int MODE>
+__device__ __noinline__ unsigned long long pshort_hits(const uint16_t* h, uint32_t len, uint32_t sl, uint32_t j,
+                                                       const uint32_t* bm, const uint2* jc, uint32_t c, uint32_t base,
+                                                       uint32_t win, uint32_t we, const RowDesc* desc) {
+  unsigned long long sum = 0;
+  for (uint32_t i = 0; i < len;) {
+    const uint32_t hb = (uint32_t)h[i] << 16, m = (uint32_t)h[i + 1] + 1;
+    if (MODE != kTri && hb >= j) break;
+    for (uint32_t k = sl; k < m; k += 8) {
+      const uint32_t y = hb | h[i + 2 + k], dy = y - base, at = dy < win ? dy : win + (y & (kHashBits - 1));
+      if (!((bm[at >> 5] >> (y & 31)) & 1u) || (MODE != kTri && y >= j)) continue;
+      if (dy >= win) {
+        uint32_t lo = 0, hi = c;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (jc[mid].y < y) lo = mid + 1;
+          else hi = mid;
+        }
+        if (lo == c || jc[lo].y != y) continue;
+      }
+      sum += MODE == kSym ? (unsigned long long)we + desc[y].card : 1ull;
+    }
+    i += m + 2;
+  }
+  return sum;
+}
+
 // This lane's part of the count of pivot i's pairs e in [e0, e1), by a group
 // of NW warps (gw: this warp's index in it): the returned count plus what went
 // into `sum`; kSym: everything goes into `wsum`, weighted.  But for kTri the rows
 // are full ones, which hold elements >= j too.  The group's slice is free for the
 // next pivot on return, bm zero.
-template <int NW, int MODE>
+template <int NW, int MODE, bool LONG>
 __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowView& A, uint32_t e0, uint32_t e1,
                                                 const Slice& s, uint32_t win, uint32_t* scan, uint32_t lane,
                                                 uint32_t gw, WordSum& sum, uint32_t card_i,
@@ -371,7 +403,7 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
     s.jc[k] = make_uint2(x < core_k ? core_offset32(x) : 0u, x);
     if (SYM) s.wt[k] = card_i + a.desc[x].card;
   };
-  if (NW == 1) warp_decode_to(A, lane, put);
+  if (NW == 1) warp_decode_to<LONG>(A, lane, put);
   else cta_decode_to<NW * 32>(A, scan, put);
   uint32_t* word32 = reinterpret_cast<uint32_t*>(s.word);
   if (NW > 1)
@@ -547,6 +579,13 @@ __device__ __forceinline__ uint32_t pivot_count(const PivotArgs& a, const RowVie
             }
           }
           n = 0;
+        } else if (LONG && type == TY_PSHORT && n <= kProbeRatio * e) {
+          const unsigned long long hits =
+              pshort_hits<MODE>(reinterpret_cast<const uint16_t*>(p), d.w & 0x3fffffffu, sl, j, s.bm, s.jc, c, base, win,
+                                SYM ? s.wt[e] : 0u, a.desc);
+          if (SYM) wsum += hits;
+          else cnt += (uint32_t)hits;
+          n = 0;
         } else if (type != TY_UINT || n > kProbeRatio * e) {
           const RowView B = load_view(a.desc, a.arena, j);
           for (uint32_t t = sl; t < e; t += 8) {
@@ -651,7 +690,7 @@ __device__ __forceinline__ void keep_below(const PivotArgs& a, RowView& A, uint3
 // L1 and have few warps at a barrier: large pivots as units of unit_span
 // positions (units; the giants' are k_pivots_heavy's) where some have more, or
 // a range of the order from pos0 on whole (units null).
-template <int NW, int MODE>
+template <int NW, int MODE, bool LONG>
 __global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivots_cta(PivotArgs a, const uint2* __restrict__ units,
                                                                uint32_t n_units, uint32_t pos0, uint32_t* counter,
                                                                uint32_t cap, uint32_t win) {
@@ -677,7 +716,7 @@ __global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivo
     const uint32_t card = A.card;
     if (MODE == kSym) keep_below(a, A, i);
     const uint32_t e0 = 1 + uu.y * a.unit_span, e1 = units ? min(A.card, e0 + a.unit_span) : A.card;
-    const uint32_t cnt = pivot_count<NW, MODE>(a, A, e0, e1, s, win, s_scan, lane, warp, sum, card, acc);
+    const uint32_t cnt = pivot_count<NW, MODE, LONG>(a, A, e0, e1, s, win, s_scan, lane, warp, sum, card, acc);
     acc += finish_pivot<MODE>(a, i, card, cnt, sum, lane);
   }
   cta_add<NW>(acc + sum.total(), a);
@@ -692,7 +731,7 @@ __global__ void __launch_bounds__(NW * 32, (MODE == kSym ? 24 : 32) / NW) k_pivo
 // pivot's card for lollipops).
 constexpr uint32_t kTinyMax = 8;
 constexpr uint32_t kTinyChunk = 16;
-template <int MODE>
+template <int MODE, bool LONG>
 __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32_t base, uint32_t g, uint32_t* mem,
                                                       uint32_t lane) {
   uint32_t* list = mem;                               // kTinyChunk * kTinyMax
@@ -726,7 +765,7 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
     RowView W = load_view(a.desc, a.arena, i);
     if (MODE == kSym) keep_below(a, W, i);
     uint32_t* to = list + poff[p];
-    warp_decode_to(W, lane, [&](uint32_t k, uint32_t x) {
+    warp_decode_to<LONG>(W, lane, [&](uint32_t k, uint32_t x) {
       if (k < W.card) to[k] = x;
     });
     __syncwarp();
@@ -750,7 +789,7 @@ __device__ __noinline__ unsigned long long tiny_chunk(const PivotArgs& a, uint32
 
 // Pivots up to light_max entries, one warp each: order[mid0, mid1) in grabs of
 // mid_chunk, then the tiny ones order[mid1, n_order) in chunks of tiny_chunk.
-template <int MODE>
+template <int MODE, bool LONG>
 __global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_warp(PivotArgs a, uint32_t mid1, uint32_t mid_chunk,
                                                                 uint32_t tiny, uint32_t cap, uint32_t win) {
   extern __shared__ __align__(16) char dyn[];
@@ -774,7 +813,7 @@ __global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_wa
       RowView A = load_view(a.desc, a.arena, i);
       const uint32_t card = A.card;
       if (MODE == kSym) keep_below(a, A, i);
-      const uint32_t cnt = pivot_count<1, MODE>(a, A, 1, A.card, s, win, nullptr, lane, 0, sum, card, acc);
+      const uint32_t cnt = pivot_count<1, MODE, LONG>(a, A, 1, A.card, s, win, nullptr, lane, 0, sum, card, acc);
       acc += finish_pivot<MODE>(a, i, card, cnt, sum, lane);
     }
   }
@@ -785,7 +824,7 @@ __global__ void __launch_bounds__(kCtaThreads, MODE == kSym ? 3 : 4) k_pivots_wa
     if (lane == 0) base = tiny0 + atomicAdd(&a.queue[3], tiny);
     base = __shfl_sync(FULL, base, 0);
     if (base >= a.n_order) break;
-    acc += tiny_chunk<MODE>(a, base, min(tiny, a.n_order - base), reinterpret_cast<uint32_t*>(mem), lane);
+    acc += tiny_chunk<MODE, LONG>(a, base, min(tiny, a.n_order - base), reinterpret_cast<uint32_t*>(mem), lane);
   }
   cta_add(acc + sum.total(), a);
   overlap_end();
@@ -1047,7 +1086,7 @@ constexpr uint64_t kSplitRows = 196608;
 static uint32_t cap_of(uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); }
 
 // One launch of k_pivots_cta: n units, or order[pos0, pos0 + n) whole.
-template <int NW, int MODE>
+template <int NW, int MODE, bool LONG>
 struct CtaLaunch {
   uint32_t n = 0, pos0 = 0, cap = 0, win = 0, bytes = 0;
   unsigned grid = 0;
@@ -1065,18 +1104,18 @@ struct CtaLaunch {
                   unsigned split, bool& overlap) const {
     if (!n) return cudaSuccess;
     static std::atomic<bool> done[64];
-    cudaError_t e = allow_smem((const void*)k_pivots_cta<NW, MODE>, slice_bytes<NW, MODE>(kCtaListCap, kCtaWindow),
+    cudaError_t e = allow_smem((const void*)k_pivots_cta<NW, MODE, LONG>, slice_bytes<NW, MODE>(kCtaListCap, kCtaWindow),
                                done, device);
     if (e != cudaSuccess) return e;
-    e = launch_overlapped(k_pivots_cta<NW, MODE>, grid, NW * 32, bytes, st, overlap, split, a, units, n, pos0, next,
+    e = launch_overlapped(k_pivots_cta<NW, MODE, LONG>, grid, NW * 32, bytes, st, overlap, split, a, units, n, pos0, next,
                           cap, win);
     overlap = true;
     return e;
   }
 };
 
-template <int MODE>
-static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_units, int most, cudaStream_t st) {
+template <int MODE, bool LONG>
+static cudaError_t launch_pivots_as(PivotArgs a, const uint2* units, uint32_t n_units, int most, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   int device = 0;
   if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
@@ -1087,8 +1126,8 @@ static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_uni
   const unsigned g_heavy =
       giants ? (unsigned)std::max(1, std::min(most, resident_grid(device, (uint32_t)sizeof(HeavySmem), 6))) : 0u;
   const uint32_t n_large = !units ? a.n_large : a.n_large > a.n_giant ? n_units : 0u;  // no list: whole pivots
-  const CtaLaunch<kLargeWarps, MODE> large(a, n_large, 0, a.max_large, kCtaWindow, most, device);
-  const CtaLaunch<kMidWarps, MODE> mid(a, a.n_heavy > a.n_large ? a.n_heavy - a.n_large : 0u, a.n_large, a.max_mid,
+  const CtaLaunch<kLargeWarps, MODE, LONG> large(a, n_large, 0, a.max_large, kCtaWindow, most, device);
+  const CtaLaunch<kMidWarps, MODE, LONG> mid(a, a.n_heavy > a.n_large ? a.n_heavy - a.n_large : 0u, a.n_large, a.max_mid,
                                        kWarpWindow, most, device);
   const uint32_t cap = cap_of(a.max_warp), win = window_bits(a.n, kWarpWindow);
   const uint32_t bytes = NWARPS * slice_bytes<1, MODE>(cap, win);
@@ -1118,15 +1157,26 @@ static cudaError_t launch_pivots(PivotArgs a, const uint2* units, uint32_t n_uni
   if (e == cudaSuccess) e = mid.run(a, nullptr, a.queue + 4, device, st, split, overlap);
   if (e == cudaSuccess && gw) {
     static std::atomic<bool> done[64];
-    e = allow_smem((const void*)k_pivots_warp<MODE>, NWARPS * slice_bytes<1, MODE>(kLightMax, kWarpWindow), done,
+    e = allow_smem((const void*)k_pivots_warp<MODE, LONG>, NWARPS * slice_bytes<1, MODE>(kLightMax, kWarpWindow), done,
                    device);
     if (e == cudaSuccess)
-      e = launch_overlapped(k_pivots_warp<MODE>, (unsigned)gw, kCtaThreads, bytes, st, overlap, split, a, mid1,
+      e = launch_overlapped(k_pivots_warp<MODE, LONG>, (unsigned)gw, kCtaThreads, bytes, st, overlap, split, a, mid1,
                             mid_chunk, tiny_grab, cap, win);
   }
   // A launch that failed leaves the others short of the last CTA: clear the queue for the next call.
   if (e != cudaSuccess) cudaMemsetAsync(a.queue, 0, kPivotQueueWords * sizeof(uint32_t), st);
   return e;
+}
+
+// The kernels for matrices of bitset or pshort rows throughout (PivotArgs::long_rows) have
+// the loops those rows want: long bitset rows four rounds in flight, pshort
+// rows streamed.  Of their own, as they cost the others up to 2% (R-MAT scale 22,
+// hybrid 5.37 against 5.49 ms); for them 23.8 against 18.2 ms (bitset) and 8.06 against 7.05
+// (pshort).
+template <int MODE>
+static cudaError_t launch_pivots(const PivotArgs& a, const uint2* units, uint32_t n_units, int most, cudaStream_t st) {
+  return a.long_rows ? launch_pivots_as<MODE, true>(a, units, n_units, most, st)
+                     : launch_pivots_as<MODE, false>(a, units, n_units, most, st);
 }
 
 cudaError_t launch_pivot_units(const RowDesc* desc, const uint32_t* order, uint32_t n_heavy,

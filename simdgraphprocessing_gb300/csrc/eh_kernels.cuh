@@ -95,6 +95,7 @@ struct PivotArgs {
   bool report;             // also move the flags to out[1] (and clear them)
   unsigned long long* out; // result; in batch mode out[num_graphs]
   uint32_t unit_span;      // pivot positions e per unit of a large pivot
+  bool long_rows;          // bitset or pshort rows whatever their density (not the hybrid layout)
   const uint32_t* graph_rows;  // batch mode: graph g owns rows [graph_rows[g], graph_rows[g+1]); else null
   uint32_t num_graphs;
   const unsigned long long* core;  // dense core bitmap of rows j < core_k (see core_row_offset), or null
