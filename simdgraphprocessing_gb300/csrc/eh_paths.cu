@@ -166,8 +166,9 @@ __global__ void k_symbiosity_find(uint32_t n, const RowDesc* __restrict__ dr, co
 // rows too long for a warp are k_symbiosity_heavy's.  Half-reciprocal R-MAT scale 21,
 // hybrid: 223 us here (latency of the lane merges and of the warp rows' first
 // blocks, about equal) and 74 us for the listed rows, where binary searches in a
-// staged row took 335 us; 541 -> 299 us a call with the two overlapped.
-__global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc* __restrict__ dr,
+// staged row took 335 us; 541 -> 279 us a call with the two overlapped (six CTAs
+// an SM; five: 299).
+__global__ void __launch_bounds__(256, 6) k_symbiosity(uint32_t n, const RowDesc* __restrict__ dr,
                                                     const uint4* __restrict__ ar, const RowDesc* __restrict__ dc,
                                                     const uint4* __restrict__ ac, SymTest test,
                                                     unsigned long long* out, uint32_t* cursor) {
@@ -176,14 +177,19 @@ __global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc
   const uint32_t lane = threadIdx.x & 31;
   unsigned long long acc = 0;
   const uint32_t chunks = (n + kSymChunk - 1) / kSymChunk;
+  const uint32_t turn = (uint32_t)(((lane >> 1) * 2654435761ull) % chunks);  // this lane's 16th starts here
   for (;;) {
     uint32_t q = 0;
     if (lane == 0) q = atomicAdd(cursor, 1u);
     q = __shfl_sync(FULL, q, 0);
     if (q >= chunks) break;
-    // Pairs of rows, 2 * chunks apart: the long rows at the front of a degree-ordered graph spread over the chunks.
-    const auto row_of = [&](uint32_t l) { return 2 * q + (l & 1) + (uint64_t)(l >> 1) * 2 * chunks; };
-    const uint64_t r = row_of(lane);
+    // Pairs of rows, one from each 16th of the matrix at a different place in it: the long
+    // rows at the front of a degree-ordered graph spread over the chunks, and so do those
+    // of raw R-MAT ids, which sit at the same places of every 16th (scale 22, directed: 493 us a call, 1,015
+    // with the pairs 2 * chunks apart).
+    uint32_t at = q + turn;
+    if (at >= chunks) at -= chunks;
+    const uint64_t r = 2 * at + (lane & 1) + (uint64_t)(lane >> 1) * 2 * chunks;
     bool warp_row = false;
     RowView A, B;
     A.p = B.p = nullptr;
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(256, 5) k_symbiosity(uint32_t n, const RowDesc
       if (lane == 0) acc += sym_above(both, A2, B2, test);
     }
     for (uint32_t wm = __ballot_sync(FULL, warp_row && !mergeable); wm; wm &= wm - 1) {
-      const uint32_t r2 = (uint32_t)row_of(__ffs(wm) - 1);
+      const uint32_t r2 = __shfl_sync(FULL, (uint32_t)r, __ffs(wm) - 1);
       const RowView A2 = load_view(dr, ar, r2);
       const RowView B2 = load_view(dc, ac, r2);
       const uint32_t both = warp_intersect_size(A2, B2, lane, &s_hdr[threadIdx.x >> 5]);  // header table: pshort rows
