@@ -430,7 +430,7 @@ def run_ours(a, rank, world, local_rank):
     peak, peak_kind = measured_peak()
     # A count launches the warp kernel, the CTA kernel for rows above light_max,
     # again for the units of rows above 512, and the giants' kernel above 2,048.
-    limits = [(shape or {}).get("light_max", 96), 512, 2048]
+    limits = [(shape or {}).get("light_max", 160 if info["matrix_size"] < 3500000 else 96), 512, 2048]
     kernels_per_count = 1 + sum(info["max_row_cardinality"] > x for x in limits)
     traffic = traffic_per_launch(work)
     fx = fixture_for(a)

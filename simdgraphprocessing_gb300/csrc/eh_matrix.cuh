@@ -112,7 +112,7 @@ struct Matrix {
 // Each pool keeps up to kPoolKeep bytes of freed memory mapped between calls:
 // the device's default pool releases it at every synchronisation, and mapping
 // 400 MB again costs about 1 ms on GB300.  16 GiB holds a rebuilt scale-22
-// matrix with its largest tuned core (4.3 GB) and its build scratch.
+// matrix with the largest core a shape may ask for (4.3 GB) and its build scratch.
 constexpr uint64_t kPoolKeep = 16ull << 30;
 // Which pool: the dense cores of work plans (large, and kept
 // for the matrix's life) come from a pool of their own.  In the same pool as
