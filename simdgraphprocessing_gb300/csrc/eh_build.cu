@@ -39,6 +39,15 @@ constexpr int kBigBlock = 1024;
 // each of them.
 constexpr uint64_t kLaneRow = 8;
 
+// Appends a row to the list of rows longer than kBigRow.  Offsets that rise fill at
+// most `cap` slots (big_row_capacity); where they fall, rows that are valid one by one
+// can be more, and those past the list are left out: the build is refused anyway.
+__device__ __forceinline__ void list_big(uint32_t* big, uint32_t* n_big, uint32_t cap, uint64_t row, uint32_t& flags) {
+  const uint32_t at = atomicAdd(n_big, 1u);
+  if (at < cap) big[at] = (uint32_t)row;
+  else flags |= ERRF_OFFSETS;
+}
+
 struct SegMeasure {
   uint32_t cnt, parts, first, last, first_hi, last_hi, flags;
 };
@@ -219,7 +228,7 @@ __global__ void __launch_bounds__(kBlock) k_measure(uint64_t n, uint64_t total, 
                                                     int layout, RowMeasure* __restrict__ meas,
                                                     BuildTotals* __restrict__ tot,
                                                     uint32_t* __restrict__ err, uint32_t* __restrict__ big,
-                                                    uint32_t* __restrict__ n_big) {
+                                                    uint32_t* __restrict__ n_big, uint32_t big_cap) {
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t nw = (uint64_t)gridDim.x * (kBlock / 32);
   uint32_t flags = 0;
@@ -262,7 +271,7 @@ __global__ void __launch_bounds__(kBlock) k_measure(uint64_t n, uint64_t total, 
       const uint64_t row = row0 + q * nw;
       const uint64_t b = __shfl_sync(FULL, my_b, q), e = __shfl_sync(FULL, my_e, q);
       if (e - b > kBigRow) {
-        if (lane == 0) big[atomicAdd(n_big, 1u)] = (uint32_t)row;
+        if (lane == 0) list_big(big, n_big, big_cap, row, flags);
         continue;
       }
       const SegMeasure sm = measure_segment(n, row, b, b, e, 0u, nbr, mask, sel, lane);
@@ -291,11 +300,11 @@ __global__ void __launch_bounds__(kBigBlock) k_measure_big(uint64_t n, const uin
                                                            BuildTotals* __restrict__ tot, uint32_t* __restrict__ err,
                                                            const uint32_t* __restrict__ big,
                                                            const uint32_t* __restrict__ big_begin,
-                                                           const uint32_t* __restrict__ big_end) {
+                                                           const uint32_t* __restrict__ big_end, uint32_t big_cap) {
   constexpr int NWB = kBigBlock / 32;
   __shared__ SegMeasure s_seg[NWB];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t nb = *big_end;
+  const uint32_t nb = min(*big_end, big_cap);
   Totals t;
   uint32_t flags = 0;
   for (uint32_t i = *big_begin + blockIdx.x; i < nb; i += gridDim.x) {
@@ -387,7 +396,8 @@ __global__ void __launch_bounds__(kBlock) k_measure_prefix(uint64_t n, uint64_t 
                                                            const uint32_t* __restrict__ nbr, int sel, int layout,
                                                            RowMeasure* __restrict__ meas,
                                                            BuildTotals* __restrict__ tot, uint32_t* __restrict__ err,
-                                                           uint32_t* __restrict__ big, uint32_t* __restrict__ n_big) {
+                                                           uint32_t* __restrict__ big, uint32_t* __restrict__ n_big,
+                                                           uint32_t big_cap) {
   const uint32_t lane = threadIdx.x & 31, sl = lane & 7, grp = lane >> 3;
   const uint64_t nw = (uint64_t)gridDim.x * (kBlock / 32);
   uint32_t flags = 0;
@@ -445,7 +455,7 @@ __global__ void __launch_bounds__(kBlock) k_measure_prefix(uint64_t n, uint64_t 
       const uint32_t q = __ffs(m) - 1;
       const uint64_t row = dealt_row(row0, q, nw), b = __shfl_sync(FULL, my_b, q), l = __shfl_sync(FULL, len, q);
       if (l > kBigRow) {
-        if (lane == 0) big[atomicAdd(n_big, 1u)] = (uint32_t)row;
+        if (lane == 0) list_big(big, n_big, big_cap, row, flags);
         continue;
       }
       const uint32_t cnt = warp_sum_u32(measure_prefix<32, uint32_t>(nbr + b, (uint32_t)l, n, row, sel, lane, flags));
@@ -468,9 +478,10 @@ __global__ void __launch_bounds__(kBigBlock) k_measure_prefix_big(uint64_t n, co
                                                                   uint32_t* __restrict__ err,
                                                                   const uint32_t* __restrict__ big,
                                                                   const uint32_t* __restrict__ big_begin,
-                                                                  const uint32_t* __restrict__ big_end) {
+                                                                  const uint32_t* __restrict__ big_end,
+                                                                  uint32_t big_cap) {
   __shared__ uint32_t s_cnt;
-  const uint32_t lane = threadIdx.x & 31, nb = *big_end;
+  const uint32_t lane = threadIdx.x & 31, nb = min(*big_end, big_cap);
   Totals t;
   uint32_t flags = 0;
   for (uint32_t i = *big_begin + blockIdx.x; i < nb; i += gridDim.x) {
@@ -1175,29 +1186,32 @@ cudaError_t launch_measure_rows(uint64_t n, uint64_t total, uint64_t r_begin, ui
                                 const uint32_t* nbr, const uint8_t* mask, int sel, int layout, RowMeasure* meas,
                                 BuildTotals* totals, uint32_t* err, uint32_t* big, uint32_t* n_big, cudaStream_t st) {
   if (r_end <= r_begin) return cudaSuccess;
+  const uint32_t cap = (uint32_t)big_row_capacity(n, total);
   if (prefix_build(sel, layout)) {
     const unsigned grid = (unsigned)std::min<uint64_t>((r_end - r_begin + kBlock - 1) / kBlock, 152 * 8);
-    k_measure_prefix<<<grid, kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, sel,
-                                                                                layout, meas, totals, err, big, n_big);
+    k_measure_prefix<<<grid, kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, sel, layout, meas, totals, err, big,
+                                              n_big, cap);
     return cudaGetLastError();
   }
   const unsigned grid = (unsigned)std::min<uint64_t>((r_end - r_begin + kBlock / 32 - 1) / (kBlock / 32), 152 * 8);
-  k_measure<<<grid, kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, mask, sel,
-                                                                        layout, meas, totals, err, big, n_big);
+  k_measure<<<grid, kBlock, 0, st>>>(n, total, r_begin, r_end, off, nbr, mask, sel, layout, meas, totals, err, big,
+                                     n_big, cap);
   return cudaGetLastError();
 }
 
-cudaError_t launch_measure_big(uint64_t n, const uint64_t* off, const uint32_t* nbr, const uint8_t* mask, int sel,
-                               int layout, RowMeasure* meas, BuildTotals* totals, uint32_t* err, const uint32_t* big,
-                               const uint32_t* big_begin, const uint32_t* big_end, cudaStream_t st) {
+cudaError_t launch_measure_big(uint64_t n, uint64_t total, const uint64_t* off, const uint32_t* nbr,
+                               const uint8_t* mask, int sel, int layout, RowMeasure* meas, BuildTotals* totals,
+                               uint32_t* err, const uint32_t* big, const uint32_t* big_begin, const uint32_t* big_end,
+                               cudaStream_t st) {
   if (n == 0) return cudaSuccess;
+  const uint32_t cap = (uint32_t)big_row_capacity(n, total);
   if (prefix_build(sel, layout)) {
     k_measure_prefix_big<<<2 * 152, kBigBlock, 0, st>>>(n, off, nbr, sel, layout, meas, totals, err, big, big_begin,
-                                                        big_end);
+                                                        big_end, cap);
     return cudaGetLastError();
   }
   k_measure_big<<<2 * 152, kBigBlock, 0, st>>>(n, off, nbr, mask, sel, layout, meas, totals, err, big, big_begin,
-                                               big_end);
+                                               big_end, cap);
   return cudaGetLastError();
 }
 

@@ -178,13 +178,13 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
       if ((e = launch_measure_rows(n, total, up->rows[c], up->rows[c + 1], d_off, d_nbr, d_mask, sel, layout, meas,
                                    tot, err, big, n_big, st)) != cudaSuccess ||
           (e = cudaMemcpyAsync(mark + c + 1, n_big, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
-          (e = launch_measure_big(n, d_off, d_nbr, d_mask, sel, layout, meas, tot, err, big, mark + c, mark + c + 1,
+          (e = launch_measure_big(n, total, d_off, d_nbr, d_mask, sel, layout, meas, tot, err, big, mark + c, mark + c + 1,
                                   st)) != cudaSuccess)
         return fail(cuda_fail(e, "measure kernel"));
     }
   } else if ((e = launch_measure_rows(n, total, 0, n, d_off, d_nbr, d_mask, sel, layout, meas, tot, err, big, n_big,
                                       st)) != cudaSuccess ||
-             (e = launch_measure_big(n, d_off, d_nbr, d_mask, sel, layout, meas, tot, err, big, mark, n_big, st)) !=
+             (e = launch_measure_big(n, total, d_off, d_nbr, d_mask, sel, layout, meas, tot, err, big, mark, n_big, st)) !=
                  cudaSuccess) {
     return fail(cuda_fail(e, "measure kernel"));
   }
