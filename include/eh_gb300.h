@@ -6,7 +6,11 @@
  * eh_last_error() (thread-local).  Handles are opaque; the library owns the
  * device memory behind them.  A handle may be used from one host thread at a
  * time.  `stream` arguments are cudaStream_t values passed as void* (NULL = the
- * legacy default stream).
+ * legacy default stream).  Counts and listings of one matrix share its work
+ * queues: called on several streams they run one after the other, in the order
+ * of the calls.  Captured ones have queues of their own and may be replayed
+ * beside direct calls (cliques only while no row is above 1,024 entries), but
+ * graphs with counts of the same matrix must not overlap each other.
  *
  * Each entry point names the reference interface it replaces
  * (chrisaberger/SIMDGraphProcessing, paths relative to that project).

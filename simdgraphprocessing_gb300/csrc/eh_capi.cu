@@ -87,28 +87,62 @@ cudaError_t upload_stream(cudaStream_t* out) {
   return cudaSuccess;
 }
 
-void note_use(Matrix* m, cudaStream_t st) {
+static bool is_capturing(cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
+  return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+static unsigned long long stream_id(cudaStream_t st) {
+  unsigned long long id = 0;
+  return cudaStreamGetId(st, &id) == cudaSuccess ? id : 0;
+}
+
+void note_use(Matrix* m, cudaStream_t st) {
+  if (is_capturing(st)) return;
+  const unsigned long long id = stream_id(st);
   std::lock_guard<std::mutex> g(m->uses_mu);
-  cudaEvent_t ev = nullptr;
+  Matrix::StreamUse* use = nullptr;
   for (auto& u : m->uses)
-    if (u.first == st) ev = u.second;
-  if (!ev) {
-    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return;
-    m->uses.emplace_back(st, ev);
+    if (u.stream == st) use = &u;
+  if (!use) {
+    cudaEvent_t ev = nullptr;
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+      cudaStreamSynchronize(st);  // nothing to wait for later
+      return;
+    }
+    m->uses.push_back({st, id, ev});
+    use = &m->uses.back();
   }
-  cudaEventRecord(ev, st);
+  if (use->id != id) {  // the handle's former stream may still run launches
+    cudaStreamWaitEvent(st, use->done, 0);
+    use->id = id;
+  }
+  cudaEventRecord(use->done, st);
 }
 
 cudaError_t wait_uses(Matrix* m, cudaStream_t st) {
+  const unsigned long long id = stream_id(st);
   std::lock_guard<std::mutex> g(m->uses_mu);
   for (auto& u : m->uses) {
-    if (u.first == st) continue;  // stream order covers it
-    const cudaError_t e = cudaStreamWaitEvent(st, u.second, 0);
+    if (u.stream == st && u.id == id) continue;  // stream order covers it
+    const cudaError_t e = cudaStreamWaitEvent(st, u.done, 0);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+eh_status own_counters(Matrix* m, cudaStream_t st, uint32_t** counters, bool* captured) {
+  *captured = is_capturing(st);
+  *counters = m->counters + (*captured ? kMatrixCounters : 0);
+  if (*captured) return EH_OK;
+  const unsigned long long id = stream_id(st);
+  std::lock_guard<std::mutex> g(m->uses_mu);
+  if (m->counted && (m->count_stream != st || m->count_id != id))
+    for (auto& u : m->uses)
+      if (u.stream == m->count_stream) CU(cudaStreamWaitEvent(st, u.done, 0), "last count");
+  m->counted = true;
+  m->count_stream = st;
+  m->count_id = id;
+  return EH_OK;
 }
 
 eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr, const uint8_t* d_mask,
@@ -210,12 +244,12 @@ eh_status build_device(uint64_t n, const uint64_t* d_off, const uint32_t* d_nbr,
   m->arena_units = m->tot.payload_units;
   if ((e = pool_alloc((void**)&m->desc, nn * sizeof(RowDesc), st)) != cudaSuccess ||
       (e = pool_alloc((void**)&m->arena, (m->arena_units + 1) * 16, st)) != cudaSuccess ||
-      (e = pool_alloc((void**)&m->counters, kMatrixCounters * sizeof(uint32_t), st)) != cudaSuccess)
+      (e = pool_alloc((void**)&m->counters, 2 * kMatrixCounters * sizeof(uint32_t), st)) != cudaSuccess)
     return fail(set_error(EH_ERR_OUT_OF_MEMORY, "matrix allocation (%llu bytes) failed: %s",
                           (unsigned long long)((m->arena_units + 1) * 16 + nn * 16), cudaGetErrorString(e)));
   m->result = reinterpret_cast<unsigned long long*>(m->counters + 16);
-  m->device_bytes = nn * sizeof(RowDesc) + (m->arena_units + 1) * 16 + 128;
-  cudaMemsetAsync(m->counters, 0, kMatrixCounters * sizeof(uint32_t), st);
+  m->device_bytes = nn * sizeof(RowDesc) + (m->arena_units + 1) * 16 + 2 * kMatrixCounters * sizeof(uint32_t);
+  cudaMemsetAsync(m->counters, 0, 2 * kMatrixCounters * sizeof(uint32_t), st);
   cudaMemsetAsync(m->arena, 0, (m->arena_units + 1) * 16, st);
   if ((e = launch_encode(n, d_off, d_nbr, d_mask, sel, layout, meas, off16, m->desc, m->arena, big, big + big_cap, st)) !=
       cudaSuccess)
@@ -431,8 +465,8 @@ PivotArgs pivot_args(Matrix* m, unsigned long long* out) {
   a.n_giant = m->plan.n_giant;
   a.giant_lists = m->plan.giant_lists;
   a.giant_off = m->plan.giant_off;
-  a.queue = m->counters + kQueueWord;
-  a.flags = m->counters + kFlagWord;
+  a.queue = nullptr;  // take_queue
+  a.flags = nullptr;
   a.ctas = 0;
   a.report = false;
   a.out = out;
@@ -530,13 +564,6 @@ static eh_status count_sync(Matrix* m, uint64_t* count, cudaStream_t st, Launch&
 eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const uint32_t* graph_rows,
                          uint32_t num_graphs, cudaStream_t st, Workspace* ws, bool list, uint32_t* tuples,
                          uint64_t capacity, unsigned long long* tri) {
-  Workspace own;
-  if (!ws) {
-    own.counters = m->counters;
-    own.clique_scratch = m->clique_scratch;
-    own.clique_scratch_words = m->clique_scratch_words;
-  }
-  Workspace& w = ws ? *ws : own;
   if (m->selection != EH_SELECT_LOWER)
     return set_error(EH_ERR_UNSUPPORTED, "clique counting needs a matrix built with EH_SELECT_LOWER");
   if (k > kCliqueMaxK)
@@ -554,6 +581,14 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
     return launch_triangle_count(m, out, nullptr, 0, st, ws);
   eh_status s = ensure_plan(m, st);
   if (s != EH_OK) return s;
+  Workspace own;
+  if (!ws) {
+    bool captured = false;
+    if ((s = own_counters(m, st, &own.counters, &captured)) != EH_OK) return s;
+    own.clique_scratch = m->clique_scratch;
+    own.clique_scratch_words = m->clique_scratch_words;
+  }
+  Workspace& w = ws ? *ws : own;
   const Plan& p = m->plan;
   const uint32_t cap = clique_smem_cap(k, m->device);
   const uint32_t nG = p.above(cap);
@@ -675,6 +710,22 @@ static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
   return EH_OK;
 }
 
+// Gives a call's pivot kernels the work-queue words of ws or the matrix's own.  The
+// kernels leave them zero, as direct launches find them; those of captured launches
+// are cleared first, since graphs that overlap may have left others.
+static eh_status take_queue(Matrix* m, Workspace* ws, PivotArgs& a, cudaStream_t st) {
+  uint32_t* counters = ws ? ws->counters : m->counters;
+  a.flags = counters + kFlagWord;
+  bool captured = false;
+  if (!ws) {
+    const eh_status s = own_counters(m, st, &counters, &captured);
+    if (s != EH_OK) return s;
+  }
+  a.queue = counters + kQueueWord;
+  if (captured) CU(cudaMemsetAsync(a.queue, 0, kPivotQueueWords * sizeof(uint32_t), st), "queue reset");
+  return EH_OK;
+}
+
 eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st, bool report) {
   eh_status s = ensure_oriented(m, st);
   if (s != EH_OK) return s;
@@ -693,15 +744,19 @@ eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t
     a.max_warp = o.largest_at_most(m->light_max);
     a.max_mid = o.largest_at_most(kMidMax);
     a.max_large = o.largest_at_most(kCtaListCap);
-    CU(launch_lollipops(a, nullptr, 0, m->grid, st), "lollipop kernel");
+    if ((s = take_queue(m, nullptr, a, st)) != EH_OK) return s;
+    const cudaError_t e = launch_lollipops(a, nullptr, 0, m->grid, st);
     note_use(m, st);
+    CU(e, "lollipop kernel");
     return EH_OK;
   }
   if ((s = ensure_plan(m, st)) != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
   a.report = report;
-  CU(launch_lollipops(a, m->plan.unit_list(), m->plan.n_units, m->grid, st), "lollipop kernel");
+  if ((s = take_queue(m, nullptr, a, st)) != EH_OK) return s;
+  const cudaError_t e = launch_lollipops(a, m->plan.unit_list(), m->plan.n_units, m->grid, st);
   note_use(m, st);
+  CU(e, "lollipop kernel");
   return EH_OK;
 }
 
@@ -713,9 +768,8 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
   if (s != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
   a.report = report;
-  uint32_t* counters = ws ? ws->counters : m->counters;
-  a.queue = counters + kQueueWord;
-  a.flags = counters + kFlagWord;
+  if ((s = take_queue(m, ws, a, st)) != EH_OK) return s;
+  uint32_t* counters = a.queue - kQueueWord;
   a.graph_rows = graph_rows;
   a.num_graphs = num_graphs;
   if (graph_rows) {
@@ -724,7 +778,9 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
     a.n_order = m->plan.above(kCliqueWarpMax);
     a.n_heavy = std::min(a.n_heavy, a.n_order);
   }
-  CU(launch_triangles(a, m->plan.unit_list(), m->plan.n_units, m->grid, st), "triangle kernel");
+  const cudaError_t e = launch_triangles(a, m->plan.unit_list(), m->plan.n_units, m->grid, st);
+  if (e != cudaSuccess) note_use(m, st);
+  CU(e, "triangle kernel");
   if (graph_rows && !large_only) {
     CliqueArgs c{m->desc, m->arena, a.order, 3, out, graph_rows, num_graphs, a.core, a.core_k, nullptr, 0, nullptr};
     int sms = 0;
@@ -1001,7 +1057,7 @@ void eh_matrix_free(eh_matrix_t mh) {
                   m->oriented.lcard, m->oriented.order};
   for (void* b : bufs)
     if (b) cudaFreeAsync(b, st);
-  for (auto& u : m->uses) cudaEventDestroy(u.second);
+  for (auto& u : m->uses) cudaEventDestroy(u.done);
   delete m;
 }
 

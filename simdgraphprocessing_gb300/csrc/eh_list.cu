@@ -147,11 +147,14 @@ extern "C" eh_status eh_list_triangles(eh_matrix_t mh, uint32_t* d_out, uint64_t
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   eh_status s = ensure_plan(m, st);
   if (s != EH_OK) return s;
+  uint32_t* counters = nullptr;
+  bool captured = false;
+  if ((s = own_counters(m, st, &counters, &captured)) != EH_OK) return s;
   const Plan& p = m->plan;
   ListArgs a{m->desc, m->arena, p.order, p.n_giant, p.giant_lists, p.giant_off, p.core, p.core_k,
-             d_out, capacity, reinterpret_cast<unsigned long long*>(d_total), m->counters + 4};
+             d_out, capacity, reinterpret_cast<unsigned long long*>(d_total), counters + 4};
   cudaError_t e = cudaMemsetAsync(d_total, 0, sizeof(uint64_t), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(m->counters + 4, 0, 2 * sizeof(uint32_t), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(counters + 4, 0, 2 * sizeof(uint32_t), st);
   if (e != cudaSuccess) return set_error(EH_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
   const uint32_t n_large = p.above(kListWarpMax);
   int sms = 0;

@@ -62,8 +62,8 @@ struct Plan : SizeOrder {
 constexpr uint32_t kMatrixCounters = 32, kFlagWord = 15, kQueueWord = 18;
 
 // Per-launch scratch: work-queue counters and the clique kernel's global slots.
-// A matrix has its own; concurrent launches on one matrix (the serving loop)
-// each bring theirs.
+// A matrix has its own, for launches that run one after the other (own_counters);
+// concurrent launches on one matrix (the serving loop) each bring theirs.
 struct Workspace {
   uint32_t* counters = nullptr;        // kMatrixCounters: as Matrix::counters
   uint32_t* clique_scratch = nullptr;
@@ -82,6 +82,7 @@ struct Matrix {
   Oriented oriented;
   // kMatrixCounters words: 0..14 the clique and list kernels' work queues, 15 device
   // error flags, 16..17 `result`, 18..25 the pivot kernels' queue (PivotArgs::queue).
+  // Another kMatrixCounters follow: the queues of captured launches.
   uint32_t* counters = nullptr;
   unsigned long long* result = nullptr;
   int grid = 0;
@@ -99,9 +100,19 @@ struct Matrix {
   // Where the matrix's buffers are read: one event per stream, recorded after
   // every launch that reads them (not while that stream is being captured).
   // Freeing or replacing a buffer makes the freeing stream wait for these
-  // events, not for the whole device.
+  // events, not for the whole device.  A handle may come back as another stream
+  // (id: cudaStreamGetId); its event then covers both.
+  struct StreamUse {
+    cudaStream_t stream;
+    unsigned long long id;
+    cudaEvent_t done;
+  };
   std::mutex uses_mu;
-  std::vector<std::pair<cudaStream_t, cudaEvent_t>> uses;
+  std::vector<StreamUse> uses;
+  // The stream of the last launch that used the matrix's own workspace.
+  bool counted = false;
+  cudaStream_t count_stream = nullptr;
+  unsigned long long count_id = 0;
 };
 
 // eh_capi.cu
@@ -150,6 +161,11 @@ eh_status ensure_vbits(Matrix* m);
 void note_use(Matrix* m, cudaStream_t st);
 // Makes st wait for every launch note_use has recorded on m, on any stream.
 cudaError_t wait_uses(Matrix* m, cudaStream_t st);
+// The counters of a launch on st that uses m's own workspace, to be followed by
+// note_use.  The last such launch has to be over before: where it was on another
+// stream, st waits for it.  A launch being captured gets the second set, which it has
+// to clear itself (*captured): when its graph runs is not known here.
+eh_status own_counters(Matrix* m, cudaStream_t st, uint32_t** counters, bool* captured);
 // eh_batch.cu: tuned work shape of this matrix's size class, if the tuner has one.
 void apply_cached_shape(Matrix* m);
 PivotArgs pivot_args(Matrix* m, unsigned long long* out);
