@@ -727,7 +727,9 @@ static eh_status take_queue(Matrix* m, Workspace* ws, PivotArgs& a, cudaStream_t
 }
 
 eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st, bool report) {
-  eh_status s = ensure_oriented(m, st);
+  // Looking at the matrix waits for the device, which a capture does not allow: there a
+  // matrix that has its plan is counted by definition unless an earlier call looked.
+  eh_status s = is_capturing(st) ? EH_OK : ensure_oriented(m, st);
   if (s != EH_OK) return s;
   if (m->oriented.state == 1) {
     if ((s = ensure_core(m, st)) != EH_OK) return s;
