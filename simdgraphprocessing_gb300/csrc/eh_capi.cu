@@ -802,15 +802,22 @@ eh_status ensure_vbits(Matrix* m) {
   uint32_t v = 0;
   eh_status s = eh_matrix_get_max_row_id(reinterpret_cast<eh_matrix_t>(m), &v);
   if (s != EH_OK) return s;
+  // Made on the library's own stream, outside any capture that the caller's stream is
+  // in, and finished here, as queries may run on any stream.
+  cudaStream_t own = nullptr;
   unsigned long long* bits = nullptr;
   const uint64_t bytes = row_bits_words(m->n) * sizeof(unsigned long long);
-  CU(pool_alloc((void**)&bits, bytes, nullptr), "similar_nodes bitmap");
-  cudaError_t e = launch_row_bits(m->n, m->desc, m->arena, v, bits, nullptr);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // queries may run on any stream
-  if (e != cudaSuccess) {
-    cudaFreeAsync(bits, nullptr);
-    return cuda_fail(e, "similar_nodes bitmap");
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CU(cudaThreadExchangeStreamCaptureMode(&mode), "similar_nodes bitmap");
+  cudaError_t e = upload_stream(&own);
+  if (e == cudaSuccess) e = pool_alloc((void**)&bits, bytes, own);
+  if (e == cudaSuccess) {
+    e = launch_row_bits(m->n, m->desc, m->arena, v, bits, own);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+    if (e != cudaSuccess) cudaFreeAsync(bits, own);
   }
+  cudaThreadExchangeStreamCaptureMode(&mode);  // the caller's again
+  if (e != cudaSuccess) return cuda_fail(e, "similar_nodes bitmap");
   m->vbits = bits;
   m->device_bytes += bytes;
   return EH_OK;

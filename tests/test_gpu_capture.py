@@ -1,6 +1,6 @@
 """Single counts captured into a CUDA graph and replayed, against the blocking calls and
 the oracle (exact).  A lollipop count needs the matrix's plan before the capture (here
-from set_shape), but no first count."""
+from set_shape) and similar_nodes its largest row, but neither a first count."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -35,6 +35,17 @@ def test_lollipops_first_counted_in_a_capture(eh, oracle, layout):
     assert captured(torch, lambda out, st: m.count_lollipops_async(out, stream=st)) == [want] * 3
     assert m.count_lollipops() == want
     assert captured(torch, lambda out, st: m.count_lollipops_async(out, stream=st)) == [want] * 3
+
+
+@pytest.mark.parametrize("layout", ["hybrid", "uint", "pshort"])
+def test_similar_nodes_first_counted_in_a_capture(eh, oracle, layout):
+    torch = pytest.importorskip("torch")
+    off, nbr = small_graph(eh)
+    want = oracle.Matrix(off, nbr, oracle.SELECT_ALL, oracle.LAYOUTS[layout]).similar_nodes(10)
+    m = eh.Matrix.build(off, nbr, selection="all", layout=layout)
+    m.max_row_id()
+    assert captured(torch, lambda out, st: m.similar_nodes_async(10, out, stream=st)) == [want] * 3
+    assert m.similar_nodes(10) == want
 
 
 @pytest.mark.parametrize("k", [0, 3, 4, 5])
