@@ -650,7 +650,8 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
 
 // Looks at the matrix once: symmetric without self-loops and with at most
 // kCtaListCap entries below the diagonal in any row, it gets the pivots of the
-// symmetric lollipop count (Oriented); any other keeps the count by definition.
+// symmetric lollipop count (Oriented); any other keeps the count by definition, and so
+// does, for this call, one that there is no memory left to look at.
 static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
   Oriented& o = m->oriented;
   if (o.state) return EH_OK;
@@ -675,6 +676,10 @@ static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
     cudaFreeAsync(o.lcard, st);
     cudaFreeAsync(o.order, st);
     o.lcard = o.order = nullptr;
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return EH_OK;
+    }
     return cuda_fail(e, "lollipop plan");
   };
   cudaError_t e;
