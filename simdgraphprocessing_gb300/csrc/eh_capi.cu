@@ -575,9 +575,8 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   if (m->tot.max_card >= kCliqueMaxPivot)
     return set_error(EH_ERR_UNSUPPORTED, "a row of %llu selected entries is above the clique kernels' limit of %u",
                      (unsigned long long)m->tot.max_card, kCliqueMaxPivot - 1);
-  // 3-cliques are triangles.  (Rows of 2^16 entries stay here: a pshort row that
-  // long is where the triangle count follows the reference's u16 counts.)
-  if (k == 3 && !list && !graph_rows && m->tot.max_card < 65536u)
+  // 3-cliques are triangles.
+  if (k == 3 && !list && !graph_rows)
     return launch_triangle_count(m, out, nullptr, 0, st, ws);
   eh_status s = ensure_plan(m, st);
   if (s != EH_OK) return s;

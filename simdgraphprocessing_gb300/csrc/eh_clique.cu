@@ -781,6 +781,21 @@ __global__ void __launch_bounds__(NT, NT == 1024 ? 1 : (GLOBAL ? 2 : 8)) k_cliqu
       }
     }
     __syncthreads();
+    // k = 3, pshort pivots of >= 65,536 entries: M[e] without what the reference's u16
+    // counts drop.  (Not for larger k, whose later levels need the whole of M[t].)
+    if (GLOBAL && top == 0 && A.type == TY_PSHORT && c >= 65536u) {
+      for (uint32_t e = 1 + warp; e < c; e += NW) {
+        const RowView B = load_view(a.desc, a.arena, list[e]);
+        if (!pshort_pair_drop(A, B, list[e])) continue;
+        uint32_t* Me = masks + mask_off(e);
+        for (uint32_t w = lane; 32 * w < e; w += 32)
+          for (uint32_t r = Me[w]; r; r &= r - 1) {
+            const uint32_t h = list[32 * w + __ffs(r) - 1] >> 16;
+            if (pshort_full_block(A, h) && pshort_full_block(B, h)) Me[w] &= ~(r & (0u - r));
+          }
+      }
+      __syncthreads();
+    }
     // phase 2: warp per e
     for (uint32_t e = 1 + warp; e < c; e += NW) {
       const uint32_t* Me = masks + mask_off(e);

@@ -168,9 +168,7 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
     const uint32_t* L =
         (A.type == TY_UINT) ? static_cast<const uint32_t*>(A.p) : a.giant_lists + a.giant_off[uu.x];
     if (bulk_words) A.p = s.words;
-    // The core path is skipped for pshort pivots of >= 65,536 entries, where the
-    // reference's u16 partition count can drop a block (see pshort_pair_drop).
-    const bool use_core = a.core_k && !(A.type == TY_PSHORT && A.card >= 65536u);
+    const bool use_core = a.core_k != 0;
     const uint32_t and_k = min(a.core_k, kCoreAndMax);
     if (use_core) {
       for (uint32_t k = threadIdx.x; k < (and_k >> 6); k += kCtaThreads) s.abits[k] = 0ull;
@@ -223,6 +221,15 @@ __global__ void __launch_bounds__(kCtaThreads, 6) k_pivots_heavy(PivotArgs a, co
         cnt = pair_count_warp(L, e, A, B, j, lane);
       }
       if (lane == 0) uacc += LOLLI ? (unsigned long long)cnt * c : (unsigned long long)cnt;
+    }
+    // Pshort pivots of >= 65,536 entries: less what the reference's u16 counts drop of the
+    // same pairs (a loop of its own: in the one above it spills registers).
+    if (A.type == TY_PSHORT && c >= 65536u) {
+      unsigned long long drop = 0;
+      for (uint32_t e = e0 + threadIdx.x; e < e1; e += kCtaThreads)
+        drop += pshort_pair_drop(A, load_view(a.desc, a.arena, L[e]), L[e]);
+      drop = warp_sum_u64(drop);
+      if (lane == 0) uacc -= LOLLI ? drop * c : drop;
     }
     if (a.graph_rows) {  // batch: this unit's count goes to its graph
       if (lane == 0 && uacc) atomicAdd(&a.out[graph_of(a.graph_rows, a.num_graphs, i)], uacc);
