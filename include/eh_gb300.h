@@ -211,6 +211,8 @@ void eh_matrix_free(eh_matrix_t m);
 /* ------------------------------------------------------------------------- */
 /* Pattern counts.  The synchronous forms write the count to host memory; the  */
 /* _async forms write it to device memory on `stream` without synchronizing.   */
+/* A device-side wait that ran out in one of those (or in a batch) is reported */
+/* by the next synchronous count of the matrix (eh_batch_matrix's).            */
 /* ------------------------------------------------------------------------- */
 /* undirected_triangle_counting<T,R>::run (apps/undirected_triangle_counting.cpp:27-65):
  * sum_i sum_{j in row(i)} |row(i) ∩ row(j)|.  Matrix built with EH_SELECT_LOWER. */

@@ -594,7 +594,7 @@ eh_status launch_cliques(Matrix* m, uint32_t k, unsigned long long* out, const u
   const uint32_t nB = p.above(kCliqueWarpMax);
   const uint32_t nL = p.above(tri ? 1 : k - 2);  // triangles need two entries, k-cliques k - 1
   CliqueArgs a{m->desc, m->arena, p.order, k, out, graph_rows, num_graphs, p.core, p.core_k, tuples, capacity, tri};
-  CU(cudaMemsetAsync(w.counters, 0, 16 * sizeof(uint32_t), st), "memset");
+  CU(cudaMemsetAsync(w.counters, 0, kFlagWord * sizeof(uint32_t), st), "memset");  // not the flags after them
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
   if (nG > 0) {
