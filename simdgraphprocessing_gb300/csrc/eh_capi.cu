@@ -801,26 +801,27 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
 }  // namespace eh
 
 namespace eh {
-eh_status ensure_vbits(Matrix* m) {
+eh_status ensure_vbits(Matrix* m, cudaStream_t st) {
   if (m->vbits) return EH_OK;
   uint32_t v = 0;
   eh_status s = eh_matrix_get_max_row_id(reinterpret_cast<eh_matrix_t>(m), &v);
   if (s != EH_OK) return s;
-  // Made on the library's own stream, outside any capture that the caller's stream is
-  // in, and finished here, as queries may run on any stream.
+  // Finished here, as queries may run on any stream, and no part of a capture that st is
+  // in: that goes on beside the library's own stream.
+  const bool capturing = is_capturing(st);
   cudaStream_t own = nullptr;
   unsigned long long* bits = nullptr;
   const uint64_t bytes = row_bits_words(m->n) * sizeof(unsigned long long);
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  CU(cudaThreadExchangeStreamCaptureMode(&mode), "similar_nodes bitmap");
-  cudaError_t e = upload_stream(&own);
+  if (capturing) CU(cudaThreadExchangeStreamCaptureMode(&mode), "similar_nodes bitmap");
+  cudaError_t e = capturing ? upload_stream(&own) : cudaSuccess;
   if (e == cudaSuccess) e = pool_alloc((void**)&bits, bytes, own);
   if (e == cudaSuccess) {
     e = launch_row_bits(m->n, m->desc, m->arena, v, bits, own);
     if (e == cudaSuccess) e = cudaStreamSynchronize(own);
     if (e != cudaSuccess) cudaFreeAsync(bits, own);
   }
-  cudaThreadExchangeStreamCaptureMode(&mode);  // the caller's again
+  if (capturing) cudaThreadExchangeStreamCaptureMode(&mode);  // the caller's again
   if (e != cudaSuccess) return cuda_fail(e, "similar_nodes bitmap");
   m->vbits = bits;
   m->device_bytes += bytes;
@@ -1106,7 +1107,7 @@ eh_status eh_similar_nodes_async(eh_matrix_t mh, uint32_t threshold, uint64_t* d
   CHECK_MATRIX(mh);
   EH_CHECK_ARG(d_count, "d_count is NULL");
   Matrix* m = MX(mh);
-  eh_status s = eh::ensure_vbits(m);
+  eh_status s = eh::ensure_vbits(m, ST(stream));
   if (s != EH_OK) return s;
   CU(eh::launch_similar(m->n, m->desc, m->arena, (uint32_t)m->vstar, m->vbits, threshold,
                         reinterpret_cast<unsigned long long*>(d_count), ST(stream)),

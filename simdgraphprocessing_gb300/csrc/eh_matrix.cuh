@@ -155,8 +155,8 @@ eh_status ensure_units(Matrix* m, uint32_t light_max, uint32_t unit_span, cudaSt
 eh_status ensure_core(Matrix* m, cudaStream_t st);
 // Frees the parts of the plan that depend on the work shape (units, dense core), so that the next ensure_plan builds them from nothing.
 eh_status drop_shape_parts(Matrix* m, cudaStream_t st);
-// The largest row's id and its bitmap (Matrix::vstar, vbits).
-eh_status ensure_vbits(Matrix* m);
+// The largest row's id and its bitmap (Matrix::vstar, vbits), before a query on st.
+eh_status ensure_vbits(Matrix* m, cudaStream_t st);
 // Records that launches reading m's buffers were just queued on st.
 void note_use(Matrix* m, cudaStream_t st);
 // Makes st wait for every launch note_use has recorded on m, on any stream.

@@ -314,7 +314,7 @@ eh_status eh_server_add_graph(eh_server_t sh, uint64_t n, const uint64_t* offset
   eh::GraphEntry ge;
   ge.low = reinterpret_cast<eh::Matrix*>(low);
   ge.all = reinterpret_cast<eh::Matrix*>(all);
-  if ((st = eh::ensure_plan(ge.low, nullptr)) == EH_OK) st = eh::ensure_vbits(ge.all);
+  if ((st = eh::ensure_plan(ge.low, nullptr)) == EH_OK) st = eh::ensure_vbits(ge.all, nullptr);
   if (st != EH_OK) {
     eh_matrix_free(low);
     eh_matrix_free(all);
