@@ -87,18 +87,19 @@ cudaError_t upload_stream(cudaStream_t* out) {
   return cudaSuccess;
 }
 
+// (The default stream is never captured and never another one: short blocking counts on
+// it are not kept waiting for these questions.)
 static bool is_capturing(cudaStream_t st) {
+  if (!st) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
 }
 static unsigned long long stream_id(cudaStream_t st) {
   unsigned long long id = 0;
-  return cudaStreamGetId(st, &id) == cudaSuccess ? id : 0;
+  return st && cudaStreamGetId(st, &id) == cudaSuccess ? id : 0;
 }
 
-void note_use(Matrix* m, cudaStream_t st) {
-  if (is_capturing(st)) return;
-  const unsigned long long id = stream_id(st);
+static void record_use(Matrix* m, cudaStream_t st, unsigned long long id) {
   std::lock_guard<std::mutex> g(m->uses_mu);
   Matrix::StreamUse* use = nullptr;
   for (auto& u : m->uses)
@@ -117,6 +118,14 @@ void note_use(Matrix* m, cudaStream_t st) {
     use->id = id;
   }
   cudaEventRecord(use->done, st);
+}
+
+void note_use(Matrix* m, cudaStream_t st) {
+  if (!is_capturing(st)) record_use(m, st, stream_id(st));
+}
+// As note_use, after take_queue.
+static void note_count(Matrix* m, cudaStream_t st, bool captured) {
+  if (!captured) record_use(m, st, m->count_id);
 }
 
 cudaError_t wait_uses(Matrix* m, cudaStream_t st) {
@@ -717,24 +726,25 @@ static eh_status ensure_oriented(Matrix* m, cudaStream_t st) {
 // Gives a call's pivot kernels the work-queue words of ws or the matrix's own.  The
 // kernels leave them zero, as direct launches find them; those of captured launches
 // are cleared first, since graphs that overlap may have left others.
-static eh_status take_queue(Matrix* m, Workspace* ws, PivotArgs& a, cudaStream_t st) {
+static eh_status take_queue(Matrix* m, Workspace* ws, PivotArgs& a, cudaStream_t st, bool* captured) {
   uint32_t* counters = ws ? ws->counters : m->counters;
   a.flags = counters + kFlagWord;
-  bool captured = false;
+  *captured = false;
   if (!ws) {
-    const eh_status s = own_counters(m, st, &counters, &captured);
+    const eh_status s = own_counters(m, st, &counters, captured);
     if (s != EH_OK) return s;
   }
   a.queue = counters + kQueueWord;
-  if (captured) CU(cudaMemsetAsync(a.queue, 0, kPivotQueueWords * sizeof(uint32_t), st), "queue reset");
+  if (*captured) CU(cudaMemsetAsync(a.queue, 0, kPivotQueueWords * sizeof(uint32_t), st), "queue reset");
   return EH_OK;
 }
 
 eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t st, bool report) {
   // Looking at the matrix waits for the device, which a capture does not allow: there a
   // matrix that has its plan is counted by definition unless an earlier call looked.
-  eh_status s = is_capturing(st) ? EH_OK : ensure_oriented(m, st);
+  eh_status s = m->oriented.state || is_capturing(st) ? EH_OK : ensure_oriented(m, st);
   if (s != EH_OK) return s;
+  bool captured = false;
   if (m->oriented.state == 1) {
     if ((s = ensure_core(m, st)) != EH_OK) return s;
     const Oriented& o = m->oriented;
@@ -750,18 +760,18 @@ eh_status launch_lollipop_count(Matrix* m, unsigned long long* out, cudaStream_t
     a.max_warp = o.largest_at_most(m->light_max);
     a.max_mid = o.largest_at_most(kMidMax);
     a.max_large = o.largest_at_most(kCtaListCap);
-    if ((s = take_queue(m, nullptr, a, st)) != EH_OK) return s;
+    if ((s = take_queue(m, nullptr, a, st, &captured)) != EH_OK) return s;
     const cudaError_t e = launch_lollipops(a, nullptr, 0, m->grid, st);
-    note_use(m, st);
+    note_count(m, st, captured);
     CU(e, "lollipop kernel");
     return EH_OK;
   }
   if ((s = ensure_plan(m, st)) != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
   a.report = report;
-  if ((s = take_queue(m, nullptr, a, st)) != EH_OK) return s;
+  if ((s = take_queue(m, nullptr, a, st, &captured)) != EH_OK) return s;
   const cudaError_t e = launch_lollipops(a, m->plan.unit_list(), m->plan.n_units, m->grid, st);
-  note_use(m, st);
+  note_count(m, st, captured);
   CU(e, "lollipop kernel");
   return EH_OK;
 }
@@ -774,7 +784,9 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
   if (s != EH_OK) return s;
   PivotArgs a = pivot_args(m, out);
   a.report = report;
-  if ((s = take_queue(m, ws, a, st)) != EH_OK) return s;
+  bool captured = false;
+  if ((s = take_queue(m, ws, a, st, &captured)) != EH_OK) return s;
+  const auto queued = [&] { ws ? note_use(m, st) : note_count(m, st, captured); };
   uint32_t* counters = a.queue - kQueueWord;
   a.graph_rows = graph_rows;
   a.num_graphs = num_graphs;
@@ -785,7 +797,7 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
     a.n_heavy = std::min(a.n_heavy, a.n_order);
   }
   const cudaError_t e = launch_triangles(a, m->plan.unit_list(), m->plan.n_units, m->grid, st);
-  if (e != cudaSuccess) note_use(m, st);
+  if (e != cudaSuccess) queued();
   CU(e, "triangle kernel");
   if (graph_rows && !large_only) {
     CliqueArgs c{m->desc, m->arena, a.order, 3, out, graph_rows, num_graphs, a.core, a.core_k, nullptr, 0, nullptr};
@@ -794,7 +806,7 @@ eh_status launch_triangle_count(Matrix* m, unsigned long long* out, const uint32
     CU(cudaMemsetAsync(counters + 11, 0, sizeof(uint32_t), st), "memset");
     CU(launch_clique_warp(c, a.n_order, m->plan.above(1), counters + 11, sms, st), "triangle kernel (warp)");
   }
-  note_use(m, st);
+  queued();
   return EH_OK;
 }
 
