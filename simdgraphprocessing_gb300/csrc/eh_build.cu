@@ -1001,8 +1001,9 @@ __global__ void k_plan_scatter(uint64_t n, const uint32_t* __restrict__ cards, u
 // Rows as pivots of the symmetric lollipop count: lcard[r] = |row(r) ∩ [0, r)|, and
 // whether the matrix is symmetric without self-loops: check[0] sums a keyed hash
 // of the pair (larger id, smaller id) over the entries below the diagonal minus
-// the same over those above it (0 for a symmetric matrix; for any other, 0 with
-// probability 2^-64 over the key), check[1] counts self-loops.  Pairs of rows are
+// the same over those above it, check[1] counts self-loops.  A symmetric matrix gives
+// 0.  Another one would give 0 with probability 2^-64 if the hash were a random
+// function; for this mixer, with a key drawn per process, that is not proven.  Pairs of rows are
 // dealt to warps round-robin; a lane takes its row of up to kLaneRow entries, the
 // warp longer ones, and a CTA of k_orient_big those over kBigRow entries, so that
 // no hub is one warp's (one row a warp, 8 rows a CTA: 614 us at R-MAT scale 20).
@@ -1010,7 +1011,7 @@ __device__ __forceinline__ unsigned long long pair_hash(unsigned long long key, 
   unsigned long long z = (((unsigned long long)hi << 32) | lo) ^ key;  // SplitMix64's finalizer (Steele, Lea, Flood 2014)
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  return (z ^ (z >> 31)) * (key | 1ull);
+  return z ^ (z >> 31);
 }
 struct OrientSum {
   unsigned long long sum = 0, self = 0;
