@@ -143,17 +143,17 @@ def measured_peak():
 
 
 def traffic_per_launch(work):
-    """DRAM bytes (read + write) per launch of the count kernel from the committed
-    ncu summary for this workload, or None."""
+    """DRAM bytes (read + write) of one count's kernels from the committed ncu summary
+    for this workload and the work shapes they were captured with, or (None, None)."""
     path = os.path.join(ROOT, "profiles", "traffic.json")
     try:
         with open(path) as f:
             t = json.load(f)
         key = "rmat_s%d_ef%d_seed%d_%s" % (work["scale"], work["undirected_edges"] >> work["scale"],
                                             work["seed"], work["layout"])
-        return t[key]["dram_bytes_per_launch"]
+        return t[key]["dram_bytes_per_launch"], t[key]["work_shapes"]
     except Exception:
-        return None
+        return None, None
 
 
 class ClockSampler:
@@ -432,7 +432,7 @@ def run_ours(a, rank, world, local_rank):
     # again for the units of rows above 512, and the giants' kernel above 2,048.
     limits = [(shape or {}).get("light_max", 160 if info["matrix_size"] < 3500000 else 96), 512, 2048]
     kernels_per_count = 1 + sum(info["max_row_cardinality"] > x for x in limits)
-    traffic = traffic_per_launch(work)
+    traffic, traffic_shapes = traffic_per_launch(work)
     fx = fixture_for(a)
     cpu = None
     if not a.no_cpu and not a.profile and world == 1:
@@ -442,14 +442,15 @@ def run_ours(a, rank, world, local_rank):
                "; C oracle port of the reference algorithm (OpenMP, build %.2f s untimed)" % tb,
                "count_matches_gpu": (ccount == count) if ccount is not None else None}
     # Roofline: the physical HBM figure is the count's DRAM traffic (ncu, the
-    # two pivot kernels of one count) over the event-timed count.  The
+    # pivot kernels of one count, at the shapes given with it) over the event-timed count.  The
     # algorithmic bytes B_tc charge every neighbour row in full per edge while
     # the kernels probe words of it (much of it from L2), so B_tc / time is an
     # effective bandwidth above what HBM can deliver, reported beside it.
     algo_gbs = btc / (ms / 1e3) / 1e9
     dram_gbs = (traffic / (ms / 1e3) / 1e9) if traffic else None
     roofline = {"bound": "hbm", "achieved": dram_gbs, "peak": peak, "unit": "GB/s",
-                "frac": (dram_gbs / peak) if dram_gbs else None, "traffic": traffic, "peak_kind": peak_kind,
+                "frac": (dram_gbs / peak) if dram_gbs else None, "traffic": traffic,
+                "traffic_work_shapes": traffic_shapes, "peak_kind": peak_kind,
                 "achieved_basis": "ncu DRAM bytes (read + write) of one count's kernels / CUDA-event count time",
                 "nominal_gbs": NOMINAL_HBM_GBS,
                 "frac_of_nominal": (dram_gbs / NOMINAL_HBM_GBS) if dram_gbs else None,

@@ -213,6 +213,9 @@ void eh_matrix_free(eh_matrix_t m);
 /* _async forms write it to device memory on `stream` without synchronizing.   */
 /* A device-side wait that ran out in one of those (or in a batch) is reported */
 /* by the next synchronous count of the matrix (eh_batch_matrix's).            */
+/* A matrix's first count builds its work plan, waits for it and so cannot be   */
+/* captured (eh_matrix_set_shape builds the plan too); a first similar_nodes    */
+/* can be once the largest row is known (eh_matrix_get_max_row_id).             */
 /* ------------------------------------------------------------------------- */
 /* undirected_triangle_counting<T,R>::run (apps/undirected_triangle_counting.cpp:27-65):
  * sum_i sum_{j in row(i)} |row(i) ∩ row(j)|.  Matrix built with EH_SELECT_LOWER. */

@@ -90,7 +90,7 @@ __device__ __forceinline__ void put_tuple(const CliqueArgs& a, unsigned long lon
 // Both are bound by instruction issue (80% of the slots with RowsArea).  A batch of
 // 256 graphs (37 M entries, rows of 18 on average): 2.24 ms with HashArea, 15.7 of 32
 // lanes active, as nearly every step met a bitset row beside a uint one and a hit to
-// look up; 1.70 ms with RowsArea, 26.7 lanes.  Where a core answers most pairs HashArea
+// look up; 1.70 ms with RowsArea, 26.7 lanes (2.50 and 1.80 ms alone under ncu).  Where a core answers most pairs HashArea
 // is the better one: 4-cliques of an R-MAT graph of 1 M vertices 0.340 against 0.347 ms
 // in this kernel, of 21,288 vertices 34 against 51 us in all, as the table's shared
 // memory (158 KB per SM against 51) keeps it from starting beside the larger pivots'
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kCtaThreads, 5) k_clique_warp(CliqueArgs a, ui
 //    bank conflicts, and the popcount unit (16 lanes per cycle and SM) sees one
 //    word in eight.
 // Bound by instruction issue.  Tensor cores do not help: the one-bit mma.sync
-// (m16n8k256, and.popc) takes 545 cycles a warp on this chip, fewer bits per cycle
+// (m16n8k256, and.popc) takes 520 to 545 cycles a warp on this chip, fewer bits per cycle
 // than the AND loop.  R-MAT, 1 M vertices, 4-cliques: phase 1 / phase 2 took 1.49 /
 // 2.73 ms with a warp per e in both.
 __host__ __device__ __forceinline__ uint32_t quad_off(uint32_t e) {

@@ -1086,8 +1086,8 @@ static cudaError_t allow_smem(const void* kernel, uint32_t bytes, std::atomic<bo
 // Kernels that ask for different splits of L1 and shared memory do not run on an SM
 // at the same time, and a short call is mostly the tails of its tiers: below
 // kSplitRows rows, if there are several, all ask for the whole of it.  R-MAT, 14 edges a vertex, uint: 60 K
-// vertices 46.9 -> 43.4 us, 130 K 80.5 -> 79.3 (hybrid 90.3 -> 86.7), 260 K even; above
-// that L1 counts for more (520 K 247 -> 270, 1 M 544 -> 623).
+// vertices 46.9 -> 43.4 us, 130 K 80.5 -> 79.3 (hybrid 90.3 -> 86.7), 260 K even (the line
+// lies halfway); above that L1 counts for more (520 K 247 -> 270, 1 M 544 -> 623).
 constexpr uint64_t kSplitRows = 196608;
 
 static uint32_t cap_of(uint32_t entries) { return std::max(32u, (entries + 31) & ~31u); }

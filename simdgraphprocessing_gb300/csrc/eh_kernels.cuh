@@ -117,7 +117,11 @@ constexpr uint32_t kWarpWindow = 8192, kCtaWindow = 65536;  // bits of the pivot
 // count: 32,768 / 40,960 / 65,536 core rows take 704 / 721 / 780 at 1 M rows, 1,193 /
 // 1,239 / 1,453 at 1.5 M (67 MB of core words stay in L2), 3,625 / 3,257 / 3,738 at
 // 3 M and 6,487 / 5,927 / 5,557 at 2^22, where streaming the bitset rows behind a
-// smaller core costs more.  A warp per pivot as far as its slice goes (light_max
+// smaller core costs more.  At the lines (light_max as here): 1,447 / 1,477 at 1.74 M
+// and 1,807 / 1,758 at 2 M; 4,469 / 4,421 at 3.49 M.  The rule sees the rows alone: with 8
+// edges a vertex 40,960 rows pay from 2.5 M on (1,060 / 1,034; 734 / 757 at 2 M) and are
+// still the best at 2^22 (1,985 with light_max 160 against the rule's 2,202), which a
+// tuned matrix gets.  A warp per pivot as far as its slice goes (light_max
 // 160; one launch for most small graphs: 2^14 rows 37 -> 21 us, 2^18 185 -> 164)
 // except at the largest sizes, where smaller slices leave more L1 for loads in flight
 // (2^22: 5,557 at 160, 5,410 at 96).

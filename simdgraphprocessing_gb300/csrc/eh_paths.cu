@@ -13,8 +13,8 @@
 //           (set_union, union.hpp:6-127); a bitset row is ORed word by word;
 //   collect takes seen AND NOT visited as the new frontier (set_difference,
 //           difference.hpp:5-84) and merges it into visited.
-// Frontier rows longer than kBfsHeavy entries are split over every warp of
-// the grid; shorter ones are taken one per warp.  Levels are launched
+// Frontier rows longer than kBfsHeavy entries are split over the warps of the
+// grid, rows above kBfsGroup over a CTA, and shorter ones take 8 lanes.  Levels are launched
 // kBfsChunk at a time: each kernel reads its frontier size from device memory
 // and does nothing once a frontier is empty, so the host checks the sizes
 // once per chunk instead of once per level.
